@@ -728,24 +728,14 @@ mdgpu_status mdgpu_tc_items(const double *h, const mdgpu_control *ctl, int *item
    KList kl;
    mdgpu_status s = build_klist(h, *ctl, kl);
    if (s) return s;
-   const int n = (int)kl.tc_item.size();
+   std::vector<int4> it, kk;
+   build_tc_items(kl, it, kk);
+   const int n = (int)it.size();
    *nitems = n;
    *nk = kl.nk;
    if (n > cap) return MDGPU_E_CAPACITY;
-   for (int i = 0; i < n; i++) {
-      if (items) {
-         items[4 * i] = kl.tc_item[i].x;
-         items[4 * i + 1] = kl.tc_item[i].y;
-         items[4 * i + 2] = kl.tc_item[i].z;
-         items[4 * i + 3] = kl.tc_item[i].w;
-      }
-      if (k0) {
-         k0[4 * i] = kl.tc_k0[i].x;
-         k0[4 * i + 1] = kl.tc_k0[i].y;
-         k0[4 * i + 2] = kl.tc_k0[i].z;
-         k0[4 * i + 3] = kl.tc_k0[i].w;
-      }
-   }
+   if (items && n > 0) std::memcpy(items, it.data(), n * sizeof(int4));
+   if (k0 && n > 0) std::memcpy(k0, kk.data(), n * sizeof(int4));
    return MDGPU_OK;
 }
 

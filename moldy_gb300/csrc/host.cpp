@@ -298,9 +298,6 @@ mdgpu_status build_klist(const double *h, const mdgpu_control &ctl, KList &kl)
    kl.coeff.clear();
    kl.coeff2.clear();
    int nk = 0;
-   std::vector<int4> cols;         // (h, k, l0, count) of each column
-   std::vector<int> col_item;      // its first item (before the sort)
-   std::vector<float2> col_kxy;
    for (int hh = 0; hh <= kl.hmax; hh++)
       for (int k = (hh == 0 ? 0 : -kl.kmax); k <= kl.kmax; k++) {
          double kx = hh * hinvp[0] + k * hinvp[3];
@@ -316,11 +313,6 @@ mdgpu_status build_klist(const double *h, const mdgpu_control &ctl, KList &kl)
                if (extend)
                   kl.item.back().w++;
                else {
-                  if (prev_l != l - 1) {   // a new column
-                     cols.push_back(make_int4(hh, k, l, 0));
-                     col_item.push_back((int)kl.item.size());
-                     col_kxy.push_back(make_float2((float)kx, (float)ky));
-                  }
                   kl.item.push_back(make_int4(hh, k, l, 1));
                   kl.item_k0.push_back(nk);
                   kl.item_kxy.push_back(make_double2(kx, ky));
@@ -345,12 +337,9 @@ mdgpu_status build_klist(const double *h, const mdgpu_control &ctl, KList &kl)
    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return kl.item[a].w > kl.item[b].w; });
    KList o;
    o.item.reserve(kl.nitems);
-   std::vector<int> new_k0(kl.nitems), pre_w(kl.nitems);
-   for (int i = 0; i < kl.nitems; i++) pre_w[i] = kl.item[i].w;
    int k0 = 0;
    for (int i : order) {
       const int4 it = kl.item[i];
-      new_k0[i] = k0;
       o.item.push_back(it);
       o.item_k0.push_back(k0);
       o.item_kxy.push_back(kl.item_kxy[i]);
@@ -368,48 +357,194 @@ mdgpu_status build_klist(const double *h, const mdgpu_control &ctl, KList &kl)
    kl.kz.swap(o.kz);
    kl.coeff.swap(o.coeff);
    kl.coeff2.swap(o.coeff2);
-   // Tensor-core items: each column cut into runs of KT from its first l,
-   // so run r holds the column's KI items 4r .. 4r+3 (contiguous k each).
-   kl.tc_item.clear();
-   kl.tc_k0.clear();
-   kl.tc_kxy.clear();
-   for (size_t c = 0; c < cols.size(); c++) {
-      const int f = col_item[c], e = c + 1 < cols.size() ? col_item[c + 1] : kl.nitems;
-      int total = 0;
-      for (int i = f; i < e; i++) total += pre_w[i];
-      for (int r = 0; r * KT < total; r++) {
-         int ki[4];
-         for (int j = 0; j < 4; j++) {
-            const int run = 4 * r + j;
-            ki[j] = run * KI < total ? new_k0[f + run] : -1;
-         }
-         kl.tc_item.push_back(make_int4(cols[c].x, cols[c].y, cols[c].z + r * KT, std::min(KT, total - r * KT)));
-         kl.tc_k0.push_back(make_int4(ki[0], ki[1], ki[2], ki[3]));
-         kl.tc_kxy.push_back(col_kxy[c]);
-      }
-   }
-   kl.tc_nitems = (int)kl.tc_item.size();
-   {
-      std::vector<int> ord(kl.tc_nitems);
-      for (int i = 0; i < kl.tc_nitems; i++) ord[i] = i;
-      std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return kl.tc_item[a].w > kl.tc_item[b].w; });
-      std::vector<int4> it2, k02;
-      std::vector<float2> kxy2;
-      for (int i : ord) {
-         it2.push_back(kl.tc_item[i]);
-         k02.push_back(kl.tc_k0[i]);
-         kxy2.push_back(kl.tc_kxy[i]);
-      }
-      while (it2.size() % 128) {
-         it2.push_back(make_int4(0, 0, 0, 0));
-         k02.push_back(make_int4(-1, -1, -1, -1));
-         kxy2.push_back(make_float2(0.f, 0.f));
-      }
-      kl.tc_item.swap(it2);
-      kl.tc_k0.swap(k02);
-      kl.tc_kxy.swap(kxy2);
-   }
+   kl.q.ns = 0;
    return MDGPU_OK;
+}
+
+void build_tc_items(const KList &kl, std::vector<int4> &item, std::vector<int4> &k0)
+{
+   // the columns' KI items in order of l
+   std::vector<int> ord(kl.nitems);
+   for (int i = 0; i < kl.nitems; i++) ord[i] = i;
+   std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) {
+      const int4 x = kl.item[a], y = kl.item[b];
+      return x.x != y.x ? x.x < y.x : x.y != y.y ? x.y < y.y : x.z < y.z;
+   });
+   std::vector<int4> it, kk;
+   for (size_t f = 0; f < ord.size();) {
+      size_t e = f + 1;   // the column's consecutive items
+      while (e < ord.size() && kl.item[ord[e]].x == kl.item[ord[f]].x && kl.item[ord[e]].y == kl.item[ord[f]].y &&
+             kl.item[ord[e]].z == kl.item[ord[e - 1]].z + kl.item[ord[e - 1]].w)
+         e++;
+      for (size_t r = f; r < e; r += KT / KI) {
+         int4 t = kl.item[ord[r]], q = make_int4(-1, -1, -1, -1);
+         t.w = 0;
+         int *qp = &q.x;
+         for (size_t j = r; j < e && j < r + KT / KI; j++) {
+            t.w += kl.item[ord[j]].w;
+            qp[j - r] = kl.item_k0[ord[j]];
+         }
+         it.push_back(t);
+         kk.push_back(q);
+      }
+      f = e;
+   }
+   std::vector<int> by(it.size());
+   for (size_t i = 0; i < by.size(); i++) by[i] = (int)i;
+   std::stable_sort(by.begin(), by.end(), [&](int a, int b) { return it[a].w > it[b].w; });
+   item.clear();
+   k0.clear();
+   for (int i : by) {
+      item.push_back(it[i]);
+      k0.push_back(kk[i]);
+   }
+   while (item.size() % 128) {
+      item.push_back(make_int4(0, 0, 0, 0));
+      k0.push_back(make_int4(-1, -1, -1, -1));
+   }
+}
+
+// The k-list as quads (h, m): the k-vectors (h, s m, r t), s, r = +-1, of one
+// quad and t share their trig products (kspace_q.cu).  A unit is four quads
+// (h, m0 .. m0 + 3), m0 a multiple of 4; its t range covers every |l| of its
+// quads.  Units run over blocks of four h, m up in one block and down in the
+// next, so that consecutive units span few h and m values (the tables a row
+// tile reads).
+void build_qlist(KList &kl, int ns)
+{
+   QList &q = kl.q;
+   q = QList();
+   q.ns = ns;
+   int hm = 0, mm = 0, lm = 0;
+   for (const int4 &it : kl.item) {
+      hm = std::max(hm, it.x);
+      mm = std::max(mm, std::abs(it.y));
+      lm = std::max(lm, std::max(std::abs(it.z), std::abs(it.z + it.w - 1)));
+   }
+   const int M4 = mm / 4 + 1;
+   std::vector<int> tr((size_t)(hm + 1) * M4, 0);   // t range of each unit
+   for (const int4 &it : kl.item) {
+      int &t = tr[(size_t)it.x * M4 + std::abs(it.y) / 4];
+      t = std::max(t, std::max(std::abs(it.z), std::abs(it.z + it.w - 1)) + 1);
+   }
+   QGeom &g = q.g;
+   g.hrows = hm + 1;
+   g.mrows = 4 * M4;
+   const int T = lm + 1;
+   if (ns == 3) {   // t-blocks of up to 40 (80 columns), equally wide
+      g.nblk = (T + 39) / 40;
+      g.TW = ((T + g.nblk - 1) / g.nblk + 7) / 8 * 8;
+      g.TP = g.TW * g.nblk;
+   } else {         // 32 wide, the last one 16 or 32
+      g.nblk = (T + 31) / 32;
+      g.TW = 32;
+      g.TP = 32 * (g.nblk - 1) + (T - 32 * (g.nblk - 1) <= 16 ? 16 : 32);
+   }
+   for (int k = 0; k < 9; k++) g.b[k] = 2 * PI * kl.hinv[k];
+   std::vector<int> uid((size_t)(hm + 1) * M4, -1);
+   for (int hb = 0; hb <= hm; hb += 4)
+      for (int j = 0; j < M4; j++) {
+         const int mb = (hb / 4) & 1 ? M4 - 1 - j : j;
+         for (int h = hb; h <= hm && h < hb + 4; h++) {
+            const int t = tr[(size_t)h * M4 + mb];
+            if (t == 0) continue;
+            uid[(size_t)h * M4 + mb] = (int)q.units.size();
+            q.units.push_back(make_int4(h, 4 * mb, t, 0));
+         }
+      }
+   const int nu = (int)q.units.size();
+   g.nquads = 4 * nu;
+   q.coeff.assign((size_t)g.nquads * g.TP * 4, make_double2(0.0, 0.0));
+   for (int i = 0; i < kl.nitems; i++)
+      for (int w = 0; w < kl.item[i].w; w++) {
+         const int4 it = kl.item[i];
+         const int k = kl.item_k0[i] + w, l = it.z + w, m = std::abs(it.y), s = it.y < 0, r = l < 0;
+         const int quad = 4 * uid[(size_t)it.x * M4 + m / 4] + m % 4;
+         q.coeff[((size_t)quad * g.TP + std::abs(l)) * 4 + 2 * s + r] = make_double2(kl.coeff[k], kl.coeff2[k]);
+      }
+   // structure-factor row tiles: up to 16 (mixed) or 8 units of a t-block
+   const int per = ns == 3 ? 16 : 8;
+   for (int b = 0; b < g.nblk; b++) {
+      QTile t;
+      int n = 0, x0 = 0, x1 = 0, y0 = 0, y1 = 0;
+      auto close = [&] {
+         if (n == 0) return;
+         t.col0 = 2 * b * g.TW;
+         t.nT = 2 * std::min(g.TW, g.TP - b * g.TW);
+         t.xlo = x0;
+         t.nx = x1 - x0 + 1;
+         t.ylo = y0;
+         t.ny = y1 - y0 + 4;
+         for (int k = n; k < 16; k++) t.unit[k] = -1;
+         q.tiles.push_back(t);
+         n = 0;
+      };
+      for (int u = 0; u < nu; u++) {
+         const int4 un = q.units[u];
+         if (un.z <= b * g.TW) continue;
+         if (n > 0) {
+            const int nx0 = std::min(x0, un.x), nx1 = std::max(x1, un.x), ny0 = std::min(y0, un.y), ny1 = std::max(y1, un.y);
+            if (n == per || nx1 - nx0 + 1 > Q_XMAX || ny1 - ny0 + 4 > Q_YMAX) close();
+         }
+         if (n == 0) {
+            x0 = x1 = un.x;
+            y0 = y1 = un.y;
+         }
+         x0 = std::min(x0, un.x);
+         x1 = std::max(x1, un.x);
+         y0 = std::min(y0, un.y);
+         y1 = std::max(y1, un.y);
+         t.unit[n++] = u;
+      }
+      close();
+   }
+   if (ns == 7) {
+      // force-pass segments: units by rising |(h, m)| in reciprocal space, so
+      // that a segment's coefficients are of similar size
+      std::vector<int> ord(nu);
+      for (int u = 0; u < nu; u++) ord[u] = u;
+      auto rad = [&](int u) {
+         const double x = q.units[u].x * g.b[0], y = (q.units[u].y + 1.5) * g.b[4];
+         return x * x + y * y;
+      };
+      std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return rad(a) < rad(b); });
+      for (int b = 0; b < g.nblk; b++) {
+         q.seg0.push_back((int)q.segs.size());
+         int n = 0;
+         QSeg s;
+         s.blk = b;
+         auto close = [&] {
+            if (n == 0) return;
+            for (; n < 8; n++) s.unit[n] = -1;
+            q.segs.push_back(s);
+            n = 0;
+         };
+         for (int u : ord)
+            if (q.units[u].z > b * g.TW) {
+               s.unit[n++] = u;
+               if (n == 8) close();
+            }
+         close();
+      }
+      q.seg0.push_back((int)q.segs.size());
+   } else {
+      // mixed force pass: per 64-wide t-block the units by falling t range,
+      // padded to item tiles of four
+      for (int b = 0; 64 * b < g.TP; b++) {
+         q.fblk.push_back((int)q.fu.size());
+         std::vector<int> ord;
+         for (int u = 0; u < nu; u++)
+            if (q.units[u].z > 64 * b) ord.push_back(u);
+         if (ord.empty()) {
+            q.fblk.pop_back();
+            break;
+         }
+         std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return q.units[x].z > q.units[y].z; });
+         for (int u : ord) q.fu.push_back(make_int4(q.units[u].x, q.units[u].y, q.units[u].z, u));
+         while (q.fu.size() % 4) q.fu.push_back(make_int4(0, 0, 0, -1));
+      }
+      q.fblk.push_back((int)q.fu.size());
+   }
 }
 
 // ---- pair potential at one distance (kernel() for one pair, poteval) -----

@@ -49,8 +49,7 @@ __device__ __forceinline__ unsigned long long to_fixed64(double s)
 // FP32 partial sums stay small even where the full sum cancels (an ionic
 // crystal listed species by species would otherwise give chunks of a
 // single charge sign).  mixed: 0 the FP64 records, 1 the FP32 records and
-// z tables, 2 the FP32 phases only (the tensor-core passes build their own
-// tables).
+// z tables.
 __global__ void k_prep(int N, int ns, const int *__restrict__ sorted, const double *__restrict__ site,
                        const double *__restrict__ chg, double hi0, double hi1, double hi2,
                        double hi3, double hi4, double hi5, double hi6, double hi7, double hi8,
@@ -73,7 +72,6 @@ __global__ void k_prep(int N, int ns, const int *__restrict__ sorted, const doub
       unsigned int uy32 = (unsigned int)((uy + 0x80000000ull) >> 32);
       unsigned int uz32 = (unsigned int)((uz + 0x80000000ull) >> 32);
       ph32[i] = make_int4((int)ux32, (int)uy32, (int)uz32, __float_as_int((float)q));
-      if (mixed == 2) return;   // the tensor-core passes build their own z tables
       double sz, cz;
       sincospi(2.0 * ((double)(long long)uz * 5.421010862427522e-20), &sz, &cz);   // 2^-64
       z32[i] = make_float2((float)cz, (float)sz);
@@ -915,12 +913,12 @@ __global__ void k_kcompact(int N, const int *__restrict__ sorted, const double *
 // -------------------------------------------------------------- host side
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
 
-mdgpu_status ks_prepare(mdgpu_ctx *c)
+// The k-list's device tables of the CUDA-core passes.
+static mdgpu_status ks_upload_list(mdgpu_ctx *c)
 {
    KsDev &d = c->kd;
    const KList &kl = c->kl;
    cudaStream_t st = c->stream;
-   const int N = c->nsites;
    if (!c->kl_uploaded) {
       const int nk = kl.nk, ni = kl.nitems;
       CK(d.item.ensure(ni));
@@ -949,34 +947,25 @@ mdgpu_status ks_prepare(mdgpu_ctx *c)
       CK(cudaMemcpyAsync(d.kz64.p, kv.data(), kv.size() * sizeof(double), cudaMemcpyHostToDevice, st));
       CK(cudaMemcpyAsync(d.coeff.p, kl.coeff.data(), nk * sizeof(double), cudaMemcpyHostToDevice, st));
       CK(cudaMemcpyAsync(d.coeff2.p, kl.coeff2.data(), nk * sizeof(double), cudaMemcpyHostToDevice, st));
-      const size_t nt = kl.tc_item.size();
-      CK(d.tc_item.ensure(nt));
-      CK(d.tc_k0.ensure(nt));
-      CK(d.tc_kxy.ensure(nt));
-      CK(d.tc_coef.ensure(nt));
-      CK(cudaMemcpyAsync(d.tc_kxy.p, kl.tc_kxy.data(), nt * sizeof(float2), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.tc_item.p, kl.tc_item.data(), nt * sizeof(int4), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.tc_k0.p, kl.tc_k0.data(), nt * sizeof(int4), cudaMemcpyHostToDevice, st));
       CK(cudaStreamSynchronize(st));
-      d.tc_ver++;
       c->kl_uploaded = true;
    }
-   if (c->prec == MDGPU_MIXED && c->tc_sfac) {
-      CK(ks_tc_init(c->device));
-      CK(d.ztab.ensure(ks_tc_ztab_len(N)));
-      CK(d.zsite.ensure(ks_tc_zsite_len(N)));
-      CK(d.utab.ensure(ks_tc_utab_len((int)kl.tc_item.size())));
+   return MDGPU_OK;
+}
+
+mdgpu_status ks_prepare(mdgpu_ctx *c)
+{
+   KsDev &d = c->kd;
+   cudaStream_t st = c->stream;
+   const int N = c->nsites;
+   if (c->tc_sfac && N == c->fw_site0) {
+      const mdgpu_status s = ks_q_prepare(c, c->prec == MDGPU_MIXED ? 3 : 7);
+      if (s) return s;
    }
-   CK(d.ph32.ensure(N + 128));
    if (!d.kcount.p) {   // k_kfinal_part's finished-block counter, zero between evaluations
       CK(d.kcount.ensure(1));
       CK(cudaMemsetAsync(d.kcount.p, 0, sizeof(unsigned int), st));
    }
-   CK(d.z32.ensure(N));
-   CK(d.zp32.ensure((size_t)N * KI));
-   CK(d.ph64a.ensure(N));
-   CK(d.ph64b.ensure(N));
-   CK(d.z64.ensure(N));
    return MDGPU_OK;
 }
 
@@ -1063,19 +1052,28 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       c->launches += 3;
       slots = d.kslots.p;
    }
-   // mixed form over the charged sites: both passes on the tensor cores
-   const bool tc = mixed && compact && c->tc_sfac;
-   k_prep<<<(Nk + 255) / 256, 256, 0, st>>>(Nk, N, slots, d_site, c->rd.chg.p, hinv[0], hinv[1], hinv[2],
-                                            hinv[3], hinv[4], hinv[5], hinv[6], hinv[7], hinv[8],
-                                            tc ? 2 : mixed ? 1 : 0, d.ph32.p, d.z32.p, d.zp32.p, d.ph64a.p,
-                                            d.ph64b.p, d.z64.p);
-   CK(cudaGetLastError());
+   // over the charged sites: both passes on the tensor cores
+   const bool tc = compact && c->tc_sfac;
+   const int ns = mixed ? 3 : 7;
+   mdgpu_status s;
+   if (!tc && (s = ks_upload_list(c)) != MDGPU_OK) return s;
    if (tc) {
-      CK(d.ztab.ensure(ks_tc_ztab_len(Nk)));
-      CK(d.zsite.ensure(ks_tc_zsite_len(Nk)));
-      CK(d.utab.ensure(ks_tc_utab_len((int)kl.tc_item.size())));
-      ks_tables_tc(st, Nk, d);
-      c->launches += 1;
+      if ((s = ks_q_tables(c, ns, Nk, slots, d_site)) != MDGPU_OK) return s;
+   } else {
+      if (mixed) {
+         CK(d.ph32.ensure(N));
+         CK(d.z32.ensure(N));
+         CK(d.zp32.ensure((size_t)N * KI));
+      } else {
+         CK(d.ph64a.ensure(N));
+         CK(d.ph64b.ensure(N));
+         CK(d.z64.ensure(N));
+      }
+      k_prep<<<(Nk + 255) / 256, 256, 0, st>>>(Nk, N, slots, d_site, c->rd.chg.p, hinv[0], hinv[1], hinv[2],
+                                               hinv[3], hinv[4], hinv[5], hinv[6], hinv[7], hinv[8],
+                                               mixed ? 1 : 0, d.ph32.p, d.z32.p, d.zp32.p, d.ph64a.p, d.ph64b.p,
+                                               d.z64.p);
+      CK(cudaGetLastError());
    }
    KsShape sh = mixed ? ks_shape(Nk, ni, 1, 2) : ks_shape(Nk, ni, 1, 1);
    if (nf > 0) {
@@ -1088,8 +1086,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    phase_mark(c, MDGPU_PH_SFAC);
    const dim3 gs((ni + 127) / 128, sh.chunks);
    if (tc) {
-      CK(d.part32.ensure((size_t)ks_tc_chunks(Nk) * nk));
-      sh.chunks = ks_sfac_tc(st, Nk, nk, d, (int)(kl.tc_item.size() / 128), c->qmax, &out->err);
+      if ((s = ks_q_sfac(c, ns, Nk, &sh.chunks)) != MDGPU_OK) return s;
    } else if (mixed) {
       CK(d.part32.ensure((size_t)sh.chunks * nk));
       k_sfac32<<<gs, 128, 0, st>>>(d.item.p, d.item_k0.p, ni, d.ph32.p, d.zp32.p, Nk, sh.chunk, nk, d.part32.p,
@@ -1111,10 +1108,12 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    }
    CK(cudaGetLastError());
    // blocks of the per-k reduction: KR_K k each (the framework form: 256)
-   const int nbk = nf > 0 ? (nk + 255) / 256 : (nk + KR_K - 1) / KR_K;
+   int nbk = nf > 0 ? (nk + 255) / 256 : (nk + KR_K - 1) / KR_K;
    CK(d.blk.ensure((size_t)nbk * 8));
    phase_mark(c, MDGPU_PH_KREDUCE);
-   if (nf > 0) {
+   if (tc) {
+      if ((s = ks_q_reduce(c, ns, sh.chunks, &nbk)) != MDGPU_OK) return s;
+   } else if (nf > 0) {
       if (mixed) {
          CK(d.kdatf32.ensure(nk));
          k_kreduce_fw<true><<<nbk, 256, 0, st>>>(nk, sh.chunks, d.part32.p, d.partf32.p, nullptr, nullptr,
@@ -1141,21 +1140,23 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       k_kfinal<<<1, 512, 0, st>>>(d.blk.p, nbk, out);
    }
    CK(cudaGetLastError());
-   if (tc) {
-      sh.splits = ks_force_tc_splits(Nk);
-      ks_coef_tc(st, d, (int)kl.tc_item.size(), (float)kl.dkz);
-      c->launches += 1;
+   if (tc && mixed) {
+      sh.splits = ks_force_tc_splits(d);
+      int np = 0;
+      for (int i = 0; i < d.q_nfblk; i++) np = std::max(np, d.q_fblk[i + 1] - d.q_fblk[i]);
+      CK(d.utab.ensure(ks_tc_utab_len(np)));
+      CK(d.tc_coef.ensure((size_t)np * 8));
    }
-   CK(d.fpart.ensure((size_t)sh.splits * 3 * Nk));
+   if (!tc || mixed) CK(d.fpart.ensure((size_t)sh.splits * 3 * Nk));
    phase_mark(c, MDGPU_PH_KFORCE);
    dim3 gf((Nk + 255) / 256, sh.splits);
    const int obase = compact ? -1 : 0;   // partial rows by slot of the charged list, or by site
-   if (tc) {
-      if (c->nsm <= 0) CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
-      const int nl = ks_force_tc(st, Nk, d, (int)kl.tc_item.size(), c->nsm, c->rd.chg.p, slots, d.fpart.p,
-                                 &out->err);
+   if (tc && mixed) {
+      const int nl = ks_force_tc(st, Nk, kl.q.g, d, c->nsm, c->rd.chg.p, slots, d.fpart.p, &out->err);
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl - 1;
+   } else if (tc) {
+      if ((s = ks_q_force64(c, Nk, slots)) != MDGPU_OK) return s;
    } else if (mixed)
       k_force32<<<gf, FT_THREADS, 0, st>>>(d.item.p, d.item_k0.p, d.item_kxy32.p, ni, nk, sh.per_split,
                                            d.kdat32.p, d.ph32.p, d.zp32.p, c->rd.chg.p, slots, Nk, obase,
@@ -1169,6 +1170,9 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    if (join) CK(cudaStreamWaitEvent(st, join, 0));
    if (compact) {
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
+      if (tc && !mixed) {
+         if ((s = ks_q_fsum64(c, Nk, slots, d_force)) != MDGPU_OK) return s;
+      } else
       k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots, d_force);
    } else {
       k_fsum<<<(3 * N + 255) / 256, 256, 0, st>>>(3 * N, sh.splits, d.fpart.p, d_force, accumulate ? 1 : 0);

@@ -1,0 +1,1242 @@
+// Reciprocal space on the tensor cores by products of one-dimensional trig
+// tables: the structure factor of both forms and the force pass of the FP64
+// form (the S(k) and force sums of ewald(), src/ewald.c:523-579).
+//
+// A quad is a pair (h, m), m = |k| >= 0: the columns (h, +-m) of the k-list.
+// With the per-site tables X = cos, sin(2 pi h s_x), Y = cos, sin(2 pi m s_y)
+// and Z = cos, sin(2 pi t s_z), t = |l|, the four k-vectors (h, s m, r t),
+// s, r = +-1, have
+//     exp(i k.r) = [(P1 - s P2) + i (P3 + s P4)] (C_t + i r S_t),
+//     P1 = ch cm, P2 = sh sm, P3 = sh cm, P4 = ch sm,
+// so the eight real sums  Q_pc = sum_j q_j P_p {C_t, S_t}  give S(k) of all
+// four (k_qreduce), and the force sums are eight real sums the other way
+// round.  Against one seed per k-column and the running l this is half the
+// tensor-core work per k-vector (both signs of l from one product) and one
+// multiplication per operand element in place of half a sine/cosine pair.
+//
+// Arithmetic.  Every operand is a fixed-point integer cut into NS balanced
+// base-256 digits d in [-128, 127], held as fp16 (exact), digit i of weight
+// 2^(-7 - 8 i).  A product of digits i and j goes to accumulator group
+// g = i + j; groups g < NS are kept.  In a group all products are integers
+// below 2^14, so the FP32 accumulators are exact while fewer than
+// 2^10 / (g + 1) terms are added; they are read back and added up in
+// wide integers (NS = 7: 96 bits, every 128 terms) or FP32 (NS = 3, every
+// 1024 terms, where only group 0 has to be exact).
+//   NS = 3  mixed form: operands to 2^-24, as the FP32 path
+//   NS = 7  FP64 form: operands to 2^-56, products left out below 2^-56:
+//           errors below the rounding of an FP64 multiply-add per term.
+// The tables themselves are integer polynomials of the exact integer phases
+// (qsincos), good to 2^-60 and 2^-29.
+// Digits laid end to end: operand B holds its NS digits as consecutive rows
+// blocks, so one MMA of digit i of A by digits 0 .. NS - 1 - i of B adds to
+// groups i .. NS - 1 at once (NS instructions per K-step in place of
+// NS (NS + 1) / 2, and A is read from shared memory NS times).
+//
+// Measured, 131,072-site water (98,304 charged sites, 69,876 k-vectors),
+// against one FP64 recurrence per k and site, or the seed-and-run bf16
+// products of the mixed form: FP64 structure factor 119.4 -> 1.41 ms, forces
+// 130.4 -> 4.86 ms; mixed structure factor 0.414 -> 0.299 ms.  Force error
+// of the FP64 form against extended precision (2048-site water; rock salt,
+// 5832 ions): 6.1e-15 -> 2.2e-15; 1.5e-14 -> 1.1e-14.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstring>
+
+#include "mdgpu_internal.h"
+#include "tc.cuh"
+
+namespace mdgpu {
+
+// ---------------------------------------------------------------- layout
+constexpr int Q_KS = 32;                          // K per stage: sites, or K-rows (two units)
+constexpr int Q_OP = 128 * Q_KS * 2;              // one digit of a 128-row operand stage: 8 KB
+constexpr int Q_BW = 16;                          // operand / read-back warps
+constexpr int Q_THREADS = 32 * (Q_BW + 3);        // and a bulk-copy warp, two MMA warps
+constexpr int Q_ERR = 8, Q_FERR = 16;             // error-word bits: structure factor, force pass
+
+template <int NS> struct QCfg;
+template <> struct QCfg<3> {
+   typedef int T;
+   static constexpr int RS = 36;                  // table row: 32 sites, padded against bank conflicts
+   static constexpr int MT = 2, NPART = 1;        // 128-row tiles per CTA, column parts of B
+   static constexpr int NB = 3;                   // stages in flight
+   static constexpr int NTMAX = 80;               // columns (2 t-width) of a t-block
+   static constexpr int SEG = 32;                 // stages between read-backs
+};
+template <> struct QCfg<7> {
+   typedef long long T;
+   static constexpr int RS = 34;
+   static constexpr int MT = 1, NPART = 2;
+   static constexpr int NB = 2;
+   static constexpr int NTMAX = 64;
+   static constexpr int SEG = 4;
+};
+// bytes: a stage's table rows, its B operand, both; the A operand; all
+template <int NS> constexpr int Q_TAB = 2 * (Q_XMAX + Q_YMAX) * QCfg<NS>::RS * (int)sizeof(typename QCfg<NS>::T);
+template <int NS> constexpr int Q_B = QCfg<NS>::NTMAX * Q_KS * 2 * NS;
+template <int NS> constexpr int Q_STAGE = Q_B<NS> + Q_TAB<NS>;
+template <int NS> constexpr int Q_A = QCfg<NS>::MT * NS * Q_OP;
+template <int NS> constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_STAGE<NS>;
+static_assert(Q_SMEM<3> <= 227 * 1024 && Q_SMEM<7> <= 227 * 1024, "one CTA's shared memory");
+static_assert(Q_STAGE<3> % 128 == 0 && Q_STAGE<7> % 128 == 0, "stage buffers stay aligned");
+
+// ------------------------------------------------------ fixed-point trig
+// sin, cos(2 pi p / 2^64) in units of 2^-63: the phase is reduced to an
+// eighth turn, p = quadrant + w (1/8), |w| <= 1, and the Taylor series of
+// sin and cos (pi w / 4) are summed in v = w^2 / 4 by 64-bit integer Horner
+// steps (coefficients (pi/4)^n 4^k / n! in units of 2^-64; terms left out
+// below 2^-62).
+__device__ __forceinline__ void qsincos(unsigned long long p, long long &s, long long &c)
+{
+   const unsigned int qd = (unsigned int)((p + (1ull << 61)) >> 62);
+   const long long r = (long long)(p - ((unsigned long long)qd << 62));
+   const unsigned long long w = (unsigned long long)(r < 0 ? -r : r) << 2;    // |w| 2^63
+   const unsigned long long v = __umul64hi(w, w);                             // w^2 / 4 in 2^-64
+   unsigned long long a = 0x355d865ull;
+   a = 0x16fadb9f1ull - __umul64hi(v, a);
+   a = 0x7a3d0d3406ull - __umul64hi(v, a);
+   a = 0x1e3074fde887ull - __umul64hi(v, a);
+   a = 0x541e0d21fb9e0ull - __umul64hi(v, a);
+   a = 0x9969667315ec2eull - __umul64hi(v, a);
+   a = 0xa335e33bad570e9ull - __umul64hi(v, a);
+   a = 0x52aef39896f94afbull - __umul64hi(v, a);
+   a = 0xc90fdaa22168c235ull - __umul64hi(v, a);
+   unsigned long long b = 0x4a8316ull;
+   b = 0x2418c586ull - __umul64hi(v, b);
+   b = 0xdb7127a26ull - __umul64hi(v, b);
+   b = 0x3f3a7146ec8ull - __umul64hi(v, b);
+   b = 0xd368f9510254ull - __umul64hi(v, b);
+   b = 0x1e1f506891babbull - __umul64hi(v, b);
+   b = 0x2aba78fc797ff40ull - __umul64hi(v, b);
+   b = 0x20783e1036b58767ull - __umul64hi(v, b);
+   b = 0x9de9e64df22ef2d2ull - __umul64hi(v, b);
+   unsigned long long sn = __umul64hi(w, a);
+   unsigned long long cs = (1ull << 63) - __umul64hi(v, b);
+   sn -= sn >> 8;                                                             // times Q_KAPPA
+   cs -= cs >> 8;
+   const long long S = r < 0 ? -(long long)sn : (long long)sn, C = (long long)cs;
+   const bool sw = qd & 1u, ng = qd & 2u;
+   s = sw ? C : S;
+   c = sw ? -S : C;
+   if (ng) {
+      s = -s;
+      c = -c;
+   }
+}
+// The same for a 32-bit phase, in units of 2^-31 (terms left out below 2^-32).
+__device__ __forceinline__ void qsincos(unsigned int p, int &s, int &c)
+{
+   const unsigned int qd = (p + (1u << 29)) >> 30;
+   const int r = (int)(p - (qd << 30));
+   const unsigned int w = (unsigned int)(r < 0 ? -r : r) << 2;
+   const unsigned int v = __umulhi(w, w);
+   unsigned int a = 0x1e30u;
+   a = 0x541e1u - __umulhi(v, a);
+   a = 0x996966u - __umulhi(v, a);
+   a = 0xa335e34u - __umulhi(v, a);
+   a = 0x52aef399u - __umulhi(v, a);
+   a = 0xc90fdaa2u - __umulhi(v, a);
+   unsigned int b = 0x3f4u;
+   b = 0xd369u - __umulhi(v, b);
+   b = 0x1e1f50u - __umulhi(v, b);
+   b = 0x2aba790u - __umulhi(v, b);
+   b = 0x20783e10u - __umulhi(v, b);
+   b = 0x9de9e64eu - __umulhi(v, b);
+   unsigned int sn = __umulhi(w, a), cs = (1u << 31) - __umulhi(v, b);
+   sn -= sn >> 8;
+   cs -= cs >> 8;
+   const int S = r < 0 ? -(int)sn : (int)sn, C = (int)cs;
+   const bool sw = qd & 1u, ng = qd & 2u;
+   s = sw ? C : S;
+   c = sw ? -S : C;
+   if (ng) {
+      s = -s;
+      c = -c;
+   }
+}
+// phase n u (n a table index) in the form's width; 32-bit phases are
+// rounded from the 64-bit product, so their error does not grow with n
+__device__ __forceinline__ void qtrig(int n, unsigned long long u, long long &s, long long &c)
+{
+   qsincos((unsigned long long)n * u, s, c);
+}
+__device__ __forceinline__ void qtrig(int n, unsigned long long u, int &s, int &c)
+{
+   qsincos((unsigned int)(((unsigned long long)n * u + 0x80000000ull) >> 32), s, c);
+}
+
+// A 64-bit table value as (signed low word, high word): ah 2^32 + al.
+__device__ __forceinline__ long long qbalance(long long v)
+{
+   const int lo = (int)v;
+   return (long long)((unsigned long long)((v - lo) & ~0xffffffffll) | (unsigned int)lo);
+}
+__device__ __forceinline__ int qbalance(int v) { return v; }
+
+// Biased product of two table values (units of 2^-31 / 2^-63 again): every
+// byte but the lowest is a digit plus 128, the lowest rounds.
+__device__ __forceinline__ unsigned int qmul(int a, int b)
+{
+   const unsigned int t = (unsigned int)__mulhi(a, b);
+   return t + t + 0x80808080u;
+}
+__device__ __forceinline__ unsigned long long qmul(long long a, long long b)   // balanced values
+{
+   const int ah = (int)(a >> 32), al = (int)a, bh = (int)(b >> 32), bl = (int)b;
+   const long long t = (long long)ah * bh + (long long)(__mulhi(ah, bl) + __mulhi(al, bh));
+   return (unsigned long long)(t + t) + 0x8080808080808080ull;
+}
+
+// Digit i of two biased values as an fp16 pair (first value in the low half).
+__device__ __forceinline__ unsigned int qpair(unsigned int bytes)   // 0x??B?A: values plus 128 in bytes 0 and 2
+{
+   unsigned int r;
+   const unsigned int v = (bytes & 0x00ff00ffu) | 0x64006400u;       // fp16 1024 + byte
+   asm("add.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0xe480e480u));   // - 1152
+   return r;
+}
+template <int I> __device__ __forceinline__ unsigned int qdigit(unsigned int a, unsigned int b)
+{
+   return qpair(__byte_perm(a, b, (3 - I) | ((7 - I) << 8)));
+}
+template <int I> __device__ __forceinline__ unsigned int qdigit(unsigned long long a, unsigned long long b)
+{
+   if (I < 4)
+      return qdigit<(I < 4 ? I : 0)>((unsigned int)(a >> 32), (unsigned int)(b >> 32));
+   return qdigit<(I >= 4 ? I - 4 : 0)>((unsigned int)a, (unsigned int)b);
+}
+// NS = 3, operand A: x in units of 2^-24 (24 bits), y of 2^-31, the product
+// rounded to 2^-23, its digits plus 128 in bytes 3, 2, 1 and the high byte
+// of fp16 1024 in byte 0, so that one byte permutation gives an fp16 pair
+// without a mask.  The ALU pipe (permutations, masks, adds; half the rate of
+// the FMA pipe) bounds the operand build: the multiplications are written so
+// that they run on the FMA pipe (c256 = 256 is not a constant to the
+// compiler, or it would shift and add on the ALU).
+struct QA {
+   unsigned int v;
+};
+__device__ __forceinline__ QA qmul_a(int x, int y, unsigned int c256)
+{
+   const long long t = (long long)x * y + 0x80000000ll;
+   QA r;
+   asm("mad.lo.u32 %0, %1, %2, %3;" : "=r"(r.v) : "r"((unsigned int)(t >> 32)), "r"(c256), "r"(0x80808064u));
+   return r;
+}
+__device__ __forceinline__ unsigned long long qmul_a(long long x, long long y, unsigned int) { return qmul(x, y); }
+template <int I> __device__ __forceinline__ unsigned int qdigit(QA a, QA b)
+{
+   unsigned int r;
+   const unsigned int v = __byte_perm(a.v, b.v, (3 - I) | ((7 - I) << 8) | (4 << 12));
+   asm("add.f16x2 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(0xe480e480u));   // - 1152
+   return r;
+}
+// The NS digits of eight values (K order) to dst + i stride.
+template <int NS, int I, typename U> struct QStore {
+   static __device__ __forceinline__ void run(unsigned char *dst, int stride, const U (&v)[8])
+   {
+      *reinterpret_cast<uint4 *>(dst) =
+         make_uint4(qdigit<I>(v[0], v[1]), qdigit<I>(v[2], v[3]), qdigit<I>(v[4], v[5]), qdigit<I>(v[6], v[7]));
+      QStore<NS, I + 1, U>::run(dst + stride, stride, v);
+   }
+};
+template <int NS, typename U> struct QStore<NS, NS, U> {
+   static __device__ __forceinline__ void run(unsigned char *, int, const U (&)[8]) {}
+};
+template <int NS, typename U> __device__ __forceinline__ void qstore(unsigned char *dst, int stride, const U (&v)[8])
+{
+   QStore<NS, 0, U>::run(dst, stride, v);
+}
+
+__device__ __forceinline__ unsigned long long q_fixed64(double s)
+{
+   // frac(s) 2^64 for |s| < 2 (as k_prep)
+   return (unsigned long long)__double2ll_rn(s * 4611686018427387904.0) << 2;
+}
+
+__device__ __forceinline__ int q_blkcols(const QGeom &g, int b) { return 2 * min(g.TW, g.TP - b * g.TW); }
+
+// ------------------------------------------------------------- per site
+// One block per 32-site stage of the charged list (slots; sites past n get
+// phase and charge zero): the X and Y tables, the structure factor's B
+// operand (digits of q z, the charge scaled by a power of two to |q| < 1),
+// and per form: NS = 3 the force pass's A operand (zsite: three bf16 terms
+// of z per 128-site tile and 64-wide t-block, [term][per 8 t: cosines,
+// sines][row group][8 sites][8 t]); NS = 7 the z values in FP64 (zd).
+template <int NS>
+__global__ void __launch_bounds__(256)
+k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__restrict__ site,
+       const double *__restrict__ chg, double hi0, double hi1, double hi2, double hi3, double hi4, double hi5,
+       double hi6, double hi7, double hi8, double qinv, typename QCfg<NS>::T *__restrict__ X,
+       typename QCfg<NS>::T *__restrict__ Y, unsigned char *__restrict__ ztab, uint4 *__restrict__ zsite,
+       double *__restrict__ zd)
+{
+   typedef typename QCfg<NS>::T T;
+   constexpr int RS = QCfg<NS>::RS;
+   __shared__ unsigned long long su[3][32];
+   __shared__ T sq[32];
+   __shared__ T sz[64][33];   // [per 8 t: 8 cosines, 8 sines][site] of a 32-wide run of t
+   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, stage = blockIdx.x;
+   if (w == 0) {
+      const int i = stage * 32 + lane;
+      unsigned long long ux = 0, uy = 0, uz = 0;
+      double q = 0.0;
+      if (i < n) {
+         const int si = slots[i];
+         const double x = site[si], y = site[ns + si], z = site[2 * (size_t)ns + si];
+         ux = q_fixed64(hi0 * x + hi1 * y + hi2 * z);
+         uy = q_fixed64(hi3 * x + hi4 * y + hi5 * z);
+         uz = q_fixed64(hi6 * x + hi7 * y + hi8 * z);
+         q = chg[si] * qinv * Q_KAPPA;
+      }
+      su[0][lane] = ux;
+      su[1][lane] = uy;
+      su[2][lane] = uz;
+      sq[lane] = NS == 3 ? (T)__double2int_rn(q * 2147483648.0)
+                         : (T)qbalance((T)__double2ll_rn(q * 9223372036854775808.0));
+   }
+   __syncthreads();
+   {
+      const unsigned long long ux = su[0][lane], uy = su[1][lane];
+      T *xb = X + (size_t)stage * 2 * g.hrows * RS + lane, *yb = Y + (size_t)stage * 2 * g.mrows * RS + lane;
+      for (int r = w; r < g.hrows + g.mrows; r += 8) {
+         const bool y = r >= g.hrows;
+         const int k = y ? r - g.hrows : r;
+         T s, c;
+         qtrig(k, y ? uy : ux, s, c);
+         if (NS == 3 && !y) {   // X in units of 2^-24
+            c = (c + 64) >> 7;
+            s = (s + 64) >> 7;
+         }
+         T *d = (y ? yb : xb) + (size_t)2 * k * RS;
+         d[0] = qbalance(c);
+         d[RS] = qbalance(s);
+      }
+   }
+   const unsigned long long uz = su[2][lane];
+   for (int t0 = 0; t0 < g.TP; t0 += 32) {
+      const int nt = min(32, g.TP - t0);   // a multiple of 8
+      __syncthreads();
+      for (int t = w; t < nt; t += 8) {
+         T s, c;
+         qtrig(t0 + t, uz, s, c);
+         const int col = 16 * (t >> 3) + (t & 7);
+         sz[col][lane] = qbalance(c);
+         sz[col + 8][lane] = qbalance(s);
+         if (NS == 7) {
+            double *d = zd + ((size_t)stage * 2 * g.TP + 2 * t0 + col) * 32 + lane;
+            d[0] = (double)c * (1.0 / (9223372036854775808.0 * Q_KAPPA));
+            d[8 * 32] = (double)s * (1.0 / (9223372036854775808.0 * Q_KAPPA));
+         }
+      }
+      __syncthreads();
+      {
+         // digits of q z: 8 sites (kg) of one column per thread
+         const int kg = tid & 3, c8 = (tid >> 2) & 7, cg = tid >> 5;
+         if (8 * cg < 2 * nt) {
+            auto qz = [&](int e) { return qmul(sq[8 * kg + e], sz[8 * cg + c8][8 * kg + e]); };
+            decltype(qz(0)) v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = qz(e);
+            const int tcol = 2 * t0 + 8 * cg, b = tcol / (2 * g.TW), lc = tcol - 2 * b * g.TW;
+            const int nT = q_blkcols(g, b), pc = nT / QCfg<NS>::NPART;   // columns of a part
+            const int part = lc / pc, pl = lc - part * pc;
+            unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * NS + (size_t)2 * b * g.TW * Q_KS * 2 * NS +
+                               ((size_t)part * NS * pc + pl) * Q_KS * 2 + kg * 128 + c8 * 16;
+            qstore<NS>(d, pc * Q_KS * 2, v);
+         }
+      }
+      if (NS == 3) {
+         // force pass: 8 t of one site per thread, cosines or sines
+         const int sl = tid & 31, cg = tid >> 5;
+         if (8 * cg < 2 * nt) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = (float)sz[8 * cg + e][sl] * (float)(1.0 / (2147483648.0 * Q_KAPPA));
+            unsigned int h[4], m[4], l[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) tc::split3(v[2 * j], v[2 * j + 1], h[j], m[j], l[j]);
+            const int i = stage * 32 + sl, tile = i >> 7, r = i & 127;
+            const int tcol = 2 * t0 + 8 * cg, fb = tcol / 128, fc = tcol - 128 * fb;   // 64-wide t-block of the force pass
+            const int fcols = min(128, 2 * g.TP - 128 * fb);
+            uint4 *d = zsite + ((size_t)tile * 2 * g.TP + 128 * fb) * 3 * 16 + (size_t)(fc >> 3) * 128 + (r >> 3) * 8 + (r & 7);
+            const size_t ts = (size_t)fcols * 16;   // uint4 per term
+            d[0] = make_uint4(h[0], h[1], h[2], h[3]);
+            d[ts] = make_uint4(m[0], m[1], m[2], m[3]);
+            d[2 * ts] = make_uint4(l[0], l[1], l[2], l[3]);
+         }
+      }
+   }
+}
+
+// ------------------------------------------------------ shared CTA parts
+__device__ __forceinline__ void q_abort(int *flag, int *err, int bit)
+{
+   *(volatile int *)flag = 1;
+   atomicOr(err, bit);
+}
+__device__ __forceinline__ bool q_aborted(const int *flag) { return *(const volatile int *)flag != 0; }
+
+struct QBars {
+   uint64_t full_b[3], empty_b[3], full_a[2], empty_a[2], accf, acce, done[2];
+};
+__device__ __forceinline__ void q_init(QBars &B)
+{
+   for (int s = 0; s < 3; s++) {
+      tc::bar_init(&B.full_b[s], 1);
+      tc::bar_init(&B.empty_b[s], 2);   // released by both MMA issuers
+   }
+   for (int s = 0; s < 2; s++) {
+      tc::bar_init(&B.full_a[s], Q_BW);
+      tc::bar_init(&B.empty_a[s], 2);
+   }
+   tc::bar_init(&B.accf, 2);
+   tc::bar_init(&B.acce, Q_BW);
+   tc::bar_init(&B.done[0], 1);
+   tc::bar_init(&B.done[1], 1);
+   tc::bar_init_fence();
+}
+
+// MMA issue of one thread (issuer p of two) over nst stages in segments of
+// SEG: NS = 3, issuer p takes 128-row tile p; NS = 7, column part p.
+// Operand stages: A [tile][digit][row group 16][kg 4][8 rows][16 B], B
+// [part][digit][col group][kg 4][8][16 B].
+template <int NS>
+__device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned char *Bbuf, unsigned int tmem, int p,
+                                        int nst, int nT, int *abort_s, int *err, int errbit)
+{
+   using namespace tc;
+   constexpr int SEG = QCfg<NS>::SEG, NB = QCfg<NS>::NB;
+   const int pc = nT / QCfg<NS>::NPART;
+   const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NS * Q_OP : 0);
+   const unsigned int b0 = saddr(Bbuf) + (QCfg<NS>::NPART == 2 ? p * NS * pc * Q_KS * 2 : 0);
+   const unsigned int d0 = tmem + 256u * p;
+   for (int st = 0; st < nst; st++) {
+      const int sa = st & 1, sb = st % NB, seg = st / SEG;
+      if (!bar_wait(&B.full_a[sa], (unsigned int)(st >> 1) & 1u) ||
+          !bar_wait(&B.full_b[sb], (unsigned int)(st / NB) & 1u) ||
+          (st % SEG == 0 && seg > 0 && !bar_wait(&B.acce, (unsigned int)(seg - 1) & 1u)) || q_aborted(abort_s)) {
+         q_abort(abort_s, err, errbit);
+         break;
+      }
+      fence_after_sync();
+#pragma unroll
+      for (int ks = 0; ks < 2; ks++)
+#pragma unroll
+         for (int i = 0; i < NS; i++)
+            mma_f16(d0 + i * pc, sdesc(a0 + sa * Q_A<NS> + i * Q_OP + ks * 256, 128, 512),
+                    sdesc(b0 + sb * Q_STAGE<NS> + ks * 256, 128, 512), idesc_f16(128, (NS - i) * pc, false),
+                    st % SEG != 0 || ks > 0 || i > 0);
+      mma_commit(&B.empty_a[sa]);
+      mma_commit(&B.empty_b[sb]);
+      if (st % SEG == SEG - 1 || st == nst - 1) mma_commit(&B.accf);
+   }
+   mma_commit(&B.done[p]);
+   bar_wait(&B.done[p], 0);   // every MMA complete before the tensor memory is released
+}
+
+// 4 consecutive FP32 columns of this thread's lane of tensor memory
+__device__ __forceinline__ void q_ld4(unsigned int taddr, float (&v)[4])
+{
+   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3])
+                : "r"(taddr)
+                : "memory");
+}
+template <int N> __device__ __forceinline__ void q_ldwait(float (&v)[N][4])
+{
+   asm volatile("tcgen05.wait::ld.sync.aligned;" : : : "memory");
+#pragma unroll
+   for (int i = 0; i < N; i++) asm volatile("" : "+f"(v[i][0]), "+f"(v[i][1]), "+f"(v[i][2]), "+f"(v[i][3]));
+}
+
+// 96-bit signed sums (three words)
+struct Q96 {
+   unsigned int w0, w1, w2;
+};
+// the seven groups of one output as an integer, group 6 of weight 1: low
+// part (groups 3..6) and high part (groups 0..2, weight 2^32)
+__device__ __forceinline__ Q96 q_combine(float d0, float d1, float d2, float d3, float d4, float d5, float d6)
+{
+   const long long lo = (long long)__float2int_rn(d6) + (long long)__float2int_rn(d5) * 256 +
+                        (long long)__float2int_rn(d4) * 65536 + (long long)__float2int_rn(d3) * 16777216;
+   const long long hi = (long long)__float2int_rn(d2) + (long long)__float2int_rn(d1) * 256 +
+                        (long long)__float2int_rn(d0) * 65536;
+   Q96 r;
+   const unsigned int sx = (unsigned int)(lo >> 63);
+   asm("add.cc.u32 %0, %3, %4;\n\taddc.u32 %1, %5, %6;\n\tmov.u32 %2, %7;"
+       : "=&r"(r.w1), "=&r"(r.w2), "=&r"(r.w0)
+       : "r"((unsigned int)(lo >> 32)), "r"((unsigned int)hi), "r"(sx), "r"((unsigned int)(hi >> 32)),
+         "r"((unsigned int)lo));
+   return r;
+}
+__device__ __forceinline__ void q_add(Q96 &a, const Q96 &b)
+{
+   asm("add.cc.u32 %0, %0, %3;\n\taddc.cc.u32 %1, %1, %4;\n\taddc.u32 %2, %2, %5;"
+       : "+r"(a.w0), "+r"(a.w1), "+r"(a.w2)
+       : "r"(b.w0), "r"(b.w1), "r"(b.w2));
+}
+__device__ __forceinline__ Q96 q_shift(Q96 v, int s)   // arithmetic shift right, 0 <= s < 96
+{
+   while (s >= 32) {
+      v.w0 = v.w1;
+      v.w1 = v.w2;
+      v.w2 = (unsigned int)((int)v.w2 >> 31);
+      s -= 32;
+   }
+   v.w0 = __funnelshift_r(v.w0, v.w1, s);
+   v.w1 = __funnelshift_r(v.w1, v.w2, s);
+   v.w2 = (unsigned int)((int)v.w2 >> s);
+   return v;
+}
+__device__ __forceinline__ double q_value(const Q96 &v)
+{
+   return (double)(long long)(((unsigned long long)v.w2 << 32) | v.w1) * 4294967296.0 + (double)v.w0;
+}
+
+// ----------------------------------------------------- structure factor
+// Grid: (row tiles, site ranges).  part[range][quad row 4 quad + p][2 TP].
+template <int NS>
+__global__ void __launch_bounds__(Q_THREADS, 1)
+k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4 *__restrict__ units, const unsigned char *__restrict__ X,
+         const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, int nstages, int per,
+         double *__restrict__ part, int *__restrict__ err)
+{
+   using namespace tc;
+   typedef typename QCfg<NS>::T T;
+   constexpr int RS = QCfg<NS>::RS, MT = QCfg<NS>::MT, NB = QCfg<NS>::NB, SEG = QCfg<NS>::SEG;
+   extern __shared__ __align__(1024) unsigned char sm[];
+   __shared__ __align__(8) QBars B;
+   __shared__ unsigned int tmem_s;
+   __shared__ int abort_s;
+   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>;
+   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+   const QTile &ti = tiles[blockIdx.x];
+   const int nT = ti.nT, st0 = blockIdx.y * per, nst = min(nstages, st0 + per) - st0;
+   if (nst <= 0) return;   // (uniform)
+   if (tid == 0) {
+      q_init(B);
+      abort_s = 0;
+   }
+   __syncwarp();
+   if (w == Q_BW + 1) tmem_alloc(&tmem_s, 512);
+   fence_before_sync();
+   __syncthreads();
+   fence_after_sync();
+   const unsigned int tmem = tmem_s;
+
+   if (w == Q_BW) {
+      // ---- bulk copies: a stage's digits of q z and the tile's table rows
+      if (lane == 0) {
+         const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * NS);
+         const unsigned int xb = (unsigned int)(2 * ti.nx * RS * sizeof(T)), yb = (unsigned int)(2 * ti.ny * RS * sizeof(T));
+         int issued = 0;
+         for (int st = 0; st < nst; st++) {
+            const int s = st % NB;
+            if ((st >= NB && !bar_wait(&B.empty_b[s], (unsigned int)(st / NB - 1) & 1u)) || q_aborted(&abort_s)) {
+               q_abort(&abort_s, err, Q_ERR);
+               break;
+            }
+            unsigned char *d = Sbuf + s * Q_STAGE<NS>;
+            const size_t sg = (size_t)(st0 + st);
+            bar_expect_tx(&B.full_b[s], bb + xb + yb);
+            bulk_load(d, ztab + (sg * 2 * g.TP + ti.col0) * Q_KS * 2 * NS, bb, &B.full_b[s]);
+            bulk_load(d + Q_B<NS>, X + (sg * g.hrows + ti.xlo) * 2 * RS * sizeof(T), xb, &B.full_b[s]);
+            bulk_load(d + Q_B<NS> + 2 * Q_XMAX * RS * sizeof(T), Y + (sg * g.mrows + ti.ylo) * 2 * RS * sizeof(T), yb,
+                      &B.full_b[s]);
+            issued = st + 1;
+         }
+         // copies still in flight complete before the CTA's shared memory goes
+         for (int st = issued > NB ? issued - NB : 0; st < issued; st++)
+            bar_wait(&B.full_b[st % NB], (unsigned int)(st / NB) & 1u);
+      }
+   } else if (w > Q_BW) {
+      if (lane == 0)
+         q_issue<NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
+   } else {
+      // ---- A operand: row 8 w + (lane & 7) of each 128-row tile (product
+      // p of a quad), sites 8 kg .. 8 kg + 7 of the stage
+      const int r = 8 * w + (lane & 7), kg = lane >> 3, p = r & 3;
+      int xo[MT], yo[MT];   // this row's table offsets
+#pragma unroll
+      for (int mt = 0; mt < MT; mt++) {
+         const int u = ti.unit[8 * mt + (r >> 4)];
+         const int4 un = u >= 0 ? units[u] : make_int4(ti.xlo, ti.ylo, 0, 0);
+         const int hx = un.x - ti.xlo, my = un.y + (u >= 0 ? (r >> 2) & 3 : 0) - ti.ylo;
+         xo[mt] = (2 * hx + (p == 1 || p == 2)) * RS + 8 * kg;
+         yo[mt] = (2 * my + (p & 1)) * RS + 8 * kg;
+      }
+      // read-back: lane quarter w % 4 (row 32 (w % 4) + lane), a quarter of
+      // the columns of each tile / part
+      const int cq = w >> 2;
+      const int ncw = nT >> 2;                    // columns per warp
+      constexpr int MAXC = QCfg<NS>::NTMAX / 16;  // chunks of four columns
+      constexpr int NACC = MT * MAXC * 4;
+      float af[NS == 3 ? NACC : 1];
+      Q96 ai[NS == 7 ? NACC : 1];
+#pragma unroll
+      for (int i = 0; i < NACC; i++) {
+         if (NS == 3) af[NS == 3 ? i : 0] = 0.f;
+         else ai[NS == 7 ? i : 0] = Q96{0u, 0u, 0u};
+      }
+      const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16);
+      // first column of this warp in tensor memory and the group stride
+      const int pc = nT / QCfg<NS>::NPART, pl = cq * ncw;
+      auto flush = [&](int seg) -> bool {
+         const bool got = bar_wait(&B.accf, (unsigned int)seg & 1u);
+         if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
+            if (lane == 0) q_abort(&abort_s, err, Q_ERR);
+            return false;
+         }
+         fence_after_sync();
+#pragma unroll
+         for (int mt = 0; mt < MT; mt++)
+#pragma unroll
+            for (int ch = 0; ch < MAXC; ch++)
+               if (4 * ch < ncw) {
+                  const int lc = pl + 4 * ch;   // column of the block
+                  const unsigned int col = MT == 2 ? 256u * mt + lc : 256u * (lc / pc) + lc % pc;
+                  float d[NS][4];
+#pragma unroll
+                  for (int k = 0; k < NS; k++) q_ld4(trow + col + k * pc, d[k]);
+                  q_ldwait(d);
+#pragma unroll
+                  for (int e = 0; e < 4; e++) {
+                     const int i = (mt * MAXC + ch) * 4 + e;
+                     if (NS == 3)
+                        af[NS == 3 ? i : 0] += fmaf(d[0][e], 65536.f, fmaf(d[1][e], 256.f, d[2][e]));
+                     else
+                        q_add(ai[NS == 7 ? i : 0], q_combine(d[0][e], d[1][e], d[2][e], d[NS > 3 ? 3 : 0][e], d[NS > 3 ? 4 : 0][e],
+                                                            d[NS > 3 ? 5 : 0][e], d[NS > 3 ? 6 : 0][e]));
+                  }
+               }
+         fence_before_sync();
+         __syncwarp();
+         if (lane == 0) bar_arrive(&B.acce);
+         return true;
+      };
+      bool live = true;
+      for (int st = 0; st < nst && live; st++) {
+         const int sa = st & 1, sb = st % NB;
+         const bool got = (st < 2 || bar_wait(&B.empty_a[sa], (unsigned int)((st >> 1) - 1) & 1u)) &&
+                          bar_wait(&B.full_b[sb], (unsigned int)(st / NB) & 1u);
+         if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
+            if (lane == 0) q_abort(&abort_s, err, Q_ERR);
+            live = false;
+            break;
+         }
+         const T *xs = reinterpret_cast<const T *>(Sbuf + sb * Q_STAGE<NS> + Q_B<NS>);
+         const T *ys = xs + 2 * Q_XMAX * RS;
+         unsigned char *A = Abuf + sa * Q_A<NS> + (r >> 3) * 512 + kg * 128 + (r & 7) * 16;
+#pragma unroll
+         for (int mt = 0; mt < MT; mt++) {
+            constexpr int PV = 16 / (int)sizeof(T);   // values per 16-byte load
+            T xv[8], yv[8];
+#pragma unroll
+            for (int e = 0; e < 8 / PV; e++) {
+               *reinterpret_cast<uint4 *>(xv + e * PV) = *reinterpret_cast<const uint4 *>(xs + xo[mt] + e * PV);
+               *reinterpret_cast<uint4 *>(yv + e * PV) = *reinterpret_cast<const uint4 *>(ys + yo[mt] + e * PV);
+            }
+            decltype(qmul_a(xv[0], yv[0], 0u)) v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = qmul_a(xv[e], yv[e], c256);
+            qstore<NS>(A + mt * NS * Q_OP, Q_OP, v);
+         }
+         fence_async_smem();
+         __syncwarp();
+         if (lane == 0) bar_arrive(&B.full_a[sa]);
+         // the previous segment is read back once the first stage of this
+         // one is built (its build overlaps the segment's last MMAs)
+         if (st > 0 && st % SEG == 0) live = flush(st / SEG - 1);
+      }
+      if (live) live = flush((nst - 1) / SEG);
+      if (live) {
+#pragma unroll
+         for (int mt = 0; mt < MT; mt++) {
+            const int row = 32 * (w & 3) + lane;
+            const int u = ti.unit[8 * mt + (row >> 4)];
+            if (u >= 0) {
+               double *dst = part + ((size_t)blockIdx.y * 4 * g.nquads + (size_t)u * 16 + (row & 15)) * 2 * g.TP + ti.col0 + pl;
+#pragma unroll
+               for (int ch = 0; ch < MAXC; ch++)
+                  if (4 * ch < ncw) {
+                     double v[4];
+#pragma unroll
+                     for (int e = 0; e < 4; e++) {
+                        const int i = (mt * MAXC + ch) * 4 + e;
+                        v[e] = NS == 3 ? (double)af[NS == 3 ? i : 0] : q_value(ai[NS == 7 ? i : 0]);
+                     }
+                     reinterpret_cast<double2 *>(dst + 4 * ch)[0] = make_double2(v[0], v[1]);
+                     reinterpret_cast<double2 *>(dst + 4 * ch)[1] = make_double2(v[2], v[3]);
+                  }
+            }
+         }
+      }
+   }
+   fence_before_sync();
+   __syncthreads();
+   if (w == Q_BW + 1) {
+      __syncwarp();
+      fence_after_sync();
+      tmem_dealloc(tmem, 512);
+   }
+}
+
+// ------------------------------------------------- per-k energy and stress
+// A block takes 32 consecutive (quad, t): its eight warps add up their eight
+// sums over the site ranges w, w + 8, ... (fixed order), then one thread per
+// (quad, t) and (s, r) forms its k-vector's S(k), energy and stress
+// (src/ewald.c:525-553) and A = coeff Re S, B = coeff Im S, laid out
+// [quad][t][s][r] (zero where there is no such k-vector).
+template <typename R>
+__global__ void __launch_bounds__(256)
+k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coeff, int nranges, double scale,
+          const double *__restrict__ part, R *__restrict__ ab, double *__restrict__ blk)
+{
+   __shared__ double sq[8][8][32];
+   __shared__ double sh[4][7];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   const int i = blockIdx.x * 32 + lane, quad = i / g.TP, t = i - quad * g.TP;
+   const int4 un = quad < g.nquads ? units[quad >> 2] : make_int4(0, 0, 0, 0);
+   const bool live = t < un.z;   // the unit's t range: its columns were computed
+   {
+      double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (live) {
+         const size_t row = 2 * (size_t)g.TP, plane = 4 * (size_t)g.nquads * row;
+         const double *p = part + (size_t)quad * 4 * row + 16 * (t >> 3) + (t & 7) + w * plane;
+         for (int c = w; c < nranges; c += 8, p += 8 * plane)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+               q[2 * k] += p[k * row];
+               q[2 * k + 1] += p[k * row + 8];
+            }
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++) sq[w][k][lane] = q[k];
+   }
+   __syncthreads();
+   {
+      // sum k = w of lane's (quad, t) over the warps
+      double v = 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; j++) v += sq[j][w][lane];
+      __syncthreads();
+      sq[0][w][lane] = v * scale;
+   }
+   __syncthreads();
+   if (w >= 4) return;
+   // (s, r) = warp w
+   double e[7] = {0, 0, 0, 0, 0, 0, 0};
+   if (quad < g.nquads) {
+      double A = 0.0, Bc = 0.0;
+      const double2 cf = live ? coeff[(size_t)i * 4 + w] : make_double2(0.0, 0.0);
+      if (cf.x != 0.0) {
+         double q[8];
+#pragma unroll
+         for (int k = 0; k < 8; k++) q[k] = sq[0][k][lane];
+         const double s = w & 2 ? -1.0 : 1.0, r = w & 1 ? -1.0 : 1.0;
+         const double C = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
+         const double S = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
+         const double hh = un.x, kk = s * (un.y + (quad & 3)), l = r * t;
+         const double kx = hh * g.b[0] + kk * g.b[3], ky = hh * g.b[1] + kk * g.b[4];
+         const double kz = hh * g.b[2] + kk * g.b[5] + l * g.b[8];
+         const double pek = 0.5 * cf.x * (C * C + S * S), pc = pek * cf.y;
+         e[0] = pek;
+         e[1] = pek - pc * kx * kx;
+         e[2] = -(pc * kx * ky);
+         e[3] = -(pc * kx * kz);
+         e[4] = pek - pc * ky * ky;
+         e[5] = -(pc * ky * kz);
+         e[6] = pek - pc * kz * kz;
+         A = cf.x * C;
+         Bc = cf.x * S;
+      }
+      ab[(size_t)i * 8 + 2 * w] = (R)A;
+      ab[(size_t)i * 8 + 2 * w + 1] = (R)Bc;
+   }
+#pragma unroll
+   for (int k = 0; k < 7; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) e[k] += __shfl_down_sync(0xffffffffu, e[k], o);
+      if (lane == 0) sh[w][k] = e[k];
+   }
+   asm volatile("bar.sync 1, 128;" : : : "memory");
+   if (threadIdx.x < 7)
+      blk[blockIdx.x * 8 + threadIdx.x] = (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
+}
+
+// ------------------------------------------------- force pass, FP64 form
+// F_j = q_j sum_k k (A sin k.r_j - B cos k.r_j) as three sums over the quad
+// rows with the integer weights h, k, l:
+//     H_a(j) = sum_col z_col(j) sum_rows P_row(j) U_a(row, col),
+// the inner sum a matrix product (sites x quad rows, built per stage from
+// the tables, times quad rows x columns), F = q b^T (H_h, H_k, H_l).
+// A segment is 8 units (128 quad rows) of one t-block, units in order of
+// rising |(h, m)| so that the coefficients of a segment, which share a
+// power-of-two scale, are of similar size.
+// Coefficients of quad (h, m) at t for one weight set: v[p] of P_p C_t and
+// v[4 + p] of P_p S_t.
+__device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m, int t, double (&v)[8])
+{
+#pragma unroll
+   for (int k = 0; k < 8; k++) v[k] = 0.0;
+#pragma unroll
+   for (int x = 0; x < 4; x++) {
+      const double s = x & 2 ? -1.0 : 1.0, r = x & 1 ? -1.0 : 1.0;
+      const double wt = set == 0 ? (double)h : set == 1 ? s * m : r * t;
+      const double A = wt * ab[2 * x], Bc = wt * ab[2 * x + 1];
+      v[0] -= Bc;
+      v[1] += s * Bc;
+      v[2] += A;
+      v[3] += s * A;
+      v[4] += r * A;
+      v[5] -= r * s * A;
+      v[6] += r * Bc;
+      v[7] += r * s * Bc;
+   }
+}
+
+// Grid: (segments, 3 sets).  The segment's B operand, [stage 4][part][digit]
+// [col group][kg 4][8 cols][8 K], and its scale exponent.
+__global__ void __launch_bounds__(256)
+k_qcoef(QGeom g, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict__ units,
+        const double *__restrict__ ab, unsigned char *__restrict__ bq, int *__restrict__ bexp)
+{
+   constexpr int NS = 7;
+   __shared__ double smax[8];
+   const int seg = blockIdx.x, set = blockIdx.y, tid = threadIdx.x;
+   const QSeg &sg = segs[seg];
+   const int nT = q_blkcols(g, sg.blk), tw = nT / 2, t0 = sg.blk * g.TW;
+   double mx = 0.0;
+   for (int i = tid; i < 32 * tw; i += 256) {
+      const int ql = i / tw, t = t0 + i % tw, u = sg.unit[ql >> 2];
+      if (u < 0) continue;
+      const int4 un = units[u];
+      if (t >= un.z) continue;
+      double v[8];
+      q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set, un.x, un.y + (ql & 3), t, v);
+#pragma unroll
+      for (int k = 0; k < 8; k++) mx = fmax(mx, fabs(v[k]));
+   }
+#pragma unroll
+   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+   if ((tid & 31) == 0) smax[tid >> 5] = mx;
+   __syncthreads();
+   mx = smax[0];
+   for (int k = 1; k < 8; k++) mx = fmax(mx, smax[k]);
+   int e = -4096;
+   if (mx > 0.0) frexp(mx, &e);
+   if (tid == 0) bexp[set * nseg + seg] = e;
+   const double sc = mx > 0.0 ? ldexp(Q_KAPPA * Q_KAPPA, 63 - e) : 0.0;
+   unsigned char *base = bq + ((size_t)set * nseg + seg) * 4 * (QCfg<NS>::NTMAX * Q_KS * 2 * NS);
+   const int pc = nT / 2;
+   // two quads (8 K values) at one t per thread
+   for (int i = tid; i < 16 * tw; i += 256) {
+      const int pr = i & 15, tl = i >> 4, t = t0 + tl;
+      unsigned long long vc[8], vs[8];
+#pragma unroll
+      for (int x = 0; x < 2; x++) {
+         const int ql = 2 * pr + x, u = sg.unit[ql >> 2];
+         double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+         if (u >= 0) {
+            const int4 un = units[u];
+            if (t < un.z) q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set, un.x, un.y + (ql & 3), t, v);
+         }
+#pragma unroll
+         for (int k = 0; k < 4; k++) {
+            vc[4 * x + k] = (unsigned long long)__double2ll_rn(v[k] * sc) + 0x8080808080808080ull;
+            vs[4 * x + k] = (unsigned long long)__double2ll_rn(v[4 + k] * sc) + 0x8080808080808080ull;
+         }
+      }
+      const int stage = pr >> 2, kg = pr & 3, lc = 16 * (tl >> 3) + (tl & 7);
+#pragma unroll
+      for (int cs = 0; cs < 2; cs++) {
+         const int col = lc + 8 * cs, part = col / pc, pl = col - part * pc;
+         unsigned char *d = base + (size_t)stage * (QCfg<NS>::NTMAX * Q_KS * 2 * NS) +
+                            ((size_t)part * NS * pc + (pl & ~7)) * Q_KS * 2 + kg * 128 + (pl & 7) * 16;
+         if (cs == 0) qstore<NS>(d, pc * Q_KS * 2, vc);
+         else qstore<NS>(d, pc * Q_KS * 2, vs);
+      }
+   }
+}
+
+// Grid: (site tiles of 128, sets, items).  hpart[item][set][n].
+__global__ void __launch_bounds__(Q_THREADS, 1)
+k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restrict__ items,
+          const int4 *__restrict__ units, const long long *__restrict__ X, const long long *__restrict__ Y,
+          const double *__restrict__ zd, const unsigned char *__restrict__ bq, const int *__restrict__ bexp, int n,
+          double *__restrict__ hpart, int *__restrict__ err)
+{
+   using namespace tc;
+   constexpr int NS = 7, RS = QCfg<NS>::RS, NB = QCfg<NS>::NB, SEG = QCfg<NS>::SEG;
+   constexpr int BST = QCfg<NS>::NTMAX * Q_KS * 2 * NS;   // a stage's B operand
+   extern __shared__ __align__(1024) unsigned char sm[];
+   __shared__ __align__(8) QBars B;
+   __shared__ unsigned int tmem_s;
+   __shared__ int abort_s;
+   __shared__ double red[4][128];
+   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>;
+   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+   const int tile = blockIdx.x, set = blockIdx.y;
+   const QItem it = items[blockIdx.z];
+   const int nst = (it.seg1 - it.seg0) * SEG;
+   const int blk = segs[it.seg0].blk, nT = q_blkcols(g, blk);
+   if (tid == 0) {
+      q_init(B);
+      abort_s = 0;
+   }
+   __syncwarp();
+   if (w == Q_BW + 1) tmem_alloc(&tmem_s, 512);
+   fence_before_sync();
+   __syncthreads();
+   fence_after_sync();
+   const unsigned int tmem = tmem_s;
+
+   if (w == Q_BW) {
+      if (lane == 0) {
+         const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * NS);
+         const unsigned char *src = bq + ((size_t)set * nseg + it.seg0) * SEG * BST;
+         int issued = 0;
+         for (int st = 0; st < nst; st++) {
+            const int s = st % NB;
+            if ((st >= NB && !bar_wait(&B.empty_b[s], (unsigned int)(st / NB - 1) & 1u)) || q_aborted(&abort_s)) {
+               q_abort(&abort_s, err, Q_FERR);
+               break;
+            }
+            bar_expect_tx(&B.full_b[s], bb);
+            bulk_load(Sbuf + s * Q_STAGE<NS>, src + (size_t)st * BST, bb, &B.full_b[s]);
+            issued = st + 1;
+         }
+         for (int st = issued > NB ? issued - NB : 0; st < issued; st++)
+            bar_wait(&B.full_b[st % NB], (unsigned int)(st / NB) & 1u);
+      }
+   } else if (w > Q_BW) {
+      if (lane == 0)
+         q_issue<NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
+   } else {
+      // ---- A operand: site j of the tile, two quads (8 K) per stage
+      const int j = tid & 127, kg = tid >> 7;
+      const size_t sg = (size_t)tile * 4 + (j >> 5);
+      const long long *xb = X + sg * 2 * g.hrows * RS + (j & 31), *yb = Y + sg * 2 * g.mrows * RS + (j & 31);
+      unsigned char *Aw = Abuf + (j >> 3) * 512 + kg * 128 + (j & 7) * 16;
+      int emax = -4096;
+      for (int k = lane; k < nseg; k += 32) emax = max(emax, bexp[set * nseg + k]);
+      emax = __reduce_max_sync(0xffffffffu, emax);
+      constexpr int MAXC = QCfg<NS>::NTMAX / 16;
+      Q96 ai[MAXC * 4];
+#pragma unroll
+      for (int i = 0; i < MAXC * 4; i++) ai[i] = Q96{0u, 0u, 0u};
+      const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16);
+      const int cq = w >> 2, ncw = nT >> 2, pc = nT / 2, pl = cq * ncw;
+      auto flush = [&](int seg) -> bool {
+         const bool got = bar_wait(&B.accf, (unsigned int)seg & 1u);
+         if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
+            if (lane == 0) q_abort(&abort_s, err, Q_FERR);
+            return false;
+         }
+         fence_after_sync();
+         const int sh = emax - bexp[set * nseg + it.seg0 + seg];
+#pragma unroll
+         for (int ch = 0; ch < MAXC; ch++)
+            if (4 * ch < ncw) {
+               const int lc = pl + 4 * ch;
+               const unsigned int col = 256u * (lc / pc) + lc % pc;
+               float d[NS][4];
+#pragma unroll
+               for (int k = 0; k < NS; k++) q_ld4(trow + col + k * pc, d[k]);
+               q_ldwait(d);
+               if (sh < 96)
+#pragma unroll
+                  for (int e = 0; e < 4; e++)
+                     q_add(ai[4 * ch + e],
+                           q_shift(q_combine(d[0][e], d[1][e], d[2][e], d[3][e], d[4][e], d[5][e], d[6][e]), sh));
+            }
+         fence_before_sync();
+         __syncwarp();
+         if (lane == 0) bar_arrive(&B.acce);
+         return true;
+      };
+      long long xv[2], yv[4];
+      auto fetch = [&](int st) {
+         const int u = segs[it.seg0 + st / SEG].unit[2 * (st % SEG) + (kg >> 1)];
+         const int4 un = u >= 0 ? units[u] : make_int4(0, 0, 0, 0);
+         const long long *x = xb + (size_t)2 * un.x * RS, *y = yb + (size_t)2 * (un.y + 2 * (kg & 1)) * RS;
+         xv[0] = __ldg(x);
+         xv[1] = __ldg(x + RS);
+#pragma unroll
+         for (int k = 0; k < 4; k++) yv[k] = __ldg(y + k * RS);
+      };
+      fetch(0);
+      bool live = true;
+      for (int st = 0; st < nst && live; st++) {
+         const int sa = st & 1;
+         unsigned long long v[8];
+#pragma unroll
+         for (int x = 0; x < 2; x++) {
+            v[4 * x] = qmul(xv[0], yv[2 * x]);
+            v[4 * x + 1] = qmul(xv[1], yv[2 * x + 1]);
+            v[4 * x + 2] = qmul(xv[1], yv[2 * x]);
+            v[4 * x + 3] = qmul(xv[0], yv[2 * x + 1]);
+         }
+         if (st + 1 < nst) fetch(st + 1);
+         const bool got = st < 2 || bar_wait(&B.empty_a[sa], (unsigned int)((st >> 1) - 1) & 1u);
+         if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
+            if (lane == 0) q_abort(&abort_s, err, Q_FERR);
+            live = false;
+            break;
+         }
+         qstore<NS>(Aw + sa * Q_A<NS>, Q_OP, v);
+         fence_async_smem();
+         __syncwarp();
+         if (lane == 0) bar_arrive(&B.full_a[sa]);
+         if (st > 0 && st % SEG == 0) live = flush(st / SEG - 1);
+      }
+      if (live) live = flush((nst - 1) / SEG);
+      // the columns contracted with the site's z values
+      double f = 0.0;
+      if (live) {
+         const int row = 32 * (w & 3) + lane;
+         const double *z = zd + (((size_t)tile * 4 + (row >> 5)) * 2 * g.TP + 2 * blk * g.TW + pl) * 32 + (row & 31);
+#pragma unroll
+         for (int i = 0; i < MAXC * 4; i++)
+            if (i < ncw) f = fma(q_value(ai[i]), z[(size_t)i * 32], f);
+      }
+      red[cq][32 * (w & 3) + lane] = f;
+      asm volatile("bar.sync 2, %0;" : : "n"(Q_BW * 32) : "memory");
+      if (tid < 128) {
+         const int i = tile * 128 + tid;
+         if (i < n && !q_aborted(&abort_s)) {
+            const double s = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
+            // units of the product: 2^-62 over the four table scales, times the coefficients' scale
+            const double sc = emax > -4096 ? ldexp(1.0 / (Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA), emax - 62) : 0.0;
+            hpart[((size_t)blockIdx.z * 3 + set) * n + i] = s * sc;
+         }
+      }
+   }
+   fence_before_sync();
+   __syncthreads();
+   if (w == Q_BW + 1) {
+      __syncwarp();
+      fence_after_sync();
+      tmem_dealloc(tmem, 512);
+   }
+}
+
+// force[site of slot i] += q b^T (H_h, H_k, H_l), the items' sums in order
+__global__ void __launch_bounds__(256)
+k_fsum_q(int n, int N, int nitems, QGeom g, const double *__restrict__ hpart, const int *__restrict__ slots,
+         const double *__restrict__ chg, double *__restrict__ force)
+{
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (i >= n) return;
+   double H[3] = {0, 0, 0};
+   for (int k = 0; k < nitems; k++)
+#pragma unroll
+      for (int s = 0; s < 3; s++) H[s] += hpart[((size_t)k * 3 + s) * n + i];
+   const int si = slots[i];
+   const double q = chg[si];
+   force[si] += q * (g.b[0] * H[0] + g.b[3] * H[1]);
+   force[N + si] += q * (g.b[1] * H[0] + g.b[4] * H[1]);
+   force[2 * (size_t)N + si] += q * (g.b[2] * H[0] + g.b[5] * H[1] + g.b[8] * H[2]);
+}
+
+// ------------------------------------------------------------- host side
+#define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
+
+// Shared-memory sizes, set once per device outside any stream capture
+// (contexts may be created from several host threads: the per-device flags
+// are atomic, and setting the attribute twice is harmless).
+static cudaError_t q_init_device(int device)
+{
+   static std::atomic<unsigned long long> done{0};
+   const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
+   if (bit && (done.load() & bit)) return cudaSuccess;
+   cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7>);
+   if (e == cudaSuccess) e = ks_force_tc_init();
+   if (e == cudaSuccess && bit) done.fetch_or(bit);
+   return e;
+}
+
+// Stages of 32 sites, padded to the force passes' 128-site tiles.
+static size_t q_stages(int n) { return (size_t)((n + 127) / 128) * 4; }
+
+// The quad list of the current k-list and its device copy.
+mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
+{
+   KsDev &d = c->kd;
+   QList &q = c->kl.q;
+   CK(q_init_device(c->device));
+   if (c->nsm <= 0) CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
+   if (q.ns == ns || c->kl.nk == 0) return MDGPU_OK;
+   build_qlist(c->kl, ns);
+   cudaStream_t st = c->stream;
+   auto up = [&](auto &buf, const auto &v) -> cudaError_t {
+      cudaError_t e = buf.ensure(v.size());
+      if (e == cudaSuccess && !v.empty())
+         e = cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st);
+      return e;
+   };
+   CK(up(d.q_units, q.units));
+   CK(up(d.q_coeff, q.coeff));
+   CK(up(d.q_tiles, q.tiles));
+   CK(up(d.q_segs, q.segs));
+   CK(up(d.q_fu, q.fu));
+   d.q_fblk = q.fblk;
+   d.q_nfblk = q.fblk.empty() ? 0 : (int)q.fblk.size() - 1;
+   CK(cudaStreamSynchronize(st));
+   d.tc_ver++;
+   return MDGPU_OK;
+}
+
+// The scale of the charges: a power of two above the largest.
+static int q_charge_exp(const mdgpu_ctx *c)
+{
+   int e = 0;
+   std::frexp(c->qmax > 0 ? c->qmax : 1.0, &e);
+   return e;
+}
+
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site)
+{
+   KsDev &d = c->kd;
+   const QGeom &g = c->kl.q.g;
+   const size_t S = q_stages(n);
+   const double *hi = c->kl.hinv;
+   const double qinv = std::ldexp(1.0, -q_charge_exp(c));
+   CK(d.q_ztab.ensure(S * 2 * g.TP * Q_KS * 2 * ns));
+   if (ns == 3) {
+      CK(d.q_x32.ensure(S * 2 * g.hrows * QCfg<3>::RS));
+      CK(d.q_y32.ensure(S * 2 * g.mrows * QCfg<3>::RS));
+      CK(d.zsite.ensure(S / 4 * 2 * g.TP * 48));
+      k_qtab<3><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
+                                                        hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x32.p,
+                                                        d.q_y32.p, d.q_ztab.p, d.zsite.p, nullptr);
+   } else {
+      CK(d.q_x64.ensure(S * 2 * g.hrows * QCfg<7>::RS));
+      CK(d.q_y64.ensure(S * 2 * g.mrows * QCfg<7>::RS));
+      CK(d.q_zd.ensure(S * 2 * g.TP * 32));
+      k_qtab<7><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
+                                                        hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x64.p,
+                                                        d.q_y64.p, d.q_ztab.p, nullptr, d.q_zd.p);
+   }
+   CK(cudaGetLastError());
+   return MDGPU_OK;
+}
+
+// Site ranges: the count for which the waves of (tile, range) CTAs, each its
+// stages plus a start-up of about six, come out shortest.
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges)
+{
+   KsDev &d = c->kd;
+   const QList &q = c->kl.q;
+   const int nst = (n + 31) / 32, nt = (int)q.tiles.size();
+   const size_t plane = 4 * (size_t)q.g.nquads * 2 * q.g.TP;
+   long long best = -1;
+   int R = 1;
+   for (int r = 1; r <= 64 && r <= nst; r++) {
+      if (r > 1 && r * plane * sizeof(double) > (256u << 20)) break;
+      const long long cost = (long long)((nt * r + c->nsm - 1) / c->nsm) * ((nst + r - 1) / r + 6);
+      if (best < 0 || cost < best) {
+         best = cost;
+         R = r;
+      }
+   }
+   const int per = (nst + R - 1) / R;
+   R = (nst + per - 1) / per;
+   CK(d.q_part.ensure(R * plane));
+   const dim3 grid(nt, R);
+   if (ns == 3)
+      k_sfac_q<3><<<grid, Q_THREADS, Q_SMEM<3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, nst, per, d.q_part.p, &c->out.p->err);
+   else
+      k_sfac_q<7><<<grid, Q_THREADS, Q_SMEM<7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, nst, per, d.q_part.p, &c->out.p->err);
+   CK(cudaGetLastError());
+   *nranges = R;
+   return MDGPU_OK;
+}
+
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges, int *nblocks)
+{
+   KsDev &d = c->kd;
+   const QGeom &g = c->kl.q.g;
+   const size_t nqt = (size_t)g.nquads * g.TP;
+   const int nb = (int)((nqt + 31) / 32);
+   const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
+   CK(d.blk.ensure((size_t)nb * 8));
+   if (ns == 3) {
+      CK(d.q_ab32.ensure(nqt * 8));
+      k_qreduce<float><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
+         std::ldexp(1.0 / k4, q_charge_exp(c) - 30), d.q_part.p, d.q_ab32.p, d.blk.p);
+   } else {
+      CK(d.q_ab64.ensure(nqt * 8));
+      k_qreduce<double><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
+         std::ldexp(1.0 / k4, q_charge_exp(c) - 62), d.q_part.p, d.q_ab64.p, d.blk.p);
+   }
+   CK(cudaGetLastError());
+   *nblocks = nb;
+   return MDGPU_OK;
+}
+
+mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
+{
+   (void)slots;
+   KsDev &d = c->kd;
+   const QList &q = c->kl.q;
+   const int nseg = (int)q.segs.size(), T = (n + 127) / 128;
+   // runs of segments: the length for which the waves of (site tile, set,
+   // run) CTAs come out shortest
+   if (d.q_items_for[0] != T || d.q_items_for[1] != (int)d.tc_ver || d.q_items_for[2] != c->nsm) {
+      int per = 1;
+      long long best = -1;
+      int mx = 1;
+      for (size_t b = 0; b + 1 < q.seg0.size(); b++) mx = std::max(mx, q.seg0[b + 1] - q.seg0[b]);
+      auto count = [&](int p) {
+         int k = 0;
+         for (size_t b = 0; b + 1 < q.seg0.size(); b++) k += (q.seg0[b + 1] - q.seg0[b] + p - 1) / p;
+         return k;
+      };
+      for (int p = 1; p <= mx; p++) {
+         const int k = count(p);
+         if (k > 16 && p < mx) continue;
+         const long long cost = (3LL * T * k + c->nsm - 1) / c->nsm * (4LL * p + 7);
+         if (best < 0 || cost < best) {
+            best = cost;
+            per = p;
+         }
+      }
+      std::vector<QItem> items;
+      for (size_t b = 0; b + 1 < q.seg0.size(); b++)
+         for (int s = q.seg0[b]; s < q.seg0[b + 1]; s += per) items.push_back(QItem{s, std::min(s + per, q.seg0[b + 1])});
+      CK(d.q_items.ensure(items.size()));
+      CK(cudaMemcpyAsync(d.q_items.p, items.data(), items.size() * sizeof(QItem), cudaMemcpyHostToDevice, c->stream));
+      CK(cudaStreamSynchronize(c->stream));
+      d.q_nitems = (int)items.size();
+      d.q_items_for[0] = T;
+      d.q_items_for[1] = (int)d.tc_ver;
+      d.q_items_for[2] = c->nsm;
+   }
+   CK(d.q_bq.ensure((size_t)3 * nseg * 4 * QCfg<7>::NTMAX * Q_KS * 2 * 7));
+   CK(d.q_bexp.ensure((size_t)3 * nseg));
+   CK(d.fpart.ensure((size_t)d.q_nitems * 3 * n));
+   k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, d.q_segs.p, nseg, d.q_units.p, d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
+   k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_SMEM<7>, c->stream>>>(
+      q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, n,
+      d.fpart.p, &c->out.p->err);
+   CK(cudaGetLastError());
+   c->launches += 1;
+   return MDGPU_OK;
+}
+
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force)
+{
+   k_fsum_q<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->nsites, c->kd.q_nitems, c->kl.q.g, c->kd.fpart.p, slots,
+                                                    c->rd.chg.p, d_force);
+   CK(cudaGetLastError());
+   return MDGPU_OK;
+}
+#undef CK
+
+}  // namespace mdgpu

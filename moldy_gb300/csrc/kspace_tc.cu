@@ -1,74 +1,15 @@
-// Reciprocal space of the mixed form on the tensor cores (tcgen05).  This
-// part: the S(k) pass of ewald() (src/ewald.c:124-141, the sums of q cos(k.r)
-// and q sin(k.r) over sites, 523-533) as a complex matrix product; the force
-// pass (src/ewald.c:557-566) follows further down.
-//
-// A tensor-core item is a run of up to KT = 64 consecutive l values of one
-// (h,k) column.  For item i, site j and offset t,
-//     exp(i k.r_j) = seed_ij z_j(t),  seed_ij = exp(2 pi i (h u_x + k u_y + l0 u_z)),
-//     z_j(t) = exp(2 pi i t u_z)
-// with the 32-bit fixed-point phases u of the FP32 path, so
-//     S(i, t) = sum_j (q_j seed_ij) z_j(t)
-// is a product of an items x sites matrix (computed per stage on the CUDA
-// cores: one polynomial sine/cosine per item and site, amortised over up to
-// 64 k-vectors) and a sites x t matrix (the per-site z tables, built once
-// per evaluation).  Complex arithmetic as real MMAs of N = 128: Ar and Ai
-// each times the whole z operand [Zr | Zi] (rows t, then 64 + t) into D1 =
-// (Ar Zr, Ar Zi) and D2 = (Ai Zr, Ai Zi), then Re S = Ar Zr - Ai Zi and
-// Im S = Ar Zi + Ai Zr in the read-back.  An MMA of 128 x N x 16 costs one
-// issuing thread the same time for any N up to 256 (measured:
-// mdgpu_tc_rate), so the products are kept wide and issued by two threads.
-//
-// Precision.  Charges are scaled by a power of two to |q| < 1, and every
-// FP32 operand is split into three bf16 terms on fixed grids (tc.cuh): the
-// hi*hi products go to their own tensor-memory accumulators (D1, D2), where
-// their sums are exact (multiples of 2^-14 below 2^10: a 1024-site partial
-// of terms of magnitude < 1), so the accumulator's round-toward-zero never
-// acts on them; hm, mh, hl, lh and mm go to a second pair, 2^-8 smaller.
-// The terms left out and the splitting are within 2^-24 of each operand, as
-// for the FP32 path.  Each CTA sums 1024 sites and writes one partial per k;
-// the partials are added in compensated FP32 and FP64 by the per-k
-// reduction.
-//
-// CTA roles (608 threads): warps 0-15 build the A operand of each 32-site
-// stage (one item row and 8 sites per thread) and, at the end, read the
-// accumulators back (a warp reaches tensor-memory lanes 32 (w % 4) ..);
-// warp 16 streams each stage's z tables and its 32 site records (bulk
-// copies, three stages in flight); warp 17 owns the tensor memory and
-// issues the Ar MMAs, warp 18 the Ai MMAs.  A operands and z tables are
-// triple-buffered on mbarriers, so the A operand of a stage is built while
-// the MMAs of the two before it run; every wait is bounded and sets bit 3
-// of the error word when it expires.
+// Force pass of the mixed form's reciprocal space on the tensor cores
+// (tcgen05; src/ewald.c:557-566).  The structure factor and the per-site
+// tables it shares are in kspace_q.cu.
 #include <atomic>
 #include <cmath>
 
 #include "mdgpu_internal.h"
-#include "phase.cuh"
 #include "tc.cuh"
 
 namespace mdgpu {
 
-constexpr int TC_KS = 32;                          // sites per stage (two MMA K-steps of 16)
-constexpr int TC_NSA = 3;                          // A-operand buffers
-constexpr int TC_NSB = 3;                          // z-table buffers (bulk copies in flight)
-constexpr int TC_TERM = 128 * TC_KS * 2;           // one 128-row bf16 operand of a stage: 8 KB
-constexpr int TC_ABYTES = 6 * TC_TERM;             // Ar, Ai x (hi, mid, lo)
-constexpr int TC_BBYTES = 3 * TC_TERM;             // [Zr | Zi] x (hi, mid, lo)
-constexpr int TC_CHUNK = 1024;                     // sites per CTA (one partial per k)
-constexpr int TC_PBYTES = TC_KS * 16;              // a stage's site records (u_x, u_y, u_z, q)
-constexpr int TC_AOFF = 0, TC_BOFF = TC_AOFF + TC_NSA * TC_ABYTES, TC_POFF = TC_BOFF + TC_NSB * TC_BBYTES;
-constexpr int TC_SMEM = TC_POFF + TC_NSB * TC_PBYTES;
-constexpr int TC_LBO = 16 * 128;                   // 8-column groups of a 128-row operand
-constexpr int TC_ERR = 8;                          // error-word bit: a stage wait expired
-constexpr int TC_AW = 16;                          // operand / read-back warps
-constexpr int TC_THREADS = 32 * (TC_AW + 3);       // and a bulk-copy warp, two MMA warps
-
-static_assert(TC_AOFF % 1024 == 0 && TC_BOFF % 1024 == 0 && TC_POFF % 16 == 0, "operand buffers stay aligned");
-static_assert(TC_SMEM <= 227 * 1024, "one CTA's shared memory");
-static_assert(TC_CHUNK % TC_KS == 0, "chunks hold whole stages");
-static_assert(KT == 4 * KI && KT <= 64, "an item is four KI runs, Zr and Zi fit 128 rows");
-
-__device__ __forceinline__ void tc_abort(int *flag, int *err, int bit = TC_ERR)
+__device__ __forceinline__ void tc_abort(int *flag, int *err, int bit)
 {
    *(volatile int *)flag = 1;
    atomicOr(err, bit);
@@ -79,231 +20,34 @@ __device__ __forceinline__ bool tc_aborted(const int *flag)
    return *(const volatile int *)flag != 0;
 }
 
-// Grid: (item tiles of 128, site chunks of TC_CHUNK).  part[chunk][k].
-__global__ void __launch_bounds__(TC_THREADS, 1)
-k_sfac_tc(const int4 *__restrict__ item, const int4 *__restrict__ item_k0, const int4 *__restrict__ ph,
-          const uint4 *__restrict__ ztab, int np, int nk, float qscale, float qunscale, float2 *__restrict__ part,
-          int *__restrict__ err)
-{
-   using namespace tc;
-   extern __shared__ __align__(1024) unsigned char sm[];
-   __shared__ __align__(8) uint64_t full_b[TC_NSB], empty_b[TC_NSB], full_a[TC_NSA], empty_a[TC_NSA], accf;
-   __shared__ unsigned int tmem_s;
-   __shared__ int abort_s;
-   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-   const int tile = blockIdx.x, chunk = blockIdx.y;
-   const int s0 = chunk * TC_CHUNK;
-   const int nst = (min(np, s0 + TC_CHUNK) - s0) / TC_KS;
-   const int ncols = (item[tile * 128].w + 15) & ~15;   // the tile's largest count, rounded up
-   if (ncols == 0 || nst <= 0) return;                  // (uniform over the CTA)
-   if (tid == 0) {
-      for (int s = 0; s < TC_NSB; s++) {
-         bar_init(&full_b[s], 1);
-         bar_init(&empty_b[s], 2);   // released by both MMA issuers
-      }
-      for (int s = 0; s < TC_NSA; s++) {
-         bar_init(&full_a[s], TC_AW);
-         bar_init(&empty_a[s], 2);
-      }
-      bar_init(&accf, 2);
-      abort_s = 0;
-      bar_init_fence();
-   }
-   __syncwarp();
-   if (w == TC_AW + 1) tmem_alloc(&tmem_s, 512);
-   fence_before_sync();
-   __syncthreads();
-   fence_after_sync();
-   const unsigned int tmem = tmem_s;
-
-   if (w == TC_AW) {
-      // ---- bulk copies: each stage's z tables and site records
-      if (lane == 0) {
-         int issued = 0;
-         for (int st = 0; st < nst; st++) {
-            const int s = st % TC_NSB;
-            if (st >= TC_NSB && !bar_wait(&empty_b[s], (unsigned int)(st / TC_NSB - 1) & 1u)) {
-               tc_abort(&abort_s, err);
-               break;
-            }
-            if (tc_aborted(&abort_s)) break;
-            bar_expect_tx(&full_b[s], TC_BBYTES + TC_PBYTES);
-            bulk_load(sm + TC_BOFF + s * TC_BBYTES, ztab + (size_t)(s0 / TC_KS + st) * (TC_BBYTES / 16), TC_BBYTES,
-                      &full_b[s]);
-            bulk_load(sm + TC_POFF + s * TC_PBYTES, ph + s0 + st * TC_KS, TC_PBYTES, &full_b[s]);
-            issued = st + 1;
-         }
-         // copies still in flight complete before the CTA's shared memory goes
-         for (int st = issued > TC_NSB ? issued - TC_NSB : 0; st < issued; st++)
-            bar_wait(&full_b[st % TC_NSB], (unsigned int)(st / TC_NSB) & 1u);
-      }
-   } else if (w == TC_AW + 1 || w == TC_AW + 2) {
-      // ---- MMA issue: warp TC_AW + 1 multiplies Ar, warp TC_AW + 2 Ai, by the
-      // whole z operand [Zr | Zi] (N = 128) into D1 = (Ar Zr, Ar Zi) and
-      // D2 = (Ai Zr, Ai Zi)
-      const int ic = w - TC_AW - 1;
-      if (lane == 0) {
-         const unsigned int idn = idesc_bf16(128, 128, false);
-         const int ta[6] = {0, 0, 1, 0, 2, 1}, tb[6] = {0, 1, 0, 2, 0, 1};
-         for (int st = 0; st < nst; st++) {
-            const int sa = st % TC_NSA, sb = st % TC_NSB;
-            if (!bar_wait(&full_a[sa], (unsigned int)(st / TC_NSA) & 1u) ||
-                !bar_wait(&full_b[sb], (unsigned int)(st / TC_NSB) & 1u)) {
-               tc_abort(&abort_s, err);
-               break;
-            }
-            fence_after_sync();
-            const unsigned int a = saddr(sm + TC_AOFF + sa * TC_ABYTES) + 3 * ic * TC_TERM;
-            const unsigned int b = saddr(sm + TC_BOFF + sb * TC_BBYTES);
-#pragma unroll
-            for (int ks = 0; ks < TC_KS / 16; ks++)
-#pragma unroll
-               for (int p = 0; p < 6; p++)
-                  mma_f16(tmem + 128u * ic + (p == 0 ? 0u : 256u),
-                           sdesc(a + ta[p] * TC_TERM + ks * 2 * TC_LBO, TC_LBO, 128),
-                           sdesc(b + tb[p] * TC_TERM + ks * 2 * TC_LBO, TC_LBO, 128), idn, st > 0 || ks > 0 || p > 1);
-            mma_commit(&empty_a[sa]);
-            mma_commit(&empty_b[sb]);
-         }
-         mma_commit(&accf);   // also after an abort: the readers wait on it
-      }
-   } else {
-      // ---- A operand: q_j seed_ij for this thread's item row and the
-      // stage's sites 8 qq .. 8 qq + 7 (one column group)
-      const int m = tid & 127, qq = tid >> 7;
-      const int4 hd = item[tile * 128 + m];
-      const unsigned int H = (unsigned int)hd.x, K = (unsigned int)hd.y, L = (unsigned int)hd.z;
-      for (int st = 0; st < nst; st++) {
-         const int s = st % TC_NSA, sb = st % TC_NSB;
-         if (tc_aborted(&abort_s)) break;
-         if ((st >= TC_NSA && !bar_wait(&empty_a[s], (unsigned int)(st / TC_NSA - 1) & 1u)) ||
-             !bar_wait(&full_b[sb], (unsigned int)(st / TC_NSB) & 1u)) {
-            tc_abort(&abort_s, err);
-            break;
-         }
-         unsigned char *A = sm + TC_AOFF + s * TC_ABYTES;
-         const int4 *P = reinterpret_cast<const int4 *>(sm + TC_POFF + sb * TC_PBYTES) + 8 * qq;
-         unsigned int hr[4], mr[4], lr[4], hi[4], mi[4], li[4];
-#pragma unroll
-         for (int jp = 0; jp < 4; jp++) {
-            const int4 v0 = P[2 * jp], v1 = P[2 * jp + 1];
-            f2x sv, cv;   // the two sites as the lanes of paired FP32 instructions
-            sincos_poly2(H * (unsigned int)v0.x + K * (unsigned int)v0.y + L * (unsigned int)v0.z,
-                         H * (unsigned int)v1.x + K * (unsigned int)v1.y + L * (unsigned int)v1.z, sv, cv);
-            const f2x q = pk2(__int_as_float(v0.w) * qscale, __int_as_float(v1.w) * qscale);
-            split3(mul2(cv, q), hr[jp], mr[jp], lr[jp]);
-            split3(mul2(sv, q), hi[jp], mi[jp], li[jp]);
-         }
-         unsigned char *row = A + qq * TC_LBO + (m >> 3) * 128 + (m & 7) * 16;
-         *reinterpret_cast<uint4 *>(row) = make_uint4(hr[0], hr[1], hr[2], hr[3]);
-         *reinterpret_cast<uint4 *>(row + TC_TERM) = make_uint4(mr[0], mr[1], mr[2], mr[3]);
-         *reinterpret_cast<uint4 *>(row + 2 * TC_TERM) = make_uint4(lr[0], lr[1], lr[2], lr[3]);
-         *reinterpret_cast<uint4 *>(row + 3 * TC_TERM) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-         *reinterpret_cast<uint4 *>(row + 4 * TC_TERM) = make_uint4(mi[0], mi[1], mi[2], mi[3]);
-         *reinterpret_cast<uint4 *>(row + 5 * TC_TERM) = make_uint4(li[0], li[1], li[2], li[3]);
-         fence_async_smem();
-         __syncwarp();
-         if (lane == 0) bar_arrive(&full_a[s]);
-      }
-      // ---- read back: item row m (lane quarter w % 4), t in [16 qq, 16 qq + 16):
-      // Re = Ar Zr - Ai Zi, Im = Ar Zi + Ai Zr, each the hh sums plus the rest
-      const bool done = bar_wait(&accf, 0);
-      const bool ok = __all_sync(0xffffffffu, done && !tc_aborted(&abort_s));
-      if (!done && lane == 0) tc_abort(&abort_s, err);
-      fence_after_sync();
-      const int t0 = 16 * qq;
-      if (ok && t0 < ncols) {
-         const int4 k0 = item_k0[tile * 128 + m];
-         const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16) + (unsigned int)t0;
-         const int kr = qq == 0 ? k0.x : qq == 1 ? k0.y : qq == 2 ? k0.z : k0.w;
-         // column pairs (hh sums, the rest): Ar Zr at t, Ar Zi at 64 + t,
-         // Ai Zr at 128 + t, Ai Zi at 192 + t; the rest 256 further on
-         auto pair_sum = [&](unsigned int col, float (&out)[16]) {
-            float u[16], v[16];
-            tmem_ld16(trow + col, u);
-            tmem_ld16(trow + col + 256, v);
-            tmem_wait2(u, v);
-#pragma unroll
-            for (int j = 0; j < 16; j++) out[j] = u[j] + v[j];
-         };
-         float re[16], im[16], x[16];
-         pair_sum(0, re);
-         pair_sum(192, x);
-#pragma unroll
-         for (int j = 0; j < 16; j++) re[j] -= x[j];
-         pair_sum(64, im);
-         pair_sum(128, x);
-#pragma unroll
-         for (int j = 0; j < 16; j++) im[j] += x[j];
-         float2 *dst = part + (size_t)chunk * nk;
-         if (kr >= 0)
-#pragma unroll
-            for (int j = 0; j < 16; j++)
-               if (t0 + j < hd.w) dst[kr + j] = make_float2(re[j] * qunscale, im[j] * qunscale);
-      }
-   }
-   fence_before_sync();
-   __syncthreads();
-   if (w == TC_AW + 1) {
-      __syncwarp();
-      fence_after_sync();
-      tmem_dealloc(tmem, 512);
-   }
-}
-
-// The structure-factor product into part32 ([chunks][nk]); returns the
-// number of chunks.
-int ks_sfac_tc(cudaStream_t st, int nsites, int nk, const KsDev &d, int ntiles, double qmax, int *err)
-{
-   const int np = (nsites + TC_KS - 1) / TC_KS * TC_KS;
-   const int nchunks = (np + TC_CHUNK - 1) / TC_CHUNK;
-   // charges scaled by a power of two to |q| <= 1 (exact), undone on the partials
-   int e = 0;
-   std::frexp(qmax > 0 ? qmax : 1.0, &e);
-   const float qs = std::ldexp(1.0f, e);
-   k_sfac_tc<<<dim3(ntiles, nchunks), TC_THREADS, TC_SMEM, st>>>(d.tc_item.p, d.tc_k0.p, d.ph32.p, d.ztab.p, np, nk,
-                                                          1.0f / qs, qs, d.part32.p, err);
-   return nchunks;
-}
-
-size_t ks_tc_ztab_len(int nsites)
-{
-   const size_t np = (size_t)(nsites + TC_KS - 1) / TC_KS * TC_KS;
-   return np / TC_KS * (TC_BBYTES / 16);
-}
-
-int ks_tc_chunks(int nsites)
-{
-   const int np = (nsites + TC_KS - 1) / TC_KS * TC_KS;
-   return (np + TC_CHUNK - 1) / TC_CHUNK;
-}
-
-
 // ------------------------------------------------------------- forces
 // The force pass of ewald() (src/ewald.c:557-566): for a charged site j,
 //     F_j = q_j sum_k k (sin(k.r_j) A_k - cos(k.r_j) B_k) = q_j sum_k k Im(e_jk U_k),
-// U_k = A_k - i B_k.  Over a tensor-core item (seed_ij, offsets t, k-vector
-// (kx, ky, kz0 + t dkz)):
-//     W1_ij = sum_t z_j(t) U_t,  W2_ij = sum_t t z_j(t) U_t,
+// U_k = A_k - i B_k.  An item i is a column (h, k) of the k-list, its
+// k-vectors (h, k, +-t) taken together: with seed_ij = exp(2 pi i (h u_x +
+// k u_y)), z_j(t) = C_t + i S_t and U+-_t the coefficients at l = +-t,
+//     W1_ij = sum_t C_t (U+ + U-) + i S_t (U+ - U-),
+//     W2_ij = sum_t t (C_t (U+ - U-) + i S_t (U+ + U-)),
 //     F_j += q_j (kx f1, ky f1, kz0 f1 + dkz f2),  f1,2 = Im(seed_ij W1,2_ij).
-// W is a product of the sites x t z tables (K = 128: the 64 cosines, then
-// the 64 sines) and four coefficient rows per item,
-//     W1re = [A | B],  W1im = [-B | A],  W2re = [tA | tB],  W2im = [-tB | tA],
-// each row scaled by a power of two to |v| <= 1 (the scale is folded into
-// the item's force coefficients).  Operands are three bf16 terms on fixed
-// grids as in the structure factor, six term products (hh into one
-// accumulator, the rest into another): the k-space force on a site is a
+// W is a product of the sites x t z tables (per 8 t: 8 cosines, 8 sines,
+// one K-step of 16) and four coefficient rows per item, real and imaginary
+// parts of W1 and W2, each pair of rows scaled by a power of two to |v| <= 1
+// (the scale is folded into the item's force coefficients).  Taking l = +-t
+// together halves K against a running l from the column's first k-vector
+// (131,072-site water: 0.50 -> 0.42 ms, then bound by the
+// epilogue's latency).  Operands are three bf16 terms on
+// fixed grids (tc.cuh), six term products (hh into one accumulator, where
+// sums are exact, the rest into another): the k-space force on a site is a
 // near-cancelling sum over k, and two fp16 terms (2^-22 per operand, three
 // products) raised the force error of the fixtures to 1.1e-5.  A CTA holds
-// one 128-site tile's z tables (96 KB) at a time and streams the
+// one 128-site tile's z tables (up to 96 KB) at a time and streams the
 // coefficient rows of 32 items (N = 128) per tile of items, two K-steps per
-// stage (only the K-steps an item tile's longest item needs; one barrier
-// wait and one commit per 12 MMAs: at one K-step per stage the issuing
-// threads' waits cost 6 % of the pass); tensor memory holds two
-// accumulator pairs, so the epilogue of one item tile (16 warps, four per
-// tensor-memory lane quarter, 8 items each: the seed sine/cosine per item
-// and site, the k-vector weights, Kahan-compensated FP32 force sums)
-// overlaps the MMAs of the next.
+// stage (only the K-steps an item tile's longest item needs); tensor memory
+// holds two accumulator pairs, so the epilogue of one item tile (16 warps,
+// four per tensor-memory lane quarter, 8 items -- one unit of four quads --
+// each: the seeds by products of the site's x and y tables, the k-vector
+// weights, Kahan-compensated FP32 force sums) overlaps the MMAs of the next.
+// Systems with more than 64 t values run once per 64-wide t-block.
 constexpr int FTC_NI = 32;                         // items per item tile (4 rows each: N = 128)
 constexpr int FTC_NSB = 2;                         // coefficient stages in flight per ring (two rings)
 constexpr int FTC_ATERM = 128 * 128 * 2;           // one term of a site tile's z tables: 32 KB
@@ -320,80 +64,75 @@ static_assert(FTC_IPW % 4 == 0, "an epilogue warp reads its items' columns 16 at
 constexpr int FTC_SPLITS = 2;                      // force slots per site (two CTAs at most per site tile)
 constexpr int FTC_ERR = 16;                        // error-word bit: a force-pass wait expired
 
-// Coefficient rows of each item from the per-k (A, B, kz): one warp per
-// item.  Layout per (item tile, K-step of 16): [term][column group 2][row
-// group 16][8 rows][8 K] bf16, row 4 i + c for item i of the tile.
+// Coefficient rows of each item from the dense per-(quad, t) A and B
+// (k_qreduce): one warp per item, 64 t from t0.  Item 8 j + 2 q + s is quad
+// q of unit fu[j] with k = +-m.  Layout per (item tile, K-step of 16): [term]
+// [cosines, sines][row group 16][8 rows][8 t] bf16, row 4 i + c for item i
+// of the tile.
 __global__ void __launch_bounds__(256)
-k_utab_tc(int nitems, const int4 *__restrict__ item, const int4 *__restrict__ item_k0,
-          const float2 *__restrict__ kxy, const float4 *__restrict__ kd, float dkz, uint4 *__restrict__ utab,
-          float4 *__restrict__ coef)
+k_utab_tc(int nitems, QGeom g, int t0, const int4 *__restrict__ fu, const float4 *__restrict__ ab,
+          uint4 *__restrict__ utab, float4 *__restrict__ coef)
 {
-   __shared__ float sv[8][64][4];
+   __shared__ float4 sv[8][64];
    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int i = blockIdx.x * 8 + wl;
    if (i >= nitems) return;   // (warp-uniform)
-   const int4 hd = item[i], k0 = item_k0[i];
-   float a[2], b[2], kz0 = 0.f, m1 = 0.f, m2 = 0.f;
+   const int4 un = fu[i >> 3];
+   const int q = (i >> 1) & 3, neg = i & 1;
+   float m1 = 0.f, m2 = 0.f;
 #pragma unroll
    for (int h = 0; h < 2; h++) {
-      const int t = lane + 32 * h;
-      a[h] = b[h] = 0.f;
-      if (t < hd.w) {
-         const int run = t >> 4;
-         const int kr = run == 0 ? k0.x : run == 1 ? k0.y : run == 2 ? k0.z : k0.w;
-         const float4 v = kd[kr + (t & 15)];
-         a[h] = v.x;
-         b[h] = v.y;
-         if (t == 0) kz0 = v.z;
-      }
-      m1 = fmaxf(m1, fmaxf(fabsf(a[h]), fabsf(b[h])));
-      m2 = fmaxf(m2, (float)t * fmaxf(fabsf(a[h]), fabsf(b[h])));
+      const int t = t0 + lane + 32 * h;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);   // A+, B+, A-, B-
+      if (un.w >= 0 && t < g.TP) v = ab[((size_t)(4 * un.w + q) * g.TP + t) * 2 + neg];
+      sv[wl][lane + 32 * h] = v;
+      const float a = fmaxf(fabsf(v.x + v.z), fabsf(v.x - v.z)), b = fmaxf(fabsf(v.y + v.w), fabsf(v.y - v.w));
+      m1 = fmaxf(m1, fmaxf(a, b));
+      m2 = fmaxf(m2, (float)t * fmaxf(a, b));
    }
 #pragma unroll
    for (int o = 16; o > 0; o >>= 1) {
       m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
       m2 = fmaxf(m2, __shfl_xor_sync(0xffffffffu, m2, o));
    }
-   kz0 = __shfl_sync(0xffffffffu, kz0, 0);
    // powers of two at or above the rows' largest magnitude
    int e1 = 0, e2 = 0;
+   // (their reciprocals stay finite: rows below 2^-100 are zeros in effect)
    if (m1 > 0.f) frexpf(m1, &e1);
    if (m2 > 0.f) frexpf(m2, &e2);
+   e1 = max(e1, -100);
+   e2 = max(e2, -100);
    const float s1 = ldexpf(1.f, e1), s2 = ldexpf(1.f, e2), i1 = ldexpf(1.f, -e1), i2 = ldexpf(1.f, -e2);
-#pragma unroll
-   for (int h = 0; h < 2; h++) {
-      const int t = lane + 32 * h;
-      sv[wl][t][0] = a[h] * i1;
-      sv[wl][t][1] = b[h] * i1;
-      sv[wl][t][2] = (float)t * a[h] * i2;
-      sv[wl][t][3] = (float)t * b[h] * i2;
-   }
    __syncwarp();
-   const int tile = i / FTC_NI, il = i % FTC_NI;
+   const int tile = i / FTC_NI, il = i % FTC_NI, c = lane & 3, ks = lane >> 2;
 #pragma unroll
-   for (int h = 0; h < 2; h++) {
-      const int id = lane + 32 * h, c = id & 3, g = id >> 2;   // row c of the item, column group g
-      const bool zi = g >= 8;                                  // the sine half of K
-      const int t0 = 8 * (g & 7);
-      // W1re = [A | B], W1im = [-B | A], W2re = [tA | tB], W2im = [-tB | tA]
-      const int src = (c & 2) + (zi ? ((c & 1) ? 0 : 1) : ((c & 1) ? 1 : 0));
-      const float sg = (!zi && (c & 1)) ? -1.f : 1.f;
+   for (int kg = 0; kg < 2; kg++) {
       float v[8];
 #pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = sg * sv[wl][t0 + e][src];
+      for (int e = 0; e < 8; e++) {
+         const float4 x = sv[wl][8 * ks + e];
+         const float As = x.x + x.z, Ad = x.x - x.z, Bs = x.y + x.w, Bd = x.y - x.w;
+         // rows W1re, W1im, W2re, W2im: cosine and sine coefficients
+         const float r = kg == 0 ? (c == 0 ? As : c == 1 ? -Bs : c == 2 ? Ad : -Bd)
+                                 : (c == 0 ? Bd : c == 1 ? Ad : c == 2 ? Bs : As);
+         v[e] = c < 2 ? r * i1 : (float)(t0 + 8 * ks + e) * r * i2;
+      }
       unsigned int hh[4], mm[4], ll[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) tc::split3(v[2 * j], v[2 * j + 1], hh[j], mm[j], ll[j]);
-      const int n = 4 * il + c, ks = g >> 1, kg = g & 1;
-      const size_t base =
-          ((size_t)tile * 8 + ks) * (FTC_BBYTES / 16) + kg * 128 + (n >> 3) * 8 + (n & 7);
+      const int n = 4 * il + c;
+      const size_t base = ((size_t)tile * 8 + ks) * (FTC_BBYTES / 16) + kg * 128 + (n >> 3) * 8 + (n & 7);
       utab[base] = make_uint4(hh[0], hh[1], hh[2], hh[3]);
       utab[base + FTC_BTERM / 16] = make_uint4(mm[0], mm[1], mm[2], mm[3]);
       utab[base + 2 * FTC_BTERM / 16] = make_uint4(ll[0], ll[1], ll[2], ll[3]);
    }
    if (lane == 0) {
-      const float2 k = kxy[i];
-      coef[i] = hd.w > 0 ? make_float4(k.x * s1, k.y * s1, kz0 * s1, dkz * s2) : make_float4(0.f, 0.f, 0.f, 0.f);
+      // the seeds' table scale (units of 2^-24 and 2^-31, times Q_KAPPA each) folded in
+      const double f2 = 1.0 / (16777216.0 * 2147483648.0 * Q_KAPPA * Q_KAPPA);
+      const double hh = un.x, kk = neg ? -(double)(un.y + q) : (double)(un.y + q);
+      coef[i] = un.w >= 0 ? make_float4((float)((hh * g.b[0] + kk * g.b[3]) * f2 * s1), (float)((hh * g.b[1] + kk * g.b[4]) * f2 * s1),
+                                        (float)((hh * g.b[2] + kk * g.b[5]) * f2 * s1), (float)(g.b[8] * f2 * s2))
+                          : make_float4(0.f, 0.f, 0.f, 0.f);
    }
 }
 
@@ -405,6 +144,13 @@ __device__ __forceinline__ void kahan_add_tc(float &s, float &c, float x)
    s = t;
 }
 
+// K-steps (8 t each) of an item tile in the t-block from t0: its first unit's
+// t range is the longest (units in order of falling range)
+__device__ __forceinline__ int ftc_ksteps(int4 un, int t0)
+{
+   return un.w < 0 ? 0 : min(max(un.z - t0 + 7, 0) >> 3, 8);
+}
+
 // Work ranges of the persistent force pass.  Unit u is (site tile u / ntl,
 // item tile u % ntl); CTA c takes units ustart[c] .. ustart[c + 1] - 1, a
 // contiguous run over the site tiles.  The runs split the units' weights
@@ -413,14 +159,14 @@ __device__ __forceinline__ void kahan_add_tc(float &s, float &c, float x)
 // a tile), so no run lies strictly inside a site tile and a tile is shared
 // by two CTAs at most.  One block; pre (after ustart[G]) holds the prefix
 // weights of the item tiles.
-__global__ void k_ftc_ranges(const int4 *__restrict__ item, int ntl, int nsite_tiles, int G, int *__restrict__ ustart)
+__global__ void k_ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *__restrict__ ustart)
 {
    int *pre = ustart + G + 1;
    if (threadIdx.x == 0) {
       int sum = 0;
       pre[0] = 0;
       for (int t = 0; t < ntl; t++) {
-         sum += 2 * ((item[t * FTC_NI].w + 15) >> 4) + 1;
+         sum += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
          pre[t + 1] = sum;
       }
    }
@@ -447,10 +193,10 @@ __global__ void k_ftc_ranges(const int4 *__restrict__ item, int ntl, int nsite_t
 // tile's forces into slot 0 of fpart, or slot 1 when the range starts inside
 // the tile (and zeros into slot 1 when the range covers the whole tile).
 __global__ void __launch_bounds__(FTC_THREADS, 1)
-k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int nitems,
-           const int4 *__restrict__ ph, const uint4 *__restrict__ zsite, const uint4 *__restrict__ utab,
-           const double *__restrict__ chg, const int *__restrict__ slots, int n, const int *__restrict__ ustart,
-           double *__restrict__ fpart, int *__restrict__ err)
+k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef, int nitems, int t0,
+           const int *__restrict__ X, const int *__restrict__ Y, const uint4 *__restrict__ zsite,
+           const uint4 *__restrict__ utab, const double *__restrict__ chg, const int *__restrict__ slots, int n,
+           const int *__restrict__ ustart, double *__restrict__ fpart, int *__restrict__ err)
 {
    using namespace tc;
    extern __shared__ __align__(1024) unsigned char sm[];
@@ -469,8 +215,11 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
    unsigned char *A = sm, *Bs = sm + FTC_ABYTES;
    // [2][FTC_EG][128][3]: per epilogue group, a site tile's force sums (by tile parity)
    float *red = reinterpret_cast<float *>(sm + FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES);
-   // per epilogue warp: its items' (h, k, l0, count) and force coefficients
-   int4 *sitem = reinterpret_cast<int4 *>(sm + FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES + 2 * FTC_EG * 128 * 3 * 4);
+   // per epilogue warp: its items' force coefficients
+   float4 *scoef = reinterpret_cast<float4 *>(sm + FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES + 2 * FTC_EG * 128 * 3 * 4);
+   // the t-block's z tables of a site tile: columns, bytes of a term
+   const int fcols = min(128, 2 * (g.TP - t0));
+   const unsigned int aterm = (unsigned int)fcols * 256u;
    if (tid == 0) {
       bar_init(&full_a, 1);
       bar_init(&a_free, 2);
@@ -494,8 +243,8 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
    __syncthreads();
    fence_after_sync();
    const unsigned int tmem = tmem_s;
-   // K-steps of a unit's item tile: ceil(longest count / 16) in each half of K
-   auto khalf = [&](int u) { return (item[(u % ntl) * FTC_NI].w + 15) >> 4; };
+   // K-steps of a unit's item tile
+   auto ksteps = [&](int u) { return ftc_ksteps(fu[(u % ntl) * (FTC_NI / 8)], t0); };
 
    if (w == FTC_EW || w == FTC_EW + 1) {
       // ---- bulk copies: warp FTC_EW + p streams the coefficient rows of the
@@ -503,7 +252,7 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
       // each site tile's z tables
       const int p = w - FTC_EW;
       if (lane == 0) {
-         int g = 0, na = 0;
+         int gi = 0, na = 0;
          bool stop = false;
          for (int T = T0; T <= T1 && !stop; T++) {
             if (p == 0) {
@@ -511,18 +260,17 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
                   tc_abort(&abort_s, err, FTC_ERR);
                   break;
                }
-               bar_expect_tx(&full_a, FTC_ABYTES);
-               bulk_load(A, zsite + (size_t)T * (FTC_ABYTES / 16), FTC_ABYTES, &full_a);
+               bar_expect_tx(&full_a, 3 * aterm);
+               bulk_load(A, zsite + ((size_t)T * 2 * g.TP + 2 * t0) * 48, 3 * aterm, &full_a);
                na++;
             }
             for (int u = ua(T); u < ue(T) && !stop; u++) {
                if (((u - u0) & 1) != p) continue;
-               const int kh = khalf(u), nt = u % ntl;
-               // stage sq: K-steps q = 2 sq, 2 sq + 1 (the unit's 2 kh K-steps
-               // are the kh lowest of each half of K)
-               for (int sq = 0; sq < kh; sq++) {
-                  const int s = g % FTC_NSB;
-                  if (g >= FTC_NSB && !bar_wait(&empty_b[p][s], (unsigned int)(g / FTC_NSB - 1) & 1u)) {
+               const int kq = ksteps(u), nt = u % ntl;
+               // stage sq: K-steps 2 sq and, within the unit's, 2 sq + 1
+               for (int sq = 0; 2 * sq < kq; sq++) {
+                  const int s = gi % FTC_NSB;
+                  if (gi >= FTC_NSB && !bar_wait(&empty_b[p][s], (unsigned int)(gi / FTC_NSB - 1) & 1u)) {
                      tc_abort(&abort_s, err, FTC_ERR);
                      stop = true;
                      break;
@@ -531,19 +279,17 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
                      stop = true;
                      break;
                   }
-                  bar_expect_tx(&full_b[p][s], FTC_SBYTES);
-                  for (int h = 0; h < 2; h++) {
-                     const int q = 2 * sq + h, ks = q < kh ? q : 4 + q - kh;
-                     bulk_load(Bs + (p * FTC_NSB + s) * FTC_SBYTES + h * FTC_BBYTES,
-                               utab + ((size_t)nt * 8 + ks) * (FTC_BBYTES / 16), FTC_BBYTES, &full_b[p][s]);
-                  }
-                  g++;
+                  const unsigned int bytes = 2 * sq + 1 < kq ? FTC_SBYTES : FTC_BBYTES;
+                  bar_expect_tx(&full_b[p][s], bytes);
+                  bulk_load(Bs + (p * FTC_NSB + s) * FTC_SBYTES, utab + ((size_t)nt * 8 + 2 * sq) * (FTC_BBYTES / 16),
+                            bytes, &full_b[p][s]);
+                  gi++;
                }
             }
          }
          // copies still in flight complete before the CTA's shared memory goes
          if (na > 0) bar_wait(&full_a, (unsigned int)(na - 1) & 1u);
-         for (int q = g > FTC_NSB ? g - FTC_NSB : 0; q < g; q++)
+         for (int q = gi > FTC_NSB ? gi - FTC_NSB : 0; q < gi; q++)
             bar_wait(&full_b[p][q % FTC_NSB], (unsigned int)(q / FTC_NSB) & 1u);
       }
    } else if (w == FTC_EW + 2 || w == FTC_EW + 3) {
@@ -555,7 +301,7 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
       const int ta[6] = {0, 0, 1, 0, 2, 1}, tb[6] = {0, 1, 0, 2, 0, 1};
       const unsigned int a0 = saddr(A), b0 = saddr(Bs + p * FTC_NSB * FTC_SBYTES);
       bool ok = true;
-      int g = 0, jj = 0;
+      int gi = 0, jj = 0;
       for (int T = T0; T <= T1; T++) {
          if (T > T0) {
             // both issuers are past the previous site tile: its z tables go
@@ -578,10 +324,10 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
                ok = false;
             }
             fence_after_sync();
-            const int kh = ok ? khalf(u) : 0;
-            for (int sq = 0; sq < kh; sq++) {
-               const int s = g % FTC_NSB;
-               if (!bar_wait(&full_b[p][s], (unsigned int)(g / FTC_NSB) & 1u)) {
+            const int kq = ok ? ksteps(u) : 0;
+            for (int sq = 0; 2 * sq < kq; sq++) {
+               const int s = gi % FTC_NSB;
+               if (!bar_wait(&full_b[p][s], (unsigned int)(gi / FTC_NSB) & 1u)) {
                   tc_abort(&abort_s, err, FTC_ERR);
                   ok = false;
                   break;
@@ -589,17 +335,18 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
                fence_after_sync();
 #pragma unroll
                for (int h = 0; h < 2; h++) {
-                  const int q = 2 * sq + h, ks = q < kh ? q : 4 + q - kh;
+                  const int ks = 2 * sq + h;
+                  if (ks >= kq) break;
                   const unsigned int bs = b0 + s * FTC_SBYTES + h * FTC_BBYTES;
 #pragma unroll
                   for (int t = 0; t < 6; t++) {
-                     const uint64_t ad = sdesc(a0 + ta[t] * FTC_ATERM + ks * 4096, 2048, 128);
+                     const uint64_t ad = sdesc(a0 + ta[t] * aterm + ks * 4096, 2048, 128);
                      const uint64_t bd = sdesc(bs + tb[t] * FTC_BTERM, 2048, 128);
-                     mma_f16(tmem + p * 256 + (t == 0 ? 0 : 128), ad, bd, idn, q > 0 || t > 1);
+                     mma_f16(tmem + p * 256 + (t == 0 ? 0 : 128), ad, bd, idn, ks > 0 || t > 1);
                   }
                }
                mma_commit(&empty_b[p][s]);
-               g++;
+               gi++;
             }
             mma_commit(&acc_full[p]);
             jj++;
@@ -614,23 +361,29 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
       // each item tile
       const int r = 32 * (w & 3) + lane, ig = w >> 2;
       const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16);
-      int4 *wi = sitem + w * 2 * FTC_IPW;   // [FTC_IPW] items, then [FTC_IPW] coefficients
-      const float4 *wc = reinterpret_cast<const float4 *>(wi + FTC_IPW);
+      float4 *wc = scoef + w * FTC_IPW;
       bool live = true;
       for (int T = T0; T <= T1; T++) {
          const int i = T * 128 + r;
-         const int4 v = i < n ? ph[i] : make_int4(0, 0, 0, 0);
-         const unsigned int ux = (unsigned int)v.x, uy = (unsigned int)v.y, uz = (unsigned int)v.z;
+         // the site's x and y tables (a stage of 32 sites, rows of 36)
+         const size_t sg = (size_t)T * 4 + (r >> 5);
+         const int *xb = X + sg * 2 * g.hrows * 36 + lane, *yb = Y + sg * 2 * g.mrows * 36 + lane;
          float Fx = 0.f, Fy = 0.f, Fz = 0.f, Cx = 0.f, Cy = 0.f, Cz = 0.f;
          for (int u = ua(T); u < ue(T) && live; u++) {
             const int j = u - u0, b = j & 1;
-            const int it0 = (u % ntl) * FTC_NI + ig * FTC_IPW;
-            // this unit's item records, fetched while its MMAs run
+            const int pos = (u % ntl) * (FTC_NI / 8) + ig;   // the warp's eight items: unit fu[pos]
+            // their tables and coefficients, fetched while the MMAs run
+            const int4 un = fu[pos];
+            const int *xp = xb + (size_t)2 * un.x * 36, *yp = yb + (size_t)2 * un.y * 36;
+            const float ch = (float)__ldg(xp), sh = (float)__ldg(xp + 36);
+            float cm[4], sm4[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+               cm[q] = (float)__ldg(yp + 2 * q * 36);
+               sm4[q] = (float)__ldg(yp + (2 * q + 1) * 36);
+            }
             __syncwarp();
-            if (lane < FTC_IPW)
-               wi[lane] = item[it0 + lane];
-            else if (lane < 2 * FTC_IPW)
-               reinterpret_cast<float4 *>(wi)[lane] = coef[it0 + lane - FTC_IPW];
+            if (lane < FTC_IPW) wc[lane] = coef[pos * FTC_IPW + lane];
             __syncwarp();
             const bool got = !tc_aborted(&abort_s) && bar_wait(&acc_full[b], (unsigned int)(j >> 1) & 1u);
             if (!__all_sync(0xffffffffu, got && !tc_aborted(&abort_s))) {
@@ -657,21 +410,18 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
             __syncwarp();
             if (lane == 0) bar_arrive(&acc_empty[b]);
             float fx = 0.f, fy = 0.f, fz = 0.f;
+            // (padding units come last; a tile whose units have no t in this
+            // block issues no MMAs, so its buffer holds an earlier unit's sums)
+            if (un.w >= 0 && un.z > t0)
 #pragma unroll
-            for (int grp = 0; grp < FTC_IPW / 4; grp++) {
+            for (int q = 0; q < 4; q++) {
+               const float a = ch * cm[q], d = sh * sm4[q], c = sh * cm[q], e = ch * sm4[q];
 #pragma unroll
-               for (int e = 0; e < 4; e++) {
-                  const int4 hd = wi[4 * grp + e];
-                  // padding items come last; a tile of padding only issues no
-                  // MMAs, so its buffer holds an earlier unit's sums (uniform)
-                  if (hd.w == 0) continue;
-                  const float4 cf = wc[4 * grp + e];
-                  float sn, cs;
-                  sincos_poly((unsigned int)hd.x * ux + (unsigned int)hd.y * uy + (unsigned int)hd.z * uz, &sn,
-                              &cs);
-                  const float w1r = wv[grp][4 * e], w1i = wv[grp][4 * e + 1];
-                  const float w2r = wv[grp][4 * e + 2], w2i = wv[grp][4 * e + 3];
-                  const float f1 = fmaf(cs, w1i, sn * w1r), f2 = fmaf(cs, w2i, sn * w2r);
+               for (int s = 0; s < 2; s++) {
+                  const float cs = s ? a + d : a - d, sn = s ? c - e : c + e;   // seed of k = +-m
+                  const float4 cf = wc[2 * q + s];
+                  const float *W = &wv[q >> 1][8 * (q & 1) + 4 * s];
+                  const float f1 = fmaf(cs, W[1], sn * W[0]), f2 = fmaf(cs, W[3], sn * W[2]);
                   fx = fmaf(cf.x, f1, fx);
                   fy = fmaf(cf.y, f1, fy);
                   fz = fmaf(cf.z, f1, fmaf(cf.w, f2, fz));
@@ -692,8 +442,8 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
          if (w < 4 && i < n && !tc_aborted(&abort_s)) {
             const double q = chg[slots[i]];
             double sx = 0.0, sy = 0.0, sz = 0.0;
-            for (int g = 0; g < FTC_EG; g++) {
-               const float *rg = rt + ((size_t)g * 128 + r) * 3;
+            for (int k = 0; k < FTC_EG; k++) {
+               const float *rg = rt + ((size_t)k * 128 + r) * 3;
                sx += (double)rg[0];
                sy += (double)rg[1];
                sz += (double)rg[2];
@@ -720,129 +470,51 @@ k_force_tc(const int4 *__restrict__ item, const float4 *__restrict__ coef, int n
    }
 }
 
-int ks_force_tc_splits(int) { return FTC_SPLITS; }
-
-// Both z tables, cos and sin of 2 pi t u_z for t = 0..63, split into three
-// bf16 terms:
-//   ztab, the structure factor's B operand per 32-site stage (np sites, a
-//     multiple of TC_KS): [term][column group (8 sites)][row group][8 rows]
-//     [8 sites], rows 0..63 the cosines and 64..127 the sines;
-//   zsite, the force pass's A operand per 128-site tile: [term][column group
-//     16][row group 16][8 rows (sites)][8 t], column groups 0..7 the
-//     cosines, 8..15 the sines.
-// A block of 256 threads takes 32 sites (one stage, a quarter of a tile).
-// Each thread computes the values of one site and 8 t (each value once),
-// writes them to zsite and to shared memory, from where the block writes
-// ztab.  Also zeroes the site records past n (padding sites have no
-// charge).
-__global__ void __launch_bounds__(256) k_ztabs_tc(int n, int np, int4 *__restrict__ ph, uint4 *__restrict__ ztab,
-                                                  uint4 *__restrict__ zsite)
+// The force pass of one t-block (its units fu0 .. fu0 + npos - 1 of the
+// list, a multiple of four) into slots 0 and 1 of fpart; returns the
+// launches, -1 if out of memory.
+static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int blk, int fu0, int npos, int nsm,
+                          const double *chg, const int *slots, double *fpart, int *err)
 {
-   __shared__ float sv[32][129];   // [site][t: cosines, then sines] (padded row)
-   const int tid = threadIdx.x, sl = tid >> 3, tg = tid & 7;
-   const int i = blockIdx.x * 32 + sl;   // site (the grid covers the 128-site tiles)
-   const unsigned int uz = i < n ? (unsigned int)ph[i].z : 0u;
-   float c[8], sn[8];
-#pragma unroll
-   for (int e = 0; e < 8; e++) sincos_rev32((unsigned int)(8 * tg + e) * uz, &sn[e], &c[e]);
-   unsigned int h[4], m[4], l[4];
-   const int tile = i >> 7, r = i & 127;
-   const size_t zb = (size_t)tile * (FTC_ABYTES / 16) + (r >> 3) * 8 + (r & 7);
-#pragma unroll
-   for (int j = 0; j < 4; j++) tc::split3(c[2 * j], c[2 * j + 1], h[j], m[j], l[j]);
-   zsite[zb + tg * 128] = make_uint4(h[0], h[1], h[2], h[3]);
-   zsite[zb + tg * 128 + FTC_ATERM / 16] = make_uint4(m[0], m[1], m[2], m[3]);
-   zsite[zb + tg * 128 + 2 * FTC_ATERM / 16] = make_uint4(l[0], l[1], l[2], l[3]);
-#pragma unroll
-   for (int j = 0; j < 4; j++) tc::split3(sn[2 * j], sn[2 * j + 1], h[j], m[j], l[j]);
-   zsite[zb + (8 + tg) * 128] = make_uint4(h[0], h[1], h[2], h[3]);
-   zsite[zb + (8 + tg) * 128 + FTC_ATERM / 16] = make_uint4(m[0], m[1], m[2], m[3]);
-   zsite[zb + (8 + tg) * 128 + 2 * FTC_ATERM / 16] = make_uint4(l[0], l[1], l[2], l[3]);
-#pragma unroll
-   for (int e = 0; e < 8; e++) {
-      sv[sl][8 * tg + e] = c[e];
-      sv[sl][64 + 8 * tg + e] = sn[e];
-   }
-   if (i >= n && i < np) ph[i] = make_int4(0, 0, 0, 0);
-   __syncthreads();
-   // B operand of the stage: (8 sites q8, row) per thread, two each
-   const int stage = blockIdx.x;
-   if (stage * TC_KS >= np) return;   // past the structure factor's padded sites (uniform)
-#pragma unroll
-   for (int k = 0; k < 2; k++) {
-      const int id = tid + 256 * k, q8 = id >> 7, row = id & 127;
-      float v[8];
-#pragma unroll
-      for (int e = 0; e < 8; e++) v[e] = sv[8 * q8 + e][row];
-#pragma unroll
-      for (int j = 0; j < 4; j++) tc::split3(v[2 * j], v[2 * j + 1], h[j], m[j], l[j]);
-      const size_t base = (size_t)stage * (TC_BBYTES / 16) + q8 * (TC_LBO / 16) + (row >> 3) * 8 + (row & 7);
-      ztab[base] = make_uint4(h[0], h[1], h[2], h[3]);
-      ztab[base + TC_TERM / 16] = make_uint4(m[0], m[1], m[2], m[3]);
-      ztab[base + 2 * TC_TERM / 16] = make_uint4(l[0], l[1], l[2], l[3]);
-   }
-}
-
-// Host side.  Per-site operand tables (after k_prep): the z tables as the
-// structure factor's B operand and as the force pass's A operand.
-void ks_tables_tc(cudaStream_t st, int nsites, const KsDev &d)
-{
-   const int np = (nsites + TC_KS - 1) / TC_KS * TC_KS;
-   const int np128 = (nsites + 127) / 128 * 128;
-   k_ztabs_tc<<<np128 / 32, 256, 0, st>>>(nsites, np, d.ph32.p, d.ztab.p, d.zsite.p);
-}
-
-// The force pass's coefficient rows (after the per-k reduction).
-void ks_coef_tc(cudaStream_t st, const KsDev &d, int nitems_padded, float dkz)
-{
-   k_utab_tc<<<(nitems_padded + 7) / 8, 256, 0, st>>>(nitems_padded, d.tc_item.p, d.tc_k0.p, d.tc_kxy.p,
-                                                      d.kdat32.p, dkz, d.utab.p, d.tc_coef.p);
-}
-
-int ks_force_tc(cudaStream_t st, int nsites, KsDev &d, int nitems_padded, int nsm, const double *chg,
-                const int *slots, double *fpart, int *err)
-{
-   const int T = (nsites + 127) / 128, ntl = nitems_padded / FTC_NI;
+   const int T = (nsites + 127) / 128, ntl = npos * 8 / FTC_NI, t0 = 64 * blk;
    const int G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
-   int launches = 1;
-   if (d.tc_rkey[0] != T || d.tc_rkey[1] != ntl || d.tc_rkey[2] != G || d.tc_rver != d.tc_ver) {
+   const int4 *fu = d.q_fu.p + fu0;
+   k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, fu, reinterpret_cast<const float4 *>(d.q_ab32.p), d.utab.p,
+                                   d.tc_coef.p);
+   int launches = 2;
+   if (blk > 0 || d.tc_rkey[0] != T || d.tc_rkey[1] != ntl || d.tc_rkey[2] != G || d.tc_rver != d.tc_ver) {
       if (d.tc_ustart.ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
-      k_ftc_ranges<<<1, 256, 0, st>>>(d.tc_item.p, ntl, T, G, d.tc_ustart.p);
+      k_ftc_ranges<<<1, 256, 0, st>>>(fu, t0, ntl, T, G, d.tc_ustart.p);
       d.tc_rkey[0] = T;
       d.tc_rkey[1] = ntl;
       d.tc_rkey[2] = G;
-      d.tc_rver = d.tc_ver;
+      d.tc_rver = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
       launches++;
    }
-   k_force_tc<<<G, FTC_THREADS, FTC_SMEM, st>>>(d.tc_item.p, d.tc_coef.p, nitems_padded, d.ph32.p, d.zsite.p,
+   k_force_tc<<<G, FTC_THREADS, FTC_SMEM, st>>>(g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p, d.q_y32.p, d.zsite.p,
                                                 d.utab.p, chg, slots, nsites, d.tc_ustart.p, fpart, err);
    return launches;
 }
 
-size_t ks_tc_zsite_len(int nsites)
+int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int nsm, const double *chg, const int *slots,
+                double *fpart, int *err)
 {
-   return (size_t)((nsites + 127) / 128) * (FTC_ABYTES / 16);
+   int launches = 0;
+   for (int b = 0; b < d.q_nfblk; b++) {
+      const int nl = force_tc_block(st, nsites, g, d, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm, chg, slots,
+                                    fpart + (size_t)b * FTC_SPLITS * 3 * nsites, err);
+      if (nl < 0) return -1;
+      launches += nl;
+   }
+   return launches;
 }
 
-size_t ks_tc_utab_len(int nitems_padded)
-{
-   return (size_t)(nitems_padded / FTC_NI) * 8 * (FTC_BBYTES / 16);
-}
+int ks_force_tc_splits(const KsDev &d) { return FTC_SPLITS * d.q_nfblk; }
+size_t ks_tc_utab_len(int npos) { return (size_t)((npos + 3) / 4) * 8 * (FTC_BBYTES / 16); }
 
-// Shared-memory sizes of the tensor-core kernels, set once per device
-// outside any stream capture (from ks_prepare).
-// (contexts may be created from several host threads: the per-device flags
-// are atomic, and setting the attribute twice is harmless)
-cudaError_t ks_tc_init(int device)
+cudaError_t ks_force_tc_init()
 {
-   static std::atomic<unsigned long long> done{0};
-   const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
-   if (bit && (done.load() & bit)) return cudaSuccess;
-   cudaError_t e = cudaFuncSetAttribute(k_sfac_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM);
-   if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_force_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, FTC_SMEM);
-   if (e == cudaSuccess && bit) done.fetch_or(bit);
-   return e;
+   return cudaFuncSetAttribute(k_force_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, FTC_SMEM);
 }
 
 }  // namespace mdgpu

@@ -14,7 +14,7 @@ namespace mdgpu {
 
 constexpr int NPOTP = 8;          // parameters per potential (src/defs.h:144)
 constexpr int KI = 16;            // k-vectors per k-space work item
-constexpr int KT = 64;            // k-vectors per tensor-core structure-factor item (4 KI runs)
+constexpr int KT = 64;            // k-vectors per item of mdgpu_tc_items (4 KI runs)
 constexpr int FT_THREADS = 128;   // k_force32: threads per block, two sites each
 constexpr double PI = 3.14159265358979323846;
 constexpr double ALPHAMIN = 1e-7; // src/defs.h:181
@@ -55,6 +55,45 @@ struct RsGeom {
 mdgpu_status build_rs_geom(const double *h, const mdgpu_control &ctl, RsGeom &g);
 mdgpu_status build_rdf_stencil(const double *h, double limit, int nx, int ny, int nz, std::vector<int4> &full);
 
+// ---- tensor-core reciprocal space: quads (kspace_q.cu) --------------------
+constexpr double Q_KAPPA = 255.0 / 256.0;   // scale of every table value: no top digit overflows
+// Geometry of one k-list's tables.
+struct QGeom {
+   int hrows, mrows;       // X and Y values per site: h = 0 .. hrows - 1, m = 0 .. mrows - 1 (a multiple of 4)
+   int TP;                 // t values (columns 2 TP: per 8 t, 8 cosines and 8 sines)
+   int TW, nblk;           // t-blocks: width, count (the last one may be narrower)
+   int nquads;             // 4 x units
+   double b[9];            // 2 pi h^-1, row-major
+};
+// Row tile of a t-block: its units (four quads (h, m0 .. m0 + 3) each, -1
+// padding) and the table ranges it reads.
+constexpr int Q_XMAX = 8, Q_YMAX = 24;   // h and m values a row tile may span
+struct QTile {
+   int col0, nT;                 // first column of its t-block, columns
+   int xlo, nx, ylo, ny;         // h and m values spanned
+   int unit[16];
+};
+// Eight units of one t-block (the K-rows between two read-backs of the FP64
+// force pass), and a run of segments.
+struct QSeg {
+   int blk;
+   int unit[8];
+};
+struct QItem {
+   int seg0, seg1;
+};
+struct QList {
+   int ns = 0;                     // digits it was built for (3 mixed, 7 FP64)
+   QGeom g{};
+   std::vector<int4> units;        // (h, m0, t range, 0)
+   std::vector<double2> coeff;     // [quad][TP][s][r]: src/ewald.c:510-511 (0: no such k-vector)
+   std::vector<QTile> tiles;       // structure factor
+   std::vector<QSeg> segs;         // FP64 force pass
+   std::vector<int> seg0;          // first segment of each t-block, and the end
+   std::vector<int4> fu;           // mixed force pass: (h, m0, t range, unit), per 64-wide t-block
+   std::vector<int> fblk;          // first entry of each of its t-blocks, and the end
+};
+
 // ---- host-side k-vector list ---------------------------------------------
 struct KList {
    int hmax = 0, kmax = 0, lmax = 0, nk = 0, nitems = 0;
@@ -67,15 +106,14 @@ struct KList {
    double key[12];                 // h, k_cutoff, alpha
    double vol = 0;
    double hinv[9];
-   // tensor-core structure factor: runs of up to KT l values of a column,
-   // largest count first, padded with empty runs to a multiple of 128
-   std::vector<int4> tc_item;      // (h, k, l0, count)
-   std::vector<int4> tc_k0;        // first k index of each KI run of the item (-1 past its end)
-   std::vector<float2> tc_kxy;     // (kx, ky) of the item's column
-   int tc_nitems = 0;              // before padding
+   QList q;
 };
 
 mdgpu_status build_klist(const double *h, const mdgpu_control &ctl, KList &kl);
+// Quads of the list for ns digits (kl.q).
+void build_qlist(KList &kl, int ns);
+// Runs of up to KT l values of one (h, k) column (mdgpu_tc_items).
+void build_tc_items(const KList &kl, std::vector<int4> &item, std::vector<int4> &k0);
 
 // ---- first-call constants (host, FP64, reference arithmetic) -------------
 double host_poteval(const double *potpar, double r, int ptype, double chgsq, double alpha);
@@ -201,16 +239,30 @@ struct KsDev {
    // charged sites only (a site without charge adds nothing to S(k) and
    // gets no k-space force): their slots in link-cell order
    DBuf<int> kslots, kscan, kbsum;
-   // tensor-core structure factor: its items and the per-site z tables as
-   // split bf16 MMA operands (kspace_tc.cu)
-   DBuf<int4> tc_item, tc_k0;
-   DBuf<float2> tc_kxy;
-   DBuf<uint4> ztab;       // structure factor: z tables as the B operand, per 16 sites
+   // tensor-core passes (kspace_q.cu, kspace_tc.cu): the quad list; the
+   // per-site tables (X, Y fixed point; z digits as the structure factor's B
+   // operand; z as the mixed force pass's A operand or in FP64); the
+   // structure-factor partials; per (quad, t) A and B; the force passes'
+   // coefficient operands
+   DBuf<int4> q_units, q_fu;
+   DBuf<double2> q_coeff;
+   DBuf<QTile> q_tiles;
+   DBuf<QSeg> q_segs;
+   DBuf<QItem> q_items;
+   DBuf<int> q_x32, q_y32, q_bexp;
+   DBuf<long long> q_x64, q_y64;
+   DBuf<unsigned char> q_ztab, q_bq;
+   DBuf<double> q_zd, q_part, q_ab64;
+   DBuf<float> q_ab32;
+   int q_nfblk = 0;                 // mixed force pass: t-blocks and their entries of q_fu
+   std::vector<int> q_fblk;
+   int q_items_for[3] = {-1, -1, -1};   // (site tiles, list upload, SMs) of q_items
+   int q_nitems = 0;
    DBuf<uint4> zsite;      // force pass: z tables as the A operand, per 128 sites
    DBuf<uint4> utab;       // force pass: per-item coefficient rows (B operand)
    DBuf<float4> tc_coef;   // per item: kx s1, ky s1, kz0 s1, dkz s2 (row scales s)
    DBuf<int> tc_ustart;    // force pass: the CTAs' work ranges (k_ftc_ranges)
-   long long tc_ver = 0;   // uploads of tc_item so far
+   long long tc_ver = 0;   // uploads of the quad list so far
    int tc_rkey[3] = {-1, -1, -1};   // (site tiles, item tiles, CTAs) of tc_ustart
    long long tc_rver = -1;          // tc_ver of tc_ustart
 };
@@ -349,8 +401,8 @@ struct mdgpu_ctx {
    // the k-space passes run over every site, not only the charged ones
    // (the adjoint's backward passes read every site's phases)
    bool ks_all_sites = false;
-   // mixed form: structure factor on the tensor cores (MDGPU_KSPACE_TC=0
-   // at context creation selects the CUDA-core pass)
+   // reciprocal space on the tensor cores (MDGPU_KSPACE_TC=0 at context
+   // creation selects the CUDA-core passes)
    bool tc_sfac = true;
    uint64_t ncharged_gen = 0;       // configuration the count below is for
    int ncharged = 0;                // sites with a nonzero charge
@@ -412,25 +464,23 @@ struct KsShape {
 // Chunks of the structure-factor pass and k-splits of a per-site pass
 // (ipt items per thread, spt sites per thread).
 KsShape ks_shape(int N, int nitems, int ipt, int spt);
-// Reciprocal-space passes on the tensor cores (kspace_tc.cu), mixed form:
-// per-site operand tables (after k_prep); the structure factor into part32
-// ([chunks][nk], returns the number of chunks); the force pass's per-item
-// coefficient rows (after the per-k reduction); the force pass, F_slot * q
-// into fpart[split][3][nsites] (returns the number of splits).
-void ks_tables_tc(cudaStream_t st, int nsites, const KsDev &d);
-int ks_sfac_tc(cudaStream_t st, int nsites, int nk, const KsDev &d, int ntiles, double qmax, int *err);
-void ks_coef_tc(cudaStream_t st, const KsDev &d, int nitems_padded, float dkz);
-int ks_force_tc(cudaStream_t st, int nsites, KsDev &d, int nitems_padded, int nsm, const double *chg,
-                const int *slots, double *fpart, int *err);
-int ks_force_tc_splits(int nsites);
-cudaError_t ks_tc_init(int device);
-size_t ks_tc_ztab_len(int nsites);
-int ks_tc_chunks(int nsites);
-size_t ks_tc_zsite_len(int nsites);
-size_t ks_tc_utab_len(int nitems_padded);
-cudaError_t ks_tc_init(int device);
-size_t ks_tc_ztab_len(int nsites);
-int ks_tc_chunks(int nsites);
+// Reciprocal-space passes on the tensor cores.  kspace_q.cu: both forms'
+// tables, structure factor and per-k sums (A and B per (quad, t), the
+// blocks' energy/stress records into d.blk; returns their number, -1 if out
+// of memory), and the FP64 form's force pass (adds the forces after join,
+// if any).  kspace_tc.cu: the mixed form's force pass, F_slot into
+// fpart[split][3][nsites] (returns the launches, -1 if out of memory).
+mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns);
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site);
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges);
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges, int *nblocks);
+mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots);
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force);
+int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int nsm, const double *chg, const int *slots,
+                double *fpart, int *err);
+int ks_force_tc_splits(const KsDev &d);
+size_t ks_tc_utab_len(int npos);
+cudaError_t ks_force_tc_init();
 // api.cu
 mdgpu_status fail(mdgpu_ctx *c, mdgpu_status s, const std::string &msg);
 mdgpu_status cuda_check(mdgpu_ctx *c, cudaError_t e, const char *what);

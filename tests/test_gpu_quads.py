@@ -1,0 +1,65 @@
+"""The tensor-core reciprocal space of both forms (products of per-axis trig
+tables, kspace_q.cu, and the mixed force pass, kspace_tc.cu) against the
+CUDA-core passes at the sizes where its tiling can go wrong: charged-site
+counts around the 32-site stages and 128-site tiles, |l| ranges around the
+column blocks (8, 16, 32, 40, 64), row tiles that span several blocks of h,
+triclinic cells (|l| not symmetric about a column's middle) and net charge.
+
+Tolerances.  FP64: both paths are FP64-accurate sums (operands to 2^-55, the
+CUDA-core recurrence a few 2^-53 per term), held to the parity tests' 1e-12
+of the RMS force.  Mixed: 1e-5 of the FP64 result, the form's bound."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def ions(n, box, kc, tilt=0.0, seed=1, net=False):
+    from moldy_gb300 import system as S
+    rng = np.random.default_rng(seed)
+    h = np.diag(np.asarray(box, float))
+    h[0, 1], h[0, 2], h[1, 2] = tilt * box[1], 0.7 * tilt * box[2], -tilt * box[2]
+    x = h @ rng.uniform(-0.499, 0.499, (3, n))
+    half = n // 2
+    species = [S.Species("A", half, np.array([1], np.int32), np.zeros((1, 3))),
+               S.Species("B", n - half, np.array([2], np.int32), np.zeros((1, 3)))]
+    species = [s for s in species if s.nmols]
+    q = np.array([0.0, 1.0, 0.7 if net else -1.0]) / S.CONV_Q
+    return S.System(h=h, species=species, ptype=S.LJPOT, potpar=np.zeros((9, 8)), site_charge=q, site=x,
+                    c_of_m=(np.linalg.inv(h) @ x).T, control=S.Control(cutoff=3.0, alpha=0.45, k_cutoff=kc))
+
+
+def lbox(trange, kc):
+    return 2 * math.pi * (trange - 0.5) / kc
+
+
+CASES = [dict(n=n, box=(9, 9, 9), kc=4.0) for n in (1, 2, 31, 32, 33, 127, 128, 129, 1025, 4097)]
+CASES += [dict(n=65, box=(7, 8, lbox(t, 3.0)), kc=3.0) for t in (3, 8, 9, 16, 17, 32, 33, 40, 41, 64, 65, 81, 130)]
+CASES += [dict(n=200, box=(lbox(t, 3.0), 7, 8), kc=3.0) for t in (33, 70)]
+CASES += [dict(n=200, box=(7, lbox(t, 3.0), 8), kc=3.0) for t in (33, 70)]
+CASES += [dict(n=300, box=(20, 22, 24), kc=3.0, tilt=t, net=net) for t in (0.1, -0.25) for net in (False, True)]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "-".join(
+    str(round(v, 1) if isinstance(v, float) else v) for v in c.values()).replace(" ", ""))
+def test_matches_cuda_core_passes(case, monkeypatch):
+    from moldy_gb300 import ForceField
+    sysm = ions(**case)
+    res = {}
+    for form in ("fp64", "mixed"):
+        for tc in ("1", "0"):
+            monkeypatch.setenv("MDGPU_KSPACE_TC", tc)
+            ff = ForceField(sysm, precision=form)
+            res[form, tc] = ff.ewald()
+            self_e = abs(ff.info()["self_energy"])
+            ff.close()
+    f0, e0, s0 = res["fp64", "0"]
+    # a single site feels no net force: the terms' own size is the scale
+    scale = max(np.sqrt((f0 ** 2).mean()), 1e-3 * self_e / sysm.nsites)
+    for form, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+        f, e, s = res[form, "1"]
+        assert np.sqrt(((f - f0) ** 2).mean()) <= tol * scale, form
+        assert abs(e - e0) <= tol * (abs(e0) + self_e), form
+        assert np.abs(s - s0).max() <= tol * (np.abs(s0).max() + self_e), form
