@@ -235,13 +235,21 @@ k_adj_kreduce(int nk, int nchunks, int loss, int fw, const float2 *__restrict__ 
    }
 }
 
-__global__ void k_adj_kfinal(const double *__restrict__ blk, int nblocks, double *__restrict__ scal)
+// scal[1 + t] = sum of the block records' component t, in a fixed order
+__global__ void __launch_bounds__(256) k_adj_kfinal(const double *__restrict__ blk, int nblocks, double *__restrict__ scal)
 {
-   const int t = threadIdx.x;
-   if (t >= 2 || blockIdx.x != 0) return;
-   double s = 0.0;
-   for (int b = 0; b < nblocks; b++) s += blk[2 * b + t];
-   scal[1 + t] = s;
+   __shared__ double sh[256];
+   double e = 0.0, l = 0.0;
+   for (int b = threadIdx.x; b < nblocks; b += 256) {
+      e += blk[2 * b];
+      l += blk[2 * b + 1];
+   }
+   e = block_sum256(e, sh);
+   l = block_sum256(l, sh);
+   if (threadIdx.x == 0) {
+      scal[1] = e;
+      scal[2] = l;
+   }
 }
 
 constexpr int AD_ITEMS = 64;     // k-vector items per shared-memory tile
@@ -438,6 +446,15 @@ static mdgpu_status ks_adjoint(mdgpu_ctx *c, bool loss)
       CK(cudaMemsetAsync(a.scal.p + 1, 0, 2 * sizeof(double), st));
       return MDGPU_OK;
    }
+   if (c->tc_sfac && !fw) {
+      int nb = 0;
+      const mdgpu_status s = ks_q_adjoint(c, loss, c->rd.sorted.p, a.gq.p + (loss ? N : 0), &nb);
+      if (s != MDGPU_OK) return s;
+      k_adj_kfinal<<<1, 256, 0, st>>>(a.blk.p, nb, a.scal.p);
+      CK(cudaGetLastError());
+      c->launches += 1;
+      return MDGPU_OK;
+   }
    // the forward's structure-factor chunks (its partial sums are reused)
    const KsShape sh = ks_shape(N, ni, 1, 1);
    const size_t plane = (size_t)sh.chunks * nk;
@@ -488,7 +505,7 @@ static mdgpu_status ks_adjoint(mdgpu_ctx *c, bool loss)
                                                 d.kz64.p, d.coeff.p, c->ctl.alpha, nullptr, nullptr, nullptr,
                                                 a.kadj64.p, a.kadjf64.p, a.blk.p);
    }
-   k_adj_kfinal<<<1, 32, 0, st>>>(a.blk.p, nbk, a.scal.p);
+   k_adj_kfinal<<<1, 256, 0, st>>>(a.blk.p, nbk, a.scal.p);
    CK(a.gkpart.ensure((size_t)sh.splits * 2 * N));
    const dim3 gs((N + AD_THREADS - 1) / AD_THREADS, sh.splits);
    if (mixed)

@@ -431,15 +431,11 @@ void build_qlist(KList &kl, int ns)
    g.hrows = hm + 1;
    g.mrows = 4 * M4;
    const int T = lm + 1;
-   if (ns == 3) {   // t-blocks of up to 40 (80 columns), equally wide
-      g.nblk = (T + 39) / 40;
-      g.TW = ((T + g.nblk - 1) / g.nblk + 7) / 8 * 8;
-      g.TP = g.TW * g.nblk;
-   } else {         // 32 wide, the last one 16 or 32
-      g.nblk = (T + 31) / 32;
-      g.TW = 32;
-      g.TP = 32 * (g.nblk - 1) + (T - 32 * (g.nblk - 1) <= 16 ? 16 : 32);
-   }
+   // t-blocks 32 wide, the last one a multiple of 8 (mixed), 16 or 32 (FP64)
+   const int gr = ns == 3 ? 8 : 16;
+   g.TW = 32;
+   g.nblk = (T + 31) / 32;
+   g.TP = 32 * (g.nblk - 1) + (T - 32 * (g.nblk - 1) + gr - 1) / gr * gr;
    for (int k = 0; k < 9; k++) g.b[k] = 2 * PI * kl.hinv[k];
    std::vector<int> uid((size_t)(hm + 1) * M4, -1);
    for (int hb = 0; hb <= hm; hb += 4)

@@ -832,16 +832,18 @@ __global__ void k_fsum(int n3, int nsplit, const double *__restrict__ fpart, dou
 }
 
 // force[comp][slots[j]] += sum over splits of fpart[split][comp][j], j < n
-// (partials by slot of the charged-site list; the other sites get nothing)
+// (partials by slot of the charged-site list; the other sites get nothing),
+// times the site's charge when chg is given
 __global__ void k_fsum_slots(int n, int N, int nsplit, const double *__restrict__ fpart,
-                             const int *__restrict__ slots, double *__restrict__ force)
+                             const int *__restrict__ slots, const double *__restrict__ chg, double *__restrict__ force)
 {
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= 3 * n) return;
    const int comp = i / n, j = i - comp * n;
    double s = 0.0;
    for (int k = 0; k < nsplit; k++) s += fpart[(size_t)k * 3 * n + i];
-   force[(size_t)comp * N + slots[j]] += s;
+   const int si = slots[j];
+   force[(size_t)comp * N + si] += chg ? chg[si] * s : s;
 }
 
 // Compaction of the link-cell order to the charged sites: per block of
@@ -1018,11 +1020,13 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    // The passes run over the charged sites only (a site without charge adds
    // nothing to S(k) and has no k-space force; rigid water's O sites are a
    // quarter of the work), kept in link-cell order -- except with a
-   // framework molecule and under the adjoint, which read every site.
+   // framework molecule and under the adjoint, which need every site.
    const bool compact = nf <= 0 && !c->ks_all_sites;
+   // both passes on the tensor cores, but with a framework molecule
+   const bool tc = nf <= 0 && c->tc_sfac;
    int Nk = N;
    const int *slots = c->rd.sorted.p;
-   if (compact) {
+   if (compact || tc) {
       if (c->ncharged_gen != c->gen) {
          int n = 0;
          double qm = 0;
@@ -1034,6 +1038,8 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
          c->qmax = qm;
          c->ncharged_gen = c->gen;
       }
+   }
+   if (compact) {
       Nk = c->ncharged;
       if (Nk == 0) {
          if (join) CK(cudaStreamWaitEvent(st, join, 0));
@@ -1052,8 +1058,6 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       c->launches += 3;
       slots = d.kslots.p;
    }
-   // over the charged sites: both passes on the tensor cores
-   const bool tc = compact && c->tc_sfac;
    const int ns = mixed ? 3 : 7;
    mdgpu_status s;
    if (!tc && (s = ks_upload_list(c)) != MDGPU_OK) return s;
@@ -1152,7 +1156,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    dim3 gf((Nk + 255) / 256, sh.splits);
    const int obase = compact ? -1 : 0;   // partial rows by slot of the charged list, or by site
    if (tc && mixed) {
-      const int nl = ks_force_tc(st, Nk, kl.q.g, d, c->nsm, c->rd.chg.p, slots, d.fpart.p, &out->err);
+      const int nl = ks_force_tc(st, Nk, kl.q.g, d, d.q_ab32.p, false, c->nsm, d.fpart.p, &out->err);
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl - 1;
    } else if (tc) {
@@ -1168,12 +1172,12 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    CK(cudaGetLastError());
    phase_mark(c, MDGPU_PH_FINAL);
    if (join) CK(cudaStreamWaitEvent(st, join, 0));
-   if (compact) {
+   if (compact || tc) {
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
       if (tc && !mixed) {
          if ((s = ks_q_fsum64(c, Nk, slots, d_force)) != MDGPU_OK) return s;
       } else
-      k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots, d_force);
+      k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots, tc ? c->rd.chg.p : nullptr, d_force);
    } else {
       k_fsum<<<(3 * N + 255) / 256, 256, 0, st>>>(3 * N, sh.splits, d.fpart.p, d_force, accumulate ? 1 : 0);
    }

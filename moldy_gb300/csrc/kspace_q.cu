@@ -35,7 +35,7 @@
 // Measured, 131,072-site water (98,304 charged sites, 69,876 k-vectors),
 // against one FP64 recurrence per k and site, or the seed-and-run bf16
 // products of the mixed form: FP64 structure factor 119.4 -> 1.41 ms, forces
-// 130.4 -> 4.86 ms; mixed structure factor 0.414 -> 0.299 ms.  Force error
+// 130.4 -> 4.86 ms; mixed structure factor 0.414 -> 0.274 ms.  Force error
 // of the FP64 form against extended precision (2048-site water; rock salt,
 // 5832 ions): 6.1e-15 -> 2.2e-15; 1.5e-14 -> 1.1e-14.
 #include <algorithm>
@@ -61,7 +61,7 @@ template <> struct QCfg<3> {
    static constexpr int RS = 36;                  // table row: 32 sites, padded against bank conflicts
    static constexpr int MT = 2, NPART = 1;        // 128-row tiles per CTA, column parts of B
    static constexpr int NB = 3;                   // stages in flight
-   static constexpr int NTMAX = 80;               // columns (2 t-width) of a t-block
+   static constexpr int NTMAX = 64;               // columns (2 t-width) of a t-block
    static constexpr int SEG = 32;                 // stages between read-backs
 };
 template <> struct QCfg<7> {
@@ -74,12 +74,13 @@ template <> struct QCfg<7> {
 };
 // bytes: a stage's table rows, its B operand, both; the A operand; all
 template <int NS> constexpr int Q_TAB = 2 * (Q_XMAX + Q_YMAX) * QCfg<NS>::RS * (int)sizeof(typename QCfg<NS>::T);
-template <int NS> constexpr int Q_B = QCfg<NS>::NTMAX * Q_KS * 2 * NS;
-template <int NS> constexpr int Q_STAGE = Q_B<NS> + Q_TAB<NS>;
+// (ND: digits of operand B, NS unless weights of a wide range need more)
+template <int ND> constexpr int Q_B = 64 * Q_KS * 2 * ND;
+template <int NS, int ND> constexpr int Q_STAGE = Q_B<ND> + Q_TAB<NS>;
 template <int NS> constexpr int Q_A = QCfg<NS>::MT * NS * Q_OP;
-template <int NS> constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_STAGE<NS>;
-static_assert(Q_SMEM<3> <= 227 * 1024 && Q_SMEM<7> <= 227 * 1024, "one CTA's shared memory");
-static_assert(Q_STAGE<3> % 128 == 0 && Q_STAGE<7> % 128 == 0, "stage buffers stay aligned");
+template <int NS, int ND> constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_STAGE<NS, ND>;
+static_assert(Q_SMEM<3, 4> <= 227 * 1024 && Q_SMEM<7, 7> <= 227 * 1024, "one CTA's shared memory");
+static_assert(Q_STAGE<3, 3> % 128 == 0 && Q_STAGE<3, 4> % 128 == 0 && Q_STAGE<7, 7> % 128 == 0, "stage buffers stay aligned");
 
 // ------------------------------------------------------ fixed-point trig
 // sin, cos(2 pi p / 2^64) in units of 2^-63: the phase is reduced to an
@@ -401,7 +402,7 @@ __device__ __forceinline__ void q_init(QBars &B)
 // SEG: NS = 3, issuer p takes 128-row tile p; NS = 7, column part p.
 // Operand stages: A [tile][digit][row group 16][kg 4][8 rows][16 B], B
 // [part][digit][col group][kg 4][8][16 B].
-template <int NS>
+template <int NS, int ND>
 __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned char *Bbuf, unsigned int tmem, int p,
                                         int nst, int nT, int *abort_s, int *err, int errbit)
 {
@@ -409,7 +410,7 @@ __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned 
    constexpr int SEG = QCfg<NS>::SEG, NB = QCfg<NS>::NB;
    const int pc = nT / QCfg<NS>::NPART;
    const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NS * Q_OP : 0);
-   const unsigned int b0 = saddr(Bbuf) + (QCfg<NS>::NPART == 2 ? p * NS * pc * Q_KS * 2 : 0);
+   const unsigned int b0 = saddr(Bbuf) + (QCfg<NS>::NPART == 2 ? p * ND * pc * Q_KS * 2 : 0);
    const unsigned int d0 = tmem + 256u * p;
    for (int st = 0; st < nst; st++) {
       const int sa = st & 1, sb = st % NB, seg = st / SEG;
@@ -425,7 +426,7 @@ __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned 
 #pragma unroll
          for (int i = 0; i < NS; i++)
             mma_f16(d0 + i * pc, sdesc(a0 + sa * Q_A<NS> + i * Q_OP + ks * 256, 128, 512),
-                    sdesc(b0 + sb * Q_STAGE<NS> + ks * 256, 128, 512), idesc_f16(128, (NS - i) * pc, false),
+                    sdesc(b0 + sb * Q_STAGE<NS, ND> + ks * 256, 128, 512), idesc_f16(128, (ND - i) * pc, false),
                     st % SEG != 0 || ks > 0 || i > 0);
       mma_commit(&B.empty_a[sa]);
       mma_commit(&B.empty_b[sb]);
@@ -495,11 +496,12 @@ __device__ __forceinline__ double q_value(const Q96 &v)
 }
 
 // ----------------------------------------------------- structure factor
-// Grid: (row tiles, site ranges).  part[range][quad row 4 quad + p][2 TP].
-template <int NS>
+// Grid: (row tiles, site ranges, channels).  part[channel][range][quad row 4
+// quad + p][2 TP]; channel c reads its own digits, zstride further on each.
+template <int NS, int ND>
 __global__ void __launch_bounds__(Q_THREADS, 1)
 k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4 *__restrict__ units, const unsigned char *__restrict__ X,
-         const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, int nstages, int per,
+         const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, size_t zstride, int nstages, int per,
          double *__restrict__ part, int *__restrict__ err)
 {
    using namespace tc;
@@ -528,7 +530,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
    if (w == Q_BW) {
       // ---- bulk copies: a stage's digits of q z and the tile's table rows
       if (lane == 0) {
-         const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * NS);
+         const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * ND);
          const unsigned int xb = (unsigned int)(2 * ti.nx * RS * sizeof(T)), yb = (unsigned int)(2 * ti.ny * RS * sizeof(T));
          int issued = 0;
          for (int st = 0; st < nst; st++) {
@@ -537,12 +539,12 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
                q_abort(&abort_s, err, Q_ERR);
                break;
             }
-            unsigned char *d = Sbuf + s * Q_STAGE<NS>;
+            unsigned char *d = Sbuf + s * Q_STAGE<NS, ND>;
             const size_t sg = (size_t)(st0 + st);
             bar_expect_tx(&B.full_b[s], bb + xb + yb);
-            bulk_load(d, ztab + (sg * 2 * g.TP + ti.col0) * Q_KS * 2 * NS, bb, &B.full_b[s]);
-            bulk_load(d + Q_B<NS>, X + (sg * g.hrows + ti.xlo) * 2 * RS * sizeof(T), xb, &B.full_b[s]);
-            bulk_load(d + Q_B<NS> + 2 * Q_XMAX * RS * sizeof(T), Y + (sg * g.mrows + ti.ylo) * 2 * RS * sizeof(T), yb,
+            bulk_load(d, ztab + blockIdx.z * zstride + (sg * 2 * g.TP + ti.col0) * Q_KS * 2 * ND, bb, &B.full_b[s]);
+            bulk_load(d + Q_B<ND>, X + (sg * g.hrows + ti.xlo) * 2 * RS * sizeof(T), xb, &B.full_b[s]);
+            bulk_load(d + Q_B<ND> + 2 * Q_XMAX * RS * sizeof(T), Y + (sg * g.mrows + ti.ylo) * 2 * RS * sizeof(T), yb,
                       &B.full_b[s]);
             issued = st + 1;
          }
@@ -552,7 +554,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
+         q_issue<NS, ND>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
    } else {
       // ---- A operand: row 8 w + (lane & 7) of each 128-row tile (product
       // p of a quad), sites 8 kg .. 8 kg + 7 of the stage
@@ -596,18 +598,19 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
                if (4 * ch < ncw) {
                   const int lc = pl + 4 * ch;   // column of the block
                   const unsigned int col = MT == 2 ? 256u * mt + lc : 256u * (lc / pc) + lc % pc;
-                  float d[NS][4];
+                  float d[ND][4];
 #pragma unroll
-                  for (int k = 0; k < NS; k++) q_ld4(trow + col + k * pc, d[k]);
+                  for (int k = 0; k < ND; k++) q_ld4(trow + col + k * pc, d[k]);
                   q_ldwait(d);
 #pragma unroll
                   for (int e = 0; e < 4; e++) {
                      const int i = (mt * MAXC + ch) * 4 + e;
-                     if (NS == 3)
-                        af[NS == 3 ? i : 0] += fmaf(d[0][e], 65536.f, fmaf(d[1][e], 256.f, d[2][e]));
-                     else
-                        q_add(ai[NS == 7 ? i : 0], q_combine(d[0][e], d[1][e], d[2][e], d[NS > 3 ? 3 : 0][e], d[NS > 3 ? 4 : 0][e],
-                                                            d[NS > 3 ? 5 : 0][e], d[NS > 3 ? 6 : 0][e]));
+                     if (NS == 3) {
+                        const float lo = ND == 3 ? d[2][e] : fmaf(d[2][e], 256.f, d[ND - 1][e]);
+                        af[NS == 3 ? i : 0] += fmaf(d[0][e], ND == 3 ? 65536.f : 16777216.f, fmaf(d[1][e], ND == 3 ? 256.f : 65536.f, lo));
+                     } else
+                        q_add(ai[NS == 7 ? i : 0], q_combine(d[0][e], d[1][e], d[2][e], d[ND > 4 ? 3 : 0][e], d[ND > 4 ? 4 : 0][e],
+                                                            d[ND > 4 ? 5 : 0][e], d[ND > 4 ? 6 : 0][e]));
                   }
                }
          fence_before_sync();
@@ -625,7 +628,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
             live = false;
             break;
          }
-         const T *xs = reinterpret_cast<const T *>(Sbuf + sb * Q_STAGE<NS> + Q_B<NS>);
+         const T *xs = reinterpret_cast<const T *>(Sbuf + sb * Q_STAGE<NS, ND> + Q_B<ND>);
          const T *ys = xs + 2 * Q_XMAX * RS;
          unsigned char *A = Abuf + sa * Q_A<NS> + (r >> 3) * 512 + kg * 128 + (r & 7) * 16;
 #pragma unroll
@@ -656,7 +659,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
             const int row = 32 * (w & 3) + lane;
             const int u = ti.unit[8 * mt + (row >> 4)];
             if (u >= 0) {
-               double *dst = part + ((size_t)blockIdx.y * 4 * g.nquads + (size_t)u * 16 + (row & 15)) * 2 * g.TP + ti.col0 + pl;
+               double *dst = part + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * 4 * g.nquads + (size_t)u * 16 + (row & 15)) * 2 * g.TP + ti.col0 + pl;
 #pragma unroll
                for (int ch = 0; ch < MAXC; ch++)
                   if (4 * ch < ncw) {
@@ -774,7 +777,7 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
 // A segment is 8 units (128 quad rows) of one t-block, units in order of
 // rising |(h, m)| so that the coefficients of a segment, which share a
 // power-of-two scale, are of similar size.
-// Coefficients of quad (h, m) at t for one weight set: v[p] of P_p C_t and
+// Coefficients of quad (h, m) at t for one weight set (h, k, l, or 1): v[p] of P_p C_t and
 // v[4 + p] of P_p S_t.
 __device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m, int t, double (&v)[8])
 {
@@ -783,7 +786,7 @@ __device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m,
 #pragma unroll
    for (int x = 0; x < 4; x++) {
       const double s = x & 2 ? -1.0 : 1.0, r = x & 1 ? -1.0 : 1.0;
-      const double wt = set == 0 ? (double)h : set == 1 ? s * m : r * t;
+      const double wt = set == 0 ? (double)h : set == 1 ? s * m : set == 2 ? r * t : 1.0;
       const double A = wt * ab[2 * x], Bc = wt * ab[2 * x + 1];
       v[0] -= Bc;
       v[1] += s * Bc;
@@ -796,10 +799,10 @@ __device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m,
    }
 }
 
-// Grid: (segments, 3 sets).  The segment's B operand, [stage 4][part][digit]
+// Grid: (segments, sets from set0).  The segment's B operand, [stage 4][part][digit]
 // [col group][kg 4][8 cols][8 K], and its scale exponent.
 __global__ void __launch_bounds__(256)
-k_qcoef(QGeom g, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict__ units,
+k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict__ units,
         const double *__restrict__ ab, unsigned char *__restrict__ bq, int *__restrict__ bexp)
 {
    constexpr int NS = 7;
@@ -814,7 +817,7 @@ k_qcoef(QGeom g, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict
       const int4 un = units[u];
       if (t >= un.z) continue;
       double v[8];
-      q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set, un.x, un.y + (ql & 3), t, v);
+      q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set0 + set, un.x, un.y + (ql & 3), t, v);
 #pragma unroll
       for (int k = 0; k < 8; k++) mx = fmax(mx, fabs(v[k]));
    }
@@ -840,7 +843,7 @@ k_qcoef(QGeom g, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict
          double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
          if (u >= 0) {
             const int4 un = units[u];
-            if (t < un.z) q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set, un.x, un.y + (ql & 3), t, v);
+            if (t < un.z) q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set0 + set, un.x, un.y + (ql & 3), t, v);
          }
 #pragma unroll
          for (int k = 0; k < 4; k++) {
@@ -904,7 +907,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
                break;
             }
             bar_expect_tx(&B.full_b[s], bb);
-            bulk_load(Sbuf + s * Q_STAGE<NS>, src + (size_t)st * BST, bb, &B.full_b[s]);
+            bulk_load(Sbuf + s * Q_STAGE<NS, NS>, src + (size_t)st * BST, bb, &B.full_b[s]);
             issued = st + 1;
          }
          for (int st = issued > NB ? issued - NB : 0; st < issued; st++)
@@ -912,7 +915,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
+         q_issue<NS, NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
    } else {
       // ---- A operand: site j of the tile, two quads (8 K) per stage
       const int j = tid & 127, kg = tid >> 7;
@@ -1009,7 +1012,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
             const double s = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
             // units of the product: 2^-62 over the four table scales, times the coefficients' scale
             const double sc = emax > -4096 ? ldexp(1.0 / (Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA), emax - 62) : 0.0;
-            hpart[((size_t)blockIdx.z * 3 + set) * n + i] = s * sc;
+            hpart[((size_t)blockIdx.z * gridDim.y + set) * n + i] = s * sc;
          }
       }
    }
@@ -1040,6 +1043,217 @@ k_fsum_q(int n, int N, int nitems, QGeom g, const double *__restrict__ hpart, co
    force[2 * (size_t)N + si] += q * (g.b[2] * H[0] + g.b[5] * H[1] + g.b[8] * H[2]);
 }
 
+// ----------------------------------------------------------------- adjoint
+// Weighted structure factors V_a = sum_j q_j v_ja exp(i k.r_j) (a = x, y, z)
+// and the per-site sums of the adjoint's reciprocal space (adjoint.cu): the
+// weights take the charges' place in operand B, one more digit than the
+// charges in the mixed form (residual weights spread over decades: a few
+// close contacts dominate them, and the digits' grid is that of the largest).
+
+// wmax[a]: bits of an FP32 upper bound of max |q v_a| (zeroed before)
+template <typename V4>
+__global__ void __launch_bounds__(256)
+k_qwmax(int n, const int *__restrict__ slots, const double *__restrict__ chg, const V4 *__restrict__ res,
+        unsigned int *__restrict__ wmax)
+{
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   float m[3] = {0.f, 0.f, 0.f};
+   if (i < n) {
+      const double q = chg[slots[i]];
+      const V4 v = res[i];
+      m[0] = __double2float_ru(fabs(q * (double)v.x));
+      m[1] = __double2float_ru(fabs(q * (double)v.y));
+      m[2] = __double2float_ru(fabs(q * (double)v.z));
+   }
+#pragma unroll
+   for (int a = 0; a < 3; a++) {
+      const unsigned int x = __reduce_max_sync(0xffffffffu, __float_as_uint(m[a]));
+      if ((threadIdx.x & 31) == 0 && x) atomicMax(&wmax[a], x);
+   }
+}
+__device__ __forceinline__ int q_wexp(unsigned int bits)   // a power of two above
+{
+   int e = 0;
+   const float m = __uint_as_float(bits);
+   if (m > 0.f) frexp((double)m, &e);
+   return e;
+}
+
+// Operand B of the three weighted channels, per 32-site stage as in k_qtab.
+template <int NS, int ND, typename V4>
+__global__ void __launch_bounds__(256)
+k_qwtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__restrict__ site,
+        const double *__restrict__ chg, double hi6, double hi7, double hi8, const V4 *__restrict__ res,
+        const unsigned int *__restrict__ wmax, unsigned char *__restrict__ ztab, size_t zstride)
+{
+   typedef typename QCfg<NS>::T T;
+   __shared__ unsigned long long su[32];
+   __shared__ T sw[3][32];
+   __shared__ T sz[64][33];
+   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, stage = blockIdx.x;
+   if (w < 4) {
+      const int i = stage * 32 + lane;
+      const int si = i < n ? slots[i] : 0;
+      if (w == 3) {
+         su[lane] = i < n ? q_fixed64(hi6 * site[si] + hi7 * site[ns + si] + hi8 * site[2 * (size_t)ns + si]) : 0ull;
+      } else {
+         double x = 0.0;
+         if (i < n) {
+            const V4 v = res[i];
+            x = chg[si] * (double)(w == 0 ? v.x : w == 1 ? v.y : v.z);
+         }
+         x = ldexp(x * Q_KAPPA, (NS == 3 ? 31 : 63) - q_wexp(wmax[w]));
+         sw[w][lane] = NS == 3 ? (T)__double2int_rn(x) : (T)qbalance((T)__double2ll_rn(x));
+      }
+   }
+   __syncthreads();
+   const unsigned long long uz = su[lane];
+   for (int t0 = 0; t0 < g.TP; t0 += 32) {
+      const int nt = min(32, g.TP - t0);
+      __syncthreads();
+      for (int t = w; t < nt; t += 8) {
+         T s, c;
+         qtrig(t0 + t, uz, s, c);
+         const int col = 16 * (t >> 3) + (t & 7);
+         sz[col][lane] = qbalance(c);
+         sz[col + 8][lane] = qbalance(s);
+      }
+      __syncthreads();
+      const int kg = tid & 3, c8 = (tid >> 2) & 7, cg = tid >> 5;
+      if (8 * cg < 2 * nt) {
+         const int tcol = 2 * t0 + 8 * cg, b = tcol / (2 * g.TW), lc = tcol - 2 * b * g.TW;
+         const int nT = q_blkcols(g, b), pc = nT / QCfg<NS>::NPART;
+         const int part = lc / pc, pl = lc - part * pc;
+         unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * ND + (size_t)2 * b * g.TW * Q_KS * 2 * ND +
+                            ((size_t)part * ND * pc + pl) * Q_KS * 2 + kg * 128 + c8 * 16;
+#pragma unroll
+         for (int a = 0; a < 3; a++) {
+            auto wz = [&](int e) { return qmul(sw[a][8 * kg + e], sz[8 * cg + c8][8 * kg + e]); };
+            decltype(wz(0)) v[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) v[e] = wz(e);
+            qstore<ND>(d + a * zstride, pc * Q_KS * 2, v);
+         }
+      }
+   }
+}
+
+// Per (quad, t) and (s, r): the alpha derivatives (blk: dE/dalpha, dG/dalpha
+// per block) and the coefficients of the per-site sum, laid out as A, B in
+// k_qreduce.  With T = sum_a k_a V_a, P + i Q = coeff T: (-P, -Q) for the
+// loss (sum_k cos Q - sin P = Im(e U), U = -P + i Q), (B, -A) for the energy
+// (A cos + B sin).  Channel sums over nr0 (charges) and nrv (weights) ranges.
+template <typename R>
+__global__ void __launch_bounds__(256)
+k_qadj(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coeff, double alpha, int loss, int nr0,
+       double scale0, const double *__restrict__ part, int nrv, double scalev, const unsigned int *__restrict__ wmax,
+       const double *__restrict__ partv, R *__restrict__ ab, double *__restrict__ blk)
+{
+   __shared__ double sq[8][8][32];
+   __shared__ double sh[4][2];
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+   const int i = blockIdx.x * 32 + lane, quad = i / g.TP, t = i - quad * g.TP;
+   const int4 un = quad < g.nquads ? units[quad >> 2] : make_int4(0, 0, 0, 0);
+   const bool live = t < un.z;
+   {
+      // warp w: channel w / 2, ranges w % 2, + 2, ...
+      const int ch = w >> 1;
+      double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      if (live && (ch == 0 || loss)) {
+         const size_t row = 2 * (size_t)g.TP, plane = 4 * (size_t)g.nquads * row;
+         const int nr = ch == 0 ? nr0 : nrv;
+         const double *p = (ch == 0 ? part : partv + (size_t)(ch - 1) * nrv * plane) + (size_t)quad * 4 * row +
+                           16 * (t >> 3) + (t & 7) + (w & 1) * plane;
+         for (int c = w & 1; c < nr; c += 2, p += 2 * plane)
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+               q[2 * k] += p[k * row];
+               q[2 * k + 1] += p[k * row + 8];
+            }
+         const double sc = ch == 0 ? scale0 : ldexp(scalev, q_wexp(wmax[ch - 1]));
+#pragma unroll
+         for (int k = 0; k < 8; k++) q[k] *= sc;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++) sq[w][k][lane] = q[k];
+   }
+   __syncthreads();
+   if (w >= 4) return;
+   double ea = 0.0, la = 0.0;
+   if (quad < g.nquads) {
+      double o0 = 0.0, o1 = 0.0;
+      const double2 cf = live ? coeff[(size_t)i * 4 + w] : make_double2(0.0, 0.0);
+      if (cf.x != 0.0) {
+         const double s = w & 2 ? -1.0 : 1.0, r = w & 1 ? -1.0 : 1.0;
+         double C[4], S[4];
+#pragma unroll
+         for (int ch = 0; ch < 4; ch++) {
+            double q[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) q[k] = sq[2 * ch][k][lane] + sq[2 * ch + 1][k][lane];
+            C[ch] = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
+            S[ch] = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
+         }
+         const double hh = un.x, kk = s * (un.y + (quad & 3)), l = r * t;
+         const double kx = hh * g.b[0] + kk * g.b[3], ky = hh * g.b[1] + kk * g.b[4];
+         const double kz = hh * g.b[2] + kk * g.b[5] + l * g.b[8];
+         const double dcf = cf.x * (kx * kx + ky * ky + kz * kz) / (2.0 * alpha * alpha * alpha);
+         ea = 0.5 * dcf * (C[0] * C[0] + S[0] * S[0]);
+         if (loss) {
+            const double Tc = kx * C[1] + ky * C[2] + kz * C[3], Ts = kx * S[1] + ky * S[2] + kz * S[3];
+            la = dcf * (C[0] * Ts - S[0] * Tc);
+            o0 = -cf.x * Tc;
+            o1 = -cf.x * Ts;
+         } else {
+            o0 = cf.x * S[0];
+            o1 = -cf.x * C[0];
+         }
+      }
+      ab[(size_t)i * 8 + 2 * w] = (R)o0;
+      ab[(size_t)i * 8 + 2 * w + 1] = (R)o1;
+   }
+#pragma unroll
+   for (int o = 16; o > 0; o >>= 1) {
+      ea += __shfl_down_sync(0xffffffffu, ea, o);
+      la += __shfl_down_sync(0xffffffffu, la, o);
+   }
+   if (lane == 0) {
+      sh[w][0] = ea;
+      sh[w][1] = la;
+   }
+   asm volatile("bar.sync 1, 128;" : : : "memory");
+   if (threadIdx.x < 2)
+      blk[blockIdx.x * 2 + threadIdx.x] = (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
+}
+
+// gq[site] += the per-site sum (items' / splits' partials s1 in order) and,
+// for the loss, v . H with H = sum_k k (A sin - B cos) of the forward's
+// force pass: FP64 items of (h, k, l) sums, or FP32-form Cartesian splits.
+template <bool MIXED, typename V4>
+__global__ void __launch_bounds__(256)
+k_qadj_site(int n, int np, QGeom g, const double *__restrict__ hpart, const double *__restrict__ s1,
+            const V4 *__restrict__ res, int loss, const int *__restrict__ slots, double *__restrict__ gq)
+{
+   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   if (i >= n) return;
+   double v = 0.0;
+   for (int k = 0; k < np; k++) v += s1[(size_t)k * (MIXED ? 3 : 1) * n + i];
+   if (loss) {
+      double H[3] = {0, 0, 0};
+      for (int k = 0; k < np; k++)
+#pragma unroll
+         for (int a = 0; a < 3; a++) H[a] += hpart[((size_t)k * 3 + a) * n + i];
+      const V4 r = res[i];
+      const double x = r.x, y = r.y, z = r.z;
+      if (MIXED)
+         v += x * H[0] + y * H[1] + z * H[2];
+      else
+         v += x * (g.b[0] * H[0] + g.b[3] * H[1]) + y * (g.b[1] * H[0] + g.b[4] * H[1]) +
+              z * (g.b[2] * H[0] + g.b[5] * H[1] + g.b[8] * H[2]);
+   }
+   gq[slots[i]] += v;
+}
+
 // ------------------------------------------------------------- host side
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
 
@@ -1051,9 +1265,10 @@ static cudaError_t q_init_device(int device)
    static std::atomic<unsigned long long> done{0};
    const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
    if (bit && (done.load() & bit)) return cudaSuccess;
-   cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3>);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7>);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7>);
+   cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 3>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<3, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 4>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
    if (e == cudaSuccess) e = ks_force_tc_init();
    if (e == cudaSuccess && bit) done.fetch_or(bit);
    return e;
@@ -1148,12 +1363,13 @@ mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges)
    CK(d.q_part.ensure(R * plane));
    const dim3 grid(nt, R);
    if (ns == 3)
-      k_sfac_q<3><<<grid, Q_THREADS, Q_SMEM<3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, nst, per, d.q_part.p, &c->out.p->err);
+      k_sfac_q<3, 3><<<grid, Q_THREADS, Q_SMEM<3, 3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, nst, per, d.q_part.p, &c->out.p->err);
    else
-      k_sfac_q<7><<<grid, Q_THREADS, Q_SMEM<7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, nst, per, d.q_part.p, &c->out.p->err);
+      k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, 0, nst, per, d.q_part.p, &c->out.p->err);
    CK(cudaGetLastError());
+   d.q_nranges = R;
    *nranges = R;
    return MDGPU_OK;
 }
@@ -1221,8 +1437,8 @@ mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
    CK(d.q_bq.ensure((size_t)3 * nseg * 4 * QCfg<7>::NTMAX * Q_KS * 2 * 7));
    CK(d.q_bexp.ensure((size_t)3 * nseg));
    CK(d.fpart.ensure((size_t)d.q_nitems * 3 * n));
-   k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, d.q_segs.p, nseg, d.q_units.p, d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
-   k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_SMEM<7>, c->stream>>>(
+   k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, 0, d.q_segs.p, nseg, d.q_units.p, d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
+   k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(
       q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, n,
       d.fpart.p, &c->out.p->err);
    CK(cudaGetLastError());
@@ -1235,6 +1451,93 @@ mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force)
    k_fsum_q<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->nsites, c->kd.q_nitems, c->kl.q.g, c->kd.fpart.p, slots,
                                                     c->rd.chg.p, d_force);
    CK(cudaGetLastError());
+   return MDGPU_OK;
+}
+
+// Reciprocal-space adjoint over all sites (slots: every site in link-cell
+// order, as the forward pass before it ran): adds into gq and writes the
+// alpha derivatives' block records into a.blk (two each; their number in
+// *nblocks).
+mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq, int *nblocks)
+{
+   KsDev &d = c->kd;
+   AdjDev &a = c->ad;
+   const QList &q = c->kl.q;
+   const QGeom &g = q.g;
+   cudaStream_t st = c->stream;
+   const int ns = q.ns, nd = ns == 3 ? 4 : 7, N = c->nsites, nst = (N + 31) / 32, nt = (int)q.tiles.size();
+   const size_t nqt = (size_t)g.nquads * g.TP, plane = 4 * (size_t)g.nquads * 2 * g.TP;
+   const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
+   const double *hi = c->kl.hinv;
+   int R = 1;
+   CK(a.wmax.ensure(3));
+   if (loss) {
+      const size_t S = q_stages(N), zstride = S * 2 * g.TP * Q_KS * 2 * nd;
+      CK(a.zw.ensure(3 * zstride));
+      CK(cudaMemsetAsync(a.wmax.p, 0, 3 * sizeof(unsigned int), st));
+      long long best = -1;
+      for (int r = 1; r <= 64 && r <= nst; r++) {
+         if (r > 1 && 3 * r * plane * sizeof(double) > (256u << 20)) break;
+         const long long cost = (long long)((3 * nt * r + c->nsm - 1) / c->nsm) * ((nst + r - 1) / r + 6);
+         if (best < 0 || cost < best) {
+            best = cost;
+            R = r;
+         }
+      }
+      const int per = (nst + R - 1) / R;
+      R = (nst + per - 1) / per;
+      CK(a.partv.ensure(3 * (size_t)R * plane));
+      const dim3 grid(nt, R, 3);
+      const int nb = (N + 255) / 256;
+      if (ns == 3) {
+         k_qwmax<float4><<<nb, 256, 0, st>>>(N, slots, c->rd.chg.p, a.res32.p, a.wmax.p);
+         k_qwtab<3, 4, float4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
+                                                    a.res32.p, a.wmax.p, a.zw.p, zstride);
+         k_sfac_q<3, 4><<<grid, Q_THREADS, Q_SMEM<3, 4>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
+            (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, a.zw.p, zstride, nst, per, a.partv.p,
+            &c->out.p->err);
+      } else {
+         k_qwmax<double4><<<nb, 256, 0, st>>>(N, slots, c->rd.chg.p, a.res64.p, a.wmax.p);
+         k_qwtab<7, 7, double4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
+                                                     a.res64.p, a.wmax.p, a.zw.p, zstride);
+         k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
+            (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, a.zw.p, zstride, nst, per, a.partv.p,
+            &c->out.p->err);
+      }
+      CK(cudaGetLastError());
+      c->launches += 3;
+   }
+   const int nb = (int)((nqt + 31) / 32);
+   *nblocks = nb;
+   CK(a.blk.ensure(2 * (size_t)nb));
+   const int e0 = q_charge_exp(c);
+   if (ns == 3) {
+      CK(a.ab32.ensure(nqt * 8));
+      k_qadj<float><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
+         std::ldexp(1.0 / k4, e0 - 30), d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, a.partv.p, a.ab32.p, a.blk.p);
+      const int sp = ks_force_tc_splits(d);
+      CK(a.gkpart.ensure((size_t)sp * 3 * N));
+      const int nl = ks_force_tc(st, N, g, d, a.ab32.p, true, c->nsm, a.gkpart.p, &c->out.p->err);
+      if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
+      c->launches += nl;
+      k_qadj_site<true, float4><<<(N + 255) / 256, 256, 0, st>>>(N, sp, g, d.fpart.p, a.gkpart.p, a.res32.p,
+                                                                 loss ? 1 : 0, slots, gq);
+   } else {
+      CK(a.ab64.ensure(nqt * 8));
+      k_qadj<double><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
+         std::ldexp(1.0 / k4, e0 - 62), d.q_part.p, R, std::ldexp(1.0 / k4, -62), a.wmax.p, a.partv.p, a.ab64.p, a.blk.p);
+      const int nseg = (int)q.segs.size(), T = (N + 127) / 128;
+      CK(a.gkpart.ensure((size_t)d.q_nitems * N));
+      k_qcoef<<<dim3(nseg, 1), 256, 0, st>>>(g, 3, d.q_segs.p, nseg, d.q_units.p, a.ab64.p, d.q_bq.p, d.q_bexp.p);
+      k_force_q<<<dim3(T, 1, d.q_nitems), Q_THREADS, Q_SMEM<7, 7>, st>>>(
+         g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, N,
+         a.gkpart.p, &c->out.p->err);
+      c->launches += 2;
+      k_qadj_site<false, double4><<<(N + 255) / 256, 256, 0, st>>>(N, d.q_nitems, g, d.fpart.p, a.gkpart.p, a.res64.p,
+                                                                   loss ? 1 : 0, slots, gq);
+   }
+   CK(cudaGetLastError());
+   c->launches += 2;
    return MDGPU_OK;
 }
 #undef CK

@@ -70,7 +70,7 @@ constexpr int FTC_ERR = 16;                        // error-word bit: a force-pa
 // [cosines, sines][row group 16][8 rows][8 t] bf16, row 4 i + c for item i
 // of the tile.
 __global__ void __launch_bounds__(256)
-k_utab_tc(int nitems, QGeom g, int t0, const int4 *__restrict__ fu, const float4 *__restrict__ ab,
+k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, const float4 *__restrict__ ab,
           uint4 *__restrict__ utab, float4 *__restrict__ coef)
 {
    __shared__ float4 sv[8][64];
@@ -130,9 +130,12 @@ k_utab_tc(int nitems, QGeom g, int t0, const int4 *__restrict__ fu, const float4
       // the seeds' table scale (units of 2^-24 and 2^-31, times Q_KAPPA each) folded in
       const double f2 = 1.0 / (16777216.0 * 2147483648.0 * Q_KAPPA * Q_KAPPA);
       const double hh = un.x, kk = neg ? -(double)(un.y + q) : (double)(un.y + q);
-      coef[i] = un.w >= 0 ? make_float4((float)((hh * g.b[0] + kk * g.b[3]) * f2 * s1), (float)((hh * g.b[1] + kk * g.b[4]) * f2 * s1),
-                                        (float)((hh * g.b[2] + kk * g.b[5]) * f2 * s1), (float)(g.b[8] * f2 * s2))
-                          : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (scalar)   // f1 alone
+         coef[i] = make_float4(un.w >= 0 ? (float)(f2 * s1) : 0.f, 0.f, 0.f, 0.f);
+      else
+         coef[i] = un.w >= 0 ? make_float4((float)((hh * g.b[0] + kk * g.b[3]) * f2 * s1), (float)((hh * g.b[1] + kk * g.b[4]) * f2 * s1),
+                                           (float)((hh * g.b[2] + kk * g.b[5]) * f2 * s1), (float)(g.b[8] * f2 * s2))
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
    }
 }
 
@@ -195,8 +198,7 @@ __global__ void k_ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int n
 __global__ void __launch_bounds__(FTC_THREADS, 1)
 k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef, int nitems, int t0,
            const int *__restrict__ X, const int *__restrict__ Y, const uint4 *__restrict__ zsite,
-           const uint4 *__restrict__ utab, const double *__restrict__ chg, const int *__restrict__ slots, int n,
-           const int *__restrict__ ustart, double *__restrict__ fpart, int *__restrict__ err)
+           const uint4 *__restrict__ utab, int n, const int *__restrict__ ustart, double *__restrict__ fpart, int *__restrict__ err)
 {
    using namespace tc;
    extern __shared__ __align__(1024) unsigned char sm[];
@@ -440,7 +442,6 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
          __syncwarp();
          asm volatile("bar.sync 2, %0;" : : "n"(FTC_EW * 32) : "memory");
          if (w < 4 && i < n && !tc_aborted(&abort_s)) {
-            const double q = chg[slots[i]];
             double sx = 0.0, sy = 0.0, sz = 0.0;
             for (int k = 0; k < FTC_EG; k++) {
                const float *rg = rt + ((size_t)k * 128 + r) * 3;
@@ -449,9 +450,9 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
                sz += (double)rg[2];
             }
             double *dst = fpart + (u0 > T * ntl ? 3 * (size_t)n : 0);
-            dst[i] = q * sx;
-            dst[n + i] = q * sy;
-            dst[2 * (size_t)n + i] = q * sz;
+            dst[i] = sx;
+            dst[n + i] = sy;
+            dst[2 * (size_t)n + i] = sz;
             if (u0 <= T * ntl && u1 >= (T + 1) * ntl) {
                double *z = fpart + 3 * (size_t)n;
                z[i] = 0.0;
@@ -473,13 +474,13 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
 // The force pass of one t-block (its units fu0 .. fu0 + npos - 1 of the
 // list, a multiple of four) into slots 0 and 1 of fpart; returns the
 // launches, -1 if out of memory.
-static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int blk, int fu0, int npos, int nsm,
-                          const double *chg, const int *slots, double *fpart, int *err)
+static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int blk,
+                          int fu0, int npos, int nsm, double *fpart, int *err)
 {
    const int T = (nsites + 127) / 128, ntl = npos * 8 / FTC_NI, t0 = 64 * blk;
    const int G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
    const int4 *fu = d.q_fu.p + fu0;
-   k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, fu, reinterpret_cast<const float4 *>(d.q_ab32.p), d.utab.p,
+   k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, scalar ? 1 : 0, fu, reinterpret_cast<const float4 *>(ab), d.utab.p,
                                    d.tc_coef.p);
    int launches = 2;
    if (blk > 0 || d.tc_rkey[0] != T || d.tc_rkey[1] != ntl || d.tc_rkey[2] != G || d.tc_rver != d.tc_ver) {
@@ -492,16 +493,16 @@ static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d,
       launches++;
    }
    k_force_tc<<<G, FTC_THREADS, FTC_SMEM, st>>>(g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p, d.q_y32.p, d.zsite.p,
-                                                d.utab.p, chg, slots, nsites, d.tc_ustart.p, fpart, err);
+                                                d.utab.p, nsites, d.tc_ustart.p, fpart, err);
    return launches;
 }
 
-int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int nsm, const double *chg, const int *slots,
+int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
                 double *fpart, int *err)
 {
    int launches = 0;
    for (int b = 0; b < d.q_nfblk; b++) {
-      const int nl = force_tc_block(st, nsites, g, d, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm, chg, slots,
+      const int nl = force_tc_block(st, nsites, g, d, ab, scalar, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm,
                                     fpart + (size_t)b * FTC_SPLITS * 3 * nsites, err);
       if (nl < 0) return -1;
       launches += nl;

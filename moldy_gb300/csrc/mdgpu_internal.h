@@ -258,6 +258,7 @@ struct KsDev {
    std::vector<int> q_fblk;
    int q_items_for[3] = {-1, -1, -1};   // (site tiles, list upload, SMs) of q_items
    int q_nitems = 0;
+   int q_nranges = 0;               // site ranges of q_part
    DBuf<uint4> zsite;      // force pass: z tables as the A operand, per 128 sites
    DBuf<uint4> utab;       // force pass: per-item coefficient rows (B operand)
    DBuf<float4> tc_coef;   // per item: kx s1, ky s1, kz0 s1, dkz s2 (row scales s)
@@ -293,6 +294,12 @@ struct AdjDev {
    DBuf<float> kz32;       // per k: k_z
    DBuf<double> gkpart;    // [splits][2][N] k-space charge-gradient partials
    DBuf<double> blk;       // per-block k-space dE/dalpha, dG/dalpha
+   // tensor-core passes: largest weights, the weights' digits, their
+   // structure factors, the per-site pass's coefficients
+   DBuf<unsigned int> wmax;
+   DBuf<unsigned char> zw;
+   DBuf<double> partv, ab64;
+   DBuf<float> ab32;
 };
 
 // Rigid-molecule dynamics (integrate.cu): one species' constants.
@@ -468,16 +475,18 @@ KsShape ks_shape(int N, int nitems, int ipt, int spt);
 // tables, structure factor and per-k sums (A and B per (quad, t), the
 // blocks' energy/stress records into d.blk; returns their number, -1 if out
 // of memory), and the FP64 form's force pass (adds the forces after join,
-// if any).  kspace_tc.cu: the mixed form's force pass, F_slot into
-// fpart[split][3][nsites] (returns the launches, -1 if out of memory).
+// if any).  kspace_tc.cu: the mixed form's force pass, F_slot / q into
+// fpart[split][3][nsites], or with scalar the sum over k of A sin - B cos
+// into its first component (returns the launches, -1 if out of memory).
 mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns);
 mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site);
 mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges);
 mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges, int *nblocks);
 mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots);
 mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force);
-int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, int nsm, const double *chg, const int *slots,
+int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
                 double *fpart, int *err);
+mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq, int *nblocks);
 int ks_force_tc_splits(const KsDev &d);
 size_t ks_tc_utab_len(int npos);
 cudaError_t ks_force_tc_init();

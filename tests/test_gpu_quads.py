@@ -63,3 +63,31 @@ def test_matches_cuda_core_passes(case, monkeypatch):
         assert np.sqrt(((f - f0) ** 2).mean()) <= tol * scale, form
         assert abs(e - e0) <= tol * (abs(e0) + self_e), form
         assert np.abs(s - s0).max() <= tol * (np.abs(s0).max() + self_e), form
+
+
+@pytest.mark.parametrize("case", [CASES[k] for k in (1, 4, 8, 13, 18, 23, 29)], ids=lambda c: "-".join(
+    str(round(v, 1) if isinstance(v, float) else v) for v in c.values()).replace(" ", ""))
+@pytest.mark.parametrize("loss", [False, True])
+def test_adjoint_matches_cuda_core_passes(case, loss, monkeypatch):
+    """Charge and alpha gradients at the tiling's edges.  The reference forces
+    are zero, so the residual is the force itself (random positions: over
+    several decades) and the mixed form's relative force error carries over:
+    the bounds of the adjoint's oracle tests, FP64 1e-9 and mixed 2e-5 of the
+    largest entry, twice that for the loss."""
+    from moldy_gb300 import ForceField
+    sysm = ions(**case)
+    fref = np.zeros((3, sysm.nsites))
+    res = {}
+    for form, tc in (("fp64", "0"), ("fp64", "1"), ("mixed", "1")):
+        monkeypatch.setenv("MDGPU_KSPACE_TC", tc)
+        ff = ForceField(sysm, precision=form)
+        res[form, tc] = ff.fm_loss_grad(fref, 0.3) if loss else ff.energy_grad()
+        ff.close()
+    v0, g0 = res["fp64", "0"]
+    for form, tol in (("fp64", 1e-9), ("mixed", 2e-5)):
+        v, g = res[form, "1"]
+        if form == "fp64" or loss:
+            assert abs(v - v0) <= 2 * tol * abs(v0), form
+        assert np.abs(g["chg"] - g0["chg"]).max() <= tol * np.abs(g0["chg"]).max(), form
+        if form == "fp64":
+            assert abs(g["alpha"] - g0["alpha"]) <= tol * (abs(g0["alpha"]) + np.abs(g0["chg"]).max())
