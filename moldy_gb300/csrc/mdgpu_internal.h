@@ -200,6 +200,7 @@ struct RsDev {
    DBuf<float4> coff;      // [e][2]: the column offsets' hi and lo parts side by side (32 B per entry)
    DBuf<int> cls_of_id, cls_pre, cs, sortc, cellc, cls_bsum;
    DBuf<float4> posc;
+   DBuf<double4> posc64;   // the FP64 form's records, class by class
    DBuf<int2> tagc;
    DBuf<unsigned long long> rdf_counts;
    double rdf_key[11] = {0};

@@ -42,6 +42,8 @@ struct RsParams {
    // (the framework's sites are binned one by one, src/force.c:458-470)
    int fw_mol, fw_site0, nmol_ent;
    int ncols;             // stencil columns (k_pairs_col)
+   int chunk;             // home slots a block takes at a time (ColHome)
+   int one_class;         // the slots are in link-cell order, one interaction class
    double hinv[9];
    double h[9];
    double rn[3];          // 1/nx, 1/ny, 1/nz
@@ -55,6 +57,8 @@ struct AdjParams {
    int loss;              // nonzero: residual weights given, loss terms wanted
    unsigned type_mask;    // bit b set: some site has identifier b
    int nslot;             // 2 max_id^2 NP + 2 gradient slots
+   int ntype;             // identifiers present, and each one's index among them
+   unsigned char type_index[MDGPU_ADJ_MAX_ID];
 };
 
 // ---------------------------------------------------------------- binning
@@ -218,7 +222,7 @@ __global__ void k_gather(RsParams P, const double *__restrict__ site, const doub
                          const int *__restrict__ siteid, const int *__restrict__ molmap,
                          const int *__restrict__ sorted, const int *__restrict__ cell_of,
                          double4 *__restrict__ pos64, float4 *__restrict__ pos32,
-                         int2 *__restrict__ tag, int *__restrict__ slot_cell)
+                         int2 *__restrict__ tag, int2 *__restrict__ tagz, int *__restrict__ slot_cell)
 {
    int p = blockIdx.x * blockDim.x + threadIdx.x;
    const int N = P.nsites;
@@ -226,6 +230,7 @@ __global__ void k_gather(RsParams P, const double *__restrict__ site, const doub
    int i = sorted[p], c = cell_of[i];
    double x = site[i], y = site[N + i], z = site[2 * N + i], q = chg[i];
    tag[p] = make_int2(siteid[i], molmap[i]);
+   if (tagz) tagz[p] = make_int2(siteid[i] | ((c % P.nz) << 16), molmap[i]);   // with the cell's z index
    slot_cell[p] = c;
    if (pos64) pos64[p] = make_double4(x, y, z, q);
    if (pos32) {
@@ -278,6 +283,62 @@ template <> struct PairMath<float, true> {
    static __device__ __forceinline__ float rsqrt(float x) { return rsqrtf(x); }
    static __device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
    static __device__ __forceinline__ float ex(float x) { return __expf(x); }
+};
+
+// FP64 form of the same: the FP64 pipe (two lanes per clock and SM) bounds
+// the pair loops, so the correctly rounded square root, divisions and exp
+// (about 55 of 110 FP64 instructions per pair) are replaced by
+//   rsqrt, rcp: the hardware's 20-bit approximation and one third-order
+//     Newton (Householder) step, e -> e^3: 5 and 3 FP64 instructions, about
+//     1 ulp;
+//   exp: Tang's table method (ACM TOMS 15, 144, 1989): x = (64 k + j) ln2/64
+//     + f, exp(x) = 2^k 2^(j/64) e^f, |f| <= ln2/128, degree 6: 12
+//     instructions, about 1 ulp.  The table of 2^(j/64) is in shared memory.
+// Arguments outside their range (r^2 zero or subnormal, |x| > 700) take the
+// general functions.
+__device__ __forceinline__ double rsqrt_n(double x)
+{
+   // (range checks on the exponent bits: a compare would take the FP64 pipe)
+   if ((unsigned int)__double2hiint(x) - 0x04000000u >= 0x78000000u) return 1.0 / sqrt(x);
+   double y;
+   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+   const double e = fma(-x, y * y, 1.0);
+   return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double rcp_n(double x)
+{
+   if (((unsigned int)__double2hiint(x) & 0x7fffffffu) - 0x04000000u >= 0x78000000u) return 1.0 / x;
+   double y;
+   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+   const double e = fma(-x, y, 1.0);
+   return fma(y, fma(e, e, e), y);
+}
+__shared__ double exp2_tab[64];   // 2^(j/64); filled by exp2_fill (kernels that use exp_n)
+__device__ __forceinline__ void exp2_fill()
+{
+   for (int j = threadIdx.x; j < 64; j += blockDim.x) exp2_tab[j] = exp2((double)j * 0.015625);
+}
+__device__ __forceinline__ double exp_n(double x)
+{
+   if (((unsigned int)__double2hiint(x) & 0x7fffffffu) >= 0x4085e000u) return exp(x);   // |x| >= 700
+   const double w = fma(x, 92.332482616893657, 6755399441055744.0);   // x 64/ln2 + 1.5 2^52
+   const int n = __double2loint(w);
+   const double nf = w - 6755399441055744.0;
+   // ln2/64 in two parts, the first with 21 trailing zero bits (nf exact in it)
+   const double f = fma(nf, -2.9815858269852933e-12, fma(nf, -0.010830424693267560, x));
+   double p = fma(f, 1.0 / 720.0, 1.0 / 120.0);
+   p = fma(f, p, 1.0 / 24.0);
+   p = fma(f, p, 1.0 / 6.0);
+   p = fma(f, p, 0.5);
+   p = fma(f * f, p, f);
+   const double t = exp2_tab[n & 63];
+   const double r = fma(t, p, t);
+   return __hiloint2double(__double2hiint(r) + ((n >> 6) << 20), __double2loint(r));
+}
+template <> struct PairMath<double, true> {
+   static __device__ __forceinline__ double rsqrt(double x) { return rsqrt_n(x); }
+   static __device__ __forceinline__ double rcp(double x) { return rcp_n(x); }
+   static __device__ __forceinline__ double ex(double x) { return exp_n(x); }
 };
 
 // One pair of kernel(): f = -U'(r)/r and U, with the erfc real-space Ewald
@@ -762,7 +823,28 @@ __global__ void __launch_bounds__(256) k_reduce_rs2(const double *__restrict__ p
 constexpr int COL_E = 3;                    // stencil columns per lane in one pass
 constexpr int COL_ROWS = 32 * COL_E * 2;    // slot runs per pass (two per column at most)
 constexpr int COL_WIN = 256;                // candidates decoded per window
-constexpr int COL_CHUNK = 16;               // consecutive home slots a block takes at a time
+constexpr int COL_CHUNK = 16;               // most consecutive home slots a block takes at a time
+
+// The home slots of a block's warp w: chunks of `chunk` consecutive slots
+// (a multiple of the block's warps) dealt to the grid's blocks in turn, a
+// chunk's slots to the block's warps in turn.
+struct ColHome {
+   int chunk, w, it, p;
+   __device__ __forceinline__ ColHome(int chunk_, int w_) : chunk(chunk_), w(w_), it(0), p((int)blockIdx.x * chunk_ + w_) {}
+   __device__ __forceinline__ void next()
+   {
+      it += PAIR_WARPS;
+      p = ((it / chunk) * (int)gridDim.x + (int)blockIdx.x) * chunk + it % chunk + w;
+   }
+};
+// Chunks of 16 (neighbouring sites share candidates and column starts in
+// L1), shorter where the grid then had blocks without a site: 500-site argon
+// in FP64 57 us with 16 against 18 us with 4.
+static int col_chunk(int N, int nblk)
+{
+   const int per = (N + nblk - 1) / nblk;
+   return std::max(PAIR_WARPS, std::min(COL_CHUNK, per / PAIR_WARPS * PAIR_WARPS));
+}
 
 // per slot (link-cell order): 1 when its identifier is in class 0; the
 // entry after the last is 0 (so the exclusive scan ends with the class-0
@@ -782,7 +864,8 @@ __global__ void k_cls_flag(int N, const int2 *__restrict__ tag, const int *__res
 __global__ void k_cls_split(RsParams P, const int *__restrict__ pre, const int *__restrict__ cls_of_id,
                             const int *__restrict__ cell_start, const float4 *__restrict__ pos32,
                             const int2 *__restrict__ tag, const int *__restrict__ sorted,
-                            const int *__restrict__ slot_cell, int *__restrict__ cs, float4 *__restrict__ posc,
+                            const int *__restrict__ slot_cell, const double4 *__restrict__ pos64,
+                            int *__restrict__ cs, float4 *__restrict__ posc, double4 *__restrict__ posc64,
                             int2 *__restrict__ tagc, int *__restrict__ sortc, int *__restrict__ cellc)
 {
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -792,6 +875,7 @@ __global__ void k_cls_split(RsParams P, const int *__restrict__ pre, const int *
       const int q = cls_of_id[t.x] == 0 ? pre[i] : n0 + (i - pre[i]);
       const int c = slot_cell[i];
       posc[q] = pos32[i];
+      if (posc64) posc64[q] = pos64[i];
       tagc[q] = make_int2(t.x | ((c % P.nz) << 16), t.y);
       sortc[q] = sorted[i];
       cellc[q] = c;
@@ -851,7 +935,7 @@ __device__ __forceinline__ ColRuns col_runs(const RsParams &P, int cx, int cy, i
 // trees.
 template <int PT, bool EW>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 8)
-k_pairs_col(RsParams P, const int *__restrict__ cell_start, const int *__restrict__ cs,
+k_pairs_col(RsParams P, const int *__restrict__ cs,
             const int *__restrict__ pre, const int4 *__restrict__ cols, const int *__restrict__ col_base,
             const float4 *__restrict__ coff, const float4 *__restrict__ posc, const int2 *__restrict__ tagc,
             const int *__restrict__ cellc,
@@ -870,7 +954,7 @@ k_pairs_col(RsParams P, const int *__restrict__ cell_start, const int *__restric
    __syncthreads();
    const R *pot = P.pot_in_smem ? pot_s : potg;
 
-   const int N = P.nsites, n0 = pre[N];
+   const int N = P.nsites, n0 = P.one_class ? N : pre[N];
    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
    int *inc = s_inc[w], *jbr = s_jb[w], *infr = s_inf[w], *cand = s_cand[w];
    // the lane's energy and virial over all its home sites (per-site sums
@@ -884,9 +968,8 @@ k_pairs_col(RsParams P, const int *__restrict__ cell_start, const int *__restric
    // chunk's slots in turn: a few resident blocks per SM take every site,
    // neighbouring sites (shared candidates and column starts in L1) at
    // about the same time
-   for (int it = 0, p = blockIdx.x * COL_CHUNK + w; p < N;
-        it++, p = ((it / (COL_CHUNK / PAIR_WARPS)) * gridDim.x + blockIdx.x) * COL_CHUNK +
-                  (it % (COL_CHUNK / PAIR_WARPS)) * PAIR_WARPS + w) {
+   for (ColHome hm(P.chunk, w); hm.p < N; hm.next()) {
+      const int p = hm.p;
       R fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
       const int *csk = cs + (p < n0 ? 0 : P.ncells + 1);
       const int c = cellc[p];
@@ -1044,6 +1127,198 @@ k_pairs_col(RsParams P, const int *__restrict__ cell_start, const int *__restric
    }
 }
 
+// The walk of k_pairs_col as a function: calls visit(j, inf) for every slot
+// j of the home cell (cx, cy, cz)'s stencil (the home slot among them), inf
+// = (offset index less the partner column's first cell) << 5 | image code:
+// the offset-table entry of slot j in cell c is c + (inf >> 5).  csk: the
+// cell starts of the slots walked.
+struct ColRows {
+   int *inc, *jb, *inf, *cand;
+};
+template <class Visit>
+__device__ __forceinline__ void walk_columns(const RsParams &P, const int *__restrict__ csk,
+                                             const int4 *__restrict__ cols, const int *__restrict__ col_base,
+                                             int cx, int cy, int cz, int lane, const ColRows &w, Visit &&visit)
+{
+   for (int base = 0; base < P.ncols; base += 32 * COL_E) {
+      int tot = 0;
+#pragma unroll
+      for (int u = 0; u < COL_E; u++) {
+         const int q0 = lane * 2 * COL_E + 2 * u;
+         w.inc[q0] = w.inc[q0 + 1] = 0;
+         w.jb[q0] = w.jb[q0 + 1] = 0;
+         w.inf[q0] = w.inf[q0 + 1] = 0;
+         const int col = base + lane * COL_E + u;
+         if (col < P.ncols) {
+            const int4 cd = __ldg(&cols[col]);
+            const int ob = __ldg(&col_base[col]);
+            const ColRuns cr = col_runs(P, cx, cy, cz, cd);
+#pragma unroll
+            for (int s = 0; s < 2; s++) {
+               if (s < cr.ns) {
+                  const int a = __ldg(&csk[cr.cc + cr.za[s]]), b = __ldg(&csk[cr.cc + cr.zb[s] + 1]);
+                  w.inc[q0 + s] = b - a;
+                  w.jb[q0 + s] = a;
+                  tot += b - a;
+                  const int eb = ob - cd.z - cz + cr.iz[s] * P.nz - cr.cc;
+                  w.inf[q0 + s] = eb * 32 | (9 * (cr.ix + 1) + 3 * (cr.iy + 1) + (cr.iz[s] + 1));
+               }
+            }
+         }
+      }
+      const int linc = warp_incl_scan(tot);
+      const int T = __shfl_sync(0xffffffffu, linc, 31);
+      int run = linc - tot;
+#pragma unroll
+      for (int r = 0; r < 2 * COL_E; r++) {
+         const int q = lane * 2 * COL_E + r;
+         w.jb[q] -= run;
+         run += w.inc[q];
+         w.inc[q] = run;
+      }
+      __syncwarp();
+      for (int w0 = 0; w0 < T; w0 += COL_WIN) {
+         const int w1 = min(T, w0 + COL_WIN);
+#pragma unroll
+         for (int r = 0; r < 2 * COL_E; r++) {
+            const int q = lane * 2 * COL_E + r;
+            const int e1 = w.inc[q], e0 = q > 0 ? w.inc[q - 1] : 0;
+            const int a = max(e0, w0), b = min(e1, w1);
+            const int jq = w.jb[q];
+            for (int t = a; t < b; t++) w.cand[t - w0] = (jq + t) | (q << 24);
+         }
+         __syncwarp();
+         for (int r0 = w0; r0 < w1; r0 += 32) {
+            const int idx = r0 + lane;
+            if (idx < w1) {
+               const int v = w.cand[idx - w0];
+               visit(v & 0xffffff, w.inf[(unsigned)v >> 24]);
+            }
+         }
+         __syncwarp();
+      }
+   }
+}
+
+// a < b for non-negative doubles, by their bits (a compare would take the
+// FP64 pipe); false when a is NaN
+__device__ __forceinline__ bool less_bits(double a, double b)
+{
+   return __double_as_longlong(a) < __double_as_longlong(b);
+}
+
+// The FP64 form by columns over one interaction class at a time: k_pairs'
+// FP64 arithmetic for r and r^2 (the reference's operation order), with the
+// cheaper square root, reciprocal and exponential of PairMath<double, true>.
+// The FP64 pipe bounds it: 131,072-site water (real-space phase) 9.75 ms
+// with k_pairs (every class, 110 FP64 instructions per pair), 4.61 ms here;
+// 2048-site water 0.220 -> 0.144 ms.
+template <int PT, bool EW>
+__global__ void __launch_bounds__(PAIR_WARPS * 32, 5)
+k_pairs_col64(RsParams P, const int *__restrict__ cs, const int *__restrict__ pre, const int4 *__restrict__ cols,
+              const int *__restrict__ col_base, const double4 *__restrict__ posc, const int2 *__restrict__ tagc,
+              const int *__restrict__ cellc, const int *__restrict__ sortc, const double *__restrict__ potg,
+              double *__restrict__ force, double *__restrict__ part, DevOut *out)
+{
+   constexpr int NP = NPar<PT>::v;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   __shared__ int s_inc[PAIR_WARPS][COL_ROWS], s_jb[PAIR_WARPS][COL_ROWS], s_inf[PAIR_WARPS][COL_ROWS];
+   __shared__ int s_cand[PAIR_WARPS][COL_WIN];
+   __shared__ double s_tot[7][PAIR_WARPS * 32];
+   __shared__ double s_reloc[27][3];
+   double *pot_s = reinterpret_cast<double *>(smem_raw);
+   if (P.pot_in_smem)
+      for (int q = threadIdx.x; q < P.max_id * P.max_id * NPOTP; q += blockDim.x) pot_s[q] = potg[q];
+   for (int q = threadIdx.x; q < 81; q += blockDim.x) s_reloc[q / 3][q % 3] = P.reloc[q / 3][q % 3];
+   if (EW || PT != 0) exp2_fill();
+#pragma unroll
+   for (int k = 0; k < 7; k++) s_tot[k][threadIdx.x] = 0.0;
+   __syncthreads();
+   const double *pot = P.pot_in_smem ? pot_s : potg;
+   const int N = P.nsites, n0 = P.one_class ? N : pre[N];
+   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   const ColRows rows{s_inc[w], s_jb[w], s_inf[w], s_cand[w]};
+   const bool strict = P.strict && !P.molpbc;
+   for (ColHome hm(P.chunk, w); hm.p < N; hm.next()) {
+      const int p = hm.p;
+      double fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
+      const int *csk = cs + (p < n0 ? 0 : P.ncells + 1);
+      const int c = cellc[p];
+      const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
+      const int2 ti = tagc[p];
+      const double *prow = pot + (size_t)(ti.x & 0xffff) * P.max_id * NPOTP;
+      const double4 xi = posc[p];
+      const int oi = sortc[p];
+      walk_columns(P, csk, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
+         const int kimg = inf & 31;
+         if (j == p && kimg == 13) return;
+         const double4 xj = posc[j];
+         const double *rl = s_reloc[kimg];
+         const double rx = __dadd_rn(__dsub_rn(xj.x, xi.x), rl[0]);
+         const double ry = __dadd_rn(__dsub_rn(xj.y, xi.y), rl[1]);
+         const double rz = __dadd_rn(__dsub_rn(xj.z, xi.z), rl[2]);
+         double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
+         const int2 tj = __ldg(&tagc[j]);
+         if (less_bits(r2, TOO_CLOSE) && ti.y != tj.y) {
+            const int oj = sortc[j];
+            if (oi < oj) note_too_close(out, oi, oj);
+         }
+         if (strict && less_bits(P.cut2, r2)) r2 = P.cut100;
+         double pp[NP];
+         const double *pj = prow + (size_t)(tj.x & 0xffff) * NPOTP;
+#pragma unroll
+         for (int k = 0; k < NP; k++) pp[k] = pj[k];
+         double f, u;
+         pair_fu<PT, EW, double, true>(r2, xj.w * xi.w, pp, P.alpha, P.norm, f, u);
+         const double wx = f * rx, wy = f * ry, wz = f * rz;
+         fx -= wx;
+         fy -= wy;
+         fz -= wz;
+         pe += u;
+         v0 = fma(wx, rx, v0);
+         v1 = fma(wx, ry, v1);
+         v2 = fma(wx, rz, v2);
+         v3 = fma(wy, ry, v3);
+         v4 = fma(wy, rz, v4);
+         v5 = fma(wz, rz, v5);
+      });
+      // the home site's force: warp trees; energy and virial (half of each
+      // evaluation) into the lane's totals
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+         fx += __shfl_down_sync(0xffffffffu, fx, o);
+         fy += __shfl_down_sync(0xffffffffu, fy, o);
+         fz += __shfl_down_sync(0xffffffffu, fz, o);
+      }
+      if (lane == 0) {
+         force[oi] = fx;
+         force[N + oi] = fy;
+         force[2 * N + oi] = fz;
+      }
+      s_tot[0][threadIdx.x] += pe;
+      s_tot[1][threadIdx.x] += v0;
+      s_tot[2][threadIdx.x] += v1;
+      s_tot[3][threadIdx.x] += v2;
+      s_tot[4][threadIdx.x] += v3;
+      s_tot[5][threadIdx.x] += v4;
+      s_tot[6][threadIdx.x] += v5;
+   }
+   __shared__ double wred[7][PAIR_WARPS];
+#pragma unroll
+   for (int k = 0; k < 7; k++) {
+      double s = s_tot[k][threadIdx.x];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) wred[k][w] = s;
+   }
+   __syncthreads();
+   if (threadIdx.x < 7) {
+      double s = 0.0;
+      for (int q = 0; q < PAIR_WARPS; q++) s += wred[threadIdx.x][q];
+      part[blockIdx.x * 8 + threadIdx.x] = 0.5 * s;
+   }
+}
+
 // The reference's evaluated pair count after a column-walk pass (which
 // leaves it out of the hot loop): per home slot the sites of every class in
 // the stencil's column runs, less the site itself, summed into
@@ -1169,17 +1444,19 @@ struct PairGrad {
    R uc, fc, duc, dfc;
 };
 
-template <int PT, bool EW, typename R>
+template <int PT, bool EW, typename R, bool FAST = false>
 __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, PairGrad<NPar<PT>::v, R> &g)
 {
-   const R r = dsqrt<R>(r2), r_r = R(1) / r, rs_r = r_r * r_r;
+   typedef PairMath<R, FAST> M;
+   const R r_f = FAST ? M::rsqrt(r2) : R(0);
+   const R r = FAST ? r2 * r_f : dsqrt<R>(r2), r_r = FAST ? r_f : R(1) / r, rs_r = r_r * r_r;
    g.uc = g.fc = g.duc = g.dfc = R(0);
    if (EW) {
       const R x = alpha * r;
-      const R t = R(1) / (R(1) + R(ASP) * x);
+      const R t = M::rcp(R(1) + R(ASP) * x);
       const R pt = R(AS1) + t * (R(AS2) + t * (R(AS3) + t * (R(AS4) + t * R(AS5))));
       const R dpt = R(AS2) + t * (R(2.0 * AS3) + t * (R(3.0 * AS4) + t * R(4.0 * AS5)));
-      const R ex = dexp<R>(-(x * x));
+      const R ex = M::ex(-(x * x));
       // d/dx [t P(t) e^{-x^2}] with dt/dx = -p t^2
       const R derfc = ex * (-R(ASP) * t * t * (pt + t * dpt) - R(2) * x * t * pt);
       g.uc = t * pt * ex * r_r;
@@ -1198,7 +1475,7 @@ __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, Pai
       g.df[0] = rs_r * R(6) * (R(2) * s12 - s6);
       g.df[1] = rs_r * R(36) * p[0] * t5 * (R(4) * s6 - R(1));
    } else if (PT == 1) {   // -p0/r^6 + p1 exp(-p2 r)
-      const R E = dexp<R>(-p[2] * r);
+      const R E = M::ex(-p[2] * r);
       const R r6 = rs_r * rs_r * rs_r;
       g.du[0] = -r6;
       g.du[1] = E;
@@ -1207,7 +1484,7 @@ __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, Pai
       g.df[1] = p[2] * E * r_r;
       g.df[2] = p[1] * E * (r_r - p[2]);
    } else if (PT == 2) {   // p0 exp(-p1 r) - p2 exp(-p3 r)
-      const R E1 = dexp<R>(-p[1] * r), E3 = dexp<R>(-p[3] * r);
+      const R E1 = M::ex(-p[1] * r), E3 = M::ex(-p[3] * r);
       const R e1 = p[0] * E1, e2 = -p[2] * E3;
       g.du[0] = E1;
       g.du[1] = -r * e1;
@@ -1218,7 +1495,7 @@ __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, Pai
       g.df[2] = -p[3] * E3 * r_r;
       g.df[3] = e2 * (r_r - p[3]);
    } else if (PT == 3) {   // p0 exp(-p1 r) + p2/r^12 - p3/r^4 - p4/r^6 - p5/r^8
-      const R E1 = dexp<R>(-p[1] * r), e1 = p[0] * E1;
+      const R E1 = M::ex(-p[1] * r), e1 = p[0] * E1;
       const R r4 = rs_r * rs_r, r6 = r4 * rs_r, r8 = r4 * r4, r12 = r6 * r6;
       g.du[0] = E1;
       g.du[1] = -r * e1;
@@ -1241,10 +1518,10 @@ __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, Pai
       g.df[1] = R(6) * rs_r * r6;
       g.df[2] = R(12) * rs_r * r12;
    } else {   // Morse: p0 e^{(p1-r)p2} - p3/r^6 + p4 (e^{-2 p5 (r-p6)} - 2 e^{-p5 (r-p6)})
-      const R E1 = dexp<R>((p[1] - r) * p[2]), e1 = p[0] * E1;
+      const R E1 = M::ex((p[1] - r) * p[2]), e1 = p[0] * E1;
       const R r6 = rs_r * rs_r * rs_r;
       const R d6 = r - p[6];
-      const R E2 = dexp<R>(R(-2) * p[5] * d6), E3 = dexp<R>(-p[5] * d6);
+      const R E2 = M::ex(R(-2) * p[5] * d6), E3 = M::ex(-p[5] * d6);
       const R e2 = p[4] * E2, e3 = R(-2) * p[4] * E3;
       g.du[0] = E1;
       g.du[1] = p[2] * e1;
@@ -1402,14 +1679,154 @@ k_pairs_adj(RsParams P, AdjParams A, const int *__restrict__ cell_start,
    for (int q = threadIdx.x; q < A.nslot; q += blockDim.x) gpart[(size_t)blockIdx.x * A.nslot + q] = s_acc[q];
 }
 
-// Slot sums over blocks, in block order.
-__global__ void k_adj_slots(const double *__restrict__ gpart, int nblocks, int nslot, double *__restrict__ slots)
+// The same over the columns of the link-cell order (both forms, without a
+// framework molecule or molecular cut-off): one walk for all partner
+// identifiers, each lane accumulating its table entries per identifier in
+// shared memory (a column of its own: no conflicts), and only the gradient
+// asked for (LOSS: of G, else of the energy).  FP64 form: the cheaper
+// primitives of PairMath<double, true>.  One walk instead of one per
+// identifier: 16,384-site water, mixed, 458 -> 137 us; 2048 sites, FP64,
+// 735 -> 250 us.  Dynamic shared memory: slot sums
+// [nslot] FP64, lane sums [types NP][threads], the potential table.
+template <int PT, bool EW, bool MIXED, bool LOSS>
+__global__ void __launch_bounds__(PAIR_WARPS * 32, MIXED ? 6 : 4)
+k_pairs_adj_col(RsParams P, AdjParams A, const int *__restrict__ cell_start, const int *__restrict__ slot_cell,
+                const int4 *__restrict__ cols, const int *__restrict__ col_base, const float4 *__restrict__ coff,
+                const double4 *__restrict__ pos64, const float4 *__restrict__ pos32, const int2 *__restrict__ tag,
+                const int *__restrict__ sorted, const double *__restrict__ site, const double *__restrict__ potg64,
+                const float *__restrict__ potg32, const double4 *__restrict__ res64, const float4 *__restrict__ res32,
+                double *__restrict__ gq, double *__restrict__ gpart)
 {
-   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-   if (q >= nslot) return;
+   typedef typename std::conditional<MIXED, float, double>::type R;
+   constexpr int NP = NPar<PT>::v, NT = PAIR_WARPS * 32;
+   extern __shared__ double s_acc[];
+   __shared__ int s_inc[PAIR_WARPS][COL_ROWS], s_jb[PAIR_WARPS][COL_ROWS], s_inf[PAIR_WARPS][COL_ROWS];
+   __shared__ int s_cand[PAIR_WARPS][COL_WIN];
+   R *s_lane = reinterpret_cast<R *>(s_acc + A.nslot), *pot = s_lane + A.ntype * NP * NT;
+   const int npot = P.max_id * P.max_id;
+   for (int q = threadIdx.x; q < A.nslot; q += NT) s_acc[q] = 0.0;
+   for (int q = threadIdx.x; q < npot * NPOTP; q += NT) pot[q] = MIXED ? (R)potg32[q] : (R)potg64[q];
+   if (!MIXED) exp2_fill();
+   __syncthreads();
+   const int N = P.nsites, T = npot * NP;
+   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   const ColRows rows{s_inc[w], s_jb[w], s_inf[w], s_cand[w]};
+   R *acc = s_lane + threadIdx.x;
+   const R alpha = MIXED ? (R)P.alphaf : (R)P.alpha, norm = MIXED ? (R)P.normf : (R)P.norm;
+   const R cut100 = (R)P.cut100;
+   for (ColHome hm(P.chunk, w); hm.p < N; hm.next()) {
+      const int p = hm.p;
+      for (int q = 0; q < A.ntype * NP; q++) acc[q * NT] = R(0);
+      const int c = slot_cell[p];
+      const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
+      const int2 ti = tag[p];
+      const R *prow = pot + (size_t)ti.x * P.max_id * NPOTP;
+      double4 xi64 = make_double4(0, 0, 0, 0);
+      float4 xi32 = make_float4(0, 0, 0, 0);
+      if (MIXED) xi32 = pos32[p]; else xi64 = pos64[p];
+      const R qi = MIXED ? (R)xi32.w : (R)xi64.w;
+      R vix = 0, viy = 0, viz = 0;
+      if (LOSS) {
+         if (MIXED) {
+            const float4 v = res32[p];
+            vix = v.x; viy = v.y; viz = v.z;
+         } else {
+            const double4 v = res64[p];
+            vix = v.x; viy = v.y; viz = v.z;
+         }
+      }
+      const int oi = sorted[p];
+      R gqs = 0, gas = 0;
+      walk_columns(P, cell_start, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
+         const int kimg = inf & 31;
+         if (j == p && kimg == 13) return;
+         const int2 tj = __ldg(&tag[j]);
+         if (!LOSS && ti.y == tj.y) return;
+         R rx, ry, rz, r2, qj;
+         if (MIXED) {
+            const float4 xj = __ldg(&pos32[j]);
+            float4 h4, l4;
+            ld_coff(coff + 2 * (__ldg(&slot_cell[j]) + (inf >> 5)), h4, l4);
+            rx = (h4.x + (xj.x - xi32.x)) + l4.x;
+            ry = (h4.y + (xj.y - xi32.y)) + l4.y;
+            rz = (h4.z + (xj.z - xi32.z)) + l4.z;
+            r2 = rx * rx + ry * ry + rz * rz;
+            qj = xj.w;
+         } else {
+            const double4 xj = pos64[j];
+            const double *rl = P.reloc[kimg];
+            rx = __dadd_rn(__dsub_rn(xj.x, xi64.x), rl[0]);
+            ry = __dadd_rn(__dsub_rn(xj.y, xi64.y), rl[1]);
+            rz = __dadd_rn(__dsub_rn(xj.z, xi64.z), rl[2]);
+            r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
+            qj = xj.w;
+         }
+         if (P.strict) {
+            bool too_close, clip;
+            pair_flags<MIXED>(P, r2, oi, j, kimg, sorted, site, too_close, clip);
+            if (clip) r2 = cut100;
+         }
+         R pp[NP];
+         const R *pj = prow + (size_t)tj.x * NPOTP;
+#pragma unroll
+         for (int q = 0; q < NP; q++) pp[q] = pj[q];
+         PairGrad<NP, R> g;
+         pair_grad<PT, EW, R, !MIXED>(r2, pp, alpha, norm, g);
+         R *aj = acc + (int)A.type_index[tj.x] * NP * NT;
+         if (LOSS) {
+            R vjx, vjy, vjz;
+            if (MIXED) {
+               const float4 v = __ldg(&res32[j]);
+               vjx = v.x; vjy = v.y; vjz = v.z;
+            } else {
+               const double4 v = res64[j];
+               vjx = v.x; vjy = v.y; vjz = v.z;
+            }
+            const R wi = vix * rx + viy * ry + viz * rz;            // v_i . r
+            const R ws = wi - (vjx * rx + vjy * ry + vjz * rz);      // (v_i - v_j) . r
+#pragma unroll
+            for (int q = 0; q < NP; q++) aj[q * NT] -= g.df[q] * wi;
+            gqs -= qj * g.fc * ws;
+            gas -= qj * g.dfc * wi;
+         } else {
+#pragma unroll
+            for (int q = 0; q < NP; q++) aj[q * NT] += g.du[q];
+            gqs += qj * g.uc;
+            gas += qj * g.duc;
+         }
+      });
+      double *se = s_acc + (LOSS ? T : 0) + (size_t)ti.x * P.max_id * NP;
+      for (int b = 0; b < P.max_id; b++) {
+         if (!((A.type_mask >> b) & 1u)) continue;
+#pragma unroll
+         for (int q = 0; q < NP; q++) {
+            const R s = warp_sum(acc[((int)A.type_index[b] * NP + q) * NT]);
+            if (lane == 0) atomicAdd(se + b * NP + q, LOSS ? (double)s : 0.5 * (double)s);
+         }
+      }
+      gqs = warp_sum(gqs);
+      gas = warp_sum(gas);
+      if (lane == 0) {
+         gq[(LOSS ? N : 0) + oi] = (double)gqs;
+         atomicAdd(s_acc + 2 * T + (LOSS ? 1 : 0), (LOSS ? 1.0 : 0.5) * (double)qi * (double)gas);
+      }
+   }
+   __syncthreads();
+   for (int q = threadIdx.x; q < A.nslot; q += NT) gpart[(size_t)blockIdx.x * A.nslot + q] = s_acc[q];
+}
+
+// Slot sums over blocks: one block per slot, in a fixed order.
+__global__ void __launch_bounds__(128) k_adj_slots(const double *__restrict__ gpart, int nblocks, int nslot,
+                                                   double *__restrict__ slots)
+{
+   __shared__ double sh[4];
+   const int q = blockIdx.x;
    double s = 0.0;
-   for (int b = 0; b < nblocks; b++) s += gpart[(size_t)b * nslot + q];
-   slots[q] = s;
+   for (int b = threadIdx.x; b < nblocks; b += 128) s += gpart[(size_t)b * nslot + q];
+   s = warp_sum(s);
+   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+   __syncthreads();
+   if (threadIdx.x == 0) slots[q] = (sh[0] + sh[1]) + (sh[2] + sh[3]);
 }
 
 // --------------------------------------------------------------------- RDF
@@ -1647,11 +2064,38 @@ static cudaError_t launch_pairs_pt(const RsParams &P, mdgpu_ctx *c, bool ew, boo
              : launch_pairs_t<PT, false, false, 0>(P, c, force, out, keys, key_cap, smem);
 }
 
+static bool col_walk_ok(const mdgpu_ctx *c);
+
+template <int PT, bool EW, bool MIXED, bool LOSS>
+static cudaError_t launch_adj_col_t(const RsParams &P, const AdjParams &A, mdgpu_ctx *c, int nblk, size_t smem)
+{
+   RsDev &d = c->rd;
+   AdjDev &a = c->ad;
+   auto kfn = k_pairs_adj_col<PT, EW, MIXED, LOSS>;
+   if (smem > 24 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   kfn<<<nblk, PAIR_WARPS * 32, smem, c->stream>>>(P, A, d.cell_start.p, d.slot_cell.p, d.cols.p, d.col_base.p,
+                                                   d.coff.p, d.pos64.p, d.pos32.p, d.tag.p, d.sorted.p, c->cur_site,
+                                                   d.pot64.p, d.pot32.p, a.res64.p, a.res32.p, a.gq.p, a.gpart.p);
+   return cudaGetLastError();
+}
+
 template <int PT, bool EW, bool MIXED>
 static cudaError_t launch_adj_t(const RsParams &P, const AdjParams &A, mdgpu_ctx *c, int nblk)
 {
    RsDev &d = c->rd;
    AdjDev &a = c->ad;
+   // the column walk keeps lane sums and the potential table in shared
+   // memory: within 160 KB (it needs 28 KB with four identifiers and two
+   // parameters, the benchmark's water)
+   const size_t smem = A.nslot * sizeof(double) +
+                       ((size_t)A.ntype * NPar<PT>::v * PAIR_WARPS * 32 + (size_t)P.max_id * P.max_id * NPOTP) *
+                          (MIXED ? sizeof(float) : sizeof(double));
+   if (col_walk_ok(c) && smem <= 160 * 1024)
+      return A.loss ? launch_adj_col_t<PT, EW, MIXED, true>(P, A, c, nblk, smem)
+                    : launch_adj_col_t<PT, EW, MIXED, false>(P, A, c, nblk, smem);
    k_pairs_adj<PT, EW, MIXED><<<nblk, PAIR_WARPS * 32, A.nslot * sizeof(double), c->stream>>>(
       P, A, d.cell_start.p, d.slot_cell.p, d.full.p, d.off_hi.p, d.off_lo.p, d.pos64.p, d.pos32.p, d.tag.p,
       d.sorted.p, c->cur_site, d.pot64.p, d.pot32.p, a.res64.p, a.res32.p, a.gq.p, a.gpart.p);
@@ -1693,8 +2137,11 @@ mdgpu_status rs_adjoint(mdgpu_ctx *c, bool loss)
    A.type_mask = 0;
    for (int id : c->site_id) A.type_mask |= 1u << id;
    A.nslot = 2 * c->max_id * c->max_id * np + 2;
+   A.ntype = 0;
+   for (int b = 0; b < MDGPU_ADJ_MAX_ID; b++) A.type_index[b] = (unsigned char)((A.type_mask >> b) & 1u ? A.ntype++ : 0);
    int nblk = (N + PAIR_WARPS - 1) / PAIR_WARPS;
    if (nblk > 4 * 152) nblk = 4 * 152;
+   P.chunk = col_chunk(N, nblk);
    CK(a.gq.ensure(2 * (size_t)N));
    CK(a.gpart.ensure((size_t)nblk * A.nslot));
    CK(a.slots.ensure((size_t)A.nslot));
@@ -1710,7 +2157,7 @@ mdgpu_status rs_adjoint(mdgpu_ctx *c, bool loss)
    default: return fail(c, MDGPU_E_PTYPE, "KERNEL called with unknown potential type");
    }
    CK(e);
-   k_adj_slots<<<(A.nslot + 255) / 256, 256, 0, st>>>(a.gpart.p, nblk, A.nslot, a.slots.p);
+   k_adj_slots<<<A.nslot, 128, 0, st>>>(a.gpart.p, nblk, A.nslot, a.slots.p);
    CK(cudaGetLastError());
    c->launches += 2;
    return MDGPU_OK;
@@ -1780,7 +2227,8 @@ mdgpu_status rs_launch(mdgpu_ctx *c, const double *d_site, const double *d_cofm,
    const bool mixed = c->prec == MDGPU_MIXED && d_keys == nullptr;
    k_gather<<<(N + 255) / 256, 256, 0, st>>>(P, d_site, d.chg.p, d.siteid.p, d.molmap.p, d.sorted.p,
                                              d.cell_of.p, mixed ? nullptr : d.pos64.p,
-                                             mixed ? d.pos32.p : nullptr, d.tag.p, d.slot_cell.p);
+                                             d_keys == nullptr ? d.pos32.p : nullptr, d.tag.p,
+                                             c->ncls == 1 || !c->rs.nbr27 ? d.tagc.p : nullptr, d.slot_cell.p);
    CK(cudaGetLastError());
    c->launches += 7;
    phase_mark(c, MDGPU_PH_PAIRS);
@@ -1789,7 +2237,7 @@ mdgpu_status rs_launch(mdgpu_ctx *c, const double *d_site, const double *d_cofm,
 #undef CK
 }
 
-// The column walk serves the mixed form without a framework molecule or
+// The column walk serves both forms without a framework molecule or
 // molecular cut-off, where every stencil column wraps the cell at most once.
 static bool col_walk_ok(const mdgpu_ctx *c)
 {
@@ -1802,55 +2250,74 @@ static bool col_walk_ok(const mdgpu_ctx *c)
 }
 
 template <int PT, bool EW>
-static cudaError_t launch_col_t(const RsParams &P, mdgpu_ctx *c, double *force, size_t smem, int nb)
+static cudaError_t launch_col_t(const RsParams &P, mdgpu_ctx *c, double *force, bool mixed, size_t smem, int nb)
 {
    RsDev &d = c->rd;
+   if (!mixed) {
+      auto kfn = k_pairs_col64<PT, EW>;
+      if (smem > 16 * 1024) {
+         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+         if (e != cudaSuccess) return e;
+      }
+      kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(
+         P, P.one_class ? d.cell_start.p : d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p,
+         P.one_class ? d.pos64.p : d.posc64.p, d.tagc.p, P.one_class ? d.slot_cell.p : d.cellc.p,
+         P.one_class ? d.sorted.p : d.sortc.p, d.pot64.p, force, d.part.p, c->out.p);
+      return cudaGetLastError();
+   }
    auto kfn = k_pairs_col<PT, EW>;
    if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
    }
-   kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, d.cell_start.p, d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p,
-                                                 d.coff.p, d.posc.p, d.tagc.p, d.cellc.p,
-                                                 d.sortc.p, c->cur_site, d.pot32.p, force, d.part.p, c->out.p);
+   kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(
+      P, P.one_class ? d.cell_start.p : d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p, d.coff.p,
+      P.one_class ? d.pos32.p : d.posc.p, d.tagc.p, P.one_class ? d.slot_cell.p : d.cellc.p,
+      P.one_class ? d.sorted.p : d.sortc.p, c->cur_site, d.pot32.p, force, d.part.p, c->out.p);
    return cudaGetLastError();
 }
 
 // Class split of the binned slots, the column-walk pair kernel and, with
 // two classes, the too-close scan across them.
-static mdgpu_status rs_pairs_col(mdgpu_ctx *c, const RsParams &P, double *d_force, bool ew, size_t smem)
+static mdgpu_status rs_pairs_col(mdgpu_ctx *c, RsParams P, double *d_force, bool ew, bool mixed, size_t smem)
 {
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
    RsDev &d = c->rd;
    cudaStream_t st = c->stream;
-   const int N = c->nsites, M = c->max_id;
+   const int N = c->nsites;
    const bool two = c->ncls == 2 && c->rs.nbr27;
-   const int *cls = d.cls_of_id.p + (two ? 0 : M);
+   const int *cls = d.cls_of_id.p;
    const int n1 = N + 1, nbs = (n1 + 1023) / 1024;
-   k_cls_flag<<<(n1 + 255) / 256, 256, 0, st>>>(N, d.tag.p, cls, d.cls_pre.p);
-   k_scan_blocks<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_pre.p, d.cls_bsum.p, n1);
-   k_scan_sums<<<1, 1024, 0, st>>>(d.cls_bsum.p, nbs, d.cls_bsum.p + nbs);
-   k_scan_add<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_bsum.p, n1);
-   const int nsplit = std::max(N, P.ncells + 1);
-   k_cls_split<<<(nsplit + 255) / 256, 256, 0, st>>>(P, d.cls_pre.p, cls, d.cell_start.p, d.pos32.p, d.tag.p,
-                                                    d.sorted.p, d.slot_cell.p, d.cs.p, d.posc.p, d.tagc.p,
-                                                    d.sortc.p, d.cellc.p);
-   CK(cudaGetLastError());
-   c->launches += 5;
+   P.one_class = !two;
+   // one class: the link-cell order as it is (k_gather wrote the packed tags)
+   if (two) {
+      k_cls_flag<<<(n1 + 255) / 256, 256, 0, st>>>(N, d.tag.p, cls, d.cls_pre.p);
+      k_scan_blocks<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_pre.p, d.cls_bsum.p, n1);
+      k_scan_sums<<<1, 1024, 0, st>>>(d.cls_bsum.p, nbs, d.cls_bsum.p + nbs);
+      k_scan_add<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_bsum.p, n1);
+      if (!mixed) CK(d.posc64.ensure(N));
+      const int nsplit = std::max(N, P.ncells + 1);
+      k_cls_split<<<(nsplit + 255) / 256, 256, 0, st>>>(P, d.cls_pre.p, cls, d.cell_start.p, d.pos32.p, d.tag.p,
+                                                       d.sorted.p, d.slot_cell.p, d.pos64.p, d.cs.p, d.posc.p,
+                                                       mixed ? nullptr : d.posc64.p, d.tagc.p, d.sortc.p, d.cellc.p);
+      CK(cudaGetLastError());
+      c->launches += 5;
+   }
    // eight resident blocks per SM (the kernel's launch bounds), each warp
    // looping over home sites: the per-block set-up and energy reduction once
    // per block instead of once per four sites
    if (c->nsm <= 0) CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
-   const int nb = std::min((N + PAIR_WARPS - 1) / PAIR_WARPS, 8 * c->nsm);
+   const int nb = std::min((N + PAIR_WARPS - 1) / PAIR_WARPS, (mixed ? 8 : 5) * c->nsm);
    c->rs_nblk = nb;
+   P.chunk = col_chunk(N, nb);
    cudaError_t e;
    switch (c->ptype) {
-   case 0: e = ew ? launch_col_t<0, true>(P, c, d_force, smem, nb) : launch_col_t<0, false>(P, c, d_force, smem, nb); break;
-   case 1: e = ew ? launch_col_t<1, true>(P, c, d_force, smem, nb) : launch_col_t<1, false>(P, c, d_force, smem, nb); break;
-   case 2: e = ew ? launch_col_t<2, true>(P, c, d_force, smem, nb) : launch_col_t<2, false>(P, c, d_force, smem, nb); break;
-   case 3: e = ew ? launch_col_t<3, true>(P, c, d_force, smem, nb) : launch_col_t<3, false>(P, c, d_force, smem, nb); break;
-   case 4: e = ew ? launch_col_t<4, true>(P, c, d_force, smem, nb) : launch_col_t<4, false>(P, c, d_force, smem, nb); break;
-   case 6: e = ew ? launch_col_t<6, true>(P, c, d_force, smem, nb) : launch_col_t<6, false>(P, c, d_force, smem, nb); break;
+   case 0: e = ew ? launch_col_t<0, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<0, false>(P, c, d_force, mixed, smem, nb); break;
+   case 1: e = ew ? launch_col_t<1, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<1, false>(P, c, d_force, mixed, smem, nb); break;
+   case 2: e = ew ? launch_col_t<2, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<2, false>(P, c, d_force, mixed, smem, nb); break;
+   case 3: e = ew ? launch_col_t<3, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<3, false>(P, c, d_force, mixed, smem, nb); break;
+   case 4: e = ew ? launch_col_t<4, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<4, false>(P, c, d_force, mixed, smem, nb); break;
+   case 6: e = ew ? launch_col_t<6, true>(P, c, d_force, mixed, smem, nb) : launch_col_t<6, false>(P, c, d_force, mixed, smem, nb); break;
    default: return fail(c, MDGPU_E_PTYPE, "KERNEL called with unknown potential type");
    }
    CK(e);
@@ -1876,7 +2343,7 @@ mdgpu_status rs_count_pairs(mdgpu_ctx *c)
    cudaStream_t st = c->stream;
    DevOut *out = c->out.p;
    CK(cudaMemsetAsync(&out->npairs2, 0, sizeof(out->npairs2), st));
-   k_count_col<<<(c->nsites + 255) / 256, 256, 0, st>>>(P, c->rd.cell_start.p, c->rd.cols.p, c->rd.cellc.p, out);
+   k_count_col<<<(c->nsites + 255) / 256, 256, 0, st>>>(P, c->rd.cell_start.p, c->rd.cols.p, c->rd.slot_cell.p, out);
    CK(cudaGetLastError());
    int64_t n2 = 0;
    CK(cudaMemcpyAsync(&n2, &out->npairs2, sizeof(n2), cudaMemcpyDeviceToHost, st));
@@ -1904,8 +2371,8 @@ mdgpu_status rs_pairs(mdgpu_ctx *c, double *d_force, unsigned long long *d_keys,
    cudaError_t e;
    c->npairs_pending = false;
    c->rs_nblk = (N + PAIR_WARPS - 1) / PAIR_WARPS;   // blocks of partial sums for the reduction
-   if (mode == 0 && mixed && col_walk_ok(c)) {
-      const mdgpu_status s = rs_pairs_col(c, P, d_force, ew, smem);
+   if (mode == 0 && col_walk_ok(c)) {
+      const mdgpu_status s = rs_pairs_col(c, P, d_force, ew, mixed, smem);
       if (s != MDGPU_OK) return s;
       c->npairs_pending = true;   // counted on demand (rs_count_pairs)
    } else {
