@@ -32,24 +32,9 @@ mdgpu_status cuda_check(mdgpu_ctx *c, cudaError_t e, const char *what)
 static const double CONV_E = 0.001 * 6.0221367e23 * 1.6605402e-27 * 1.0e4;
 static const double CONV_Q = (4.07497263794495e-14 * 1.0e-3 * 1.05482230112e-05) / 1.60217733e-19;
 
-__global__ void k_finalize(const DevOut *out, double eintra, double self, double sheet_v,
-                           int has_ewald, double *pe_out, double *stress_out)
+__global__ void k_finalize(DevOut *out, FinArgs fin)
 {
-   if (threadIdx.x != 0) return;
-   pe_out[0] = -eintra + out->pe_rs;
-   pe_out[1] = has_ewald ? (-self + sheet_v) + out->pe_k : 0.0;
-   const double *v = out->vir_rs, *s = out->st_k;
-   const double d = has_ewald ? sheet_v : 0.0;
-   const double e = has_ewald ? 1.0 : 0.0;
-   stress_out[0] = v[0] + e * s[0] + d;
-   stress_out[1] = v[1] + e * s[1];
-   stress_out[2] = v[2] + e * s[2];
-   stress_out[3] = 0.0;
-   stress_out[4] = v[3] + e * s[3] + d;
-   stress_out[5] = v[4] + e * s[4];
-   stress_out[6] = 0.0;
-   stress_out[7] = 0.0;
-   stress_out[8] = v[5] + e * s[5] + d;
+   if (threadIdx.x == 0) finalize_eval(out, fin);
 }
 
 // f += f_in and sum_i x_i (x) f_in_i, the part of the reference's virial
@@ -82,13 +67,14 @@ __global__ void k_add_in(int N, const double *__restrict__ site, const double *_
    }
 }
 
+// one warp per component, a fixed order
 __global__ void k_sum_in(const double *__restrict__ part, int nb, DevOut *out)
 {
-   int k = threadIdx.x;
-   if (k >= 6) return;
+   const int k = threadIdx.x >> 5;
    double s = 0;
-   for (int b = 0; b < nb; b++) s += part[b * 8 + k];
-   out->vir_in[k] = s;
+   for (int b = threadIdx.x & 31; b < nb; b += 32) s += part[b * 8 + k];
+   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+   if ((threadIdx.x & 31) == 0) out->vir_in[k] = s;
 }
 
 }  // namespace mdgpu
@@ -230,11 +216,53 @@ mdgpu_status mdgpu::sync_out(mdgpu_ctx *c)
 
 #define CKR(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
 
-static mdgpu_status upload_sites(mdgpu_ctx *c, double *const site[3], const double *c_of_m)
+// The reference-style calls pass six host arrays in and three out.  Small
+// ones are gathered into one buffer first, one copy each way instead of nine
+// (each costs the host 5-15 us of its own); larger ones go directly.
+static const size_t STAGE_MAX = 1u << 18;   // doubles
+
+static bool stage(mdgpu_ctx *c, size_t n)
+{
+   if (n > STAGE_MAX) return false;
+   if (c->h_stage.size() < n) c->h_stage.resize(n);
+   return true;
+}
+
+// parts[k][N], k < np, to dst[np][N] (the staging buffer's last use is over:
+// every host call that stages also waits)
+static mdgpu_status copy_in(mdgpu_ctx *c, double *dst, const double *const *parts, int np, size_t at, bool staged)
 {
    const size_t N = c->nsites;
-   for (int k = 0; k < 3; k++)
-      CKR(cudaMemcpyAsync(c->site.p + k * N, site[k], N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+   if (staged) {
+      double *h = c->h_stage.data() + at;
+      for (int k = 0; k < np; k++) std::memcpy(h + k * N, parts[k], N * sizeof(double));
+      CKR(cudaMemcpyAsync(dst, h, np * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+      return MDGPU_OK;
+   }
+   for (int k = 0; k < np; k++)
+      CKR(cudaMemcpyAsync(dst + k * N, parts[k], N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+   return MDGPU_OK;
+}
+
+// The forces back into the caller's arrays, waiting for the stream.
+static mdgpu_status copy_out_sync(mdgpu_ctx *c, double *const force[3], bool staged)
+{
+   const size_t N = c->nsites;
+   if (staged) {
+      CKR(cudaMemcpyAsync(c->h_stage.data(), c->force.p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+   } else {
+      for (int k = 0; k < 3; k++)
+         CKR(cudaMemcpyAsync(force[k], c->force.p + k * N, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+   }
+   const mdgpu_status s = sync_out(c);
+   if (s != MDGPU_OK) return s;
+   if (staged)
+      for (int k = 0; k < 3; k++) std::memcpy(force[k], c->h_stage.data() + k * N, N * sizeof(double));
+   return MDGPU_OK;
+}
+
+static mdgpu_status upload_cofm(mdgpu_ctx *c, const double *c_of_m)
+{
    if (c->ctl.molpbc) {
       if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       c->last_cofm.assign(c_of_m, c_of_m + 3 * (size_t)c->nmols);
@@ -470,8 +498,16 @@ mdgpu_status mdgpu_forces_device(mdgpu_ctx *c, const double *h, const double *d_
    mdgpu_status s = ensure_ready(c, h, true, true);
    if (s) return s;
    for (bool &m : c->ev_marked) m = false;
-   CKR(cudaMemsetAsync(c->out.p, 0, sizeof(DevOut), c->stream));
    const bool ew = c->ctl.alpha > ALPHAMIN;
+   // the evaluation's last kernel adds its parts up
+   c->fin = FinArgs();
+   c->fin.on = 1;
+   c->fin.has_ewald = ew ? 1 : 0;
+   c->fin.eintra = eintra_subtracted(c);
+   c->fin.self = c->self_energy;
+   c->fin.sheet_v = ew ? c->sheet_energy / c->kl.vol : 0.0;
+   c->fin.pe = d_pe;
+   c->fin.st = d_stress;
    // With Ewald, the k-space passes (FP32-pipe-bound) run on a second,
    // high-priority stream beside the pair kernel (latency- and integer-bound),
    // so their blocks fill the SMs as pair blocks retire; the k-space force
@@ -480,18 +516,39 @@ mdgpu_status mdgpu_forces_device(mdgpu_ctx *c, const double *h, const double *d_
    // overlap: the fork event is recorded as soon as the link-cell order is
    // complete, so the per-slot records of the pair kernel are built beside
    // the first k-space passes
+   struct FinOff {   // (not left on for a later call, whatever happens)
+      mdgpu_ctx *c;
+      ~FinOff()
+      {
+         c->fin.on = 0;
+         c->pairs_after_tables = nullptr;
+      }
+   } fin_off{c};
    s = rs_launch(c, d_site, d_cofm, d_force, overlap, nullptr, 0, overlap ? c->ev_fork : nullptr);
    if (s) return s;
    if (overlap) {
       cudaStream_t main = c->stream;
       CKR(cudaStreamWaitEvent(c->side_stream, c->ev_fork, 0));
-      s = rs_pairs(c, d_force, nullptr, 0);
-      if (s) return s;
-      CKR(cudaEventRecord(c->ev_pairs, main));
+      // A pair kernel that fills the GPU waits for the k-space tables, so that
+      // the structure factor's CTAs (one per SM, on the stream of higher
+      // priority) start before the pair blocks take every SM: those then fill
+      // what is left.  Below 8 x 152 x 4 sites both start at once (131,072-site
+      // water, mixed: 1.153 ms with the pair kernel first, 1.138 ms so).
+      c->pairs_after_tables = c->nsites >= 32 * 152 && c->tc_sfac && c->nsites == c->fw_site0 ? main : nullptr;
+      if (!c->pairs_after_tables) {
+         s = rs_pairs(c, d_force, nullptr, 0);
+         if (s) return s;
+         CKR(cudaEventRecord(c->ev_pairs, main));
+      }
       c->stream = c->side_stream;
       s = ks_launch(c, d_site, d_force, true, c->ev_pairs);
       c->stream = main;
       if (s) return s;
+      if (c->pairs_after_tables) {   // no k-space pass ran
+         c->pairs_after_tables = nullptr;
+         s = rs_pairs(c, d_force, nullptr, 0);
+         if (s) return s;
+      }
       CKR(cudaEventRecord(c->ev_join, c->side_stream));
       CKR(cudaStreamWaitEvent(main, c->ev_join, 0));
    } else if (ew) {
@@ -500,10 +557,12 @@ mdgpu_status mdgpu_forces_device(mdgpu_ctx *c, const double *h, const double *d_
    } else {
       phase_mark(c, MDGPU_PH_FINAL);
    }
-   k_finalize<<<1, 32, 0, c->stream>>>(c->out.p, eintra_subtracted(c), c->self_energy,
-                                       ew ? c->sheet_energy / c->kl.vol : 0.0, ew ? 1 : 0, d_pe, d_stress);
-   CKR(cudaGetLastError());
-   c->launches += 1;
+   if (c->fin.on) {
+      k_finalize<<<1, 32, 0, c->stream>>>(c->out.p, c->fin);
+      CKR(cudaGetLastError());
+      c->launches += 1;
+      c->fin.on = 0;
+   }
    phase_mark(c, MDGPU_NPHASES);
    return MDGPU_OK;
 }
@@ -525,13 +584,11 @@ mdgpu_status mdgpu_forces(mdgpu_ctx *c, const double *h, const double *site_soa,
    s = mdgpu_forces_device(c, h, c->site.p, c->cofm_in.p, c->force.p, d_small, d_small + 2);
    if (s) return s;
    CKR(cudaMemcpyAsync(force_out, c->force.p, 3 * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-   double small[11];
-   CKR(cudaMemcpyAsync(small, d_small, sizeof small, cudaMemcpyDeviceToHost, c->stream));
    s = sync_out(c);
    if (s) return s;
-   pe_out[0] = small[0];
-   pe_out[1] = small[1];
-   std::memcpy(stress_out, small + 2, 9 * sizeof(double));
+   pe_out[0] = c->h_out->fin[0];
+   pe_out[1] = c->h_out->fin[1];
+   std::memcpy(stress_out, c->h_out->fin + 2, 9 * sizeof(double));
    return MDGPU_OK;
 }
 
@@ -543,21 +600,18 @@ mdgpu_status mdgpu_force_calc(mdgpu_ctx *c, const double *h, double *const site[
    mdgpu_status s = ensure_ready(c, h, true, false);
    if (s) return s;
    const size_t N = c->nsites;
-   s = upload_sites(c, site, c_of_m);
-   if (s) return s;
-   for (int k = 0; k < 3; k++)
-      CKR(cudaMemcpyAsync(c->force_in.p + k * N, site_force[k], N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-   CKR(cudaMemsetAsync(c->out.p, 0, sizeof(DevOut), c->stream));
+   const bool staged = stage(c, 6 * N);
+   if ((s = copy_in(c, c->site.p, site, 3, 0, staged)) != MDGPU_OK || (s = upload_cofm(c, c_of_m)) != MDGPU_OK ||
+       (s = copy_in(c, c->force_in.p, site_force, 3, 3 * N, staged)) != MDGPU_OK)
+      return s;
    s = rs_launch(c, c->site.p, c->cofm_in.p, c->force.p, false, nullptr, 0, nullptr);
    if (s) return s;
    const int nb = (int)((N + 255) / 256);
    CKR(c->rd.part.ensure((size_t)nb * 8 > c->rd.part.n ? (size_t)nb * 8 : c->rd.part.n));
    k_add_in<<<nb, 256, 0, c->stream>>>((int)N, c->site.p, c->force_in.p, c->force.p, c->rd.part.p);
-   k_sum_in<<<1, 32, 0, c->stream>>>(c->rd.part.p, nb, c->out.p);
+   k_sum_in<<<1, 192, 0, c->stream>>>(c->rd.part.p, nb, c->out.p);
    CKR(cudaGetLastError());
-   for (int k = 0; k < 3; k++)
-      CKR(cudaMemcpyAsync(site_force[k], c->force.p + k * N, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-   s = sync_out(c);
+   s = copy_out_sync(c, site_force, staged);
    if (s) return s;
    const DevOut &o = *c->h_out;
    *pe -= eintra_subtracted(c);
@@ -576,24 +630,20 @@ mdgpu_status mdgpu_ewald(mdgpu_ctx *c, const double *h, double *const site[3],
    mdgpu_status s = ensure_ready(c, h, true, true);
    if (s) return s;
    const size_t N = c->nsites;
-   for (int k = 0; k < 3; k++) {
-      CKR(cudaMemcpyAsync(c->site.p + k * N, site[k], N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-      CKR(cudaMemcpyAsync(c->force.p + k * N, site_force[k], N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-   }
+   const bool staged = stage(c, 6 * N);
+   if ((s = copy_in(c, c->site.p, site, 3, 0, staged)) != MDGPU_OK || (s = copy_in(c, c->force.p, site_force, 3, 3 * N, staged)) != MDGPU_OK)
+      return s;
    if (c->ctl.molpbc) {   // binning by molecule: the centres of mass are on the host record only
       if (c->last_cofm.size() != 3 * (size_t)c->nmols)
          return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass (call force_calc first)");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c->last_cofm.data(), 3 * c->nmols * sizeof(double),
                           cudaMemcpyHostToDevice, c->stream));
    }
-   CKR(cudaMemsetAsync(c->out.p, 0, sizeof(DevOut), c->stream));
    s = rs_launch(c, c->site.p, c->cofm_in.p, c->force.p, true, nullptr, 0, nullptr);
    if (s) return s;
    s = ks_launch(c, c->site.p, c->force.p, true);
    if (s) return s;
-   for (int k = 0; k < 3; k++)
-      CKR(cudaMemcpyAsync(site_force[k], c->force.p + k * N, N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-   s = sync_out(c);
+   s = copy_out_sync(c, site_force, staged);
    if (s) return s;
    const DevOut &o = *c->h_out;
    const double sv = c->sheet_energy / c->kl.vol;
@@ -637,8 +687,10 @@ mdgpu_status mdgpu_rdf_counts(mdgpu_ctx *c, const double *h, const double *site_
       if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c_of_m, 3 * c->nmols * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    }
-   CKR(cudaMemsetAsync(c->out.p, 0, sizeof(DevOut), c->stream));
-   if ((s = rs_launch(c, c->site.p, c->cofm_in.p, c->force.p, true, nullptr, 0, nullptr)) != MDGPU_OK) return s;
+   c->link_order = true;
+   s = rs_launch(c, c->site.p, c->cofm_in.p, c->force.p, true, nullptr, 0, nullptr);
+   c->link_order = false;
+   if (s) return s;
    if ((s = rs_rdf(c, limit, nbins)) != MDGPU_OK) return s;
    std::vector<unsigned long long> full;
    if ((s = rdf_download(c, nbins, full)) != MDGPU_OK) return s;
@@ -702,7 +754,6 @@ mdgpu_status mdgpu_pair_keys(mdgpu_ctx *c, const double *h, const double *site_s
       CKR(cudaMemcpyAsync(c->cofm_in.p, c_of_m, 3 * c->nmols * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    }
    CKR(c->rd.keys.ensure(cap > 0 ? (size_t)cap : 1));
-   CKR(cudaMemsetAsync(c->out.p, 0, sizeof(DevOut), c->stream));
    s = rs_launch(c, c->site.p, c->cofm_in.p, c->force.p, false, c->rd.keys.p, cap, nullptr);
    if (s) return s;
    s = sync_out(c);

@@ -834,9 +834,12 @@ __global__ void k_fsum(int n3, int nsplit, const double *__restrict__ fpart, dou
 // force[comp][slots[j]] += sum over splits of fpart[split][comp][j], j < n
 // (partials by slot of the charged-site list; the other sites get nothing),
 // times the site's charge when chg is given
+// (and the evaluation's result: every sum is complete here)
 __global__ void k_fsum_slots(int n, int N, int nsplit, const double *__restrict__ fpart,
-                             const int *__restrict__ slots, const double *__restrict__ chg, double *__restrict__ force)
+                             const int *__restrict__ slots, const double *__restrict__ chg, double *__restrict__ force,
+                             FinArgs fin, DevOut *out)
 {
+   if (fin.on && blockIdx.x == 0 && threadIdx.x == blockDim.x - 1) finalize_eval(out, fin);
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= 3 * n) return;
    const int comp = i / n, j = i - comp * n;
@@ -847,8 +850,8 @@ __global__ void k_fsum_slots(int n, int N, int nsplit, const double *__restrict_
 }
 
 // Compaction of the link-cell order to the charged sites: per block of
-// 1024 slots an exclusive scan of the flags (charge != 0), the block totals
-// scanned by one block, then each charged slot's site written to its place.
+// 1024 slots an exclusive scan of the flags (charge != 0), then each charged
+// slot's site written to its place (every block adds up the totals before it).
 __device__ __forceinline__ int block_scan_1024(int v, int *sh)   // exclusive, blockDim 1024
 {
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -885,31 +888,21 @@ __global__ void __launch_bounds__(1024) k_kflag_scan(int N, const int *__restric
    if (threadIdx.x == 1023) bsum[blockIdx.x] = e + f;
 }
 
-__global__ void __launch_bounds__(1024) k_kbsum_scan(int nb, int *__restrict__ bsum)
+__global__ void __launch_bounds__(1024) k_kcompact(int N, const int *__restrict__ sorted, const double *__restrict__ chg,
+                                                   const int *__restrict__ ex, const int *__restrict__ bsum,
+                                                   int *__restrict__ slots)
 {
    __shared__ int sh[32];
-   __shared__ int carry;
-   if (threadIdx.x == 0) carry = 0;
+   int s = 0;   // charged slots of the blocks before
+   for (int k = threadIdx.x; k < (int)blockIdx.x; k += 1024) s += bsum[k];
+   s = __reduce_add_sync(0xffffffffu, s);
+   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
    __syncthreads();
-   for (int b0 = 0; b0 < nb; b0 += 1024) {
-      const int i = b0 + threadIdx.x;
-      const int v = i < nb ? bsum[i] : 0;
-      const int e = block_scan_1024(v, sh);
-      const int c0 = carry;
-      __syncthreads();
-      if (i < nb) bsum[i] = c0 + e;
-      if (threadIdx.x == 1023) carry = c0 + e + v;
-      __syncthreads();
-   }
-}
-
-__global__ void k_kcompact(int N, const int *__restrict__ sorted, const double *__restrict__ chg,
-                           const int *__restrict__ ex, const int *__restrict__ bsum, int *__restrict__ slots)
-{
-   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+   s = __reduce_add_sync(0xffffffffu, sh[threadIdx.x & 31]);
+   const int i = blockIdx.x * 1024 + threadIdx.x;
    if (i >= N) return;
    const int si = sorted[i];
-   if (chg[si] != 0.0) slots[bsum[i >> 10] + ex[i]] = si;
+   if (chg[si] != 0.0) slots[s + ex[i]] = si;
 }
 
 // -------------------------------------------------------------- host side
@@ -1009,7 +1002,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    const bool mixed = c->prec == MDGPU_MIXED;
    DevOut *out = c->out.p;
    if (nk == 0) {
-      if (join) CK(cudaStreamWaitEvent(st, join, 0));
+      if (join && !c->pairs_after_tables) CK(cudaStreamWaitEvent(st, join, 0));
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
       return MDGPU_OK;
    }
@@ -1035,6 +1028,8 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
             qm = std::max(qm, std::fabs(q));
          }
          c->ncharged = n;
+         c->n_class0 = 0;
+         for (int id : c->site_id) c->n_class0 += c->cls_of_id[id] == 0;
          c->qmax = qm;
          c->ncharged_gen = c->gen;
       }
@@ -1042,27 +1037,39 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    if (compact) {
       Nk = c->ncharged;
       if (Nk == 0) {
-         if (join) CK(cudaStreamWaitEvent(st, join, 0));
+         if (join && !c->pairs_after_tables) CK(cudaStreamWaitEvent(st, join, 0));
          if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
          return MDGPU_OK;
       }
-      const int nb = (N + 1023) / 1024;
-      CK(d.kslots.ensure(N));   // room for every site whatever the device-side count
-      CK(d.kscan.ensure(N));
-      CK(d.kbsum.ensure(nb));
-      k_kflag_scan<<<nb, 1024, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p);
-      k_kbsum_scan<<<1, 1024, 0, st>>>(nb, d.kbsum.p);
-      k_kcompact<<<(N + 255) / 256, 256, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p,
-                                                  d.kslots.p);
-      CK(cudaGetLastError());
-      c->launches += 3;
-      slots = d.kslots.p;
+      // all sites charged, or all of class 0 and the slots class by class
+      // (rigid water): the charged sites come first as they are
+      if (Nk < N && !(c->class_major && c->n_class0 == Nk)) {
+         const int nb = (N + 1023) / 1024;
+         CK(d.kslots.ensure(N));   // room for every site whatever the device-side count
+         CK(d.kscan.ensure(N));
+         CK(d.kbsum.ensure(nb));
+         k_kflag_scan<<<nb, 1024, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p);
+         k_kcompact<<<nb, 1024, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p, d.kslots.p);
+         CK(cudaGetLastError());
+         c->launches += 2;
+         slots = d.kslots.p;
+      }
    }
    const int ns = mixed ? 3 : 7;
    mdgpu_status s;
    if (!tc && (s = ks_upload_list(c)) != MDGPU_OK) return s;
    if (tc) {
       if ((s = ks_q_tables(c, ns, Nk, slots, d_site)) != MDGPU_OK) return s;
+      if (cudaStream_t main = c->pairs_after_tables) {
+         CK(cudaEventRecord(c->ev_fork, st));
+         CK(cudaStreamWaitEvent(main, c->ev_fork, 0));
+         c->pairs_after_tables = nullptr;
+         c->stream = main;
+         s = rs_pairs(c, d_force, nullptr, 0);
+         c->stream = st;
+         if (s != MDGPU_OK) return s;
+         CK(cudaEventRecord(c->ev_pairs, main));
+      }
    } else {
       if (mixed) {
          CK(d.ph32.ensure(N));
@@ -1116,7 +1123,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    CK(d.blk.ensure((size_t)nbk * 8));
    phase_mark(c, MDGPU_PH_KREDUCE);
    if (tc) {
-      if ((s = ks_q_reduce(c, ns, sh.chunks, &nbk)) != MDGPU_OK) return s;
+      if ((s = ks_q_reduce(c, ns, sh.chunks)) != MDGPU_OK) return s;
    } else if (nf > 0) {
       if (mixed) {
          CK(d.kdatf32.ensure(nk));
@@ -1137,7 +1144,8 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       k_kreduce<false><<<nbk, KR_K * KR_W, 0, st>>>(nk, sh.chunks, nullptr, d.part64.p, d.kz64.p, d.coeff.p,
                                             d.coeff2.p, nullptr, d.kdat64.p, d.blk.p);
    }
-   if (nbk > 4 * KF_PARTS) {
+   if (tc) {   // summed by the reduction's last block
+   } else if (nbk > 4 * KF_PARTS) {
       CK(d.blk2.ensure(8 * (size_t)KF_PARTS));
       k_kfinal_part<<<KF_PARTS, 128, 0, st>>>(d.blk.p, nbk, d.blk2.p, d.kcount.p, out);
    } else {
@@ -1175,9 +1183,11 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    if (compact || tc) {
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
       if (tc && !mixed) {
-         if ((s = ks_q_fsum64(c, Nk, slots, d_force)) != MDGPU_OK) return s;
+         if ((s = ks_q_fsum64(c, Nk, slots, d_force, c->fin)) != MDGPU_OK) return s;
       } else
-      k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots, tc ? c->rd.chg.p : nullptr, d_force);
+      k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots,
+                                                            tc ? c->rd.chg.p : nullptr, d_force, c->fin, out);
+      c->fin.on = 0;
    } else {
       k_fsum<<<(3 * N + 255) / 256, 256, 0, st>>>(3 * N, sh.splits, d.fpart.p, d_force, accumulate ? 1 : 0);
    }

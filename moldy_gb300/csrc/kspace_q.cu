@@ -58,6 +58,7 @@ constexpr int Q_ERR = 8, Q_FERR = 16;             // error-word bits: structure 
 template <int NS> struct QCfg;
 template <> struct QCfg<3> {
    typedef int T;
+   typedef float P;                               // structure-factor partials
    static constexpr int RS = 36;                  // table row: 32 sites, padded against bank conflicts
    static constexpr int MT = 2, NPART = 1;        // 128-row tiles per CTA, column parts of B
    static constexpr int NB = 3;                   // stages in flight
@@ -66,6 +67,7 @@ template <> struct QCfg<3> {
 };
 template <> struct QCfg<7> {
    typedef long long T;
+   typedef double P;
    static constexpr int RS = 34;
    static constexpr int MT = 1, NPART = 2;
    static constexpr int NB = 2;
@@ -502,7 +504,7 @@ template <int NS, int ND>
 __global__ void __launch_bounds__(Q_THREADS, 1)
 k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4 *__restrict__ units, const unsigned char *__restrict__ X,
          const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, size_t zstride, int nstages, int per,
-         double *__restrict__ part, int *__restrict__ err)
+         typename QCfg<NS>::P *__restrict__ part, int *__restrict__ err)
 {
    using namespace tc;
    typedef typename QCfg<NS>::T T;
@@ -659,18 +661,19 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
             const int row = 32 * (w & 3) + lane;
             const int u = ti.unit[8 * mt + (row >> 4)];
             if (u >= 0) {
-               double *dst = part + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * 4 * g.nquads + (size_t)u * 16 + (row & 15)) * 2 * g.TP + ti.col0 + pl;
+               typename QCfg<NS>::P *dst =
+                  part + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * 4 * g.nquads + (size_t)u * 16 + (row & 15)) * 2 * g.TP +
+                  ti.col0 + pl;
 #pragma unroll
                for (int ch = 0; ch < MAXC; ch++)
                   if (4 * ch < ncw) {
-                     double v[4];
-#pragma unroll
-                     for (int e = 0; e < 4; e++) {
-                        const int i = (mt * MAXC + ch) * 4 + e;
-                        v[e] = NS == 3 ? (double)af[NS == 3 ? i : 0] : q_value(ai[NS == 7 ? i : 0]);
+                     const int i = (mt * MAXC + ch) * 4;
+                     if constexpr (NS == 3) {
+                        *reinterpret_cast<float4 *>(dst + 4 * ch) = make_float4(af[i], af[i + 1], af[i + 2], af[i + 3]);
+                     } else {
+                        reinterpret_cast<double2 *>(dst + 4 * ch)[0] = make_double2(q_value(ai[i]), q_value(ai[i + 1]));
+                        reinterpret_cast<double2 *>(dst + 4 * ch)[1] = make_double2(q_value(ai[i + 2]), q_value(ai[i + 3]));
                      }
-                     reinterpret_cast<double2 *>(dst + 4 * ch)[0] = make_double2(v[0], v[1]);
-                     reinterpret_cast<double2 *>(dst + 4 * ch)[1] = make_double2(v[2], v[3]);
                   }
             }
          }
@@ -686,57 +689,62 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
 }
 
 // ------------------------------------------------- per-k energy and stress
-// A block takes 32 consecutive (quad, t): its eight warps add up their eight
-// sums over the site ranges w, w + 8, ... (fixed order), then one thread per
+// Sum of nr values a plane apart: FP32 partials compensated (an FP64 add or
+// conversion per partial would bound the per-k pass), FP64 ones plainly.
+__device__ __forceinline__ double q_rangesum(const float *p, size_t plane, int nr)
+{
+   float s = 0.f, c = 0.f;
+#pragma unroll 4
+   for (int k = 0; k < nr; k++) {
+      const float y = __ldg(p + k * plane) - c, t = s + y;
+      c = (t - s) - y;
+      s = t;
+   }
+   return (double)s - (double)c;
+}
+__device__ __forceinline__ double q_rangesum(const double *p, size_t plane, int nr)
+{
+   double s = 0.0;
+#pragma unroll 4
+   for (int k = 0; k < nr; k++) s += __ldg(p + k * plane);
+   return s;
+}
+
+// A block takes 32 consecutive (quad, t) at a time (the energy and stress of
+// all its groups in one reduction: FP64 instructions bound this kernel): warp
+// k adds up sum k of each over the site ranges, then one thread per
 // (quad, t) and (s, r) forms its k-vector's S(k), energy and stress
 // (src/ewald.c:525-553) and A = coeff Re S, B = coeff Im S, laid out
 // [quad][t][s][r] (zero where there is no such k-vector).
 template <typename R>
 __global__ void __launch_bounds__(256)
 k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coeff, int nranges, double scale,
-          const double *__restrict__ part, R *__restrict__ ab, double *__restrict__ blk)
+          const R *__restrict__ part, R *__restrict__ ab, double *__restrict__ blk, unsigned int *__restrict__ sync,
+          DevOut *__restrict__ out)
 {
-   __shared__ double sq[8][8][32];
-   __shared__ double sh[4][7];
+   __shared__ double sq[8][32];
+   __shared__ double sh[4][7], sl[7][8];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-   const int i = blockIdx.x * 32 + lane, quad = i / g.TP, t = i - quad * g.TP;
+   double e[7] = {0, 0, 0, 0, 0, 0, 0};
+   for (int grp = blockIdx.x; grp * 32 < g.nquads * g.TP; grp += gridDim.x) {
+   const int i = grp * 32 + lane, quad = i / g.TP, t = i - quad * g.TP;
    const int4 un = quad < g.nquads ? units[quad >> 2] : make_int4(0, 0, 0, 0);
    const bool live = t < un.z;   // the unit's t range: its columns were computed
    {
-      double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (live) {
-         const size_t row = 2 * (size_t)g.TP, plane = 4 * (size_t)g.nquads * row;
-         const double *p = part + (size_t)quad * 4 * row + 16 * (t >> 3) + (t & 7) + w * plane;
-         for (int c = w; c < nranges; c += 8, p += 8 * plane)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-               q[2 * k] += p[k * row];
-               q[2 * k + 1] += p[k * row + 8];
-            }
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) sq[w][k][lane] = q[k];
+      const size_t row = 2 * (size_t)g.TP;
+      sq[w][lane] = live ? scale * q_rangesum(part + ((size_t)quad * 4 + (w >> 1)) * row + 16 * (t >> 3) + 8 * (w & 1) + (t & 7),
+                                              4 * (size_t)g.nquads * row, nranges)
+                         : 0.0;
    }
    __syncthreads();
-   {
-      // sum k = w of lane's (quad, t) over the warps
-      double v = 0.0;
-#pragma unroll
-      for (int j = 0; j < 8; j++) v += sq[j][w][lane];
-      __syncthreads();
-      sq[0][w][lane] = v * scale;
-   }
-   __syncthreads();
-   if (w >= 4) return;
-   // (s, r) = warp w
-   double e[7] = {0, 0, 0, 0, 0, 0, 0};
-   if (quad < g.nquads) {
+   // (s, r) = warp w of the first four
+   if (w < 4 && quad < g.nquads) {
       double A = 0.0, Bc = 0.0;
       const double2 cf = live ? coeff[(size_t)i * 4 + w] : make_double2(0.0, 0.0);
       if (cf.x != 0.0) {
          double q[8];
 #pragma unroll
-         for (int k = 0; k < 8; k++) q[k] = sq[0][k][lane];
+         for (int k = 0; k < 8; k++) q[k] = sq[k][lane];
          const double s = w & 2 ? -1.0 : 1.0, r = w & 1 ? -1.0 : 1.0;
          const double C = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
          const double S = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
@@ -744,28 +752,51 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
          const double kx = hh * g.b[0] + kk * g.b[3], ky = hh * g.b[1] + kk * g.b[4];
          const double kz = hh * g.b[2] + kk * g.b[5] + l * g.b[8];
          const double pek = 0.5 * cf.x * (C * C + S * S), pc = pek * cf.y;
-         e[0] = pek;
-         e[1] = pek - pc * kx * kx;
-         e[2] = -(pc * kx * ky);
-         e[3] = -(pc * kx * kz);
-         e[4] = pek - pc * ky * ky;
-         e[5] = -(pc * ky * kz);
-         e[6] = pek - pc * kz * kz;
+         const double px = pc * kx, py = pc * ky;
+         e[0] += pek;
+         e[1] += pek - px * kx;
+         e[2] -= px * ky;
+         e[3] -= px * kz;
+         e[4] += pek - py * ky;
+         e[5] -= py * kz;
+         e[6] += pek - pc * kz * kz;
          A = cf.x * C;
          Bc = cf.x * S;
       }
       ab[(size_t)i * 8 + 2 * w] = (R)A;
       ab[(size_t)i * 8 + 2 * w + 1] = (R)Bc;
    }
+   __syncthreads();
+   }
+   if (w < 4)
+#pragma unroll
+      for (int k = 0; k < 7; k++) {
+#pragma unroll
+         for (int o = 16; o > 0; o >>= 1) e[k] += __shfl_down_sync(0xffffffffu, e[k], o);
+         if (lane == 0) sh[w][k] = e[k];
+      }
+   __syncthreads();
+   if (threadIdx.x < 7)
+      blk[blockIdx.x * 8 + threadIdx.x] = (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
+   // energy and stress by the last block: blocks t, t + 256, ... per thread, then trees
+   if (!last_block(&sync[SYNC_KRED])) return;
+   double v[7] = {0, 0, 0, 0, 0, 0, 0};
+   for (int b = threadIdx.x; b < (int)gridDim.x; b += 256)
+#pragma unroll
+      for (int k = 0; k < 7; k++) v[k] += __ldcg(&blk[b * 8 + k]);
 #pragma unroll
    for (int k = 0; k < 7; k++) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) e[k] += __shfl_down_sync(0xffffffffu, e[k], o);
-      if (lane == 0) sh[w][k] = e[k];
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      if (lane == 0) sl[k][w] = v[k];
    }
-   asm volatile("bar.sync 1, 128;" : : : "memory");
-   if (threadIdx.x < 7)
-      blk[blockIdx.x * 8 + threadIdx.x] = (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
+   __syncthreads();
+   if (threadIdx.x < 7) {
+      double s = 0.0;
+      for (int j = 0; j < 8; j++) s += sl[threadIdx.x][j];
+      if (threadIdx.x == 0) out->pe_k = s;
+      else out->st_k[threadIdx.x - 1] = s;
+   }
 }
 
 // ------------------------------------------------- force pass, FP64 form
@@ -1028,8 +1059,9 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
 // force[site of slot i] += q b^T (H_h, H_k, H_l), the items' sums in order
 __global__ void __launch_bounds__(256)
 k_fsum_q(int n, int N, int nitems, QGeom g, const double *__restrict__ hpart, const int *__restrict__ slots,
-         const double *__restrict__ chg, double *__restrict__ force)
+         const double *__restrict__ chg, double *__restrict__ force, FinArgs fin, DevOut *out)
 {
+   if (fin.on && blockIdx.x == 0 && threadIdx.x == 255) finalize_eval(out, fin);   // every sum is complete
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= n) return;
    double H[3] = {0, 0, 0};
@@ -1146,36 +1178,24 @@ k_qwtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__r
 template <typename R>
 __global__ void __launch_bounds__(256)
 k_qadj(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coeff, double alpha, int loss, int nr0,
-       double scale0, const double *__restrict__ part, int nrv, double scalev, const unsigned int *__restrict__ wmax,
-       const double *__restrict__ partv, R *__restrict__ ab, double *__restrict__ blk)
+       double scale0, const R *__restrict__ part, int nrv, double scalev, const unsigned int *__restrict__ wmax,
+       const R *__restrict__ partv, R *__restrict__ ab, double *__restrict__ blk)
 {
-   __shared__ double sq[8][8][32];
+   __shared__ double sq[4][8][32];
    __shared__ double sh[4][2];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    const int i = blockIdx.x * 32 + lane, quad = i / g.TP, t = i - quad * g.TP;
    const int4 un = quad < g.nquads ? units[quad >> 2] : make_int4(0, 0, 0, 0);
    const bool live = t < un.z;
    {
-      // warp w: channel w / 2, ranges w % 2, + 2, ...
-      const int ch = w >> 1;
-      double q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-      if (live && (ch == 0 || loss)) {
-         const size_t row = 2 * (size_t)g.TP, plane = 4 * (size_t)g.nquads * row;
-         const int nr = ch == 0 ? nr0 : nrv;
-         const double *p = (ch == 0 ? part : partv + (size_t)(ch - 1) * nrv * plane) + (size_t)quad * 4 * row +
-                           16 * (t >> 3) + (t & 7) + (w & 1) * plane;
-         for (int c = w & 1; c < nr; c += 2, p += 2 * plane)
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-               q[2 * k] += p[k * row];
-               q[2 * k + 1] += p[k * row + 8];
-            }
-         const double sc = ch == 0 ? scale0 : ldexp(scalev, q_wexp(wmax[ch - 1]));
-#pragma unroll
-         for (int k = 0; k < 8; k++) q[k] *= sc;
-      }
-#pragma unroll
-      for (int k = 0; k < 8; k++) sq[w][k][lane] = q[k];
+      // warp w: sum w of every channel
+      const size_t row = 2 * (size_t)g.TP, plane = 4 * (size_t)g.nquads * row;
+      const size_t at = ((size_t)quad * 4 + (w >> 1)) * row + 16 * (t >> 3) + 8 * (w & 1) + (t & 7);
+      sq[0][w][lane] = live ? scale0 * q_rangesum(part + at, plane, nr0) : 0.0;
+      for (int ch = 1; ch < 4; ch++)
+         sq[ch][w][lane] = live && loss ? ldexp(scalev, q_wexp(wmax[ch - 1])) *
+                                             q_rangesum(partv + (size_t)(ch - 1) * nrv * plane + at, plane, nrv)
+                                        : 0.0;
    }
    __syncthreads();
    if (w >= 4) return;
@@ -1190,7 +1210,7 @@ k_qadj(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coef
          for (int ch = 0; ch < 4; ch++) {
             double q[8];
 #pragma unroll
-            for (int k = 0; k < 8; k++) q[k] = sq[2 * ch][k][lane] + sq[2 * ch + 1][k][lane];
+            for (int k = 0; k < 8; k++) q[k] = sq[ch][k][lane];
             C[ch] = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
             S[ch] = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
          }
@@ -1347,11 +1367,11 @@ mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges)
    KsDev &d = c->kd;
    const QList &q = c->kl.q;
    const int nst = (n + 31) / 32, nt = (int)q.tiles.size();
-   const size_t plane = 4 * (size_t)q.g.nquads * 2 * q.g.TP;
+   const size_t plane = 4 * (size_t)q.g.nquads * 2 * q.g.TP, psz = ns == 3 ? sizeof(float) : sizeof(double);
    long long best = -1;
    int R = 1;
    for (int r = 1; r <= 64 && r <= nst; r++) {
-      if (r > 1 && r * plane * sizeof(double) > (256u << 20)) break;
+      if (r > 1 && r * plane * psz > (256u << 20)) break;
       const long long cost = (long long)((nt * r + c->nsm - 1) / c->nsm) * ((nst + r - 1) / r + 6);
       if (best < 0 || cost < best) {
          best = cost;
@@ -1360,39 +1380,38 @@ mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges)
    }
    const int per = (nst + R - 1) / R;
    R = (nst + per - 1) / per;
-   CK(d.q_part.ensure(R * plane));
+   CK(d.q_part.ensure(R * plane * psz));
    const dim3 grid(nt, R);
    if (ns == 3)
       k_sfac_q<3, 3><<<grid, Q_THREADS, Q_SMEM<3, 3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, nst, per, d.q_part.p, &c->out.p->err);
+         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, nst, per, (float *)d.q_part.p, &c->out.p->err);
    else
       k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, 0, nst, per, d.q_part.p, &c->out.p->err);
+         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, 0, nst, per, (double *)d.q_part.p, &c->out.p->err);
    CK(cudaGetLastError());
    d.q_nranges = R;
    *nranges = R;
    return MDGPU_OK;
 }
 
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges, int *nblocks)
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges)
 {
    KsDev &d = c->kd;
    const QGeom &g = c->kl.q.g;
    const size_t nqt = (size_t)g.nquads * g.TP;
-   const int nb = (int)((nqt + 31) / 32);
+   const int nb = (int)std::min<size_t>((nqt + 31) / 32, 4 * (size_t)c->nsm);
    const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
    CK(d.blk.ensure((size_t)nb * 8));
    if (ns == 3) {
       CK(d.q_ab32.ensure(nqt * 8));
       k_qreduce<float><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
-         std::ldexp(1.0 / k4, q_charge_exp(c) - 30), d.q_part.p, d.q_ab32.p, d.blk.p);
+         std::ldexp(1.0 / k4, q_charge_exp(c) - 30), (const float *)d.q_part.p, d.q_ab32.p, d.blk.p, c->rd.sync.p, c->out.p);
    } else {
       CK(d.q_ab64.ensure(nqt * 8));
       k_qreduce<double><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
-         std::ldexp(1.0 / k4, q_charge_exp(c) - 62), d.q_part.p, d.q_ab64.p, d.blk.p);
+         std::ldexp(1.0 / k4, q_charge_exp(c) - 62), (const double *)d.q_part.p, d.q_ab64.p, d.blk.p, c->rd.sync.p, c->out.p);
    }
    CK(cudaGetLastError());
-   *nblocks = nb;
    return MDGPU_OK;
 }
 
@@ -1446,10 +1465,10 @@ mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
    return MDGPU_OK;
 }
 
-mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force)
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force, const FinArgs &fin)
 {
    k_fsum_q<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->nsites, c->kd.q_nitems, c->kl.q.g, c->kd.fpart.p, slots,
-                                                    c->rd.chg.p, d_force);
+                                                    c->rd.chg.p, d_force, fin, c->out.p);
    CK(cudaGetLastError());
    return MDGPU_OK;
 }
@@ -1469,6 +1488,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    const size_t nqt = (size_t)g.nquads * g.TP, plane = 4 * (size_t)g.nquads * 2 * g.TP;
    const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
    const double *hi = c->kl.hinv;
+   const size_t psz = ns == 3 ? sizeof(float) : sizeof(double);
    int R = 1;
    CK(a.wmax.ensure(3));
    if (loss) {
@@ -1477,7 +1497,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
       CK(cudaMemsetAsync(a.wmax.p, 0, 3 * sizeof(unsigned int), st));
       long long best = -1;
       for (int r = 1; r <= 64 && r <= nst; r++) {
-         if (r > 1 && 3 * r * plane * sizeof(double) > (256u << 20)) break;
+         if (r > 1 && 3 * r * plane * psz > (256u << 20)) break;
          const long long cost = (long long)((3 * nt * r + c->nsm - 1) / c->nsm) * ((nst + r - 1) / r + 6);
          if (best < 0 || cost < best) {
             best = cost;
@@ -1486,7 +1506,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
       }
       const int per = (nst + R - 1) / R;
       R = (nst + per - 1) / per;
-      CK(a.partv.ensure(3 * (size_t)R * plane));
+      CK(a.partv.ensure(3 * (size_t)R * plane * psz));
       const dim3 grid(nt, R, 3);
       const int nb = (N + 255) / 256;
       if (ns == 3) {
@@ -1494,15 +1514,15 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
          k_qwtab<3, 4, float4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
                                                     a.res32.p, a.wmax.p, a.zw.p, zstride);
          k_sfac_q<3, 4><<<grid, Q_THREADS, Q_SMEM<3, 4>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
-            (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, a.zw.p, zstride, nst, per, a.partv.p,
-            &c->out.p->err);
+            (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, a.zw.p, zstride, nst, per,
+            (float *)a.partv.p, &c->out.p->err);
       } else {
          k_qwmax<double4><<<nb, 256, 0, st>>>(N, slots, c->rd.chg.p, a.res64.p, a.wmax.p);
          k_qwtab<7, 7, double4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
                                                      a.res64.p, a.wmax.p, a.zw.p, zstride);
          k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
-            (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, a.zw.p, zstride, nst, per, a.partv.p,
-            &c->out.p->err);
+            (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, a.zw.p, zstride, nst, per,
+            (double *)a.partv.p, &c->out.p->err);
       }
       CK(cudaGetLastError());
       c->launches += 3;
@@ -1514,7 +1534,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    if (ns == 3) {
       CK(a.ab32.ensure(nqt * 8));
       k_qadj<float><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
-         std::ldexp(1.0 / k4, e0 - 30), d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, a.partv.p, a.ab32.p, a.blk.p);
+         std::ldexp(1.0 / k4, e0 - 30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
       const int sp = ks_force_tc_splits(d);
       CK(a.gkpart.ensure((size_t)sp * 3 * N));
       const int nl = ks_force_tc(st, N, g, d, a.ab32.p, true, c->nsm, a.gkpart.p, &c->out.p->err);
@@ -1525,7 +1545,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    } else {
       CK(a.ab64.ensure(nqt * 8));
       k_qadj<double><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
-         std::ldexp(1.0 / k4, e0 - 62), d.q_part.p, R, std::ldexp(1.0 / k4, -62), a.wmax.p, a.partv.p, a.ab64.p, a.blk.p);
+         std::ldexp(1.0 / k4, e0 - 62), (const double *)d.q_part.p, R, std::ldexp(1.0 / k4, -62), a.wmax.p, (const double *)a.partv.p, a.ab64.p, a.blk.p);
       const int nseg = (int)q.segs.size(), T = (N + 127) / 128;
       CK(a.gkpart.ensure((size_t)d.q_nitems * N));
       k_qcoef<<<dim3(nseg, 1), 256, 0, st>>>(g, 3, d.q_segs.p, nseg, d.q_units.p, a.ab64.p, d.q_bq.p, d.q_bexp.p);

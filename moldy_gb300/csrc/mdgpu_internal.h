@@ -174,7 +174,21 @@ struct DevOut {
    int n_too_close;
    int64_t npairs2;       // full-list pair evaluations (2x reference count)
    int too_close[MAX_TOO_CLOSE_REC][2];
+   double fin[11];        // energies [2] and stress [9] of mdgpu_forces
 };
+
+// What the last kernel of an evaluation adds up (finalize_eval): the
+// first-call constants and where the energies and the stress go besides
+// DevOut::fin (pe null: nowhere).  on: the kernel's last block does it.
+struct FinArgs {
+   int on = 0, has_ewald = 0;
+   double eintra = 0, self = 0, sheet_v = 0;
+   double *pe = nullptr, *st = nullptr;
+};
+
+// Device counters of kernels whose last block to finish has a task of its
+// own; each is zero between evaluations (that block resets it).
+enum { SYNC_BIN = 0, SYNC_BINERR, SYNC_PAIRS, SYNC_KRED, SYNC_FSUM, SYNC_N };
 
 struct RsDev {
    DBuf<int> cell_of, cell_count, cell_start, slot_cell, sorted, blocksum;
@@ -192,16 +206,16 @@ struct RsDev {
    DBuf<unsigned long long> keys;
    DBuf<int4> rdf_full;    // RDF stencil (strict, at the RDF limit)
    // column walk of the mixed pair kernel (k_pairs_col): the stencil's
-   // columns and their offsets; the slots re-laid class by class (class 0:
-   // the sites that interact with charged sites; class 1: the rest), each
-   // class in link-cell order, with per-class cell starts cs[2][ncells+1]
+   // columns and their offsets (where it runs with two interaction classes
+   // the slots are laid class by class: cell_start then holds class 0's
+   // cells, class 1's, and the end)
    DBuf<int4> cols;
    DBuf<int> col_base;
    DBuf<float4> coff;      // [e][2]: the column offsets' hi and lo parts side by side (32 B per entry)
-   DBuf<int> cls_of_id, cls_pre, cs, sortc, cellc, cls_bsum;
-   DBuf<float4> posc;
-   DBuf<double4> posc64;   // the FP64 form's records, class by class
-   DBuf<int2> tagc;
+   DBuf<int2> tagc;        // per slot: site id with the cell's z index above 16 bits, molecule
+   DBuf<int> site_cls;     // interaction class of every site
+   DBuf<int> rank, unsorted;   // place of a site among its cell's, slots before the sort within cells
+   DBuf<unsigned int> sync;    // counters (SYNC_*)
    DBuf<unsigned long long> rdf_counts;
    double rdf_key[11] = {0};
    int rdf_nfull = 0;
@@ -252,8 +266,8 @@ struct KsDev {
    DBuf<QItem> q_items;
    DBuf<int> q_x32, q_y32, q_bexp;
    DBuf<long long> q_x64, q_y64;
-   DBuf<unsigned char> q_ztab, q_bq;
-   DBuf<double> q_zd, q_part, q_ab64;
+   DBuf<unsigned char> q_ztab, q_bq, q_part;
+   DBuf<double> q_zd, q_ab64;
    DBuf<float> q_ab32;
    int q_nfblk = 0;                 // mixed force pass: t-blocks and their entries of q_fu
    std::vector<int> q_fblk;
@@ -298,8 +312,8 @@ struct AdjDev {
    // tensor-core passes: largest weights, the weights' digits, their
    // structure factors, the per-site pass's coefficients
    DBuf<unsigned int> wmax;
-   DBuf<unsigned char> zw;
-   DBuf<double> partv, ab64;
+   DBuf<unsigned char> zw, partv;
+   DBuf<double> ab64;
    DBuf<float> ab32;
 };
 
@@ -387,6 +401,11 @@ struct mdgpu_ctx {
    bool rs_valid = false, rs_uploaded = false;
    mdgpu::KList kl;
    bool kl_valid = false, kl_uploaded = false;
+   bool class_major = false;      // the slots of the last binning are laid class by class
+   bool link_order = false;       // binning in plain link-cell order wanted (RDF)
+   bool counts_clean = false;     // cell_count is all zero (k_place leaves it so)
+   mdgpu::FinArgs fin;            // of the evaluation in progress
+   cudaStream_t pairs_after_tables = nullptr;   // ks_launch starts the pair kernel on this stream
    bool npairs_pending = false;   // the last real-space pass left the pair count to rs_count_pairs
    int rs_nblk = 0;               // blocks (energy/virial partials) of the last real-space pass
 
@@ -397,11 +416,10 @@ struct mdgpu_ctx {
    mdgpu::MdDev md;
    mdgpu::DBuf<double> site, force, force_in, cofm_in, small;
    const double *cur_site = nullptr;   // site array of the launch in progress
+   std::vector<double> h_stage;        // small host arrays of the reference-style calls, gathered
    std::vector<double> last_cofm;      // centres of mass of the last force_calc
    mdgpu::DBuf<mdgpu::DevOut> out;
    mdgpu::DevOut *h_out = nullptr;  // pinned mirror
-   double *h_stage = nullptr;       // pinned staging for 6*nsites doubles
-   size_t h_stage_n = 0;
 
    mdgpu_info info{};
    int64_t launches = 0;
@@ -414,6 +432,7 @@ struct mdgpu_ctx {
    bool tc_sfac = true;
    uint64_t ncharged_gen = 0;       // configuration the count below is for
    int ncharged = 0;                // sites with a nonzero charge
+   int n_class0 = 0;                // sites of interaction class 0
    double qmax = 0;                 // and their largest |q|
    cudaEvent_t ev[MDGPU_NPHASES + 1] = {};
    // second (high-priority) stream: the k-space passes run on it beside
@@ -473,18 +492,16 @@ struct KsShape {
 // (ipt items per thread, spt sites per thread).
 KsShape ks_shape(int N, int nitems, int ipt, int spt);
 // Reciprocal-space passes on the tensor cores.  kspace_q.cu: both forms'
-// tables, structure factor and per-k sums (A and B per (quad, t), the
-// blocks' energy/stress records into d.blk; returns their number, -1 if out
-// of memory), and the FP64 form's force pass (adds the forces after join,
-// if any).  kspace_tc.cu: the mixed form's force pass, F_slot / q into
+// tables, structure factor and per-k sums (A and B per (quad, t), energy
+// and stress into DevOut), and the FP64 form's force pass.  kspace_tc.cu: the mixed form's force pass, F_slot / q into
 // fpart[split][3][nsites], or with scalar the sum over k of A sin - B cos
 // into its first component (returns the launches, -1 if out of memory).
 mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns);
 mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site);
 mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges);
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges, int *nblocks);
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges);
 mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots);
-mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force);
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force, const FinArgs &fin);
 int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
                 double *fpart, int *err);
 mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq, int *nblocks);
@@ -508,4 +525,49 @@ inline void phase_mark(mdgpu_ctx *c, int i)
    cudaEventRecord(c->ev[i], c->stream);
    c->ev_marked[i] = true;
 }
+
+#ifdef __CUDACC__
+// True in every thread of the grid's last block to get here (all its threads
+// call it, once); count (zero before) is reset.  What the other blocks wrote
+// before their call is visible to the last one through L2 (__ldcg).
+__device__ __forceinline__ bool last_block(unsigned int *count)
+{
+   __shared__ bool last;
+   __threadfence();
+   __syncthreads();
+   if (threadIdx.x == 0) {
+      last = atomicAdd(count, 1u) == gridDim.x * gridDim.y * gridDim.z - 1;
+      if (last) *count = 0u;
+   }
+   __syncthreads();
+   if (last) __threadfence();
+   return last;
+}
+
+// Energies and stress of an evaluation from its sums (one thread).
+__device__ __forceinline__ void finalize_eval(DevOut *out, const FinArgs &f)
+{
+   double r[11];
+   const double e = f.has_ewald ? 1.0 : 0.0, d = f.has_ewald ? f.sheet_v : 0.0;
+   r[0] = -f.eintra + __ldcg(&out->pe_rs);
+   r[1] = f.has_ewald ? (-f.self + f.sheet_v) + __ldcg(&out->pe_k) : 0.0;
+   double v[6];
+   for (int k = 0; k < 6; k++) v[k] = __ldcg(&out->vir_rs[k]) + (f.has_ewald ? e * __ldcg(&out->st_k[k]) : 0.0);
+   r[2] = v[0] + d;
+   r[3] = v[1];
+   r[4] = v[2];
+   r[5] = 0.0;
+   r[6] = v[3] + d;
+   r[7] = v[4];
+   r[8] = 0.0;
+   r[9] = 0.0;
+   r[10] = v[5] + d;
+   for (int k = 0; k < 11; k++) out->fin[k] = r[k];
+   if (f.pe) {
+      f.pe[0] = r[0];
+      f.pe[1] = r[1];
+      for (int k = 0; k < 9; k++) f.st[k] = r[2 + k];
+   }
+}
+#endif
 }  // namespace mdgpu

@@ -87,40 +87,98 @@ __device__ __forceinline__ double hrow(const double *m, double a0, double a1, do
    return __dadd_rn(__dadd_rn(__dmul_rn(m[0], a0), __dmul_rn(m[1], a1)), __dmul_rn(m[2], a2));
 }
 
-__global__ void k_bin(RsParams P, const double *__restrict__ site, const double *__restrict__ cofm,
-                      const int *__restrict__ mol_first, const int *__restrict__ mol_n,
-                      int *__restrict__ cell_of, int *__restrict__ cell_count, DevOut *out)
+// Also the set-up of the evaluation's result record, by the last block, and
+// on small grids (SCAN_ONE cells) the scan of the cell counts and on small
+// systems (SCATTER_ONE sites) the placement: launches are the cost there.
+constexpr int SCAN_ONE = 8192, SCATTER_ONE = 2048;
+
+__device__ __forceinline__ int warp_incl_scan(int v);
+__device__ void block_excl_scan(int v, int *out_excl);
+
+__global__ void __launch_bounds__(256)
+k_bin(RsParams P, const double *__restrict__ site, const double *__restrict__ cofm,
+      const int *__restrict__ mol_first, const int *__restrict__ mol_n, const int *__restrict__ site_cls,
+      int *__restrict__ cell_of, int *__restrict__ rank, int *__restrict__ cell_count, int *__restrict__ cell_start,
+      int ncount, int *__restrict__ unsorted, unsigned int *__restrict__ sync, DevOut *out)
 {
-   int e = blockIdx.x * blockDim.x + threadIdx.x;
-   if (e >= P.nent) return;
-   int bad = 0;
-   double s0, s1, s2;
-   const bool by_site = !P.molpbc || e >= P.nmol_ent;
-   const int si = !P.molpbc ? e : P.fw_site0 + (e - P.nmol_ent);   // site of a site entity
-   if (by_site) {
-      const int N = P.nsites;
-      double x = site[si], y = site[N + si], z = site[2 * N + si];
-      s0 = hrow(P.hinv, x, y, z);
-      s1 = hrow(P.hinv + 3, x, y, z);
-      s2 = hrow(P.hinv + 6, x, y, z);
-   } else {
-      s0 = cofm[3 * e];
-      s1 = cofm[3 * e + 1];
-      s2 = cofm[3 * e + 2];
+   const int e = blockIdx.x * blockDim.x + threadIdx.x;
+   if (e < P.nent) {
+      int bad = 0;
+      double s0, s1, s2;
+      const bool by_site = !P.molpbc || e >= P.nmol_ent;
+      const int si = !P.molpbc ? e : P.fw_site0 + (e - P.nmol_ent);   // site of a site entity
+      if (by_site) {
+         const int N = P.nsites;
+         double x = site[si], y = site[N + si], z = site[2 * N + si];
+         s0 = hrow(P.hinv, x, y, z);
+         s1 = hrow(P.hinv + 3, x, y, z);
+         s2 = hrow(P.hinv + 6, x, y, z);
+      } else {
+         s0 = cofm[3 * e];
+         s1 = cofm[3 * e + 1];
+         s2 = cofm[3 * e + 2];
+      }
+      int cx = cellbin_dev(s0, P.nx, (double)P.nx, &bad);
+      int cy = cellbin_dev(s1, P.ny, (double)P.ny, &bad);
+      int cz = cellbin_dev(s2, P.nz, (double)P.nz, &bad);
+      int c = cz + P.nz * (cy + P.ny * cx);
+      if (bad) atomicOr(&sync[SYNC_BINERR], 1u);
+      if (by_site) {
+         if (site_cls) c += site_cls[si] * P.ncells;   // class by class
+         cell_of[si] = c;
+         rank[si] = atomicAdd(&cell_count[c], 1);
+      } else {
+         int f = mol_first[e], n = mol_n[e];
+         const int r = atomicAdd(&cell_count[c], n);
+         for (int s = 0; s < n; s++) {
+            cell_of[f + s] = c;
+            rank[f + s] = r + s;
+         }
+      }
    }
-   int cx = cellbin_dev(s0, P.nx, (double)P.nx, &bad);
-   int cy = cellbin_dev(s1, P.ny, (double)P.ny, &bad);
-   int cz = cellbin_dev(s2, P.nz, (double)P.nz, &bad);
-   int c = cz + P.nz * (cy + P.ny * cx);
-   if (bad) atomicOr(&out->err, 1);
-   if (by_site) {
-      cell_of[si] = c;
-      atomicAdd(&cell_count[c], 1);
-   } else {
-      int f = mol_first[e], n = mol_n[e];
-      for (int s = 0; s < n; s++) cell_of[f + s] = c;
-      atomicAdd(&cell_count[c], n);
+   if (!last_block(&sync[SYNC_BIN])) return;
+   const int t = threadIdx.x;
+   unsigned int *o = reinterpret_cast<unsigned int *>(out);
+   for (int q = t; q < (int)(sizeof(DevOut) / 4); q += blockDim.x) o[q] = 0u;
+   __syncthreads();
+   if (t == 0) {
+      out->err = (int)__ldcg(&sync[SYNC_BINERR]);
+      sync[SYNC_BINERR] = 0u;
    }
+   if (ncount > SCAN_ONE) return;
+   // four consecutive counts per thread and round
+   __shared__ int wsum[8], carry_s;
+   if (t == 0) carry_s = 0;
+   __syncthreads();
+   const int lane = t & 31, w = t >> 5;
+   for (int b0 = 0; b0 <= ncount; b0 += 1024) {
+      int v[4], sum = 0;
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+         const int i = b0 + 4 * t + k;
+         v[k] = i < ncount ? __ldcg(&cell_count[i]) : 0;
+         sum += v[k];
+      }
+      const int inc = warp_incl_scan(sum);
+      if (lane == 31) wsum[w] = inc;
+      __syncthreads();
+      int ex = inc - sum + carry_s, tot = 0;
+      for (int k = 0; k < 8; k++) {
+         if (k < w) ex += wsum[k];
+         tot += wsum[k];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+         const int i = b0 + 4 * t + k;
+         if (i <= ncount) cell_start[i] = ex;
+         ex += v[k];
+      }
+      __syncthreads();
+      if (t == 0) carry_s += tot;
+      __syncthreads();
+   }
+   if (P.nsites > SCATTER_ONE) return;
+   for (int i = t; i < P.nsites; i += blockDim.x) unsorted[cell_start[__ldcg(&cell_of[i])] + __ldcg(&rank[i])] = i;
 }
 
 // ---------------------------------------------------------- exclusive scan
@@ -153,11 +211,12 @@ __device__ void block_excl_scan(int v, int *out_excl)
    __syncthreads();
 }
 
+// (nin values in, n out: entry nin receives the total)
 __global__ void __launch_bounds__(1024) k_scan_blocks(const int *__restrict__ in, int *__restrict__ out,
-                                                      int *__restrict__ bsum, int n)
+                                                      int *__restrict__ bsum, int nin, int n)
 {
    int i = blockIdx.x * 1024 + threadIdx.x;
-   int v = i < n ? in[i] : 0, ex;
+   int v = i < nin ? in[i] : 0, ex;
    __shared__ int last;
    block_excl_scan(v, &ex);
    if (threadIdx.x == 1023) last = ex + v;
@@ -166,71 +225,52 @@ __global__ void __launch_bounds__(1024) k_scan_blocks(const int *__restrict__ in
    if (threadIdx.x == 0) bsum[blockIdx.x] = last;
 }
 
-__global__ void __launch_bounds__(1024) k_scan_sums(int *__restrict__ bsum, int nb, int *__restrict__ total)
+// The block sums before each block added to its scanned values (entry n,
+// the total, among them).
+__global__ void __launch_bounds__(1024) k_scan_add(int *__restrict__ out, const int *__restrict__ bsum, int n)
 {
-   __shared__ int carry_s;
-   if (threadIdx.x == 0) carry_s = 0;
+   __shared__ int sh[32];
+   int s = 0;
+   for (int k = threadIdx.x; k < (int)blockIdx.x; k += 1024) s += bsum[k];
+   s = __reduce_add_sync(0xffffffffu, s);
+   if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
    __syncthreads();
-   for (int b0 = 0; b0 < nb; b0 += 1024) {
-      int i = b0 + threadIdx.x;
-      int v = i < nb ? bsum[i] : 0, ex;
-      __shared__ int last;
-      block_excl_scan(v, &ex);
-      if (threadIdx.x == 1023) last = ex + v;
-      __syncthreads();
-      int carry = carry_s;
-      if (i < nb) bsum[i] = ex + carry;
-      __syncthreads();
-      if (threadIdx.x == 0) carry_s = carry + last;
-      __syncthreads();
-   }
-   if (threadIdx.x == 0) *total = carry_s;
-}
-
-__global__ void k_scan_add(int *__restrict__ out, const int *__restrict__ bsum, int n)
-{
-   int i = blockIdx.x * 1024 + threadIdx.x;
-   if (i < n) out[i] += bsum[blockIdx.x];
+   s = __reduce_add_sync(0xffffffffu, sh[threadIdx.x & 31]);
+   const int i = blockIdx.x * 1024 + threadIdx.x;
+   if (i < n) out[i] += s;
 }
 
 // ------------------------------------------------------ placement by cell
 __global__ void k_scatter(int n, const int *__restrict__ cell_of, const int *__restrict__ cell_start,
-                          int *__restrict__ cursor, int *__restrict__ sorted)
+                          const int *__restrict__ rank, int *__restrict__ unsorted)
 {
    int i = blockIdx.x * blockDim.x + threadIdx.x;
-   if (i >= n) return;
-   int c = cell_of[i];
-   sorted[cell_start[c] + atomicAdd(&cursor[c], 1)] = i;
+   if (i < n) unsorted[cell_start[cell_of[i]] + rank[i]] = i;
 }
 
-__global__ void k_cellsort(int ncells, const int *__restrict__ cell_start, int *__restrict__ sorted)
+// Each cell's sites in ascending order (a site's place: the count of its
+// cell's sites before it) and the per-slot records; leaves the cell counts
+// zero for the next binning.  Null pointers: records not wanted.
+__global__ void k_place(RsParams P, const double *__restrict__ site, const double *__restrict__ chg,
+                        const int *__restrict__ siteid, const int *__restrict__ molmap,
+                        const int *__restrict__ unsorted, const int *__restrict__ cell_of,
+                        const int *__restrict__ cell_start, int *__restrict__ cell_count, int ncount,
+                        int *__restrict__ sorted, double4 *__restrict__ pos64, float4 *__restrict__ pos32,
+                        int2 *__restrict__ tag, int2 *__restrict__ tagz, int *__restrict__ slot_cell)
 {
-   int c = blockIdx.x * blockDim.x + threadIdx.x;
-   if (c >= ncells) return;
-   int a = cell_start[c], b = cell_start[c + 1];
-   for (int i = a + 1; i < b; i++) {
-      int v = sorted[i], j = i - 1;
-      while (j >= a && sorted[j] > v) {
-         sorted[j + 1] = sorted[j];
-         j--;
-      }
-      sorted[j + 1] = v;
-   }
-}
-
-__global__ void k_gather(RsParams P, const double *__restrict__ site, const double *__restrict__ chg,
-                         const int *__restrict__ siteid, const int *__restrict__ molmap,
-                         const int *__restrict__ sorted, const int *__restrict__ cell_of,
-                         double4 *__restrict__ pos64, float4 *__restrict__ pos32,
-                         int2 *__restrict__ tag, int2 *__restrict__ tagz, int *__restrict__ slot_cell)
-{
-   int p = blockIdx.x * blockDim.x + threadIdx.x;
+   const int t = blockIdx.x * blockDim.x + threadIdx.x;
+   for (int q = t; q < ncount; q += gridDim.x * blockDim.x) cell_count[q] = 0;
    const int N = P.nsites;
-   if (p >= N) return;
-   int i = sorted[p], c = cell_of[i];
+   if (t >= N) return;
+   const int i = unsorted[t], cc = cell_of[i], a = cell_start[cc], b = cell_start[cc + 1];
+   int p = a;
+   for (int q = a; q < b; q++) p += unsorted[q] < i;
+   sorted[p] = i;
+   const int c = cc >= P.ncells ? cc - P.ncells : cc;
+   const int id = siteid[i], mol = molmap[i];
    double x = site[i], y = site[N + i], z = site[2 * N + i], q = chg[i];
-   tag[p] = make_int2(siteid[i], molmap[i]);
-   if (tagz) tagz[p] = make_int2(siteid[i] | ((c % P.nz) << 16), molmap[i]);   // with the cell's z index
+   if (tag) tag[p] = make_int2(id, mol);
+   if (tagz) tagz[p] = make_int2(id | ((c % P.nz) << 16), mol);   // with the cell's z index
    slot_cell[p] = c;
    if (pos64) pos64[p] = make_double4(x, y, z, q);
    if (pos32) {
@@ -769,20 +809,36 @@ __global__ void __launch_bounds__(256) k_reduce_rs(const double *__restrict__ pa
    if (t < 7) part2[blockIdx.x * 8 + t] = sh[t][0];
 }
 
-// One block over all the partials (few blocks: the column walk's grid of a
-// few blocks per SM): thread t takes blocks t, t + 256, ..., then the tree.
-__global__ void __launch_bounds__(256) k_reduce_rs1(const double *__restrict__ part, int nblocks, DevOut *out)
+// The column walks' energy and virial by their last block (few blocks):
+// thread t adds up blocks t, t + 128, ..., then fixed-shape trees; the
+// evaluation's result too where nothing follows.
+__device__ __forceinline__ void reduce_pairs_last(const double *__restrict__ part, int nblocks, unsigned int *sync,
+                                                  DevOut *out, const FinArgs &fin)
 {
-   __shared__ double sh[7][256];
-   const int t = threadIdx.x;
+   if (!last_block(&sync[SYNC_PAIRS])) return;
+   __shared__ double sh[7][PAIR_WARPS];
+   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
    double s[7] = {0, 0, 0, 0, 0, 0, 0};
-   for (int b = t; b < nblocks; b += 256)
-      for (int k = 0; k < 7; k++) s[k] += part[b * 8 + k];
-   for (int k = 0; k < 7; k++) sh[k][t] = s[k];
-   tree7(sh, t);
-   if (t == 0) {
-      out->pe_rs = sh[0][0];
-      for (int k = 0; k < 6; k++) out->vir_rs[k] = sh[k + 1][0];
+   for (int b = t; b < nblocks; b += PAIR_WARPS * 32)
+#pragma unroll
+      for (int k = 0; k < 7; k++) s[k] += __ldcg(&part[b * 8 + k]);
+#pragma unroll
+   for (int k = 0; k < 7; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[k] += __shfl_down_sync(0xffffffffu, s[k], o);
+      if (lane == 0) sh[k][w] = s[k];
+   }
+   __syncthreads();
+   if (t < 7) {
+      double v = 0.0;
+      for (int k = 0; k < PAIR_WARPS; k++) v += sh[t][k];
+      if (t == 0) out->pe_rs = v;
+      else out->vir_rs[t - 1] = v;
+   }
+   if (fin.on) {
+      __threadfence();
+      __syncthreads();
+      if (t == 0) finalize_eval(out, fin);
    }
 }
 
@@ -846,47 +902,6 @@ static int col_chunk(int N, int nblk)
    return std::max(PAIR_WARPS, std::min(COL_CHUNK, per / PAIR_WARPS * PAIR_WARPS));
 }
 
-// per slot (link-cell order): 1 when its identifier is in class 0; the
-// entry after the last is 0 (so the exclusive scan ends with the class-0
-// count)
-__global__ void k_cls_flag(int N, const int2 *__restrict__ tag, const int *__restrict__ cls_of_id,
-                           int *__restrict__ flag)
-{
-   const int p = blockIdx.x * blockDim.x + threadIdx.x;
-   if (p < N) flag[p] = cls_of_id[tag[p].x] == 0 ? 1 : 0;
-   else if (p == N) flag[p] = 0;
-}
-
-// Slots re-laid class by class (stable): class 0 first, then class 1, each
-// in link-cell order; per-class cell starts cs[K][c].  pre[p] is the number
-// of class-0 slots before p (pre[N] their total).  The per-slot tag carries
-// the identifier in its low 16 bits and the cell's z index above them.
-__global__ void k_cls_split(RsParams P, const int *__restrict__ pre, const int *__restrict__ cls_of_id,
-                            const int *__restrict__ cell_start, const float4 *__restrict__ pos32,
-                            const int2 *__restrict__ tag, const int *__restrict__ sorted,
-                            const int *__restrict__ slot_cell, const double4 *__restrict__ pos64,
-                            int *__restrict__ cs, float4 *__restrict__ posc, double4 *__restrict__ posc64,
-                            int2 *__restrict__ tagc, int *__restrict__ sortc, int *__restrict__ cellc)
-{
-   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-   const int N = P.nsites, n0 = pre[N];
-   if (i < N) {
-      const int2 t = tag[i];
-      const int q = cls_of_id[t.x] == 0 ? pre[i] : n0 + (i - pre[i]);
-      const int c = slot_cell[i];
-      posc[q] = pos32[i];
-      if (posc64) posc64[q] = pos64[i];
-      tagc[q] = make_int2(t.x | ((c % P.nz) << 16), t.y);
-      sortc[q] = sorted[i];
-      cellc[q] = c;
-   }
-   if (i <= P.ncells) {
-      const int a = cell_start[i], b = pre[a];
-      cs[i] = b;
-      cs[P.ncells + 1 + i] = n0 + (a - b);
-   }
-}
-
 // A column offset's hi and lo parts (32 bytes, 32-byte aligned) in one load.
 __device__ __forceinline__ void ld_coff(const float4 *p, float4 &h, float4 &l)
 {
@@ -935,12 +950,11 @@ __device__ __forceinline__ ColRuns col_runs(const RsParams &P, int cx, int cy, i
 // trees.
 template <int PT, bool EW>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 8)
-k_pairs_col(RsParams P, const int *__restrict__ cs,
-            const int *__restrict__ pre, const int4 *__restrict__ cols, const int *__restrict__ col_base,
+k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__restrict__ cols, const int *__restrict__ col_base,
             const float4 *__restrict__ coff, const float4 *__restrict__ posc, const int2 *__restrict__ tagc,
             const int *__restrict__ cellc,
             const int *__restrict__ sortc, const double *__restrict__ site, const float *__restrict__ potg,
-            double *__restrict__ force, double *__restrict__ part, DevOut *out)
+            double *__restrict__ force, double *__restrict__ part, unsigned int *__restrict__ sync, DevOut *out)
 {
    typedef float R;
    constexpr int NP = NPar<PT>::v;
@@ -954,7 +968,7 @@ k_pairs_col(RsParams P, const int *__restrict__ cs,
    __syncthreads();
    const R *pot = P.pot_in_smem ? pot_s : potg;
 
-   const int N = P.nsites, n0 = P.one_class ? N : pre[N];
+   const int N = P.nsites, n0 = P.one_class ? N : cs[P.ncells];
    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
    int *inc = s_inc[w], *jbr = s_jb[w], *infr = s_inf[w], *cand = s_cand[w];
    // the lane's energy and virial over all its home sites (per-site sums
@@ -971,7 +985,7 @@ k_pairs_col(RsParams P, const int *__restrict__ cs,
    for (ColHome hm(P.chunk, w); hm.p < N; hm.next()) {
       const int p = hm.p;
       R fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
-      const int *csk = cs + (p < n0 ? 0 : P.ncells + 1);
+      const int *csk = cs + (p < n0 ? 0 : P.ncells);
       const int c = cellc[p];
       const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
       const int2 ti = tagc[p];
@@ -1125,6 +1139,7 @@ k_pairs_col(RsParams P, const int *__restrict__ cs,
       for (int q = 0; q < PAIR_WARPS; q++) s += (double)wred[threadIdx.x][q];
       part[blockIdx.x * 8 + threadIdx.x] = s;
    }
+   reduce_pairs_last(part, gridDim.x, sync, out, fin);
 }
 
 // The walk of k_pairs_col as a function: calls visit(j, inf) for every slot
@@ -1215,10 +1230,10 @@ __device__ __forceinline__ bool less_bits(double a, double b)
 // 2048-site water 0.220 -> 0.144 ms.
 template <int PT, bool EW>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 5)
-k_pairs_col64(RsParams P, const int *__restrict__ cs, const int *__restrict__ pre, const int4 *__restrict__ cols,
+k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__restrict__ cols,
               const int *__restrict__ col_base, const double4 *__restrict__ posc, const int2 *__restrict__ tagc,
               const int *__restrict__ cellc, const int *__restrict__ sortc, const double *__restrict__ potg,
-              double *__restrict__ force, double *__restrict__ part, DevOut *out)
+              double *__restrict__ force, double *__restrict__ part, unsigned int *__restrict__ sync, DevOut *out)
 {
    constexpr int NP = NPar<PT>::v;
    extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1235,14 +1250,14 @@ k_pairs_col64(RsParams P, const int *__restrict__ cs, const int *__restrict__ pr
    for (int k = 0; k < 7; k++) s_tot[k][threadIdx.x] = 0.0;
    __syncthreads();
    const double *pot = P.pot_in_smem ? pot_s : potg;
-   const int N = P.nsites, n0 = P.one_class ? N : pre[N];
+   const int N = P.nsites, n0 = P.one_class ? N : cs[P.ncells];
    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const ColRows rows{s_inc[w], s_jb[w], s_inf[w], s_cand[w]};
    const bool strict = P.strict && !P.molpbc;
    for (ColHome hm(P.chunk, w); hm.p < N; hm.next()) {
       const int p = hm.p;
       double fx = 0, fy = 0, fz = 0, pe = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0, v4 = 0, v5 = 0;
-      const int *csk = cs + (p < n0 ? 0 : P.ncells + 1);
+      const int *csk = cs + (p < n0 ? 0 : P.ncells);
       const int c = cellc[p];
       const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
       const int2 ti = tagc[p];
@@ -1317,6 +1332,7 @@ k_pairs_col64(RsParams P, const int *__restrict__ cs, const int *__restrict__ pr
       for (int q = 0; q < PAIR_WARPS; q++) s += wred[threadIdx.x][q];
       part[blockIdx.x * 8 + threadIdx.x] = 0.5 * s;
    }
+   reduce_pairs_last(part, gridDim.x, sync, out, fin);
 }
 
 // The reference's evaluated pair count after a column-walk pass (which
@@ -1335,8 +1351,12 @@ k_count_col(RsParams P, const int *__restrict__ cell_start, const int4 *__restri
       const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
       for (int col = 0; col < P.ncols; col++) {
          const ColRuns cr = col_runs(P, cx, cy, cz, __ldg(&cols[col]));
-         for (int s = 0; s < cr.ns; s++)
-            n += (unsigned long long)(__ldg(&cell_start[cr.cc + cr.zb[s] + 1]) - __ldg(&cell_start[cr.cc + cr.za[s]]));
+         for (int s = 0; s < cr.ns; s++) {
+            const int *cs = cell_start + cr.cc;
+            n += (unsigned long long)(__ldg(&cs[cr.zb[s] + 1]) - __ldg(&cs[cr.za[s]]));
+            if (!P.one_class)   // class 1's cells
+               n += (unsigned long long)(__ldg(&cs[P.ncells + cr.zb[s] + 1]) - __ldg(&cs[P.ncells + cr.za[s]]));
+         }
       }
       n -= 1;   // the home site itself
    }
@@ -1367,17 +1387,16 @@ struct NbCols {
 };
 
 __global__ void __launch_bounds__(256)
-k_tooclose_x(RsParams P, NbCols nb, const int *__restrict__ cs, const int *__restrict__ pre,
-             const int4 *__restrict__ cols, const int *__restrict__ col_base,
+k_tooclose_x(RsParams P, NbCols nb, const int *__restrict__ cs, const int4 *__restrict__ cols, const int *__restrict__ col_base,
              const float4 *__restrict__ coff, const float4 *__restrict__ posc, const int2 *__restrict__ tagc,
              const int *__restrict__ cellc,
              const int *__restrict__ sortc, const double *__restrict__ site, DevOut *out)
 {
    const int t = blockIdx.x * blockDim.x + threadIdx.x;
    const int p = t / 9, d = t - 9 * p;   // one column of the neighbourhood per thread
-   const int N = P.nsites, n0 = pre[N];
+   const int N = P.nsites, n0 = cs[P.ncells];
    if (p >= n0) return;
-   const int *cs1 = cs + P.ncells + 1;
+   const int *cs1 = cs + P.ncells;
    const int c = cellc[p];
    const int cx = c / (P.ny * P.nz), cy = (c / P.nz) % P.ny, cz = c % P.nz;
    const float4 xi = posc[p];
@@ -1885,6 +1904,8 @@ k_rdf(RsParams P, const int *__restrict__ cell_start, const int *__restrict__ sl
 }
 
 // -------------------------------------------------------------- host side
+static bool col_walk_ok(const mdgpu_ctx *c);
+
 static RsParams make_params(mdgpu_ctx *c)
 {
    RsParams P;
@@ -1975,7 +1996,7 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
          if (g0 < 0)
             for (int a = 0; a < M; a++)
                if (gpop[root(a)] > best) best = gpop[g0 = root(a)];
-         c->cls_of_id.assign(2 * (size_t)M, 0);   // second half: every identifier in class 0
+         c->cls_of_id.assign(M, 0);
          c->ncls = 1;
          for (int a = 0; a < M; a++)
             if (pop[a] > 0 && root(a) != g0) {
@@ -1984,22 +2005,29 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
             }
          for (int a = 0; a < M; a++)
             if (pop[a] == 0) c->cls_of_id[a] = 0;
-         CK(d.cls_of_id.ensure(2 * (size_t)M));
-         CK(cudaMemcpyAsync(d.cls_of_id.p, c->cls_of_id.data(), 2 * (size_t)M * sizeof(int),
-                            cudaMemcpyHostToDevice, st));
+         std::vector<int> sc(N);
+         for (int i = 0; i < N; i++) sc[i] = c->cls_of_id[c->site_id[i]];
+         CK(d.site_cls.ensure(N));
+         CK(cudaMemcpyAsync(d.site_cls.p, sc.data(), N * sizeof(int), cudaMemcpyHostToDevice, st));
+         CK(cudaStreamSynchronize(st));
       }
       CK(cudaStreamSynchronize(st));
       CK(d.cell_of.ensure(N));
       CK(d.sorted.ensure(N));
-      CK(d.pos64.ensure(N));
+      CK(d.rank.ensure(N));
+      CK(d.unsorted.ensure(N));
       CK(d.pos32.ensure(N));
       CK(d.tag.ensure(N));
+      CK(d.tagc.ensure(N));
       CK(d.slot_cell.ensure(N));
    }
    if (c->rs_valid && !c->rs_uploaded) {
-      CK(d.cell_count.ensure(g.ncells + 1));
-      CK(d.cell_start.ensure(g.ncells + 1));
-      CK(d.blocksum.ensure((g.ncells + 1 + 1023) / 1024 + 2));
+      if (2 * (size_t)g.ncells > d.cell_count.n) {
+         CK(d.cell_count.ensure(2 * (size_t)g.ncells));
+         c->counts_clean = false;
+      }
+      CK(d.cell_start.ensure(2 * (size_t)g.ncells + 1));
+      CK(d.blocksum.ensure((2 * (size_t)g.ncells + 1 + 1023) / 1024 + 2));
       CK(d.full.ensure(g.full.size()));
       CK(d.off_hi.ensure(g.full.size()));
       CK(d.off_lo.ensure(g.full.size()));
@@ -2017,19 +2045,15 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
       CK(cudaMemcpyAsync(d.cols.p, g.cols.data(), g.cols.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
       CK(cudaMemcpyAsync(d.col_base.p, g.col_base.data(), g.col_base.size() * sizeof(int), cudaMemcpyHostToDevice, st));
       CK(cudaMemcpyAsync(d.coff.p, coff.data(), coff.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-      CK(d.cs.ensure(2 * ((size_t)g.ncells + 1)));
       CK(cudaStreamSynchronize(st));
       c->rs_uploaded = true;
    }
    const int nb = (N + PAIR_WARPS - 1) / PAIR_WARPS;
    CK(d.part.ensure((size_t)nb * 8));
-   if (c->sys_dirty) {
-      CK(d.cls_pre.ensure((size_t)N + 1));
-      CK(d.cls_bsum.ensure(((size_t)N + 1 + 1023) / 1024 + 2));
-      CK(d.sortc.ensure(N));
-      CK(d.cellc.ensure(N));
-      CK(d.posc.ensure(N));
-      CK(d.tagc.ensure(N));
+   if (c->prec == MDGPU_FP64) CK(d.pos64.ensure(N));
+   if (!d.sync.p) {
+      CK(d.sync.ensure(SYNC_N));
+      CK(cudaMemsetAsync(d.sync.p, 0, SYNC_N * sizeof(unsigned int), st));
    }
    return MDGPU_OK;
 }
@@ -2063,8 +2087,6 @@ static cudaError_t launch_pairs_pt(const RsParams &P, mdgpu_ctx *c, bool ew, boo
    return ew ? launch_pairs_t<PT, true, false, 0>(P, c, force, out, keys, key_cap, smem)
              : launch_pairs_t<PT, false, false, 0>(P, c, force, out, keys, key_cap, smem);
 }
-
-static bool col_walk_ok(const mdgpu_ctx *c);
 
 template <int PT, bool EW, bool MIXED, bool LOSS>
 static cudaError_t launch_adj_col_t(const RsParams &P, const AdjParams &A, mdgpu_ctx *c, int nblk, size_t smem)
@@ -2169,6 +2191,12 @@ mdgpu_status rs_rdf(mdgpu_ctx *c, double limit, int nbins)
    const RsGeom &g = c->rs;
    cudaStream_t st = c->stream;
    if (!(limit > 0.0) || nbins <= 0) return fail(c, MDGPU_E_ARG, "RDF limit and bin count must be positive");
+   if (c->class_major) {   // binned for a force call: again in link-cell order
+      c->link_order = true;
+      const mdgpu_status s = rs_launch(c, c->cur_site, c->cofm_in.p, c->force.p, true, nullptr, 0, nullptr);
+      c->link_order = false;
+      if (s != MDGPU_OK) return s;
+   }
    double key[11];
    std::memcpy(key, g.h, 9 * sizeof(double));
    key[9] = limit;
@@ -2211,26 +2239,35 @@ mdgpu_status rs_launch(mdgpu_ctx *c, const double *d_site, const double *d_cofm,
    DevOut *out = c->out.p;
    c->cur_site = d_site;
    phase_mark(c, MDGPU_PH_CELLS);
-   CK(cudaMemsetAsync(d.cell_count.p, 0, (g.ncells + 1) * sizeof(int), st));
-   const int nent = P.nent;
+   // class by class where the column walk follows; the adjoint, the RDF and
+   // the key listing read the plain link-cell order
+   c->class_major = c->ncls == 2 && g.nbr27 && col_walk_ok(c) && !d_keys && !c->ks_all_sites && !c->link_order;
+   const int ncount = g.ncells * (c->class_major ? 2 : 1), nent = P.nent;
+   if (!c->counts_clean) CK(cudaMemsetAsync(d.cell_count.p, 0, d.cell_count.n * sizeof(int), st));
+   c->counts_clean = false;
    k_bin<<<(nent + 255) / 256, 256, 0, st>>>(P, d_site, d_cofm, d.ent_mol.p, d.ent_mol.p + c->nmols,
-                                             d.cell_of.p, d.cell_count.p, out);
-   const int n = g.ncells + 1, nbs = (n + 1023) / 1024;
-   k_scan_blocks<<<nbs, 1024, 0, st>>>(d.cell_count.p, d.cell_start.p, d.blocksum.p, n);
-   k_scan_sums<<<1, 1024, 0, st>>>(d.blocksum.p, nbs, d.blocksum.p + nbs);
-   k_scan_add<<<nbs, 1024, 0, st>>>(d.cell_start.p, d.blocksum.p, n);
-   CK(cudaMemsetAsync(d.cell_count.p, 0, (g.ncells + 1) * sizeof(int), st));
-   k_scatter<<<(N + 255) / 256, 256, 0, st>>>(N, d.cell_of.p, d.cell_start.p, d.cell_count.p, d.sorted.p);
-   k_cellsort<<<(g.ncells + 255) / 256, 256, 0, st>>>(g.ncells, d.cell_start.p, d.sorted.p);
-   // the link-cell order is all the k-space passes need from here
-   if (sorted_ready) CK(cudaEventRecord(sorted_ready, st));
+                                             c->class_major ? d.site_cls.p : nullptr, d.cell_of.p, d.rank.p,
+                                             d.cell_count.p, d.cell_start.p, ncount, d.unsorted.p, d.sync.p, out);
+   c->launches += 2;
+   if (ncount > SCAN_ONE) {
+      const int n = ncount + 1, nbs = (n + 1023) / 1024;
+      k_scan_blocks<<<nbs, 1024, 0, st>>>(d.cell_count.p, d.cell_start.p, d.blocksum.p, ncount, n);
+      k_scan_add<<<nbs, 1024, 0, st>>>(d.cell_start.p, d.blocksum.p, n);
+      c->launches += 2;
+   }
+   if (ncount > SCAN_ONE || N > SCATTER_ONE) {
+      k_scatter<<<(N + 255) / 256, 256, 0, st>>>(N, d.cell_of.p, d.cell_start.p, d.rank.p, d.unsorted.p);
+      c->launches += 1;
+   }
    const bool mixed = c->prec == MDGPU_MIXED && d_keys == nullptr;
-   k_gather<<<(N + 255) / 256, 256, 0, st>>>(P, d_site, d.chg.p, d.siteid.p, d.molmap.p, d.sorted.p,
-                                             d.cell_of.p, mixed ? nullptr : d.pos64.p,
-                                             d_keys == nullptr ? d.pos32.p : nullptr, d.tag.p,
-                                             c->ncls == 1 || !c->rs.nbr27 ? d.tagc.p : nullptr, d.slot_cell.p);
+   if (!mixed) CK(d.pos64.ensure(N));
+   k_place<<<(N + 127) / 128, 128, 0, st>>>(P, d_site, d.chg.p, d.siteid.p, d.molmap.p, d.unsorted.p, d.cell_of.p,
+                                            d.cell_start.p, d.cell_count.p, ncount, d.sorted.p,
+                                            mixed ? nullptr : d.pos64.p, d_keys == nullptr ? d.pos32.p : nullptr,
+                                            c->class_major ? nullptr : d.tag.p, d.tagc.p, d.slot_cell.p);
    CK(cudaGetLastError());
-   c->launches += 7;
+   c->counts_clean = true;
+   if (sorted_ready) CK(cudaEventRecord(sorted_ready, st));
    phase_mark(c, MDGPU_PH_PAIRS);
    if (cells_only) return MDGPU_OK;
    return rs_pairs(c, d_force, d_keys, key_cap);
@@ -2253,16 +2290,17 @@ template <int PT, bool EW>
 static cudaError_t launch_col_t(const RsParams &P, mdgpu_ctx *c, double *force, bool mixed, size_t smem, int nb)
 {
    RsDev &d = c->rd;
+   FinArgs fin = c->fin;   // nothing follows without Ewald
+   fin.on = fin.on && !fin.has_ewald;
    if (!mixed) {
       auto kfn = k_pairs_col64<PT, EW>;
       if (smem > 16 * 1024) {
          cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
          if (e != cudaSuccess) return e;
       }
-      kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(
-         P, P.one_class ? d.cell_start.p : d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p,
-         P.one_class ? d.pos64.p : d.posc64.p, d.tagc.p, P.one_class ? d.slot_cell.p : d.cellc.p,
-         P.one_class ? d.sorted.p : d.sortc.p, d.pot64.p, force, d.part.p, c->out.p);
+      kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, fin, d.cell_start.p, d.cols.p, d.col_base.p, d.pos64.p, d.tagc.p,
+                                                    d.slot_cell.p, d.sorted.p, d.pot64.p, force, d.part.p, d.sync.p,
+                                                    c->out.p);
       return cudaGetLastError();
    }
    auto kfn = k_pairs_col<PT, EW>;
@@ -2270,10 +2308,9 @@ static cudaError_t launch_col_t(const RsParams &P, mdgpu_ctx *c, double *force, 
       cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
    }
-   kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(
-      P, P.one_class ? d.cell_start.p : d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p, d.coff.p,
-      P.one_class ? d.pos32.p : d.posc.p, d.tagc.p, P.one_class ? d.slot_cell.p : d.cellc.p,
-      P.one_class ? d.sorted.p : d.sortc.p, c->cur_site, d.pot32.p, force, d.part.p, c->out.p);
+   kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, fin, d.cell_start.p, d.cols.p, d.col_base.p, d.coff.p, d.pos32.p,
+                                                 d.tagc.p, d.slot_cell.p, d.sorted.p, c->cur_site, d.pot32.p, force,
+                                                 d.part.p, d.sync.p, c->out.p);
    return cudaGetLastError();
 }
 
@@ -2285,24 +2322,8 @@ static mdgpu_status rs_pairs_col(mdgpu_ctx *c, RsParams P, double *d_force, bool
    RsDev &d = c->rd;
    cudaStream_t st = c->stream;
    const int N = c->nsites;
-   const bool two = c->ncls == 2 && c->rs.nbr27;
-   const int *cls = d.cls_of_id.p;
-   const int n1 = N + 1, nbs = (n1 + 1023) / 1024;
+   const bool two = c->class_major;
    P.one_class = !two;
-   // one class: the link-cell order as it is (k_gather wrote the packed tags)
-   if (two) {
-      k_cls_flag<<<(n1 + 255) / 256, 256, 0, st>>>(N, d.tag.p, cls, d.cls_pre.p);
-      k_scan_blocks<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_pre.p, d.cls_bsum.p, n1);
-      k_scan_sums<<<1, 1024, 0, st>>>(d.cls_bsum.p, nbs, d.cls_bsum.p + nbs);
-      k_scan_add<<<nbs, 1024, 0, st>>>(d.cls_pre.p, d.cls_bsum.p, n1);
-      if (!mixed) CK(d.posc64.ensure(N));
-      const int nsplit = std::max(N, P.ncells + 1);
-      k_cls_split<<<(nsplit + 255) / 256, 256, 0, st>>>(P, d.cls_pre.p, cls, d.cell_start.p, d.pos32.p, d.tag.p,
-                                                       d.sorted.p, d.slot_cell.p, d.pos64.p, d.cs.p, d.posc.p,
-                                                       mixed ? nullptr : d.posc64.p, d.tagc.p, d.sortc.p, d.cellc.p);
-      CK(cudaGetLastError());
-      c->launches += 5;
-   }
    // eight resident blocks per SM (the kernel's launch bounds), each warp
    // looping over home sites: the per-block set-up and energy reduction once
    // per block instead of once per four sites
@@ -2325,8 +2346,8 @@ static mdgpu_status rs_pairs_col(mdgpu_ctx *c, RsParams P, double *d_force, bool
    if (two) {
       NbCols nb;
       for (int k = 0; k < 9; k++) nb.col[k] = c->rs.nbcol[k];
-      k_tooclose_x<<<(9 * N + 255) / 256, 256, 0, st>>>(P, nb, d.cs.p, d.cls_pre.p, d.cols.p, d.col_base.p, d.coff.p,
-                                                    d.posc.p, d.tagc.p, d.cellc.p, d.sortc.p,
+      k_tooclose_x<<<(9 * N + 255) / 256, 256, 0, st>>>(P, nb, d.cell_start.p, d.cols.p, d.col_base.p, d.coff.p,
+                                                    d.pos32.p, d.tagc.p, d.slot_cell.p, d.sorted.p,
                                                     c->cur_site, c->out.p);
       CK(cudaGetLastError());
       c->launches += 1;
@@ -2339,7 +2360,8 @@ mdgpu_status rs_count_pairs(mdgpu_ctx *c)
 {
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
    if (!c->npairs_pending) return MDGPU_OK;
-   const RsParams P = make_params(c);
+   RsParams P = make_params(c);
+   P.one_class = !c->class_major;
    cudaStream_t st = c->stream;
    DevOut *out = c->out.p;
    CK(cudaMemsetAsync(&out->npairs2, 0, sizeof(out->npairs2), st));
@@ -2375,6 +2397,9 @@ mdgpu_status rs_pairs(mdgpu_ctx *c, double *d_force, unsigned long long *d_keys,
       const mdgpu_status s = rs_pairs_col(c, P, d_force, ew, mixed, smem);
       if (s != MDGPU_OK) return s;
       c->npairs_pending = true;   // counted on demand (rs_count_pairs)
+      if (c->fin.on && !c->fin.has_ewald) c->fin.on = 0;   // its last block has summed the evaluation up
+      phase_mark(c, MDGPU_PH_KPREP);
+      return MDGPU_OK;
    } else {
    switch (c->ptype) {
    case 0: e = launch_pairs_pt<0>(P, c, ew, mixed, mode, d_force, out, d_keys, key_cap, smem); break;
@@ -2389,15 +2414,10 @@ mdgpu_status rs_pairs(mdgpu_ctx *c, double *d_force, unsigned long long *d_keys,
    c->launches += 1;
    }
    if (mode == 0) {
-      if (c->rs_nblk <= 8 * 256) {
-         k_reduce_rs1<<<1, 256, 0, st>>>(d.part.p, c->rs_nblk, out);
-         c->launches += 1;
-      } else {
-         CK(d.part2.ensure(8 * RS_RED));
-         k_reduce_rs<<<RS_RED, 256, 0, st>>>(d.part.p, c->rs_nblk, d.part2.p);
-         k_reduce_rs2<<<1, 256, 0, st>>>(d.part2.p, RS_RED, out);
-         c->launches += 2;
-      }
+      CK(d.part2.ensure(8 * RS_RED));
+      k_reduce_rs<<<RS_RED, 256, 0, st>>>(d.part.p, c->rs_nblk, d.part2.p);
+      k_reduce_rs2<<<1, 256, 0, st>>>(d.part2.p, RS_RED, out);
+      c->launches += 2;
       CK(cudaGetLastError());
    }
    phase_mark(c, MDGPU_PH_KPREP);
