@@ -50,16 +50,20 @@ __device__ __forceinline__ bool tc_aborted(const int *flag)
 // Systems with more than 64 t values run once per 64-wide t-block.
 constexpr int FTC_NI = 32;                         // items per item tile (4 rows each: N = 128)
 constexpr int FTC_NSB = 2;                         // coefficient stages in flight per ring (two rings)
+constexpr int FTC_KSMAX = 512;                     // item tiles whose K-step counts are kept in shared memory
 constexpr int FTC_ATERM = 128 * 128 * 2;           // one term of a site tile's z tables: 32 KB
-constexpr int FTC_ABYTES = 3 * FTC_ATERM;          // 96 KB
 constexpr int FTC_BTERM = 128 * 16 * 2;            // one term of a coefficient stage: 4 KB
 constexpr int FTC_BBYTES = 3 * FTC_BTERM;          // 12 KB
 constexpr int FTC_SBYTES = 2 * FTC_BBYTES;         // a stage: two K-steps (24 KB), one wait and commit per 12 MMAs
 constexpr int FTC_EG = 4;                          // epilogue warps per tensor-memory lane quarter
 constexpr int FTC_IPW = FTC_NI / FTC_EG;           // items of a tile per epilogue warp
 constexpr int FTC_EW = 4 * FTC_EG;                 // epilogue warps
-constexpr int FTC_SMEM = FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES + 2 * FTC_EG * 128 * 3 * 4 + FTC_EW * FTC_IPW * 32;
-constexpr int FTC_THREADS = 32 * (FTC_EW + 4);     // epilogue warps, two bulk-copy warps, two MMA warps
+constexpr int FTC_XBYTES = 2 * FTC_EG * 128 * 3 * 4 + FTC_EW * FTC_IPW * 16;   // force sums, coefficients
+// Shared memory for z tables of aterm bytes a term: no more than needed, the
+// rest of the SM's 256 KB caches the x and y tables (131,072-site water:
+// 0.346 ms at 208 KB, 0.377 ms with a third coefficient stage, 226 KB).
+__host__ __device__ constexpr int ftc_smem(int aterm) { return 3 * aterm + 2 * FTC_NSB * FTC_SBYTES + FTC_XBYTES; }
+constexpr int FTC_THREADS = 32 * (FTC_EW + 3);     // epilogue warps, a bulk-copy warp, two MMA warps
 static_assert(FTC_IPW % 4 == 0, "an epilogue warp reads its items' columns 16 at a time");
 constexpr int FTC_SPLITS = 2;                      // force slots per site (two CTAs at most per site tile)
 constexpr int FTC_ERR = 16;                        // error-word bit: a force-pass wait expired
@@ -67,11 +71,13 @@ constexpr int FTC_ERR = 16;                        // error-word bit: a force-pa
 // Coefficient rows of each item from the dense per-(quad, t) A and B
 // (k_qreduce): one warp per item, 64 t from t0.  Item 8 j + 2 q + s is quad
 // q of unit fu[j] with k = +-m.  Layout per (item tile, K-step of 16): [term]
-// [cosines, sines][row group 16][8 rows][8 t] bf16, row 4 i + c for item i
-// of the tile.
+// [cosines, sines][row group 16][8 rows][8 t] bf16, row 8 q + 2 c + s for
+// the items (q, s) of the tile: the two signs of k side by side, as the
+// epilogue takes them in paired FP32 instructions; the force coefficients
+// likewise, per q (x+ x- y+ y-), (z0+ z0- dz+ dz-).
 __global__ void __launch_bounds__(256)
 k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, const float4 *__restrict__ ab,
-          uint4 *__restrict__ utab, float4 *__restrict__ coef)
+          uint4 *__restrict__ utab, float *__restrict__ coef)
 {
    __shared__ float4 sv[8][64];
    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -120,7 +126,7 @@ k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, 
       unsigned int hh[4], mm[4], ll[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) tc::split3(v[2 * j], v[2 * j + 1], hh[j], mm[j], ll[j]);
-      const int n = 4 * il + c;
+      const int n = 8 * (il >> 1) + 2 * c + (il & 1);
       const size_t base = ((size_t)tile * 8 + ks) * (FTC_BBYTES / 16) + kg * 128 + (n >> 3) * 8 + (n & 7);
       utab[base] = make_uint4(hh[0], hh[1], hh[2], hh[3]);
       utab[base + FTC_BTERM / 16] = make_uint4(mm[0], mm[1], mm[2], mm[3]);
@@ -130,12 +136,19 @@ k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, 
       // the seeds' table scale (units of 2^-24 and 2^-31, times Q_KAPPA each) folded in
       const double f2 = 1.0 / (16777216.0 * 2147483648.0 * Q_KAPPA * Q_KAPPA);
       const double hh = un.x, kk = neg ? -(double)(un.y + q) : (double)(un.y + q);
-      if (scalar)   // f1 alone
-         coef[i] = make_float4(un.w >= 0 ? (float)(f2 * s1) : 0.f, 0.f, 0.f, 0.f);
-      else
-         coef[i] = un.w >= 0 ? make_float4((float)((hh * g.b[0] + kk * g.b[3]) * f2 * s1), (float)((hh * g.b[1] + kk * g.b[4]) * f2 * s1),
-                                           (float)((hh * g.b[2] + kk * g.b[5]) * f2 * s1), (float)(g.b[8] * f2 * s2))
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (un.w >= 0) {
+         if (scalar) {   // f1 alone
+            v[0] = (float)(f2 * s1);
+         } else {
+            v[0] = (float)((hh * g.b[0] + kk * g.b[3]) * f2 * s1);
+            v[1] = (float)((hh * g.b[1] + kk * g.b[4]) * f2 * s1);
+            v[2] = (float)((hh * g.b[2] + kk * g.b[5]) * f2 * s1);
+            v[3] = (float)(g.b[8] * f2 * s2);
+         }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) coef[(i >> 1) * 8 + 2 * k + (i & 1)] = v[k];
    }
 }
 
@@ -204,6 +217,7 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    extern __shared__ __align__(1024) unsigned char sm[];
    __shared__ __align__(8) uint64_t full_a, a_free, full_b[2][FTC_NSB], empty_b[2][FTC_NSB], acc_full[2],
        acc_empty[2], done[2];
+   __shared__ unsigned char s_ks[FTC_KSMAX];
    __shared__ unsigned int tmem_s;
    __shared__ int abort_s;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
@@ -214,14 +228,15 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    // the range's units of site tile T: ua(T) .. ue(T) - 1; local index u - u0
    auto ua = [&](int T) { return max(u0, T * ntl); };
    auto ue = [&](int T) { return min(u1, (T + 1) * ntl); };
-   unsigned char *A = sm, *Bs = sm + FTC_ABYTES;
-   // [2][FTC_EG][128][3]: per epilogue group, a site tile's force sums (by tile parity)
-   float *red = reinterpret_cast<float *>(sm + FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES);
-   // per epilogue warp: its items' force coefficients
-   float4 *scoef = reinterpret_cast<float4 *>(sm + FTC_ABYTES + 2 * FTC_NSB * FTC_SBYTES + 2 * FTC_EG * 128 * 3 * 4);
    // the t-block's z tables of a site tile: columns, bytes of a term
    const int fcols = min(128, 2 * (g.TP - t0));
    const unsigned int aterm = (unsigned int)fcols * 256u;
+   constexpr int nsb = FTC_NSB;
+   unsigned char *A = sm, *Bs = sm + 3 * aterm;
+   // [2][FTC_EG][128][3]: per epilogue group, a site tile's force sums (by tile parity)
+   float *red = reinterpret_cast<float *>(Bs + 2 * nsb * FTC_SBYTES);
+   // per epilogue warp: its items' force coefficients
+   float4 *scoef = reinterpret_cast<float4 *>(Bs + 2 * nsb * FTC_SBYTES + 2 * FTC_EG * 128 * 3 * 4);
    if (tid == 0) {
       bar_init(&full_a, 1);
       bar_init(&a_free, 2);
@@ -234,74 +249,68 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
          bar_init(&acc_full[b], 1);
          bar_init(&acc_empty[b], FTC_EW);
       }
-      bar_init(&done[0], 1);
-      bar_init(&done[1], 1);
+      for (int k = 0; k < 2; k++) bar_init(&done[k], 1);
       abort_s = 0;
       bar_init_fence();
    }
+   for (int t = tid; t < ntl && t < FTC_KSMAX; t += FTC_THREADS) s_ks[t] = (unsigned char)ftc_ksteps(fu[t * (FTC_NI / 8)], t0);
    __syncwarp();
-   if (w == FTC_EW + 2) tmem_alloc(&tmem_s, 512);   // two buffers x (hh sums, smaller terms) x 128 columns
+   if (w == FTC_EW + 1) tmem_alloc(&tmem_s, 512);   // two buffers x (hh sums, smaller terms) x 128 columns
    fence_before_sync();
    __syncthreads();
    fence_after_sync();
    const unsigned int tmem = tmem_s;
    // K-steps of a unit's item tile
-   auto ksteps = [&](int u) { return ftc_ksteps(fu[(u % ntl) * (FTC_NI / 8)], t0); };
+   auto ksteps = [&](int nt) { return nt < FTC_KSMAX ? (int)s_ks[nt] : ftc_ksteps(fu[nt * (FTC_NI / 8)], t0); };
 
-   if (w == FTC_EW || w == FTC_EW + 1) {
-      // ---- bulk copies: warp FTC_EW + p streams the coefficient rows of the
-      // range's units of local parity p into ring p; warp FTC_EW also loads
-      // each site tile's z tables
-      const int p = w - FTC_EW;
+   if (w == FTC_EW) {
+      // ---- bulk copies: each site tile's z tables, and the coefficient rows
+      // of the range's units, those of local parity p into ring p
       if (lane == 0) {
-         int gi = 0, na = 0;
+         int gi[2] = {0, 0}, na = 0;
          bool stop = false;
          for (int T = T0; T <= T1 && !stop; T++) {
-            if (p == 0) {
-               if (T > T0 && !bar_wait(&a_free, (unsigned int)(T - T0 - 1) & 1u)) {
-                  tc_abort(&abort_s, err, FTC_ERR);
-                  break;
-               }
-               bar_expect_tx(&full_a, 3 * aterm);
-               bulk_load(A, zsite + ((size_t)T * 2 * g.TP + 2 * t0) * 48, 3 * aterm, &full_a);
-               na++;
+            if (T > T0 && !bar_wait(&a_free, (unsigned int)(T - T0 - 1) & 1u)) {
+               tc_abort(&abort_s, err, FTC_ERR);
+               break;
             }
-            for (int u = ua(T); u < ue(T) && !stop; u++) {
-               if (((u - u0) & 1) != p) continue;
-               const int kq = ksteps(u), nt = u % ntl;
+            bar_expect_tx(&full_a, 3 * aterm);
+            bulk_load(A, zsite + ((size_t)T * 2 * g.TP + 2 * t0) * 48, 3 * aterm, &full_a);
+            na++;
+            int nt = ua(T) - T * ntl;
+            for (int u = ua(T); u < ue(T) && !stop; u++, nt++) {
+               const int p = (u - u0) & 1, kq = ksteps(nt);
                // stage sq: K-steps 2 sq and, within the unit's, 2 sq + 1
                for (int sq = 0; 2 * sq < kq; sq++) {
-                  const int s = gi % FTC_NSB;
-                  if (gi >= FTC_NSB && !bar_wait(&empty_b[p][s], (unsigned int)(gi / FTC_NSB - 1) & 1u)) {
+                  const int k = gi[p], s = k % nsb;
+                  if ((k >= nsb && !bar_wait(&empty_b[p][s], (unsigned int)(k / nsb - 1) & 1u)) ||
+                      tc_aborted(&abort_s)) {
                      tc_abort(&abort_s, err, FTC_ERR);
-                     stop = true;
-                     break;
-                  }
-                  if (tc_aborted(&abort_s)) {
                      stop = true;
                      break;
                   }
                   const unsigned int bytes = 2 * sq + 1 < kq ? FTC_SBYTES : FTC_BBYTES;
                   bar_expect_tx(&full_b[p][s], bytes);
-                  bulk_load(Bs + (p * FTC_NSB + s) * FTC_SBYTES, utab + ((size_t)nt * 8 + 2 * sq) * (FTC_BBYTES / 16),
+                  bulk_load(Bs + (p * nsb + s) * FTC_SBYTES, utab + ((size_t)nt * 8 + 2 * sq) * (FTC_BBYTES / 16),
                             bytes, &full_b[p][s]);
-                  gi++;
+                  gi[p]++;
                }
             }
          }
          // copies still in flight complete before the CTA's shared memory goes
          if (na > 0) bar_wait(&full_a, (unsigned int)(na - 1) & 1u);
-         for (int q = gi > FTC_NSB ? gi - FTC_NSB : 0; q < gi; q++)
-            bar_wait(&full_b[p][q % FTC_NSB], (unsigned int)(q / FTC_NSB) & 1u);
+         for (int p = 0; p < 2; p++)
+            for (int q = gi[p] > nsb ? gi[p] - nsb : 0; q < gi[p]; q++)
+               bar_wait(&full_b[p][q % nsb], (unsigned int)(q / nsb) & 1u);
       }
-   } else if (w == FTC_EW + 2 || w == FTC_EW + 3) {
-      // ---- MMA issue: warp FTC_EW + 2 + p takes the units of local parity
-      // p into tensor-memory buffer p (one issuing thread sustains half the
-      // tensor pipe's rate at N = 128; two keep it busy)
-      const int p = w - FTC_EW - 2;
+   } else if (w > FTC_EW) {
+      // ---- MMA issue: warp FTC_EW + 1 + p takes the units of local parity p
+      // into tensor-memory buffer p (a thread issues one MMA per 150 cycles
+      // whatever its N; the tensor pipe needs two at N = 128)
+      const int p = w - FTC_EW - 1;
       const unsigned int idn = idesc_bf16(128, 128, false);
       const int ta[6] = {0, 0, 1, 0, 2, 1}, tb[6] = {0, 1, 0, 2, 0, 1};
-      const unsigned int a0 = saddr(A), b0 = saddr(Bs + p * FTC_NSB * FTC_SBYTES);
+      const unsigned int a0 = saddr(A), b0 = saddr(Bs + p * nsb * FTC_SBYTES);
       bool ok = true;
       int gi = 0, jj = 0;
       for (int T = T0; T <= T1; T++) {
@@ -318,7 +327,8 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
             ok = false;
          }
          fence_after_sync();
-         for (int u = ua(T); u < ue(T); u++) {
+         int nt = ua(T) - T * ntl;
+         for (int u = ua(T); u < ue(T); u++, nt++) {
             if (((u - u0) & 1) != p) continue;
             if (ok && (tc_aborted(&abort_s) ||
                        (jj >= 1 && !bar_wait(&acc_empty[p], (unsigned int)(jj - 1) & 1u)))) {
@@ -326,10 +336,10 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
                ok = false;
             }
             fence_after_sync();
-            const int kq = ok ? ksteps(u) : 0;
+            const int kq = ok ? ksteps(nt) : 0;
             for (int sq = 0; 2 * sq < kq; sq++) {
-               const int s = gi % FTC_NSB;
-               if (!bar_wait(&full_b[p][s], (unsigned int)(gi / FTC_NSB) & 1u)) {
+               const int s = gi % nsb;
+               if (!bar_wait(&full_b[p][s], (unsigned int)(gi / nsb) & 1u)) {
                   tc_abort(&abort_s, err, FTC_ERR);
                   ok = false;
                   break;
@@ -371,22 +381,41 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
          const size_t sg = (size_t)T * 4 + (r >> 5);
          const int *xb = X + sg * 2 * g.hrows * 36 + lane, *yb = Y + sg * 2 * g.mrows * 36 + lane;
          float Fx = 0.f, Fy = 0.f, Fz = 0.f, Cx = 0.f, Cy = 0.f, Cz = 0.f;
-         for (int u = ua(T); u < ue(T) && live; u++) {
-            const int j = u - u0, b = j & 1;
-            const int pos = (u % ntl) * (FTC_NI / 8) + ig;   // the warp's eight items: unit fu[pos]
-            // their tables and coefficients, fetched while the MMAs run
-            const int4 un = fu[pos];
+         // a unit's tables: the site's x and y values, loaded one unit ahead
+         int tx[2], ty[8];
+         int4 un = make_int4(0, 0, 0, -1);
+         float4 cnext = make_float4(0.f, 0.f, 0.f, 0.f);
+         auto fetch = [&](int nt) {
+            const int pos = nt * (FTC_NI / 8) + ig;   // the warp's eight items
+            un = __ldg(&fu[pos]);
+            if (lane < FTC_IPW) cnext = __ldg(&coef[pos * FTC_IPW + lane]);
             const int *xp = xb + (size_t)2 * un.x * 36, *yp = yb + (size_t)2 * un.y * 36;
-            const float ch = (float)__ldg(xp), sh = (float)__ldg(xp + 36);
-            float cm[4], sm4[4];
+            tx[0] = __ldg(xp);
+            tx[1] = __ldg(xp + 36);
+#pragma unroll
+            for (int q = 0; q < 8; q++) ty[q] = __ldg(yp + q * 36);
+         };
+         int nt = ua(T) - T * ntl;
+         fetch(nt);
+         for (int u = ua(T); u < ue(T) && live; u++, nt++) {
+            const int j = u - u0, b = j & 1;
+            // padding units come last; a tile whose units have no t in this
+            // block issues no MMAs, so its buffer holds an earlier unit's sums
+            const bool real = un.w >= 0 && un.z > t0;
+            // the seeds' factors, per quad (P1, P2) and (P3, P4)
+            const float ch = (float)tx[0], sh = (float)tx[1];
+            float2 sd[4], sn[4];
 #pragma unroll
             for (int q = 0; q < 4; q++) {
-               cm[q] = (float)__ldg(yp + 2 * q * 36);
-               sm4[q] = (float)__ldg(yp + (2 * q + 1) * 36);
+               const float cm = (float)ty[2 * q], sm4 = (float)ty[2 * q + 1];
+               const float a = ch * cm, d = sh * sm4, c = sh * cm, e = ch * sm4;
+               sd[q] = make_float2(a - d, a + d);   // cosine of the seed, k = +-m
+               sn[q] = make_float2(c + e, c - e);   // sine
             }
             __syncwarp();
-            if (lane < FTC_IPW) wc[lane] = coef[pos * FTC_IPW + lane];
+            if (lane < FTC_IPW) wc[lane] = cnext;
             __syncwarp();
+            if (u + 1 < ue(T)) fetch(nt + 1);
             const bool got = !tc_aborted(&abort_s) && bar_wait(&acc_full[b], (unsigned int)(j >> 1) & 1u);
             if (!__all_sync(0xffffffffu, got && !tc_aborted(&abort_s))) {
                if (lane == 0) tc_abort(&abort_s, err, FTC_ERR);
@@ -397,7 +426,7 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
             // the warp's accumulator columns (hh sums plus the rest) into
             // registers, then the buffer goes back to its MMA warp at once:
             // the next unit's MMAs into it overlap this unit's arithmetic
-            float wv[FTC_IPW / 4][16];
+            f2x wv[FTC_IPW / 4][8];
 #pragma unroll
             for (int grp = 0; grp < FTC_IPW / 4; grp++) {
                float mv[16], cv[16];
@@ -406,32 +435,31 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
                tmem_ld16(trow + col + 128, cv);
                tmem_wait2(mv, cv);
 #pragma unroll
-               for (int c = 0; c < 16; c++) wv[grp][c] = mv[c] + cv[c];
+               for (int c = 0; c < 8; c++) wv[grp][c] = add2(pk2(mv[2 * c], mv[2 * c + 1]), pk2(cv[2 * c], cv[2 * c + 1]));
             }
             fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&acc_empty[b]);
-            float fx = 0.f, fy = 0.f, fz = 0.f;
-            // (padding units come last; a tile whose units have no t in this
-            // block issues no MMAs, so its buffer holds an earlier unit's sums)
-            if (un.w >= 0 && un.z > t0)
+            if (real) {
+               f2x fx = 0ull, fy = 0ull, fz = 0ull;
 #pragma unroll
-            for (int q = 0; q < 4; q++) {
-               const float a = ch * cm[q], d = sh * sm4[q], c = sh * cm[q], e = ch * sm4[q];
-#pragma unroll
-               for (int s = 0; s < 2; s++) {
-                  const float cs = s ? a + d : a - d, sn = s ? c - e : c + e;   // seed of k = +-m
-                  const float4 cf = wc[2 * q + s];
-                  const float *W = &wv[q >> 1][8 * (q & 1) + 4 * s];
-                  const float f1 = fmaf(cs, W[1], sn * W[0]), f2 = fmaf(cs, W[3], sn * W[2]);
-                  fx = fmaf(cf.x, f1, fx);
-                  fy = fmaf(cf.y, f1, fy);
-                  fz = fmaf(cf.z, f1, fmaf(cf.w, f2, fz));
+               for (int q = 0; q < 4; q++) {
+                  const f2x *W = &wv[q >> 1][4 * (q & 1)];
+                  const f2x cs = pk2(sd[q].x, sd[q].y), sv = pk2(sn[q].x, sn[q].y);
+                  const f2x f1 = fma2(cs, W[1], mul2(sv, W[0])), f2 = fma2(cs, W[3], mul2(sv, W[2]));
+                  const float4 c0 = wc[2 * q], c1 = wc[2 * q + 1];
+                  fx = fma2(pk2(c0.x, c0.y), f1, fx);
+                  fy = fma2(pk2(c0.z, c0.w), f1, fy);
+                  fz = fma2(pk2(c1.x, c1.y), f1, fma2(pk2(c1.z, c1.w), f2, fz));
                }
+               float a, d;
+               upk2(fx, a, d);
+               kahan_add_tc(Fx, Cx, a + d);
+               upk2(fy, a, d);
+               kahan_add_tc(Fy, Cy, a + d);
+               upk2(fz, a, d);
+               kahan_add_tc(Fz, Cz, a + d);
             }
-            kahan_add_tc(Fx, Cx, fx);
-            kahan_add_tc(Fy, Cy, fy);
-            kahan_add_tc(Fz, Cz, fz);
          }
          float *rt = red + (size_t)(T & 1) * FTC_EG * 128 * 3;
          float *rr = rt + ((size_t)ig * 128 + r) * 3;
@@ -464,7 +492,7 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    }
    fence_before_sync();
    __syncthreads();
-   if (w == FTC_EW + 2) {
+   if (w == FTC_EW + 1) {
       __syncwarp();
       fence_after_sync();
       tmem_dealloc(tmem, 512);
@@ -481,7 +509,7 @@ static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d,
    const int G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
    const int4 *fu = d.q_fu.p + fu0;
    k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, scalar ? 1 : 0, fu, reinterpret_cast<const float4 *>(ab), d.utab.p,
-                                   d.tc_coef.p);
+                                   reinterpret_cast<float *>(d.tc_coef.p));
    int launches = 2;
    if (blk > 0 || d.tc_rkey[0] != T || d.tc_rkey[1] != ntl || d.tc_rkey[2] != G || d.tc_rver != d.tc_ver) {
       if (d.tc_ustart.ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
@@ -492,7 +520,7 @@ static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d,
       d.tc_rver = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
       launches++;
    }
-   k_force_tc<<<G, FTC_THREADS, FTC_SMEM, st>>>(g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p, d.q_y32.p, d.zsite.p,
+   k_force_tc<<<G, FTC_THREADS, ftc_smem(256 * std::min(128, 2 * (g.TP - t0))), st>>>(g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p, d.q_y32.p, d.zsite.p,
                                                 d.utab.p, nsites, d.tc_ustart.p, fpart, err);
    return launches;
 }
@@ -515,7 +543,7 @@ size_t ks_tc_utab_len(int npos) { return (size_t)((npos + 3) / 4) * 8 * (FTC_BBY
 
 cudaError_t ks_force_tc_init()
 {
-   return cudaFuncSetAttribute(k_force_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, FTC_SMEM);
+   return cudaFuncSetAttribute(k_force_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, ftc_smem(FTC_ATERM));
 }
 
 }  // namespace mdgpu
