@@ -187,7 +187,10 @@ __device__ __forceinline__ unsigned int qmul(int a, int b)
 __device__ __forceinline__ unsigned long long qmul(long long a, long long b)   // balanced values
 {
    const int ah = (int)(a >> 32), al = (int)a, bh = (int)(b >> 32), bl = (int)b;
-   const long long t = (long long)ah * bh + (long long)(__mulhi(ah, bl) + __mulhi(al, bh));
+   int m;
+   long long t;
+   asm("mad.hi.s32 %0, %1, %2, %3;" : "=r"(m) : "r"(al), "r"(bh), "r"(__mulhi(ah, bl)));
+   asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(t) : "r"(ah), "r"(bh), "l"((long long)m));
    return (unsigned long long)(t + t) + 0x8080808080808080ull;
 }
 

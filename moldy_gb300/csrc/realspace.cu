@@ -331,11 +331,104 @@ template <> struct PairMath<float, true> {
 //   rsqrt, rcp: the hardware's 20-bit approximation and one third-order
 //     Newton (Householder) step, e -> e^3: 5 and 3 FP64 instructions, about
 //     1 ulp;
-//   exp: Tang's table method (ACM TOMS 15, 144, 1989): x = (64 k + j) ln2/64
-//     + f, exp(x) = 2^k 2^(j/64) e^f, |f| <= ln2/128, degree 6: 12
-//     instructions, about 1 ulp.  The table of 2^(j/64) is in shared memory.
+//   exp: Tang's table method (ACM TOMS 15, 144, 1989): x = (256 k + j)
+//     ln2/256 + f, exp(x) = 2^k 2^(j/256) e^f, |f| <= ln2/512, degree 4, the
+//     rounding residue of 2^(j/256) added to f: 10 instructions, 0.52 ulp (a
+//     64-entry table without residues and degree 6 took 12, for 0.87 ulp).
+//     The table is in shared memory.
 // Arguments outside their range (r^2 zero or subnormal, |x| > 700) take the
 // general functions.
+// 2^(j/256), j = 0 .. 255, rounded from 400-bit repeated square roots, and the
+// relative residue of the rounding; ln2/256 in two parts and 256/ln2
+__device__ const double2 g_exp2_tab[256] = {
+   {1.0, 0.000000e+00}, {1.0027112750502025, -3.626783e-17}, {1.0054299011128027, 9.447885e-17},
+   {1.0081558981184175, -3.225750e-17}, {1.0108892860517005, -1.507067e-17}, {1.0136300849514894, 9.158765e-18},
+   {1.016378314910953, -5.679155e-17}, {1.019133996077738, 3.534280e-17}, {1.0218971486541166, 4.999745e-17},
+   {1.0246677928971357, -7.379570e-17}, {1.0274459491187637, -4.823684e-17}, {1.030231637686041, 3.222411e-17},
+   {1.0330248790212284, 7.357847e-18}, {1.0358256936019572, -7.536772e-17}, {1.0386341019613787, 5.773230e-17},
+   {1.041450124688316, 3.634193e-17}, {1.0442737824274138, 8.189318e-17}, {1.0471050958792898, 6.949710e-17},
+   {1.0499440858006872, 5.326891e-17}, {1.0527907730046264, -9.146625e-17}, {1.0556451783605572, 1.666588e-18},
+   {1.0585073227945128, -6.757300e-17}, {1.061377227289262, -1.128113e-17}, {1.0642549128844645, 4.772122e-17},
+   {1.0671404006768237, -7.402825e-17}, {1.0700337118202419, -9.286775e-17}, {1.0729348675259756, -3.578660e-18},
+   {1.075843889062791, -9.297554e-18}, {1.0787607977571199, -6.170655e-17}, {1.0816856149932152, -4.421455e-17},
+   {1.0846183622133092, 2.919140e-17}, {1.0875590609177697, 4.973844e-18}, {1.0905077326652577, -2.793911e-17},
+   {1.0934643990728858, 1.318192e-17}, {1.0964290818163769, -5.399285e-17}, {1.099401802630222, 6.522146e-17},
+   {1.102382583307841, 4.776959e-17}, {1.1053714457017412, 7.453864e-17}, {1.1083684117236787, -7.927701e-17},
+   {1.1113735033448175, 5.006368e-17}, {1.1143867425958924, 9.341711e-17}, {1.1174081515673693, -7.138668e-17},
+   {1.1204377524096067, -5.534521e-17}, {1.12347556733302, -8.633688e-17}, {1.1265216186082418, 4.585670e-17},
+   {1.129575928566288, 5.942766e-17}, {1.1326385195987192, 2.858243e-17}, {1.1357094141578055, 4.461176e-17},
+   {1.1387886347566916, 7.826573e-17}, {1.1418762039695616, 4.073201e-17}, {1.1449721444318042, 4.053627e-17},
+   {1.148076478840179, 6.008084e-17}, {1.1511892299529827, 2.823784e-17}, {1.154310420590216, 9.024547e-17},
+   {1.1574400736337511, -7.882802e-17}, {1.1605782120274988, -2.809841e-17}, {1.1637248587775775, 3.290473e-17},
+   {1.1668800369524817, -7.534519e-17}, {1.1700437696832502, -1.579209e-18}, {1.1732160801636373, -6.211612e-17},
+   {1.1763969916502812, 4.721368e-17}, {1.1795865274628758, 8.555805e-17}, {1.182784710984341, 1.304528e-17},
+   {1.1859915656609938, -7.765238e-18}, {1.189207115002721, 3.348462e-17}, {1.1924313825831512, 3.687886e-17},
+   {1.1956643920398273, 3.861120e-17}, {1.1989061670743806, -8.181786e-17}, {1.202156731452703, 5.527550e-17},
+   {1.2054161090051239, -2.785156e-17}, {1.2086843236265816, -3.927184e-17}, {1.2119613992768012, -4.035286e-17},
+   {1.215247359980469, -6.346552e-17}, {1.2185422298274085, -7.391395e-17}, {1.2218460329727576, -8.684418e-17},
+   {1.2251587936371455, -7.267249e-17}, {1.22848053610687, -1.545634e-17}, {1.2318112847340759, 5.998794e-17},
+   {1.2351510639369334, -8.707635e-17}, {1.2384998981998165, 2.234721e-17}, {1.241857812073484, 3.750854e-17},
+   {1.245224830175258, -3.756141e-17}, {1.2486009771892048, -6.616855e-17}, {1.2519862778663162, 3.861198e-17},
+   {1.255380757024691, -5.346099e-18}, {1.2587844395497165, -6.690409e-17}, {1.2621973503942507, -2.443726e-17},
+   {1.2656195145788063, 3.358495e-17}, {1.2690509571917332, 2.102305e-18}, {1.2724917033894028, -8.312759e-18},
+   {1.275941778396392, 7.771068e-17}, {1.2794012075056693, -7.627861e-17}, {1.2828700160787783, 1.335751e-17},
+   {1.2863482295460256, -2.656322e-17}, {1.2898358734066657, 6.938292e-17}, {1.2933329732290895, -2.299942e-17},
+   {1.2968395546510096, 1.957259e-17}, {1.3003556433796506, 4.367058e-17}, {1.3038812651919358, 6.632257e-17},
+   {1.3074164459346773, -5.611560e-17}, {1.3109612115247644, -5.478069e-17}, {1.3145155879493546, 1.725003e-17},
+   {1.318079601266064, -4.140839e-17}, {1.3216532776031575, -1.876921e-17}, {1.3252366431597413, -2.157148e-17},
+   {1.3288297242059544, 3.077209e-17}, {1.3324325470831615, -3.828777e-17}, {1.3360451382041458, -4.409931e-17},
+   {1.339667524053303, 6.663805e-17}, {1.3432997311868353, -4.319647e-17}, {1.3469417862329458, 2.393619e-17},
+   {1.3505937158920345, -6.135902e-17}, {1.3542555469368927, 5.686481e-17}, {1.3579273062129011, -7.017780e-17},
+   {1.3616090206382248, 1.126452e-18}, {1.365300717204012, -7.328322e-17}, {1.3690024229745905, 7.007875e-17},
+   {1.3727141650876684, -3.275234e-17}, {1.3764359707545302, -5.011921e-17}, {1.380167867260238, 7.615244e-17},
+   {1.383909881963832, -4.892307e-17}, {1.387662042298529, 6.069910e-17}, {1.3914243757719262, -3.526009e-17},
+   {1.3951969099662003, -6.686752e-17}, {1.3989796725383112, -6.872304e-17}, {1.4027726912202048, -3.775226e-17},
+   {1.4065759938190154, 5.001447e-18}, {1.4103896082172707, 2.954183e-17}, {1.4142135623730951, -6.835809e-17},
+   {1.4180478843204152, 1.603922e-17}, {1.4218926021691656, -1.130734e-17}, {1.4257477441054942, 6.930182e-17},
+   {1.42961333839197, -8.416012e-18}, {1.433489413367789, -4.047783e-17}, {1.4373759974489824, -2.924798e-17},
+   {1.4412731191286257, 3.887191e-18}, {1.4451808069770467, -2.092304e-17}, {1.449099089642035, -4.319515e-17},
+   {1.4530279958490526, -3.977865e-17}, {1.4569675544014438, 3.877011e-17}, {1.460917794180647, -3.833465e-17},
+   {1.4648787441464057, 6.506182e-17}, {1.4688504333369818, 5.763611e-17}, {1.4728328908693675, 4.543471e-17},
+   {1.4768261459394993, -2.359109e-17}, {1.4808302278224719, -6.541568e-17}, {1.4848451658727524, 7.260075e-17},
+   {1.488870989524397, 4.134252e-17}, {1.4929077282912648, 9.506897e-18}, {1.4969554117672355, -1.911656e-17},
+   {1.5010140696264256, -4.272956e-17}, {1.5050837316234065, 4.700543e-17}, {1.5091644275934228, -6.735219e-17},
+   {1.5132561874526098, 5.871113e-17}, {1.5173590411982147, -2.839604e-17}, {1.5214730189088146, -3.941173e-18},
+   {1.5255981507445384, -7.226635e-17}, {1.529734466947287, 2.474803e-17}, {1.533881997840956, 5.786121e-17},
+   {1.5380407738316568, 6.615346e-17}, {1.5422108254079407, 5.154830e-17}, {1.5463921831410214, 6.908959e-17},
+   {1.550584877685, -9.416258e-18}, {1.5547889397770887, -5.147426e-17}, {1.559004400237837, 2.425399e-17},
+   {1.5632312899713576, 4.788017e-17}, {1.567469639965553, -6.604314e-17}, {1.5717194812923414, -2.126960e-17},
+   {1.5759808451078865, -6.432132e-18}, {1.5802537626528246, -3.267452e-17}, {1.5845382652524937, -1.220401e-17},
+   {1.588834384317164, -3.773175e-18}, {1.593142151342267, -6.336162e-17}, {1.597461597908627, 1.556744e-17},
+   {1.6017927556826934, -3.780088e-17}, {1.606135656416771, -6.446868e-17}, {1.6104903319492543, 1.534141e-17},
+   {1.6148568142048607, -4.530843e-17}, {1.6192351351948637, 1.293286e-17}, {1.6236253270173289, -2.207722e-17},
+   {1.6280274218573478, -4.123367e-17}, {1.632441451987275, 6.035634e-17}, {1.6368674497669644, 4.703084e-17},
+   {1.6413054476440063, -5.634277e-17}, {1.645755478153965, -6.152603e-17}, {1.6502175739206177, 5.534591e-18},
+   {1.6546917676561943, 5.827849e-17}, {1.6591780921616162, -4.385030e-17}, {1.6636765803267364, 3.540948e-17},
+   {1.6681872651305825, 2.559172e-17}, {1.6727101796415966, -3.274157e-17}, {1.6772453570178785, 4.950945e-17},
+   {1.681792830507429, 4.875161e-17}, {1.6863526334483934, -4.258577e-17}, {1.6909247992693053, -5.718570e-17},
+   {1.6955093614893326, 4.269170e-17}, {1.7001063537185235, -4.719540e-18}, {1.7047158096580513, -1.600785e-17},
+   {1.709337763100463, -5.773452e-17}, {1.713972247929926, 3.777176e-17}, {1.718619298122478, -1.077249e-17},
+   {1.723278947746274, -5.525585e-17}, {1.7279512309618377, -6.221809e-17}, {1.732636182022311, -9.800390e-19},
+   {1.7373338352737062, 1.821405e-17}, {1.7420442251551564, -8.759589e-19}, {1.746767386199169, -6.155537e-17},
+   {1.7515033530318782, -2.925744e-17}, {1.7562521603732995, 1.685487e-17}, {1.761013843037584, -4.510614e-17},
+   {1.7657884359332727, 5.358125e-17}, {1.7705759740635547, 3.367150e-17}, {1.7753764925265212, 3.621616e-17},
+   {1.7801900265154245, -2.968575e-17}, {1.785016611318935, 8.588380e-18}, {1.789856282321401, -2.321055e-17},
+   {1.7947090750031072, 1.015622e-17}, {1.7995750249405351, -1.404159e-17}, {1.804454167806624, -2.869135e-17},
+   {1.809346539371032, -4.992212e-17}, {1.8142521755003989, -5.495119e-17}, {1.8191711121586085, 4.069258e-17},
+   {1.8241033854070534, -5.569656e-17}, {1.8290490314048973, 3.766544e-17}, {1.8340080864093424, 1.790127e-17},
+   {1.8389805867758937, 3.762394e-18}, {1.843966568958626, -3.221177e-17}, {1.8489660695104508, 4.882502e-17},
+   {1.8539791250833855, 5.265371e-17}, {1.8590057724288205, -5.125700e-17}, {1.864046048397789, 3.508987e-17},
+   {1.8690999899412386, -5.317268e-17}, {1.8741676341103, -3.266924e-17}, {1.8792490180565602, -8.634468e-18},
+   {1.8843441790323345, -4.365759e-17}, {1.8894531543909392, -4.766018e-17}, {1.8945759815869656, 1.796393e-17},
+   {1.8997126981765553, -2.031749e-17}, {1.9048633418176741, 3.430093e-17}, {1.9100279502703899, -3.094032e-17},
+   {1.9152065613971474, -5.545066e-17}, {1.9203992131630474, 3.705834e-17}, {1.925605943636125, -5.149010e-17},
+   {1.930826790987627, 3.194046e-17}, {1.9360617934922943, 5.336806e-17}, {1.9413109895286405, -3.419354e-17},
+   {1.9465744175792332, 3.498979e-17}, {1.9518521162309783, -1.126631e-17}, {1.9571441241754002, 4.578492e-17},
+   {1.9624504802089273, 5.593437e-17}, {1.9677712232331759, -5.241935e-17}, {1.9731063922552343, -3.776592e-18},
+   {1.978456026387951, 2.041428e-17}, {1.9838201648502194, -1.110713e-17}, {1.9891988469672663, 4.124843e-18},
+   {1.9945921121709402, 8.979134e-18},
+};
+constexpr double EXP_HI = 0.00270760617331689, EXP_LO = 7.453964567463233e-13, EXP_INV = 369.3299304675746;
 __device__ __forceinline__ double rsqrt_n(double x)
 {
    // (range checks on the exponent bits: a compare would take the FP64 pipe)
@@ -353,27 +446,26 @@ __device__ __forceinline__ double rcp_n(double x)
    const double e = fma(-x, y, 1.0);
    return fma(y, fma(e, e, e), y);
 }
-__shared__ double exp2_tab[64];   // 2^(j/64); filled by exp2_fill (kernels that use exp_n)
+__shared__ double2 exp2_tab[256];   // g_exp2_tab; filled by exp2_fill (kernels that use exp_n)
 __device__ __forceinline__ void exp2_fill()
 {
-   for (int j = threadIdx.x; j < 64; j += blockDim.x) exp2_tab[j] = exp2((double)j * 0.015625);
+   for (int j = threadIdx.x; j < 256; j += blockDim.x) exp2_tab[j] = g_exp2_tab[j];
 }
 __device__ __forceinline__ double exp_n(double x)
 {
    if (((unsigned int)__double2hiint(x) & 0x7fffffffu) >= 0x4085e000u) return exp(x);   // |x| >= 700
-   const double w = fma(x, 92.332482616893657, 6755399441055744.0);   // x 64/ln2 + 1.5 2^52
+   const double w = fma(x, EXP_INV, 6755399441055744.0);   // x 256/ln2 + 1.5 2^52
    const int n = __double2loint(w);
    const double nf = w - 6755399441055744.0;
-   // ln2/64 in two parts, the first with 21 trailing zero bits (nf exact in it)
-   const double f = fma(nf, -2.9815858269852933e-12, fma(nf, -0.010830424693267560, x));
-   double p = fma(f, 1.0 / 720.0, 1.0 / 120.0);
-   p = fma(f, p, 1.0 / 24.0);
-   p = fma(f, p, 1.0 / 6.0);
+   // ln2/256 in two parts, the first with 21 trailing zero bits (nf exact in it)
+   const double f = fma(nf, -EXP_LO, fma(nf, -EXP_HI, x));
+   // (cubic coefficient: 1/6 and the best fit of f^5/120 by f^3 over the range)
+   const double2 t = exp2_tab[n & 255];
+   double p = fma(f, 1.0 / 24.0, 0.16666667994052387);
    p = fma(f, p, 0.5);
-   p = fma(f * f, p, f);
-   const double t = exp2_tab[n & 63];
-   const double r = fma(t, p, t);
-   return __hiloint2double(__double2hiint(r) + ((n >> 6) << 20), __double2loint(r));
+   p = fma(f * f, p, f + t.y);
+   const double r = fma(t.x, p, t.x);
+   return __hiloint2double(__double2hiint(r) + ((n >> 8) << 20), __double2loint(r));
 }
 template <> struct PairMath<double, true> {
    static __device__ __forceinline__ double rsqrt(double x) { return rsqrt_n(x); }
@@ -401,11 +493,28 @@ __device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm,
       rs_r = M::rcp(r2);
    }
    if (EW) {
-      R ar = alpha * r;
-      t = M::rcp(R(1) + R(ASP) * ar);
-      ef = qq * M::ex(-(ar * ar));
+      if (FAST && sizeof(R) == 8) {   // one product fewer (FP64)
+         t = M::rcp(fma((R(ASP) * alpha), r, R(1)));
+         ef = qq * M::ex(-(alpha * alpha) * r2);
+      } else {
+         R ar = alpha * r;
+         t = M::rcp(R(1) + R(ASP) * ar);
+         ef = qq * M::ex(-(ar * ar));
+      }
       t = (t * (R(AS1) + t * (R(AS2) + t * (R(AS3) + t * (R(AS4) + t * R(AS5)))))) * ef * r_r;
       ef = t + norm * ef;
+   }
+   if (EW && FAST && sizeof(R) == 8) {
+      // FP64: a potential whose parameters are all zero adds exactly nothing
+      // (rigid water's H and M: 9 of 10 pairs of their class)
+      unsigned long long any = 0;
+#pragma unroll
+      for (int k = 0; k < NPar<PT>::v; k++) any |= (unsigned long long)__double_as_longlong((double)p[k]) << 1;
+      if (any == 0) {
+         u = t;
+         f = rs_r * ef;
+         return;
+      }
    }
    if (PT == 0) {
       R r6 = (p[1] * p[1]) * rs_r;
@@ -1225,9 +1334,11 @@ __device__ __forceinline__ bool less_bits(double a, double b)
 // The FP64 form by columns over one interaction class at a time: k_pairs'
 // FP64 arithmetic for r and r^2 (the reference's operation order), with the
 // cheaper square root, reciprocal and exponential of PairMath<double, true>.
-// The FP64 pipe bounds it: 131,072-site water (real-space phase) 9.75 ms
-// with k_pairs (every class, 110 FP64 instructions per pair), 4.61 ms here;
-// 2048-site water 0.220 -> 0.144 ms.
+// The FP64 pipe bounds it (79 % busy at 32,000 sites): 131,072-site water
+// (real-space phase) 9.75 ms with k_pairs (every class, 110 FP64 instructions
+// per pair), 4.61 ms with 81 of them, 3.79 ms without those of a potential of
+// zero parameters and with the shorter exponential; 2048-site water
+// 0.220 -> 0.105 ms.
 template <int PT, bool EW>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 5)
 k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__restrict__ cols,
