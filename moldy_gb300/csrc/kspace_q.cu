@@ -34,8 +34,11 @@
 //
 // Measured, 131,072-site water (98,304 charged sites, 69,876 k-vectors),
 // against one FP64 recurrence per k and site, or the seed-and-run bf16
-// products of the mixed form: FP64 structure factor 119.4 -> 1.41 ms, forces
-// 130.4 -> 4.86 ms; mixed structure factor 0.414 -> 0.274 ms.  Force error
+// products of the mixed form: FP64 structure factor 119.4 -> 1.30 ms, forces
+// 130.4 -> 4.80 ms; mixed structure factor 0.414 -> 0.262 ms.  What bounds the
+// FP64 passes: each of the two A buffers goes round build (1500 cycles), MMAs
+// (1800) and two barriers; the read-back of a segment (its conversions) is a
+// quarter of the force pass.  Force error
 // of the FP64 form against extended precision (2048-site water; rock salt,
 // 5832 ions): 6.1e-15 -> 2.2e-15; 1.5e-14 -> 1.1e-14.
 #include <algorithm>
@@ -60,8 +63,8 @@ template <> struct QCfg<3> {
    typedef int T;
    typedef float P;                               // structure-factor partials
    static constexpr int RS = 36;                  // table row: 32 sites, padded against bank conflicts
-   static constexpr int MT = 2, NPART = 1;        // 128-row tiles per CTA, column parts of B
-   static constexpr int NB = 3;                   // stages in flight
+   static constexpr int MT = 2;                   // 128-row tiles per CTA
+   static constexpr int NB = 3;                   // B operands in flight; one table buffer more
    static constexpr int NTMAX = 64;               // columns (2 t-width) of a t-block
    static constexpr int SEG = 32;                 // stages between read-backs
 };
@@ -69,20 +72,21 @@ template <> struct QCfg<7> {
    typedef long long T;
    typedef double P;
    static constexpr int RS = 34;
-   static constexpr int MT = 1, NPART = 2;
+   static constexpr int MT = 1;
    static constexpr int NB = 2;
    static constexpr int NTMAX = 64;
    static constexpr int SEG = 4;
 };
-// bytes: a stage's table rows, its B operand, both; the A operand; all
+// bytes: a stage's table rows, its B operand; the A operand; all
 template <int NS> constexpr int Q_TAB = 2 * (Q_XMAX + Q_YMAX) * QCfg<NS>::RS * (int)sizeof(typename QCfg<NS>::T);
 // (ND: digits of operand B, NS unless weights of a wide range need more)
 template <int ND> constexpr int Q_B = 64 * Q_KS * 2 * ND;
-template <int NS, int ND> constexpr int Q_STAGE = Q_B<ND> + Q_TAB<NS>;
 template <int NS> constexpr int Q_A = QCfg<NS>::MT * NS * Q_OP;
-template <int NS, int ND> constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_STAGE<NS, ND>;
-static_assert(Q_SMEM<3, 4> <= 227 * 1024 && Q_SMEM<7, 7> <= 227 * 1024, "one CTA's shared memory");
-static_assert(Q_STAGE<3, 3> % 128 == 0 && Q_STAGE<3, 4> % 128 == 0 && Q_STAGE<7, 7> % 128 == 0, "stage buffers stay aligned");
+template <int NS, int ND>
+constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_B<ND> + (QCfg<NS>::NB + 1) * Q_TAB<NS>;
+constexpr int Q_FNB = 3, Q_FSMEM = 2 * Q_A<7> + Q_FNB * Q_B<7>;   // FP64 force pass: no table rows in shared memory
+static_assert(Q_SMEM<3, 4> <= 226 * 1024 && Q_SMEM<7, 7> <= 226 * 1024 && Q_FSMEM <= 220 * 1024, "one CTA's shared memory");
+static_assert(Q_B<3> % 128 == 0 && Q_TAB<3> % 128 == 0 && Q_TAB<7> % 128 == 0, "stage buffers stay aligned");
 
 // ------------------------------------------------------ fixed-point trig
 // sin, cos(2 pi p / 2^64) in units of 2^-63: the phase is reduced to an
@@ -345,11 +349,10 @@ k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__re
 #pragma unroll
             for (int e = 0; e < 8; e++) v[e] = qz(e);
             const int tcol = 2 * t0 + 8 * cg, b = tcol / (2 * g.TW), lc = tcol - 2 * b * g.TW;
-            const int nT = q_blkcols(g, b), pc = nT / QCfg<NS>::NPART;   // columns of a part
-            const int part = lc / pc, pl = lc - part * pc;
+            const int nT = q_blkcols(g, b);
             unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * NS + (size_t)2 * b * g.TW * Q_KS * 2 * NS +
-                               ((size_t)part * NS * pc + pl) * Q_KS * 2 + kg * 128 + c8 * 16;
-            qstore<NS>(d, pc * Q_KS * 2, v);
+                               (size_t)lc * Q_KS * 2 + kg * 128 + c8 * 16;
+            qstore<NS>(d, nT * Q_KS * 2, v);
          }
       }
       if (NS == 3) {
@@ -384,7 +387,7 @@ __device__ __forceinline__ void q_abort(int *flag, int *err, int bit)
 __device__ __forceinline__ bool q_aborted(const int *flag) { return *(const volatile int *)flag != 0; }
 
 struct QBars {
-   uint64_t full_b[3], empty_b[3], full_a[2], empty_a[2], accf, acce, done[2];
+   uint64_t full_b[3], empty_b[3], full_t[4], full_a[2], empty_a[2], accf, acce, done[2];
 };
 __device__ __forceinline__ void q_init(QBars &B)
 {
@@ -392,6 +395,7 @@ __device__ __forceinline__ void q_init(QBars &B)
       tc::bar_init(&B.full_b[s], 1);
       tc::bar_init(&B.empty_b[s], 2);   // released by both MMA issuers
    }
+   for (int s = 0; s < 4; s++) tc::bar_init(&B.full_t[s], 1);
    for (int s = 0; s < 2; s++) {
       tc::bar_init(&B.full_a[s], Q_BW);
       tc::bar_init(&B.empty_a[s], 2);
@@ -404,19 +408,21 @@ __device__ __forceinline__ void q_init(QBars &B)
 }
 
 // MMA issue of one thread (issuer p of two) over nst stages in segments of
-// SEG: NS = 3, issuer p takes 128-row tile p; NS = 7, column part p.
+// SEG.  NS = 3: issuer p takes 128-row tile p, its groups in columns 256 p
+// on.  NS = 7: issuer 0 adds to groups 0 .. 3, issuer 1 to groups 4 .. 6 (a
+// thread issues an MMA about every 150 cycles whatever its width: 11 wide
+// ones per K-step, 4 and 7, where halves of the columns took 14 narrow ones).
 // Operand stages: A [tile][digit][row group 16][kg 4][8 rows][16 B], B
-// [part][digit][col group][kg 4][8][16 B].
-template <int NS, int ND>
+// [digit][col group][kg 4][8][16 B].
+template <int NS, int ND, int NB>
 __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned char *Bbuf, unsigned int tmem, int p,
                                         int nst, int nT, int *abort_s, int *err, int errbit)
 {
    using namespace tc;
-   constexpr int SEG = QCfg<NS>::SEG, NB = QCfg<NS>::NB;
-   const int pc = nT / QCfg<NS>::NPART;
-   const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NS * Q_OP : 0);
-   const unsigned int b0 = saddr(Bbuf) + (QCfg<NS>::NPART == 2 ? p * ND * pc * Q_KS * 2 : 0);
-   const unsigned int d0 = tmem + 256u * p;
+   constexpr int SEG = QCfg<NS>::SEG;
+   const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NS * Q_OP : 0), b0 = saddr(Bbuf);
+   const unsigned int d0 = tmem + (QCfg<NS>::MT == 2 ? 256u * p : 0u);
+   const int g0 = NS == 7 && p == 1 ? 4 : 0, g1 = NS == 7 && p == 0 ? 4 : ND;   // this issuer's groups
    for (int st = 0; st < nst; st++) {
       const int sa = st & 1, sb = st % NB, seg = st / SEG;
       if (!bar_wait(&B.full_a[sa], (unsigned int)(st >> 1) & 1u) ||
@@ -429,10 +435,13 @@ __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned 
 #pragma unroll
       for (int ks = 0; ks < 2; ks++)
 #pragma unroll
-         for (int i = 0; i < NS; i++)
-            mma_f16(d0 + i * pc, sdesc(a0 + sa * Q_A<NS> + i * Q_OP + ks * 256, 128, 512),
-                    sdesc(b0 + sb * Q_STAGE<NS, ND> + ks * 256, 128, 512), idesc_f16(128, (ND - i) * pc, false),
-                    st % SEG != 0 || ks > 0 || i > 0);
+         for (int i = 0; i < NS; i++) {
+            const int ga = max(i, g0);   // first group of digit i of A
+            if (ga < g1)
+               mma_f16(d0 + ga * nT, sdesc(a0 + sa * Q_A<NS> + i * Q_OP + ks * 256, 128, 512),
+                       sdesc(b0 + sb * Q_B<ND> + (ga - i) * nT * Q_KS * 2 + ks * 256, 128, 512),
+                       idesc_f16(128, (g1 - ga) * nT, false), st % SEG != 0 || ks > 0 || i > 0);
+         }
       mma_commit(&B.empty_a[sa]);
       mma_commit(&B.empty_b[sb]);
       if (st % SEG == SEG - 1 || st == nst - 1) mma_commit(&B.accf);
@@ -511,12 +520,12 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
 {
    using namespace tc;
    typedef typename QCfg<NS>::T T;
-   constexpr int RS = QCfg<NS>::RS, MT = QCfg<NS>::MT, NB = QCfg<NS>::NB, SEG = QCfg<NS>::SEG;
+   constexpr int RS = QCfg<NS>::RS, MT = QCfg<NS>::MT, NB = QCfg<NS>::NB, NTB = NB + 1, SEG = QCfg<NS>::SEG;
    extern __shared__ __align__(1024) unsigned char sm[];
    __shared__ __align__(8) QBars B;
    __shared__ unsigned int tmem_s;
    __shared__ int abort_s;
-   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>;
+   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>, *Tbuf = Sbuf + NB * Q_B<ND>;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
    const QTile &ti = tiles[blockIdx.x];
    const int nT = ti.nT, st0 = blockIdx.y * per, nst = min(nstages, st0 + per) - st0;
@@ -533,33 +542,44 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
    const unsigned int tmem = tmem_s;
 
    if (w == Q_BW) {
-      // ---- bulk copies: a stage's digits of q z and the tile's table rows
+      // ---- bulk copies: a stage's digits of q z, and the tile's table rows
+      // a stage ahead of them (the operand is built from them before its
+      // MMAs; the rows of stage st - NB were read before its MMAs, so the
+      // wait for those frees them too)
       if (lane == 0) {
          const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * ND);
          const unsigned int xb = (unsigned int)(2 * ti.nx * RS * sizeof(T)), yb = (unsigned int)(2 * ti.ny * RS * sizeof(T));
-         int issued = 0;
+         auto table = [&](int st) {
+            unsigned char *d = Tbuf + (st % NTB) * Q_TAB<NS>;
+            const size_t sg = (size_t)(st0 + st);
+            bar_expect_tx(&B.full_t[st % NTB], xb + yb);
+            bulk_load(d, X + (sg * g.hrows + ti.xlo) * 2 * RS * sizeof(T), xb, &B.full_t[st % NTB]);
+            bulk_load(d + 2 * Q_XMAX * RS * sizeof(T), Y + (sg * g.mrows + ti.ylo) * 2 * RS * sizeof(T), yb,
+                      &B.full_t[st % NTB]);
+         };
+         int issued = 0, tabs = 1;
+         table(0);
          for (int st = 0; st < nst; st++) {
             const int s = st % NB;
             if ((st >= NB && !bar_wait(&B.empty_b[s], (unsigned int)(st / NB - 1) & 1u)) || q_aborted(&abort_s)) {
                q_abort(&abort_s, err, Q_ERR);
                break;
             }
-            unsigned char *d = Sbuf + s * Q_STAGE<NS, ND>;
-            const size_t sg = (size_t)(st0 + st);
-            bar_expect_tx(&B.full_b[s], bb + xb + yb);
-            bulk_load(d, ztab + blockIdx.z * zstride + (sg * 2 * g.TP + ti.col0) * Q_KS * 2 * ND, bb, &B.full_b[s]);
-            bulk_load(d + Q_B<ND>, X + (sg * g.hrows + ti.xlo) * 2 * RS * sizeof(T), xb, &B.full_b[s]);
-            bulk_load(d + Q_B<ND> + 2 * Q_XMAX * RS * sizeof(T), Y + (sg * g.mrows + ti.ylo) * 2 * RS * sizeof(T), yb,
-                      &B.full_b[s]);
+            bar_expect_tx(&B.full_b[s], bb);
+            bulk_load(Sbuf + s * Q_B<ND>, ztab + blockIdx.z * zstride + ((size_t)(st0 + st) * 2 * g.TP + ti.col0) * Q_KS * 2 * ND,
+                      bb, &B.full_b[s]);
             issued = st + 1;
+            if (tabs < nst) table(tabs++);
          }
          // copies still in flight complete before the CTA's shared memory goes
          for (int st = issued > NB ? issued - NB : 0; st < issued; st++)
             bar_wait(&B.full_b[st % NB], (unsigned int)(st / NB) & 1u);
+         for (int st = tabs > NTB ? tabs - NTB : 0; st < tabs; st++)
+            bar_wait(&B.full_t[st % NTB], (unsigned int)(st / NTB) & 1u);
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS, ND>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
+         q_issue<NS, ND, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
    } else {
       // ---- A operand: row 8 w + (lane & 7) of each 128-row tile (product
       // p of a quad), sites 8 kg .. 8 kg + 7 of the stage
@@ -588,7 +608,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
       }
       const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16);
       // first column of this warp in tensor memory and the group stride
-      const int pc = nT / QCfg<NS>::NPART, pl = cq * ncw;
+      const int pl = cq * ncw;
       auto flush = [&](int seg) -> bool {
          const bool got = bar_wait(&B.accf, (unsigned int)seg & 1u);
          if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
@@ -602,10 +622,10 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
             for (int ch = 0; ch < MAXC; ch++)
                if (4 * ch < ncw) {
                   const int lc = pl + 4 * ch;   // column of the block
-                  const unsigned int col = MT == 2 ? 256u * mt + lc : 256u * (lc / pc) + lc % pc;
+                  const unsigned int col = 256u * mt + lc;
                   float d[ND][4];
 #pragma unroll
-                  for (int k = 0; k < ND; k++) q_ld4(trow + col + k * pc, d[k]);
+                  for (int k = 0; k < ND; k++) q_ld4(trow + col + k * nT, d[k]);
                   q_ldwait(d);
 #pragma unroll
                   for (int e = 0; e < 4; e++) {
@@ -625,15 +645,15 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
       };
       bool live = true;
       for (int st = 0; st < nst && live; st++) {
-         const int sa = st & 1, sb = st % NB;
+         const int sa = st & 1, sb = st % NTB;
          const bool got = (st < 2 || bar_wait(&B.empty_a[sa], (unsigned int)((st >> 1) - 1) & 1u)) &&
-                          bar_wait(&B.full_b[sb], (unsigned int)(st / NB) & 1u);
+                          bar_wait(&B.full_t[sb], (unsigned int)(st / NTB) & 1u);
          if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
             if (lane == 0) q_abort(&abort_s, err, Q_ERR);
             live = false;
             break;
          }
-         const T *xs = reinterpret_cast<const T *>(Sbuf + sb * Q_STAGE<NS, ND> + Q_B<ND>);
+         const T *xs = reinterpret_cast<const T *>(Tbuf + sb * Q_TAB<NS>);
          const T *ys = xs + 2 * Q_XMAX * RS;
          unsigned char *A = Abuf + sa * Q_A<NS> + (r >> 3) * 512 + kg * 128 + (r & 7) * 16;
 #pragma unroll
@@ -833,7 +853,7 @@ __device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m,
    }
 }
 
-// Grid: (segments, sets from set0).  The segment's B operand, [stage 4][part][digit]
+// Grid: (segments, sets from set0).  The segment's B operand, [stage 4][digit]
 // [col group][kg 4][8 cols][8 K], and its scale exponent.
 __global__ void __launch_bounds__(256)
 k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict__ units,
@@ -866,7 +886,6 @@ k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *
    if (tid == 0) bexp[set * nseg + seg] = e;
    const double sc = mx > 0.0 ? ldexp(Q_KAPPA * Q_KAPPA, 63 - e) : 0.0;
    unsigned char *base = bq + ((size_t)set * nseg + seg) * 4 * (QCfg<NS>::NTMAX * Q_KS * 2 * NS);
-   const int pc = nT / 2;
    // two quads (8 K values) at one t per thread
    for (int i = tid; i < 16 * tw; i += 256) {
       const int pr = i & 15, tl = i >> 4, t = t0 + tl;
@@ -888,11 +907,11 @@ k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *
       const int stage = pr >> 2, kg = pr & 3, lc = 16 * (tl >> 3) + (tl & 7);
 #pragma unroll
       for (int cs = 0; cs < 2; cs++) {
-         const int col = lc + 8 * cs, part = col / pc, pl = col - part * pc;
+         const int col = lc + 8 * cs;
          unsigned char *d = base + (size_t)stage * (QCfg<NS>::NTMAX * Q_KS * 2 * NS) +
-                            ((size_t)part * NS * pc + (pl & ~7)) * Q_KS * 2 + kg * 128 + (pl & 7) * 16;
-         if (cs == 0) qstore<NS>(d, pc * Q_KS * 2, vc);
-         else qstore<NS>(d, pc * Q_KS * 2, vs);
+                            (size_t)(col & ~7) * Q_KS * 2 + kg * 128 + (col & 7) * 16;
+         if (cs == 0) qstore<NS>(d, nT * Q_KS * 2, vc);
+         else qstore<NS>(d, nT * Q_KS * 2, vs);
       }
    }
 }
@@ -905,7 +924,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
           double *__restrict__ hpart, int *__restrict__ err)
 {
    using namespace tc;
-   constexpr int NS = 7, RS = QCfg<NS>::RS, NB = QCfg<NS>::NB, SEG = QCfg<NS>::SEG;
+   constexpr int NS = 7, RS = QCfg<NS>::RS, NB = Q_FNB, SEG = QCfg<NS>::SEG;
    constexpr int BST = QCfg<NS>::NTMAX * Q_KS * 2 * NS;   // a stage's B operand
    extern __shared__ __align__(1024) unsigned char sm[];
    __shared__ __align__(8) QBars B;
@@ -941,7 +960,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
                break;
             }
             bar_expect_tx(&B.full_b[s], bb);
-            bulk_load(Sbuf + s * Q_STAGE<NS, NS>, src + (size_t)st * BST, bb, &B.full_b[s]);
+            bulk_load(Sbuf + s * Q_B<NS>, src + (size_t)st * BST, bb, &B.full_b[s]);
             issued = st + 1;
          }
          for (int st = issued > NB ? issued - NB : 0; st < issued; st++)
@@ -949,7 +968,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS, NS>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
+         q_issue<NS, NS, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
    } else {
       // ---- A operand: site j of the tile, two quads (8 K) per stage
       const int j = tid & 127, kg = tid >> 7;
@@ -964,7 +983,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
 #pragma unroll
       for (int i = 0; i < MAXC * 4; i++) ai[i] = Q96{0u, 0u, 0u};
       const unsigned int trow = tmem + ((unsigned int)(32 * (w & 3)) << 16);
-      const int cq = w >> 2, ncw = nT >> 2, pc = nT / 2, pl = cq * ncw;
+      const int cq = w >> 2, ncw = nT >> 2, pl = cq * ncw;
       auto flush = [&](int seg) -> bool {
          const bool got = bar_wait(&B.accf, (unsigned int)seg & 1u);
          if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
@@ -976,11 +995,10 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
 #pragma unroll
          for (int ch = 0; ch < MAXC; ch++)
             if (4 * ch < ncw) {
-               const int lc = pl + 4 * ch;
-               const unsigned int col = 256u * (lc / pc) + lc % pc;
+               const unsigned int col = pl + 4 * ch;
                float d[NS][4];
 #pragma unroll
-               for (int k = 0; k < NS; k++) q_ld4(trow + col + k * pc, d[k]);
+               for (int k = 0; k < NS; k++) q_ld4(trow + col + k * nT, d[k]);
                q_ldwait(d);
                if (sh < 96)
 #pragma unroll
@@ -993,17 +1011,21 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
          if (lane == 0) bar_arrive(&B.acce);
          return true;
       };
+      // a stage's table values are fetched a stage ahead, its unit two stages
       long long xv[2], yv[4];
-      auto fetch = [&](int st) {
+      auto unit = [&](int st) {
          const int u = segs[it.seg0 + st / SEG].unit[2 * (st % SEG) + (kg >> 1)];
-         const int4 un = u >= 0 ? units[u] : make_int4(0, 0, 0, 0);
+         return u >= 0 ? *reinterpret_cast<const int2 *>(units + u) : make_int2(0, 0);
+      };
+      auto fetch = [&](int2 un) {
          const long long *x = xb + (size_t)2 * un.x * RS, *y = yb + (size_t)2 * (un.y + 2 * (kg & 1)) * RS;
          xv[0] = __ldg(x);
          xv[1] = __ldg(x + RS);
 #pragma unroll
          for (int k = 0; k < 4; k++) yv[k] = __ldg(y + k * RS);
       };
-      fetch(0);
+      fetch(unit(0));
+      int2 next = unit(min(1, nst - 1));
       bool live = true;
       for (int st = 0; st < nst && live; st++) {
          const int sa = st & 1;
@@ -1015,7 +1037,10 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
             v[4 * x + 2] = qmul(xv[1], yv[2 * x]);
             v[4 * x + 3] = qmul(xv[0], yv[2 * x + 1]);
          }
-         if (st + 1 < nst) fetch(st + 1);
+         if (st + 1 < nst) {
+            fetch(next);
+            next = unit(min(st + 2, nst - 1));
+         }
          const bool got = st < 2 || bar_wait(&B.empty_a[sa], (unsigned int)((st >> 1) - 1) & 1u);
          if (!__all_sync(0xffffffffu, got && !q_aborted(&abort_s))) {
             if (lane == 0) q_abort(&abort_s, err, Q_FERR);
@@ -1157,17 +1182,16 @@ k_qwtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__r
       const int kg = tid & 3, c8 = (tid >> 2) & 7, cg = tid >> 5;
       if (8 * cg < 2 * nt) {
          const int tcol = 2 * t0 + 8 * cg, b = tcol / (2 * g.TW), lc = tcol - 2 * b * g.TW;
-         const int nT = q_blkcols(g, b), pc = nT / QCfg<NS>::NPART;
-         const int part = lc / pc, pl = lc - part * pc;
+         const int nT = q_blkcols(g, b);
          unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * ND + (size_t)2 * b * g.TW * Q_KS * 2 * ND +
-                            ((size_t)part * ND * pc + pl) * Q_KS * 2 + kg * 128 + c8 * 16;
+                            (size_t)lc * Q_KS * 2 + kg * 128 + c8 * 16;
 #pragma unroll
          for (int a = 0; a < 3; a++) {
             auto wz = [&](int e) { return qmul(sw[a][8 * kg + e], sz[8 * cg + c8][8 * kg + e]); };
             decltype(wz(0)) v[8];
 #pragma unroll
             for (int e = 0; e < 8; e++) v[e] = wz(e);
-            qstore<ND>(d + a * zstride, pc * Q_KS * 2, v);
+            qstore<ND>(d + a * zstride, nT * Q_KS * 2, v);
          }
       }
    }
@@ -1291,7 +1315,7 @@ static cudaError_t q_init_device(int device)
    cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 3>);
    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<3, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 4>);
    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_FSMEM);
    if (e == cudaSuccess) e = ks_force_tc_init();
    if (e == cudaSuccess && bit) done.fetch_or(bit);
    return e;
@@ -1460,7 +1484,7 @@ mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
    CK(d.q_bexp.ensure((size_t)3 * nseg));
    CK(d.fpart.ensure((size_t)d.q_nitems * 3 * n));
    k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, 0, d.q_segs.p, nseg, d.q_units.p, d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
-   k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(
+   k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_FSMEM, c->stream>>>(
       q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, n,
       d.fpart.p, &c->out.p->err);
    CK(cudaGetLastError());
@@ -1552,7 +1576,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
       const int nseg = (int)q.segs.size(), T = (N + 127) / 128;
       CK(a.gkpart.ensure((size_t)d.q_nitems * N));
       k_qcoef<<<dim3(nseg, 1), 256, 0, st>>>(g, 3, d.q_segs.p, nseg, d.q_units.p, a.ab64.p, d.q_bq.p, d.q_bexp.p);
-      k_force_q<<<dim3(T, 1, d.q_nitems), Q_THREADS, Q_SMEM<7, 7>, st>>>(
+      k_force_q<<<dim3(T, 1, d.q_nitems), Q_THREADS, Q_FSMEM, st>>>(
          g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, N,
          a.gkpart.p, &c->out.p->err);
       c->launches += 2;
