@@ -712,7 +712,8 @@ k_force64(const int4 *__restrict__ item, const int *__restrict__ item_k0,
 // framework sites are the last ones, site index >= fw0), each channel gets
 // its own structure-factor pass, and the framework sites' forces are
 // corrected by a force pass over them alone with the framework
-// coefficients negated.
+// coefficients negated.  (The adjoint's forward pass, which needs these
+// records; without the adjoint the tensor-core passes serve, see ks_launch.)
 __global__ void k_fw_split(int N, int fw0, const int *__restrict__ sorted, int mixed, int4 *__restrict__ ph32,
                            int4 *__restrict__ phf32, ulonglong2 *__restrict__ ph64b,
                            ulonglong2 *__restrict__ phf64b, int *__restrict__ fslot)
@@ -849,7 +850,8 @@ __global__ void k_fsum_slots(int n, int N, int nsplit, const double *__restrict_
    force[(size_t)comp * N + si] += chg ? chg[si] * s : s;
 }
 
-// Compaction of the link-cell order to the charged sites: per block of
+// Compaction of the link-cell order to the charged sites below fw0 (those of
+// no framework): per block of
 // 1024 slots an exclusive scan of the flags (charge != 0), then each charged
 // slot's site written to its place (every block adds up the totals before it).
 __device__ __forceinline__ int block_scan_1024(int v, int *sh)   // exclusive, blockDim 1024
@@ -876,19 +878,20 @@ __device__ __forceinline__ int block_scan_1024(int v, int *sh)   // exclusive, b
    return x - v + (w > 0 ? sh[w - 1] : 0);
 }
 
-__global__ void __launch_bounds__(1024) k_kflag_scan(int N, const int *__restrict__ sorted,
+__global__ void __launch_bounds__(1024) k_kflag_scan(int N, int fw0, const int *__restrict__ sorted,
                                                      const double *__restrict__ chg, int *__restrict__ ex,
                                                      int *__restrict__ bsum)
 {
    __shared__ int sh[32];
    const int i = blockIdx.x * 1024 + threadIdx.x;
-   const int f = (i < N && chg[sorted[i]] != 0.0) ? 1 : 0;
+   const int si = i < N ? sorted[i] : fw0;
+   const int f = (si < fw0 && chg[si] != 0.0) ? 1 : 0;
    const int e = block_scan_1024(f, sh);
    if (i < N) ex[i] = e;
    if (threadIdx.x == 1023) bsum[blockIdx.x] = e + f;
 }
 
-__global__ void __launch_bounds__(1024) k_kcompact(int N, const int *__restrict__ sorted, const double *__restrict__ chg,
+__global__ void __launch_bounds__(1024) k_kcompact(int N, int fw0, const int *__restrict__ sorted, const double *__restrict__ chg,
                                                    const int *__restrict__ ex, const int *__restrict__ bsum,
                                                    int *__restrict__ slots)
 {
@@ -902,7 +905,7 @@ __global__ void __launch_bounds__(1024) k_kcompact(int N, const int *__restrict_
    const int i = blockIdx.x * 1024 + threadIdx.x;
    if (i >= N) return;
    const int si = sorted[i];
-   if (chg[si] != 0.0) slots[s + ex[i]] = si;
+   if (si < fw0 && chg[si] != 0.0) slots[s + ex[i]] = si;
 }
 
 // -------------------------------------------------------------- host side
@@ -948,14 +951,50 @@ static mdgpu_status ks_upload_list(mdgpu_ctx *c)
    return MDGPU_OK;
 }
 
+// First slot of a framework's charged sites after n others: a tile of 128
+// begins there, never the first one (slot 0 on are the others).
+static int fw_slot0(int n) { return std::max(128, (n + 127) & ~127); }
+
+static void count_charged(mdgpu_ctx *c)
+{
+   if (c->ncharged_gen == c->gen) return;
+   int n = 0, nfw = 0;
+   double qm = 0;
+   for (size_t i = 0; i < c->chg.size(); i++) {
+      const double q = c->chg[i];
+      n += q != 0.0;
+      nfw += q != 0.0 && (int)i >= c->fw_site0;
+      qm = std::max(qm, std::fabs(q));
+   }
+   c->ncharged = n;
+   c->ncharged_fw = nfw;
+   c->n_class0 = 0;
+   for (int id : c->site_id) c->n_class0 += c->cls_of_id[id] == 0;
+   c->qmax = qm;
+   c->ncharged_gen = c->gen;
+}
+
 mdgpu_status ks_prepare(mdgpu_ctx *c)
 {
    KsDev &d = c->kd;
    cudaStream_t st = c->stream;
    const int N = c->nsites;
-   if (c->tc_sfac && N == c->fw_site0) {
+   if (c->tc_sfac) {
       const mdgpu_status s = ks_q_prepare(c, c->prec == MDGPU_MIXED ? 3 : 7);
       if (s) return s;
+   }
+   // a framework's charged sites: their slots never change (the fillers
+   // before them neither)
+   if (c->tc_sfac && c->fw_site0 < N && d.kslots_gen != c->gen) {
+      count_charged(c);
+      const int n = c->ncharged - c->ncharged_fw, f0 = fw_slot0(n);
+      std::vector<int> v((size_t)f0 - n, -1);
+      for (int i = c->fw_site0; i < N; i++)
+         if (c->chg[i] != 0.0) v.push_back(i);
+      CK(d.kslots.ensure((size_t)N + 256));
+      if (!v.empty()) CK(cudaMemcpyAsync(d.kslots.p + n, v.data(), v.size() * sizeof(int), cudaMemcpyHostToDevice, st));
+      CK(cudaStreamSynchronize(st));
+      d.kslots_gen = c->gen;
    }
    if (!d.kcount.p) {   // k_kfinal_part's finished-block counter, zero between evaluations
       CK(d.kcount.ensure(1));
@@ -1013,43 +1052,36 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    // The passes run over the charged sites only (a site without charge adds
    // nothing to S(k) and has no k-space force; rigid water's O sites are a
    // quarter of the work), kept in link-cell order -- except with a
-   // framework molecule and under the adjoint, which need every site.
-   const bool compact = nf <= 0 && !c->ks_all_sites;
-   // both passes on the tensor cores, but with a framework molecule
-   const bool tc = nf <= 0 && c->tc_sfac;
+   // framework molecule on the CUDA-core passes and under the adjoint, which
+   // need every site.  A framework's charged sites follow the others at a
+   // whole 128-site tile: the structure factor sums them apart and the force
+   // pass takes them with the other sites' coefficients (water on a charged
+   // wall, 1044 sites, mixed: an evaluation took 200 us with two CUDA-core
+   // structure-factor passes and a correcting force pass, 146 us so).
+   const bool tc = c->tc_sfac && (nf <= 0 || !c->ks_all_sites);
+   const bool compact = (nf <= 0 || tc) && !c->ks_all_sites;
    int Nk = N;
    const int *slots = c->rd.sorted.p;
-   if (compact || tc) {
-      if (c->ncharged_gen != c->gen) {
-         int n = 0;
-         double qm = 0;
-         for (double q : c->chg) {
-            n += q != 0.0;
-            qm = std::max(qm, std::fabs(q));
-         }
-         c->ncharged = n;
-         c->n_class0 = 0;
-         for (int id : c->site_id) c->n_class0 += c->cls_of_id[id] == 0;
-         c->qmax = qm;
-         c->ncharged_gen = c->gen;
-      }
-   }
+   if (compact || tc) count_charged(c);
+   int f0 = 0, nfc = 0;   // the framework's charged sites: first slot, number
    if (compact) {
-      Nk = c->ncharged;
-      if (Nk == 0) {
+      Nk = c->ncharged - c->ncharged_fw;
+      nfc = c->ncharged_fw;
+      f0 = fw_slot0(Nk);
+      if (c->ncharged == 0) {
          if (join && !c->pairs_after_tables) CK(cudaStreamWaitEvent(st, join, 0));
          if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
          return MDGPU_OK;
       }
       // all sites charged, or all of class 0 and the slots class by class
       // (rigid water): the charged sites come first as they are
-      if (Nk < N && !(c->class_major && c->n_class0 == Nk)) {
+      if (Nk < N && !(nf <= 0 && c->class_major && c->n_class0 == Nk)) {
          const int nb = (N + 1023) / 1024;
-         CK(d.kslots.ensure(N));   // room for every site whatever the device-side count
+         CK(d.kslots.ensure((size_t)N + 256));   // room for every site whatever the device-side count
          CK(d.kscan.ensure(N));
          CK(d.kbsum.ensure(nb));
-         k_kflag_scan<<<nb, 1024, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p);
-         k_kcompact<<<nb, 1024, 0, st>>>(N, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p, d.kslots.p);
+         k_kflag_scan<<<nb, 1024, 0, st>>>(N, fw0, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p);
+         k_kcompact<<<nb, 1024, 0, st>>>(N, fw0, c->rd.sorted.p, c->rd.chg.p, d.kscan.p, d.kbsum.p, d.kslots.p);
          CK(cudaGetLastError());
          c->launches += 2;
          slots = d.kslots.p;
@@ -1059,7 +1091,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    mdgpu_status s;
    if (!tc && (s = ks_upload_list(c)) != MDGPU_OK) return s;
    if (tc) {
-      if ((s = ks_q_tables(c, ns, Nk, slots, d_site)) != MDGPU_OK) return s;
+      if ((s = ks_q_tables(c, ns, nfc ? f0 + nfc : Nk, nf > 0, slots, d_site)) != MDGPU_OK) return s;
       if (cudaStream_t main = c->pairs_after_tables) {
          CK(cudaEventRecord(c->ev_fork, st));
          CK(cudaStreamWaitEvent(main, c->ev_fork, 0));
@@ -1087,7 +1119,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       CK(cudaGetLastError());
    }
    KsShape sh = mixed ? ks_shape(Nk, ni, 1, 2) : ks_shape(Nk, ni, 1, 1);
-   if (nf > 0) {
+   if (nf > 0 && !tc) {
       CK(d.fslot.ensure(nf));
       if (mixed) CK(d.phf32.ensure(N)); else CK(d.phf64b.ensure(N));
       k_fw_split<<<(N + 255) / 256, 256, 0, st>>>(N, fw0, c->rd.sorted.p, mixed ? 1 : 0, d.ph32.p, d.phf32.p,
@@ -1097,7 +1129,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    phase_mark(c, MDGPU_PH_SFAC);
    const dim3 gs((ni + 127) / 128, sh.chunks);
    if (tc) {
-      if ((s = ks_q_sfac(c, ns, Nk, &sh.chunks)) != MDGPU_OK) return s;
+      if ((s = ks_q_sfac(c, ns, Nk, nf > 0, f0, nfc)) != MDGPU_OK) return s;
    } else if (mixed) {
       CK(d.part32.ensure((size_t)sh.chunks * nk));
       k_sfac32<<<gs, 128, 0, st>>>(d.item.p, d.item_k0.p, ni, d.ph32.p, d.zp32.p, Nk, sh.chunk, nk, d.part32.p,
@@ -1123,7 +1155,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    CK(d.blk.ensure((size_t)nbk * 8));
    phase_mark(c, MDGPU_PH_KREDUCE);
    if (tc) {
-      if ((s = ks_q_reduce(c, ns, sh.chunks)) != MDGPU_OK) return s;
+      if ((s = ks_q_reduce(c, ns, nf > 0)) != MDGPU_OK) return s;
    } else if (nf > 0) {
       if (mixed) {
          CK(d.kdatf32.ensure(nk));
@@ -1158,17 +1190,25 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       for (int i = 0; i < d.q_nfblk; i++) np = std::max(np, d.q_fblk[i + 1] - d.q_fblk[i]);
       CK(d.utab.ensure(ks_tc_utab_len(np)));
       CK(d.tc_coef.ensure((size_t)np * 8));
+      if (nfc) CK(d.fpartf.ensure((size_t)sh.splits * 3 * nfc));
    }
    if (!tc || mixed) CK(d.fpart.ensure((size_t)sh.splits * 3 * Nk));
    phase_mark(c, MDGPU_PH_KFORCE);
    dim3 gf((Nk + 255) / 256, sh.splits);
    const int obase = compact ? -1 : 0;   // partial rows by slot of the charged list, or by site
    if (tc && mixed) {
-      const int nl = ks_force_tc(st, Nk, kl.q.g, d, d.q_ab32.p, false, c->nsm, d.fpart.p, &out->err);
+      int nl = 0;
+      for (int f = 0; f < 2 && nl >= 0; f++)
+         if (f ? nfc : Nk) {
+            const int k = ks_force_tc(st, f ? nfc : Nk, f ? f0 : 0, kl.q.g, d, f ? d.q_abf32.p : d.q_ab32.p, false, c->nsm,
+                                      f ? d.fpartf.p : d.fpart.p, &out->err);
+            nl = k < 0 ? -1 : nl + k;
+         }
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl - 1;
    } else if (tc) {
-      if ((s = ks_q_force64(c, Nk, slots)) != MDGPU_OK) return s;
+      if (Nk && (s = ks_q_force64(c, Nk, 0)) != MDGPU_OK) return s;
+      if (nfc && (s = ks_q_force64(c, nfc, f0)) != MDGPU_OK) return s;
    } else if (mixed)
       k_force32<<<gf, FT_THREADS, 0, st>>>(d.item.p, d.item_k0.p, d.item_kxy32.p, ni, nk, sh.per_split,
                                            d.kdat32.p, d.ph32.p, d.zp32.p, c->rd.chg.p, slots, Nk, obase,
@@ -1182,17 +1222,25 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    if (join) CK(cudaStreamWaitEvent(st, join, 0));
    if (compact || tc) {
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
-      if (tc && !mixed) {
-         if ((s = ks_q_fsum64(c, Nk, slots, d_force, c->fin)) != MDGPU_OK) return s;
-      } else
-      k_fsum_slots<<<(3 * Nk + 255) / 256, 256, 0, st>>>(Nk, N, sh.splits, d.fpart.p, slots,
-                                                            tc ? c->rd.chg.p : nullptr, d_force, c->fin, out);
+      for (int f = 0; f < 2; f++) {
+         const int n = f ? nfc : Nk;
+         if (n == 0) continue;
+         FinArgs fin = c->fin;
+         fin.on = fin.on && (f || !nfc);   // by the last of them
+         if (tc && !mixed) {
+            if ((s = ks_q_fsum64(c, n, f ? f0 : 0, slots, d_force, fin)) != MDGPU_OK) return s;
+         } else {
+            k_fsum_slots<<<(3 * n + 255) / 256, 256, 0, st>>>(n, N, sh.splits, f ? d.fpartf.p : d.fpart.p,
+                                                              slots + (f ? f0 : 0), tc ? c->rd.chg.p : nullptr, d_force,
+                                                              fin, out);
+         }
+      }
       c->fin.on = 0;
    } else {
       k_fsum<<<(3 * N + 255) / 256, 256, 0, st>>>(3 * N, sh.splits, d.fpart.p, d_force, accumulate ? 1 : 0);
    }
    CK(cudaGetLastError());
-   if (nf > 0) {
+   if (nf > 0 && !tc) {
       // the framework sites' framework-framework k-space forces, taken off
       const KsShape shf = ks_shape(nf, ni, 1, mixed ? 2 : 1);
       CK(d.sortedc.ensure(nf));

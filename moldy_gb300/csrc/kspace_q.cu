@@ -81,11 +81,11 @@ template <> struct QCfg<7> {
 template <int NS> constexpr int Q_TAB = 2 * (Q_XMAX + Q_YMAX) * QCfg<NS>::RS * (int)sizeof(typename QCfg<NS>::T);
 // (ND: digits of operand B, NS unless weights of a wide range need more)
 template <int ND> constexpr int Q_B = 64 * Q_KS * 2 * ND;
-template <int NS> constexpr int Q_A = QCfg<NS>::MT * NS * Q_OP;
-template <int NS, int ND>
-constexpr int Q_SMEM = 2 * Q_A<NS> + QCfg<NS>::NB * Q_B<ND> + (QCfg<NS>::NB + 1) * Q_TAB<NS>;
+template <int NS, int NA = NS> constexpr int Q_A = QCfg<NS>::MT * NA * Q_OP;
+template <int NS, int ND, int NA = NS>
+constexpr int Q_SMEM = 2 * Q_A<NS, NA> + QCfg<NS>::NB * Q_B<ND> + (QCfg<NS>::NB + 1) * Q_TAB<NS>;
 constexpr int Q_FNB = 3, Q_FSMEM = 2 * Q_A<7> + Q_FNB * Q_B<7>;   // FP64 force pass: no table rows in shared memory
-static_assert(Q_SMEM<3, 4> <= 226 * 1024 && Q_SMEM<7, 7> <= 226 * 1024 && Q_FSMEM <= 220 * 1024, "one CTA's shared memory");
+static_assert(Q_SMEM<3, 4, 4> <= 226 * 1024 && Q_SMEM<7, 7> <= 226 * 1024 && Q_FSMEM <= 220 * 1024, "one CTA's shared memory");
 static_assert(Q_B<3> % 128 == 0 && Q_TAB<3> % 128 == 0 && Q_TAB<7> % 128 == 0, "stage buffers stay aligned");
 
 // ------------------------------------------------------ fixed-point trig
@@ -151,8 +151,8 @@ __device__ __forceinline__ void qsincos(unsigned int p, int &s, int &c)
    b = 0x20783e10u - __umulhi(v, b);
    b = 0x9de9e64eu - __umulhi(v, b);
    unsigned int sn = __umulhi(w, a), cs = (1u << 31) - __umulhi(v, b);
-   sn -= sn >> 8;
-   cs -= cs >> 8;
+   sn -= (sn + 128) >> 8;   // (rounded: truncation biases the energy by 1e-9 of the self-energy)
+   cs -= (cs + 128) >> 8;
    const int S = r < 0 ? -(int)sn : (int)sn, C = (int)cs;
    const bool sw = qd & 1u, ng = qd & 2u;
    s = sw ? C : S;
@@ -273,13 +273,13 @@ __device__ __forceinline__ int q_blkcols(const QGeom &g, int b) { return 2 * min
 // and per form: NS = 3 the force pass's A operand (zsite: three bf16 terms
 // of z per 128-site tile and 64-wide t-block, [term][per 8 t: cosines,
 // sines][row group][8 sites][8 t]); NS = 7 the z values in FP64 (zd).
-template <int NS>
+template <int NS, int ND>
 __global__ void __launch_bounds__(256)
 k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__restrict__ site,
        const double *__restrict__ chg, double hi0, double hi1, double hi2, double hi3, double hi4, double hi5,
        double hi6, double hi7, double hi8, double qinv, typename QCfg<NS>::T *__restrict__ X,
        typename QCfg<NS>::T *__restrict__ Y, unsigned char *__restrict__ ztab, uint4 *__restrict__ zsite,
-       double *__restrict__ zd)
+       double *__restrict__ zd, int *__restrict__ XW)
 {
    typedef typename QCfg<NS>::T T;
    constexpr int RS = QCfg<NS>::RS;
@@ -291,8 +291,8 @@ k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__re
       const int i = stage * 32 + lane;
       unsigned long long ux = 0, uy = 0, uz = 0;
       double q = 0.0;
-      if (i < n) {
-         const int si = slots[i];
+      const int si = i < n ? slots[i] : -1;   // (-1: filler before a framework's sites)
+      if (si >= 0) {
          const double x = site[si], y = site[ns + si], z = site[2 * (size_t)ns + si];
          ux = q_fixed64(hi0 * x + hi1 * y + hi2 * z);
          uy = q_fixed64(hi3 * x + hi4 * y + hi5 * z);
@@ -314,6 +314,11 @@ k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__re
          const int k = y ? r - g.hrows : r;
          T s, c;
          qtrig(k, y ? uy : ux, s, c);
+         if (ND == 4 && !y) {   // and in full for the four-digit structure factor
+            int *d = XW + ((size_t)stage * 2 * g.hrows + 2 * k) * RS + lane;
+            d[0] = c;
+            d[RS] = s;
+         }
          if (NS == 3 && !y) {   // X in units of 2^-24
             c = (c + 64) >> 7;
             s = (s + 64) >> 7;
@@ -350,9 +355,9 @@ k_qtab(int n, int ns, QGeom g, const int *__restrict__ slots, const double *__re
             for (int e = 0; e < 8; e++) v[e] = qz(e);
             const int tcol = 2 * t0 + 8 * cg, b = tcol / (2 * g.TW), lc = tcol - 2 * b * g.TW;
             const int nT = q_blkcols(g, b);
-            unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * NS + (size_t)2 * b * g.TW * Q_KS * 2 * NS +
+            unsigned char *d = ztab + (size_t)stage * 2 * g.TP * Q_KS * 2 * ND + (size_t)2 * b * g.TW * Q_KS * 2 * ND +
                                (size_t)lc * Q_KS * 2 + kg * 128 + c8 * 16;
-            qstore<NS>(d, nT * Q_KS * 2, v);
+            qstore<ND>(d, nT * Q_KS * 2, v);
          }
       }
       if (NS == 3) {
@@ -414,13 +419,13 @@ __device__ __forceinline__ void q_init(QBars &B)
 // ones per K-step, 4 and 7, where halves of the columns took 14 narrow ones).
 // Operand stages: A [tile][digit][row group 16][kg 4][8 rows][16 B], B
 // [digit][col group][kg 4][8][16 B].
-template <int NS, int ND, int NB>
+template <int NS, int ND, int NA, int NB>
 __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned char *Bbuf, unsigned int tmem, int p,
                                         int nst, int nT, int *abort_s, int *err, int errbit)
 {
    using namespace tc;
    constexpr int SEG = QCfg<NS>::SEG;
-   const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NS * Q_OP : 0), b0 = saddr(Bbuf);
+   const unsigned int a0 = saddr(Abuf) + (QCfg<NS>::MT == 2 ? p * NA * Q_OP : 0), b0 = saddr(Bbuf);
    const unsigned int d0 = tmem + (QCfg<NS>::MT == 2 ? 256u * p : 0u);
    const int g0 = NS == 7 && p == 1 ? 4 : 0, g1 = NS == 7 && p == 0 ? 4 : ND;   // this issuer's groups
    for (int st = 0; st < nst; st++) {
@@ -435,10 +440,10 @@ __device__ __forceinline__ void q_issue(QBars &B, unsigned char *Abuf, unsigned 
 #pragma unroll
       for (int ks = 0; ks < 2; ks++)
 #pragma unroll
-         for (int i = 0; i < NS; i++) {
+         for (int i = 0; i < NA; i++) {
             const int ga = max(i, g0);   // first group of digit i of A
             if (ga < g1)
-               mma_f16(d0 + ga * nT, sdesc(a0 + sa * Q_A<NS> + i * Q_OP + ks * 256, 128, 512),
+               mma_f16(d0 + ga * nT, sdesc(a0 + sa * Q_A<NS, NA> + i * Q_OP + ks * 256, 128, 512),
                        sdesc(b0 + sb * Q_B<ND> + (ga - i) * nT * Q_KS * 2 + ks * 256, 128, 512),
                        idesc_f16(128, (g1 - ga) * nT, false), st % SEG != 0 || ks > 0 || i > 0);
          }
@@ -510,12 +515,18 @@ __device__ __forceinline__ double q_value(const Q96 &v)
 }
 
 // ----------------------------------------------------- structure factor
-// Grid: (row tiles, site ranges, channels).  part[channel][range][quad row 4
+// Grid: (row tiles, site ranges, channels).  The first r0 ranges share stages
+// 0 .. n0 - 1, the others those from s1 to nstages - 1 (a framework's).  part[channel][range][quad row 4
 // quad + p][2 TP]; channel c reads its own digits, zstride further on each.
-template <int NS, int ND>
+// NA = 4 (mixed form with a framework molecule): 32-bit operands.  The energy
+// and stress there are differences of the framework's large and the other
+// sites' small sums, and charges of any ratio share the digits' grid: with
+// three digits the stress of a clay (500 sites) was 1.5e-5 off, with FP32
+// sums over the sites 2.1e-6.
+template <int NS, int ND, int NA>
 __global__ void __launch_bounds__(Q_THREADS, 1)
 k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4 *__restrict__ units, const unsigned char *__restrict__ X,
-         const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, size_t zstride, int nstages, int per,
+         const unsigned char *__restrict__ Y, const unsigned char *__restrict__ ztab, size_t zstride, int r0, int n0, int s1, int nstages, int per,
          typename QCfg<NS>::P *__restrict__ part, int *__restrict__ err)
 {
    using namespace tc;
@@ -525,10 +536,12 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
    __shared__ __align__(8) QBars B;
    __shared__ unsigned int tmem_s;
    __shared__ int abort_s;
-   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>, *Tbuf = Sbuf + NB * Q_B<ND>;
+   unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS, NA>, *Tbuf = Sbuf + NB * Q_B<ND>;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
    const QTile &ti = tiles[blockIdx.x];
-   const int nT = ti.nT, st0 = blockIdx.y * per, nst = min(nstages, st0 + per) - st0;
+   const bool fw = (int)blockIdx.y >= r0;
+   const int nT = ti.nT, st0 = fw ? s1 + ((int)blockIdx.y - r0) * per : blockIdx.y * per;
+   const int nst = min(fw ? nstages : n0, st0 + per) - st0;
    if (nst <= 0) return;   // (uniform)
    if (tid == 0) {
       q_init(B);
@@ -579,7 +592,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS, ND, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
+         q_issue<NS, ND, NA, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_ERR);
    } else {
       // ---- A operand: row 8 w + (lane & 7) of each 128-row tile (product
       // p of a quad), sites 8 kg .. 8 kg + 7 of the stage
@@ -655,7 +668,7 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
          }
          const T *xs = reinterpret_cast<const T *>(Tbuf + sb * Q_TAB<NS>);
          const T *ys = xs + 2 * Q_XMAX * RS;
-         unsigned char *A = Abuf + sa * Q_A<NS> + (r >> 3) * 512 + kg * 128 + (r & 7) * 16;
+         unsigned char *A = Abuf + sa * Q_A<NS, NA> + (r >> 3) * 512 + kg * 128 + (r & 7) * 16;
 #pragma unroll
          for (int mt = 0; mt < MT; mt++) {
             constexpr int PV = 16 / (int)sizeof(T);   // values per 16-byte load
@@ -665,10 +678,14 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
                *reinterpret_cast<uint4 *>(xv + e * PV) = *reinterpret_cast<const uint4 *>(xs + xo[mt] + e * PV);
                *reinterpret_cast<uint4 *>(yv + e * PV) = *reinterpret_cast<const uint4 *>(ys + yo[mt] + e * PV);
             }
-            decltype(qmul_a(xv[0], yv[0], 0u)) v[8];
+            auto mul = [&](int e) {
+               if constexpr (NA == 4) return qmul(xv[e], yv[e]);
+               else return qmul_a(xv[e], yv[e], c256);
+            };
+            decltype(mul(0)) v[8];
 #pragma unroll
-            for (int e = 0; e < 8; e++) v[e] = qmul_a(xv[e], yv[e], c256);
-            qstore<NS>(A + mt * NS * Q_OP, Q_OP, v);
+            for (int e = 0; e < 8; e++) v[e] = mul(e);
+            qstore<NA>(A + mt * NA * Q_OP, Q_OP, v);
          }
          fence_async_smem();
          __syncwarp();
@@ -739,13 +756,17 @@ __device__ __forceinline__ double q_rangesum(const double *p, size_t plane, int 
 // (quad, t) and (s, r) forms its k-vector's S(k), energy and stress
 // (src/ewald.c:525-553) and A = coeff Re S, B = coeff Im S, laid out
 // [quad][t][s][r] (zero where there is no such k-vector).
-template <typename R>
+// FW: with a framework molecule, whose sums are in the nrf ranges after the
+// others, framework-framework terms are left out (src/ewald.c:528-579): the
+// energy is 1/2 coeff (Cn (Cn + 2 Cf) + Sn (Sn + 2 Sf)), the framework sites
+// feel the others' sums alone (abf).
+template <typename R, bool FW>
 __global__ void __launch_bounds__(256)
 k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coeff, int nranges, double scale,
-          const R *__restrict__ part, R *__restrict__ ab, double *__restrict__ blk, unsigned int *__restrict__ sync,
-          DevOut *__restrict__ out)
+          const R *__restrict__ part, int nrf, R *__restrict__ ab, R *__restrict__ abf, double *__restrict__ blk,
+          unsigned int *__restrict__ sync, DevOut *__restrict__ out)
 {
-   __shared__ double sq[8][32];
+   __shared__ double sq[FW ? 16 : 8][32];
    __shared__ double sh[4][7], sl[7][8];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    double e[7] = {0, 0, 0, 0, 0, 0, 0};
@@ -755,14 +776,15 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
    const bool live = t < un.z;   // the unit's t range: its columns were computed
    {
       const size_t row = 2 * (size_t)g.TP;
-      sq[w][lane] = live ? scale * q_rangesum(part + ((size_t)quad * 4 + (w >> 1)) * row + 16 * (t >> 3) + 8 * (w & 1) + (t & 7),
-                                              4 * (size_t)g.nquads * row, nranges)
-                         : 0.0;
+      const size_t plane = 4 * (size_t)g.nquads * row;
+      const R *src = part + ((size_t)quad * 4 + (w >> 1)) * row + 16 * (t >> 3) + 8 * (w & 1) + (t & 7);
+      sq[w][lane] = live ? scale * q_rangesum(src, plane, nranges) : 0.0;
+      if (FW) sq[(FW ? 8 : 0) + w][lane] = live ? scale * q_rangesum(src + nranges * plane, plane, nrf) : 0.0;
    }
    __syncthreads();
    // (s, r) = warp w of the first four
    if (w < 4 && quad < g.nquads) {
-      double A = 0.0, Bc = 0.0;
+      double A = 0.0, Bc = 0.0, An = 0.0, Bn = 0.0;
       const double2 cf = live ? coeff[(size_t)i * 4 + w] : make_double2(0.0, 0.0);
       if (cf.x != 0.0) {
          double q[8];
@@ -774,7 +796,14 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
          const double hh = un.x, kk = s * (un.y + (quad & 3)), l = r * t;
          const double kx = hh * g.b[0] + kk * g.b[3], ky = hh * g.b[1] + kk * g.b[4];
          const double kz = hh * g.b[2] + kk * g.b[5] + l * g.b[8];
-         const double pek = 0.5 * cf.x * (C * C + S * S), pc = pek * cf.y;
+         double Cf = 0.0, Sf = 0.0;
+         if (FW) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) q[k] = sq[(FW ? 8 : 0) + k][lane];
+            Cf = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
+            Sf = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
+         }
+         const double pek = 0.5 * cf.x * (FW ? C * (C + Cf + Cf) + S * (S + Sf + Sf) : C * C + S * S), pc = pek * cf.y;
          const double px = pc * kx, py = pc * ky;
          e[0] += pek;
          e[1] += pek - px * kx;
@@ -783,11 +812,17 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
          e[4] += pek - py * ky;
          e[5] -= py * kz;
          e[6] += pek - pc * kz * kz;
-         A = cf.x * C;
-         Bc = cf.x * S;
+         An = cf.x * C;
+         Bn = cf.x * S;
+         A = FW ? cf.x * (C + Cf) : An;
+         Bc = FW ? cf.x * (S + Sf) : Bn;
       }
       ab[(size_t)i * 8 + 2 * w] = (R)A;
       ab[(size_t)i * 8 + 2 * w + 1] = (R)Bc;
+      if (FW) {
+         abf[(size_t)i * 8 + 2 * w] = (R)An;
+         abf[(size_t)i * 8 + 2 * w + 1] = (R)Bn;
+      }
    }
    __syncthreads();
    }
@@ -968,7 +1003,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
       }
    } else if (w > Q_BW) {
       if (lane == 0)
-         q_issue<NS, NS, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
+         q_issue<NS, NS, NS, NB>(B, Abuf, Sbuf, tmem, w - Q_BW - 1, nst, nT, &abort_s, err, Q_FERR);
    } else {
       // ---- A operand: site j of the tile, two quads (8 K) per stage
       const int j = tid & 127, kg = tid >> 7;
@@ -1312,9 +1347,10 @@ static cudaError_t q_init_device(int device)
    static std::atomic<unsigned long long> done{0};
    const unsigned long long bit = device >= 0 && device < 64 ? 1ull << device : 0ull;
    if (bit && (done.load() & bit)) return cudaSuccess;
-   cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 3>);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<3, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 4>);
-   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
+   cudaError_t e = cudaFuncSetAttribute(k_sfac_q<3, 3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 3>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<3, 4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 4, 4>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<3, 4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<3, 4>);
+   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_sfac_q<7, 7, 7>, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_SMEM<7, 7>);
    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_force_q, cudaFuncAttributeMaxDynamicSharedMemorySize, Q_FSMEM);
    if (e == cudaSuccess) e = ks_force_tc_init();
    if (e == cudaSuccess && bit) done.fetch_or(bit);
@@ -1352,105 +1388,135 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    return MDGPU_OK;
 }
 
-// The scale of the charges: a power of two above the largest.
-static int q_charge_exp(const mdgpu_ctx *c)
+// The scale of the charges: FP64, a power of two above the largest; mixed,
+// the largest itself (its 31-bit fixed point then holds charges in simple
+// ratios, rigid water's 1 : -2, exactly: their rounding is the same at every
+// site of a kind and does not average out).
+static double q_charge_scale(const mdgpu_ctx *c, int ns)
 {
    int e = 0;
-   std::frexp(c->qmax > 0 ? c->qmax : 1.0, &e);
-   return e;
+   const double q = c->qmax > 0 ? c->qmax : 1.0;
+   std::frexp(q, &e);
+   return ns == 3 ? q : std::ldexp(1.0, e);
 }
 
-mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site)
+// (fw: the mixed form's structure factor in four digits)
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool fw, const int *slots, const double *d_site)
 {
    KsDev &d = c->kd;
    const QGeom &g = c->kl.q.g;
    const size_t S = q_stages(n);
    const double *hi = c->kl.hinv;
-   const double qinv = std::ldexp(1.0, -q_charge_exp(c));
-   CK(d.q_ztab.ensure(S * 2 * g.TP * Q_KS * 2 * ns));
+   const double qinv = 1.0 / q_charge_scale(c, ns);
+   CK(d.q_ztab.ensure(S * 2 * g.TP * Q_KS * 2 * (ns == 3 && fw ? 4 : ns)));
    if (ns == 3) {
       CK(d.q_x32.ensure(S * 2 * g.hrows * QCfg<3>::RS));
       CK(d.q_y32.ensure(S * 2 * g.mrows * QCfg<3>::RS));
       CK(d.zsite.ensure(S / 4 * 2 * g.TP * 48));
-      k_qtab<3><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
-                                                        hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x32.p,
-                                                        d.q_y32.p, d.q_ztab.p, d.zsite.p, nullptr);
+      if (fw) {
+         CK(d.q_xw32.ensure(S * 2 * g.hrows * QCfg<3>::RS));
+         k_qtab<3, 4><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
+                                                           hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x32.p,
+                                                           d.q_y32.p, d.q_ztab.p, d.zsite.p, nullptr, d.q_xw32.p);
+      } else {
+         k_qtab<3, 3><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
+                                                           hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x32.p,
+                                                           d.q_y32.p, d.q_ztab.p, d.zsite.p, nullptr, nullptr);
+      }
    } else {
       CK(d.q_x64.ensure(S * 2 * g.hrows * QCfg<7>::RS));
       CK(d.q_y64.ensure(S * 2 * g.mrows * QCfg<7>::RS));
       CK(d.q_zd.ensure(S * 2 * g.TP * 32));
-      k_qtab<7><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
+      k_qtab<7, 7><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
                                                         hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x64.p,
-                                                        d.q_y64.p, d.q_ztab.p, nullptr, d.q_zd.p);
+                                                        d.q_y64.p, d.q_ztab.p, nullptr, d.q_zd.p, nullptr);
    }
    CK(cudaGetLastError());
    return MDGPU_OK;
 }
 
 // Site ranges: the count for which the waves of (tile, range) CTAs, each its
-// stages plus a start-up of about six, come out shortest.
-mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges)
+// stages plus a start-up of about six, come out shortest.  A framework's
+// sites (slots f0 on) have ranges of their own.
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool fw, int f0, int nf)
 {
    KsDev &d = c->kd;
    const QList &q = c->kl.q;
-   const int nst = (n + 31) / 32, nt = (int)q.tiles.size();
+   const int n0 = (n + 31) / 32, s1 = f0 / 32, nstf = (nf + 31) / 32, nst = n0 + nstf, nt = (int)q.tiles.size();
    const size_t plane = 4 * (size_t)q.g.nquads * 2 * q.g.TP, psz = ns == 3 ? sizeof(float) : sizeof(double);
    long long best = -1;
-   int R = 1;
+   int per = nst;
    for (int r = 1; r <= 64 && r <= nst; r++) {
-      if (r > 1 && r * plane * psz > (256u << 20)) break;
-      const long long cost = (long long)((nt * r + c->nsm - 1) / c->nsm) * ((nst + r - 1) / r + 6);
+      if (r > 1 && (r + 1) * plane * psz > (256u << 20)) break;
+      const int p = (nst + r - 1) / r, nr = (n0 + p - 1) / p + (nstf + p - 1) / p;
+      const long long cost = (long long)((nt * nr + c->nsm - 1) / c->nsm) * (p + 6);
       if (best < 0 || cost < best) {
          best = cost;
-         R = r;
+         per = p;
       }
    }
-   const int per = (nst + R - 1) / R;
-   R = (nst + per - 1) / per;
+   const int R0 = (n0 + per - 1) / per, R = R0 + (nstf + per - 1) / per;
    CK(d.q_part.ensure(R * plane * psz));
    const dim3 grid(nt, R);
-   if (ns == 3)
-      k_sfac_q<3, 3><<<grid, Q_THREADS, Q_SMEM<3, 3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, nst, per, (float *)d.q_part.p, &c->out.p->err);
+   if (ns == 3 && fw)
+      k_sfac_q<3, 4, 4><<<grid, Q_THREADS, Q_SMEM<3, 4, 4>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_xw32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, R0, n0, s1, s1 + nstf, per,
+         (float *)d.q_part.p, &c->out.p->err);
+   else if (ns == 3)
+      k_sfac_q<3, 3, 3><<<grid, Q_THREADS, Q_SMEM<3, 3>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, R0, n0, s1, s1 + nstf, per,
+         (float *)d.q_part.p, &c->out.p->err);
    else
-      k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
-         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, 0, nst, per, (double *)d.q_part.p, &c->out.p->err);
+      k_sfac_q<7, 7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
+         (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, d.q_ztab.p, 0, R0, n0, s1, s1 + nstf, per,
+         (double *)d.q_part.p, &c->out.p->err);
    CK(cudaGetLastError());
-   d.q_nranges = R;
-   *nranges = R;
+   d.q_nranges = R0;
+   d.q_nrangesf = R - R0;
    return MDGPU_OK;
 }
 
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges)
+template <typename R, bool FW>
+static void q_reduce(mdgpu_ctx *c, int nb, double scale, DBuf<R> &ab, DBuf<R> &abf)
+{
+   KsDev &d = c->kd;
+   k_qreduce<R, FW><<<nb, 256, 0, c->stream>>>(c->kl.q.g, d.q_units.p, d.q_coeff.p, d.q_nranges, scale,
+                                               (const R *)d.q_part.p, d.q_nrangesf, ab.p, abf.p, d.blk.p,
+                                               c->rd.sync.p, c->out.p);
+}
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw)
 {
    KsDev &d = c->kd;
    const QGeom &g = c->kl.q.g;
    const size_t nqt = (size_t)g.nquads * g.TP;
    const int nb = (int)std::min<size_t>((nqt + 31) / 32, 4 * (size_t)c->nsm);
    const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
+   const double scale = q_charge_scale(c, ns) * std::ldexp(1.0 / k4, ns == 7 ? -62 : fw ? -38 : -30);
    CK(d.blk.ensure((size_t)nb * 8));
    if (ns == 3) {
       CK(d.q_ab32.ensure(nqt * 8));
-      k_qreduce<float><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
-         std::ldexp(1.0 / k4, q_charge_exp(c) - 30), (const float *)d.q_part.p, d.q_ab32.p, d.blk.p, c->rd.sync.p, c->out.p);
+      if (fw) CK(d.q_abf32.ensure(nqt * 8));
+      if (fw) q_reduce<float, true>(c, nb, scale, d.q_ab32, d.q_abf32);
+      else q_reduce<float, false>(c, nb, scale, d.q_ab32, d.q_abf32);
    } else {
       CK(d.q_ab64.ensure(nqt * 8));
-      k_qreduce<double><<<nb, 256, 0, c->stream>>>(g, d.q_units.p, d.q_coeff.p, nranges,
-         std::ldexp(1.0 / k4, q_charge_exp(c) - 62), (const double *)d.q_part.p, d.q_ab64.p, d.blk.p, c->rd.sync.p, c->out.p);
+      if (fw) CK(d.q_abf64.ensure(nqt * 8));
+      if (fw) q_reduce<double, true>(c, nb, scale, d.q_ab64, d.q_abf64);
+      else q_reduce<double, false>(c, nb, scale, d.q_ab64, d.q_abf64);
    }
    CK(cudaGetLastError());
    return MDGPU_OK;
 }
 
-mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
+// (a framework's sites take the runs chosen for the others')
+mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0)
 {
-   (void)slots;
    KsDev &d = c->kd;
    const QList &q = c->kl.q;
    const int nseg = (int)q.segs.size(), T = (n + 127) / 128;
    // runs of segments: the length for which the waves of (site tile, set,
    // run) CTAs come out shortest
-   if (d.q_items_for[0] != T || d.q_items_for[1] != (int)d.tc_ver || d.q_items_for[2] != c->nsm) {
+   if ((d.q_items_for[0] != T && f0 == 0) || d.q_items_for[1] != (int)d.tc_ver || d.q_items_for[2] != c->nsm) {
       int per = 1;
       long long best = -1;
       int mx = 1;
@@ -1482,19 +1548,23 @@ mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots)
    }
    CK(d.q_bq.ensure((size_t)3 * nseg * 4 * QCfg<7>::NTMAX * Q_KS * 2 * 7));
    CK(d.q_bexp.ensure((size_t)3 * nseg));
-   CK(d.fpart.ensure((size_t)d.q_nitems * 3 * n));
-   k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, 0, d.q_segs.p, nseg, d.q_units.p, d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
+   DBuf<double> &hpart = f0 > 0 ? d.fpartf : d.fpart;
+   CK(hpart.ensure((size_t)d.q_nitems * 3 * n));
+   k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, 0, d.q_segs.p, nseg, d.q_units.p,
+                                                 f0 > 0 ? d.q_abf64.p : d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
    k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_FSMEM, c->stream>>>(
-      q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, n,
-      d.fpart.p, &c->out.p->err);
+      q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p + (size_t)f0 / 32 * 2 * q.g.hrows * QCfg<7>::RS,
+      d.q_y64.p + (size_t)f0 / 32 * 2 * q.g.mrows * QCfg<7>::RS, d.q_zd.p + (size_t)f0 / 32 * 2 * q.g.TP * 32, d.q_bq.p,
+      d.q_bexp.p, n, hpart.p, &c->out.p->err);
    CK(cudaGetLastError());
    c->launches += 1;
    return MDGPU_OK;
 }
 
-mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force, const FinArgs &fin)
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, int f0, const int *slots, double *d_force, const FinArgs &fin)
 {
-   k_fsum_q<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->nsites, c->kd.q_nitems, c->kl.q.g, c->kd.fpart.p, slots,
+   const double *hpart = f0 > 0 ? c->kd.fpartf.p : c->kd.fpart.p;
+   k_fsum_q<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->nsites, c->kd.q_nitems, c->kl.q.g, hpart, slots + f0,
                                                     c->rd.chg.p, d_force, fin, c->out.p);
    CK(cudaGetLastError());
    return MDGPU_OK;
@@ -1540,15 +1610,15 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
          k_qwmax<float4><<<nb, 256, 0, st>>>(N, slots, c->rd.chg.p, a.res32.p, a.wmax.p);
          k_qwtab<3, 4, float4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
                                                     a.res32.p, a.wmax.p, a.zw.p, zstride);
-         k_sfac_q<3, 4><<<grid, Q_THREADS, Q_SMEM<3, 4>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
-            (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, a.zw.p, zstride, nst, per,
+         k_sfac_q<3, 4, 3><<<grid, Q_THREADS, Q_SMEM<3, 4>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
+            (const unsigned char *)d.q_x32.p, (const unsigned char *)d.q_y32.p, a.zw.p, zstride, R, nst, 0, nst, per,
             (float *)a.partv.p, &c->out.p->err);
       } else {
          k_qwmax<double4><<<nb, 256, 0, st>>>(N, slots, c->rd.chg.p, a.res64.p, a.wmax.p);
          k_qwtab<7, 7, double4><<<nst, 256, 0, st>>>(N, N, g, slots, c->cur_site, c->rd.chg.p, hi[6], hi[7], hi[8],
                                                      a.res64.p, a.wmax.p, a.zw.p, zstride);
-         k_sfac_q<7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
-            (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, a.zw.p, zstride, nst, per,
+         k_sfac_q<7, 7, 7><<<grid, Q_THREADS, Q_SMEM<7, 7>, st>>>(g, 256u, d.q_tiles.p, d.q_units.p,
+            (const unsigned char *)d.q_x64.p, (const unsigned char *)d.q_y64.p, a.zw.p, zstride, R, nst, 0, nst, per,
             (double *)a.partv.p, &c->out.p->err);
       }
       CK(cudaGetLastError());
@@ -1557,14 +1627,14 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    const int nb = (int)((nqt + 31) / 32);
    *nblocks = nb;
    CK(a.blk.ensure(2 * (size_t)nb));
-   const int e0 = q_charge_exp(c);
+   const double qs = q_charge_scale(c, ns);
    if (ns == 3) {
       CK(a.ab32.ensure(nqt * 8));
       k_qadj<float><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
-         std::ldexp(1.0 / k4, e0 - 30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
+         qs * std::ldexp(1.0 / k4, -30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
       const int sp = ks_force_tc_splits(d);
       CK(a.gkpart.ensure((size_t)sp * 3 * N));
-      const int nl = ks_force_tc(st, N, g, d, a.ab32.p, true, c->nsm, a.gkpart.p, &c->out.p->err);
+      const int nl = ks_force_tc(st, N, 0, g, d, a.ab32.p, true, c->nsm, a.gkpart.p, &c->out.p->err);
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl;
       k_qadj_site<true, float4><<<(N + 255) / 256, 256, 0, st>>>(N, sp, g, d.fpart.p, a.gkpart.p, a.res32.p,
@@ -1572,7 +1642,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    } else {
       CK(a.ab64.ensure(nqt * 8));
       k_qadj<double><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
-         std::ldexp(1.0 / k4, e0 - 62), (const double *)d.q_part.p, R, std::ldexp(1.0 / k4, -62), a.wmax.p, (const double *)a.partv.p, a.ab64.p, a.blk.p);
+         qs * std::ldexp(1.0 / k4, -62), (const double *)d.q_part.p, R, std::ldexp(1.0 / k4, -62), a.wmax.p, (const double *)a.partv.p, a.ab64.p, a.blk.p);
       const int nseg = (int)q.segs.size(), T = (N + 127) / 128;
       CK(a.gkpart.ensure((size_t)d.q_nitems * N));
       k_qcoef<<<dim3(nseg, 1), 256, 0, st>>>(g, 3, d.q_segs.p, nseg, d.q_units.p, a.ab64.p, d.q_bq.p, d.q_bexp.p);

@@ -499,38 +499,41 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    }
 }
 
-// The force pass of one t-block (its units fu0 .. fu0 + npos - 1 of the
+// The force pass of one t-block, sites from slot f0 on (its units fu0 .. fu0 + npos - 1 of the
 // list, a multiple of four) into slots 0 and 1 of fpart; returns the
 // launches, -1 if out of memory.
-static int force_tc_block(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int blk,
+static int force_tc_block(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int blk,
                           int fu0, int npos, int nsm, double *fpart, int *err)
 {
    const int T = (nsites + 127) / 128, ntl = npos * 8 / FTC_NI, t0 = 64 * blk;
    const int G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
    const int4 *fu = d.q_fu.p + fu0;
+   const int f = f0 > 0;
    k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, scalar ? 1 : 0, fu, reinterpret_cast<const float4 *>(ab), d.utab.p,
                                    reinterpret_cast<float *>(d.tc_coef.p));
    int launches = 2;
-   if (blk > 0 || d.tc_rkey[0] != T || d.tc_rkey[1] != ntl || d.tc_rkey[2] != G || d.tc_rver != d.tc_ver) {
-      if (d.tc_ustart.ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
-      k_ftc_ranges<<<1, 256, 0, st>>>(fu, t0, ntl, T, G, d.tc_ustart.p);
-      d.tc_rkey[0] = T;
-      d.tc_rkey[1] = ntl;
-      d.tc_rkey[2] = G;
-      d.tc_rver = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
+   if (blk > 0 || d.tc_rkey[f][0] != T || d.tc_rkey[f][1] != ntl || d.tc_rkey[f][2] != G || d.tc_rver[f] != d.tc_ver) {
+      if (d.tc_ustart[f].ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
+      k_ftc_ranges<<<1, 256, 0, st>>>(fu, t0, ntl, T, G, d.tc_ustart[f].p);
+      d.tc_rkey[f][0] = T;
+      d.tc_rkey[f][1] = ntl;
+      d.tc_rkey[f][2] = G;
+      d.tc_rver[f] = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
       launches++;
    }
-   k_force_tc<<<G, FTC_THREADS, ftc_smem(256 * std::min(128, 2 * (g.TP - t0))), st>>>(g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p, d.q_y32.p, d.zsite.p,
-                                                d.utab.p, nsites, d.tc_ustart.p, fpart, err);
+   k_force_tc<<<G, FTC_THREADS, ftc_smem(256 * std::min(128, 2 * (g.TP - t0))), st>>>(g, fu, d.tc_coef.p, npos * 8, t0,
+                                                d.q_x32.p + (size_t)f0 / 32 * 2 * g.hrows * 36, d.q_y32.p + (size_t)f0 / 32 * 2 * g.mrows * 36,
+                                                d.zsite.p + (size_t)f0 / 128 * 2 * g.TP * 48,
+                                                d.utab.p, nsites, d.tc_ustart[f].p, fpart, err);
    return launches;
 }
 
-int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
+int ks_force_tc(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
                 double *fpart, int *err)
 {
    int launches = 0;
    for (int b = 0; b < d.q_nfblk; b++) {
-      const int nl = force_tc_block(st, nsites, g, d, ab, scalar, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm,
+      const int nl = force_tc_block(st, nsites, f0, g, d, ab, scalar, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm,
                                     fpart + (size_t)b * FTC_SPLITS * 3 * nsites, err);
       if (nl < 0) return -1;
       launches += nl;

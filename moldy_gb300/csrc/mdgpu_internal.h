@@ -273,14 +273,18 @@ struct KsDev {
    std::vector<int> q_fblk;
    int q_items_for[3] = {-1, -1, -1};   // (site tiles, list upload, SMs) of q_items
    int q_nitems = 0;
-   int q_nranges = 0;               // site ranges of q_part
+   int q_nranges = 0, q_nrangesf = 0;   // site ranges of q_part, the framework's after them
+   DBuf<double> q_abf64;   // the framework sites' coefficients (whole S(k) without the framework's)
+   DBuf<float> q_abf32;
+   DBuf<int> q_xw32;       // X in full width (mixed form, framework)
+   uint64_t kslots_gen = 0;   // configuration the framework part of kslots is for
    DBuf<uint4> zsite;      // force pass: z tables as the A operand, per 128 sites
    DBuf<uint4> utab;       // force pass: per-item coefficient rows (B operand)
    DBuf<float4> tc_coef;   // per item: kx s1, ky s1, kz0 s1, dkz s2 (row scales s)
-   DBuf<int> tc_ustart;    // force pass: the CTAs' work ranges (k_ftc_ranges)
+   DBuf<int> tc_ustart[2]; // force pass: the CTAs' work ranges (k_ftc_ranges), of the framework's sites
    long long tc_ver = 0;   // uploads of the quad list so far
-   int tc_rkey[3] = {-1, -1, -1};   // (site tiles, item tiles, CTAs) of tc_ustart
-   long long tc_rver = -1;          // tc_ver of tc_ustart
+   int tc_rkey[2][3] = {{-1, -1, -1}, {-1, -1, -1}};   // (site tiles, item tiles, CTAs) of tc_ustart
+   long long tc_rver[2] = {-1, -1};                    // tc_ver of tc_ustart
 };
 
 // Buffers of the adjoint (parameter-gradient) passes.
@@ -432,6 +436,7 @@ struct mdgpu_ctx {
    bool tc_sfac = true;
    uint64_t ncharged_gen = 0;       // configuration the count below is for
    int ncharged = 0;                // sites with a nonzero charge
+   int ncharged_fw = 0;             // of them, of the framework molecule
    int n_class0 = 0;                // sites of interaction class 0
    double qmax = 0;                 // and their largest |q|
    cudaEvent_t ev[MDGPU_NPHASES + 1] = {};
@@ -497,12 +502,14 @@ KsShape ks_shape(int N, int nitems, int ipt, int spt);
 // fpart[split][3][nsites], or with scalar the sum over k of A sin - B cos
 // into its first component (returns the launches, -1 if out of memory).
 mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns);
-mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, const int *slots, const double *d_site);
-mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, int *nranges);
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, int nranges);
-mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, const int *slots);
-mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, const int *slots, double *d_force, const FinArgs &fin);
-int ks_force_tc(cudaStream_t st, int nsites, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool fw, const int *slots, const double *d_site);
+// n sites and, from slot f0 (a multiple of 128) on, nf of a framework molecule
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool fw, int f0, int nf);
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw);
+// sites from slot f0 (zero or the framework's first) on
+mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0);
+mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, int f0, const int *slots, double *d_force, const FinArgs &fin);
+int ks_force_tc(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
                 double *fpart, int *err);
 mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq, int *nblocks);
 int ks_force_tc_splits(const KsDev &d);

@@ -91,3 +91,35 @@ def test_adjoint_matches_cuda_core_passes(case, loss, monkeypatch):
         assert np.abs(g["chg"] - g0["chg"]).max() <= tol * np.abs(g0["chg"]).max(), form
         if form == "fp64":
             assert abs(g["alpha"] - g0["alpha"]) <= tol * (abs(g0["alpha"]) + np.abs(g0["chg"]).max())
+
+
+@pytest.mark.parametrize("nside,nwall,wall_charge,water_charge", [
+    (6, 7, 0.4, True), (7, 8, 0.4, True), (8, 12, 0.3, True), (6, 5, 0.0, True), (6, 7, 0.4, False)])
+def test_framework_matches_cuda_core_passes(nside, nwall, wall_charge, water_charge, monkeypatch):
+    """A framework molecule: its charged sites in tiles of their own, fewer
+    and more than one, none, and nothing else charged."""
+    import dataclasses
+
+    from moldy_gb300 import ForceField
+    from moldy_gb300 import system as S
+    sysm = S.water_on_framework(nside=nside, nlayers=nside - 2, nwall=nwall, seed=3, wall_charge=wall_charge)
+    if not water_charge:
+        q = np.array(sysm.site_charge)
+        q[1:4] = 0.0
+        sysm = dataclasses.replace(sysm, site_charge=q)
+    res = {}
+    for form in ("fp64", "mixed"):
+        for tc in ("1", "0"):
+            monkeypatch.setenv("MDGPU_KSPACE_TC", tc)
+            ff = ForceField(sysm, precision=form)
+            res[form, tc] = ff.ewald() + (ff.forces(),)
+            self_e = abs(ff.info()["self_energy"])
+            ff.close()
+    f0, e0, s0, t0 = res["fp64", "0"]
+    scale = max(np.sqrt((f0 ** 2).mean()), 1e-3 * self_e / sysm.nsites)
+    for form, tol in (("fp64", 1e-12), ("mixed", 1e-5)):
+        f, e, s, t = res[form, "1"]
+        assert np.sqrt(((f - f0) ** 2).mean()) <= tol * scale, form
+        assert abs(e - e0) <= tol * (abs(e0) + self_e), form
+        assert np.abs(s - s0).max() <= tol * (np.abs(s0).max() + self_e), form
+        assert np.abs(t[1] - t0[1]).max() <= tol * (np.abs(t0[1]).max() + self_e), form
