@@ -731,27 +731,49 @@ k_sfac_q(QGeom g, unsigned int c256, const QTile *__restrict__ tiles, const int4
 // ------------------------------------------------- per-k energy and stress
 // Sum of nr values a plane apart: FP32 partials compensated (an FP64 add or
 // conversion per partial would bound the per-k pass), FP64 ones plainly.
+// Sixteen loads in flight: the latency of the loads is what a small system's
+// sum takes (48 ranges at 2048 sites).
+template <typename R, typename F> __device__ __forceinline__ void q_ranges(const R *p, size_t plane, int nr, F &&add)
+{
+   int k = 0;
+   for (; k + 16 <= nr; k += 16) {
+      R v[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) v[j] = __ldg(p + (k + j) * plane);
+#pragma unroll
+      for (int j = 0; j < 16; j++) add(v[j]);
+   }
+   R v[15];
+#pragma unroll
+   for (int j = 0; j < 15; j++) v[j] = k + j < nr ? __ldg(p + (k + j) * plane) : R(0);
+#pragma unroll
+   for (int j = 0; j < 15; j++)
+      if (k + j < nr) add(v[j]);
+}
 __device__ __forceinline__ double q_rangesum(const float *p, size_t plane, int nr)
 {
    float s = 0.f, c = 0.f;
-#pragma unroll 4
-   for (int k = 0; k < nr; k++) {
-      const float y = __ldg(p + k * plane) - c, t = s + y;
+   q_ranges(p, plane, nr, [&](float v) {
+      const float y = v - c, t = s + y;
       c = (t - s) - y;
       s = t;
-   }
+   });
    return (double)s - (double)c;
 }
 __device__ __forceinline__ double q_rangesum(const double *p, size_t plane, int nr)
 {
    double s = 0.0;
-#pragma unroll 4
-   for (int k = 0; k < nr; k++) s += __ldg(p + k * plane);
+   q_ranges(p, plane, nr, [&](double v) { s += v; });
    return s;
 }
 
-// A block takes 32 consecutive (quad, t) at a time (the energy and stress of
-// all its groups in one reduction: FP64 instructions bound this kernel): warp
+// Energy and stress come from seven sums over the k-vectors, of the energy e
+// and of e c2 times the products of the integers (h, k, l) (the last block
+// brings those to Cartesian axes): FP64 instructions, 16 cycles each for a
+// warp, and their latency bound this kernel.
+// A block takes 32 consecutive (quad, t) at a time (all its groups in one
+// reduction, a warp per sum; 2048-site water 23 us with shuffles of seven
+// sums in four warps and four loads in flight, 10.7 us so): warp
 // k adds up sum k of each over the site ranges, then one thread per
 // (quad, t) and (s, r) forms its k-vector's S(k), energy and stress
 // (src/ewald.c:525-553) and A = coeff Re S, B = coeff Im S, laid out
@@ -767,7 +789,7 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
           unsigned int *__restrict__ sync, DevOut *__restrict__ out)
 {
    __shared__ double sq[FW ? 16 : 8][32];
-   __shared__ double sh[4][7], sl[7][8];
+   __shared__ double se[7][128], sl[8];
    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
    double e[7] = {0, 0, 0, 0, 0, 0, 0};
    for (int grp = blockIdx.x; grp * 32 < g.nquads * g.TP; grp += gridDim.x) {
@@ -794,8 +816,6 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
          const double C = (q[0] - s * q[2]) - r * (q[5] + s * q[7]);
          const double S = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
          const double hh = un.x, kk = s * (un.y + (quad & 3)), l = r * t;
-         const double kx = hh * g.b[0] + kk * g.b[3], ky = hh * g.b[1] + kk * g.b[4];
-         const double kz = hh * g.b[2] + kk * g.b[5] + l * g.b[8];
          double Cf = 0.0, Sf = 0.0;
          if (FW) {
 #pragma unroll
@@ -804,14 +824,14 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
             Sf = (q[4] + s * q[6]) + r * (q[1] - s * q[3]);
          }
          const double pek = 0.5 * cf.x * (FW ? C * (C + Cf + Cf) + S * (S + Sf + Sf) : C * C + S * S), pc = pek * cf.y;
-         const double px = pc * kx, py = pc * ky;
+         const double ph = pc * hh, pk = pc * kk, pl = pc * l;
          e[0] += pek;
-         e[1] += pek - px * kx;
-         e[2] -= px * ky;
-         e[3] -= px * kz;
-         e[4] += pek - py * ky;
-         e[5] -= py * kz;
-         e[6] += pek - pc * kz * kz;
+         e[1] = fma(ph, hh, e[1]);
+         e[2] = fma(ph, kk, e[2]);
+         e[3] = fma(ph, l, e[3]);
+         e[4] = fma(pk, kk, e[4]);
+         e[5] = fma(pk, l, e[5]);
+         e[6] = fma(pl, l, e[6]);
          An = cf.x * C;
          Bn = cf.x * S;
          A = FW ? cf.x * (C + Cf) : An;
@@ -828,32 +848,36 @@ k_qreduce(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ c
    }
    if (w < 4)
 #pragma unroll
-      for (int k = 0; k < 7; k++) {
-#pragma unroll
-         for (int o = 16; o > 0; o >>= 1) e[k] += __shfl_down_sync(0xffffffffu, e[k], o);
-         if (lane == 0) sh[w][k] = e[k];
-      }
+      for (int k = 0; k < 7; k++) se[k][threadIdx.x] = e[k];
    __syncthreads();
-   if (threadIdx.x < 7)
-      blk[blockIdx.x * 8 + threadIdx.x] = (sh[0][threadIdx.x] + sh[1][threadIdx.x]) + (sh[2][threadIdx.x] + sh[3][threadIdx.x]);
-   // energy and stress by the last block: blocks t, t + 256, ... per thread, then trees
+   if (w < 7) {
+      double v = (se[w][lane] + se[w][lane + 32]) + (se[w][lane + 64] + se[w][lane + 96]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) blk[blockIdx.x * 8 + w] = v;
+   }
+   // the blocks' sums by the last block, a warp per sum
    if (!last_block(&sync[SYNC_KRED])) return;
-   double v[7] = {0, 0, 0, 0, 0, 0, 0};
-   for (int b = threadIdx.x; b < (int)gridDim.x; b += 256)
+   if (w < 7) {
+      double v = 0.0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) v += __ldcg(&blk[b * 8 + w]);
 #pragma unroll
-      for (int k = 0; k < 7; k++) v[k] += __ldcg(&blk[b * 8 + k]);
-#pragma unroll
-   for (int k = 0; k < 7; k++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-      if (lane == 0) sl[k][w] = v[k];
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) sl[w] = v;
    }
    __syncthreads();
    if (threadIdx.x < 7) {
-      double s = 0.0;
-      for (int j = 0; j < 8; j++) s += sl[threadIdx.x][j];
-      if (threadIdx.x == 0) out->pe_k = s;
-      else out->st_k[threadIdx.x - 1] = s;
+      // stress (x, y) = delta e - sum over axes of b[axis][x] b[axis'][y] times the products' sums
+      const int k = threadIdx.x, x = k < 4 ? 0 : k < 6 ? 1 : 2, y = k < 4 ? k - 1 : k < 6 ? k - 3 : 2;
+      if (k == 0) {
+         out->pe_k = sl[0];
+      } else {
+         const double m[9] = {sl[1], sl[2], sl[3], sl[2], sl[4], sl[5], sl[3], sl[5], sl[6]};
+         double v = x == y ? sl[0] : 0.0;
+         for (int i = 0; i < 3; i++)
+            for (int j = 0; j < 3; j++) v -= g.b[3 * i + x] * g.b[3 * j + y] * m[3 * i + j];
+         out->st_k[k - 1] = v;
+      }
    }
 }
 

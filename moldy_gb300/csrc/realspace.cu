@@ -89,7 +89,10 @@ __device__ __forceinline__ double hrow(const double *m, double a0, double a1, do
 
 // Also the set-up of the evaluation's result record, by the last block, and
 // on small grids (SCAN_ONE cells) the scan of the cell counts and on small
-// systems (SCATTER_ONE sites) the placement: launches are the cost there.
+// systems (SCATTER_ONE sites) the placement: launches are the cost there, and
+// in the last block the latency of its loads, so every thread has all of its
+// own in flight (2048 sites: 14.8 us in rounds of 1024 counts and 256 sites,
+// 9.5 us so; the three separate kernels 11.8 us and two more launches).
 constexpr int SCAN_ONE = 8192, SCATTER_ONE = 2048;
 
 __device__ __forceinline__ int warp_incl_scan(int v);
@@ -146,39 +149,69 @@ k_bin(RsParams P, const double *__restrict__ site, const double *__restrict__ co
       sync[SYNC_BINERR] = 0u;
    }
    if (ncount > SCAN_ONE) return;
-   // four consecutive counts per thread and round
-   __shared__ int wsum[8], carry_s;
-   if (t == 0) carry_s = 0;
+   // one round: a run of consecutive counts per thread (a multiple of four,
+   // all its loads in flight), then the sites, eight per thread in flight
+   static_assert(SCAN_ONE <= 8192, "36 counts a thread");
+   __shared__ int wsum[8];
+   const int lane = t & 31, w = t >> 5, run = (ncount / 256 + 4) & ~3, i0 = t * run;   // 256 run > ncount
+   int4 v[9];
+   int sum = 0;
+#pragma unroll
+   for (int k = 0; k < 9; k++) {
+      v[k] = make_int4(0, 0, 0, 0);
+      const int i = i0 + 4 * k;
+      if (4 * k < run) {
+         if (i + 3 < ncount) {
+            v[k] = __ldcg(reinterpret_cast<const int4 *>(cell_count + i));
+         } else {
+            if (i < ncount) v[k].x = __ldcg(&cell_count[i]);
+            if (i + 1 < ncount) v[k].y = __ldcg(&cell_count[i + 1]);
+            if (i + 2 < ncount) v[k].z = __ldcg(&cell_count[i + 2]);
+         }
+         sum += (v[k].x + v[k].y) + (v[k].z + v[k].w);
+      }
+   }
+   const int inc = warp_incl_scan(sum);
+   if (lane == 31) wsum[w] = inc;
    __syncthreads();
-   const int lane = t & 31, w = t >> 5;
-   for (int b0 = 0; b0 <= ncount; b0 += 1024) {
-      int v[4], sum = 0;
+   int ex = inc - sum;
+   for (int k = 0; k < w; k++) ex += wsum[k];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-         const int i = b0 + 4 * t + k;
-         v[k] = i < ncount ? __ldcg(&cell_count[i]) : 0;
-         sum += v[k];
+   for (int k = 0; k < 9; k++) {
+      const int i = i0 + 4 * k;
+      if (4 * k < run) {
+         int4 o4;
+         o4.x = ex;
+         o4.y = ex + v[k].x;
+         o4.z = o4.y + v[k].y;
+         o4.w = o4.z + v[k].z;
+         ex = o4.w + v[k].w;
+         if (i + 3 <= ncount) {
+            *reinterpret_cast<int4 *>(cell_start + i) = o4;
+         } else {
+            if (i <= ncount) cell_start[i] = o4.x;
+            if (i + 1 <= ncount) cell_start[i + 1] = o4.y;
+            if (i + 2 <= ncount) cell_start[i + 2] = o4.z;
+         }
       }
-      const int inc = warp_incl_scan(sum);
-      if (lane == 31) wsum[w] = inc;
-      __syncthreads();
-      int ex = inc - sum + carry_s, tot = 0;
-      for (int k = 0; k < 8; k++) {
-         if (k < w) ex += wsum[k];
-         tot += wsum[k];
-      }
-#pragma unroll
-      for (int k = 0; k < 4; k++) {
-         const int i = b0 + 4 * t + k;
-         if (i <= ncount) cell_start[i] = ex;
-         ex += v[k];
-      }
-      __syncthreads();
-      if (t == 0) carry_s += tot;
-      __syncthreads();
    }
    if (P.nsites > SCATTER_ONE) return;
-   for (int i = t; i < P.nsites; i += blockDim.x) unsorted[cell_start[__ldcg(&cell_of[i])] + __ldcg(&rank[i])] = i;
+   __syncthreads();
+   for (int b0 = t; b0 < P.nsites; b0 += 8 * 256) {
+      int c[8], r[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+         const int i = b0 + 256 * k;
+         c[k] = i < P.nsites ? __ldcg(&cell_of[i]) : -1;
+         r[k] = i < P.nsites ? __ldcg(&rank[i]) : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+         if (c[k] >= 0) r[k] += cell_start[c[k]];
+#pragma unroll
+      for (int k = 0; k < 8; k++)
+         if (c[k] >= 0) unsorted[r[k]] = b0 + 256 * k;
+   }
 }
 
 // ---------------------------------------------------------- exclusive scan
