@@ -243,6 +243,35 @@ __device__ __forceinline__ void mol_sites(const MdStepParams &P, const double *c
    }
 }
 
+// Threads per block of the per-molecule kernels.  They are long chains of
+// FP64 instructions (the FP64 pipe takes a warp's in 16 cycles), so a small
+// system spreads over the SMs a warp to a block (216 molecules: kicks 17 us
+// in a block of 256, 11 us in seven of 32; half drift, whose chain of
+// rotations is the latency of one warp, 19 and 17.5 us; kinetic stress 6.1
+// and 4.3 us; site virial 9 and 5.3 us), and a large one keeps the number of
+// partial sums down.
+static int md_threads(int nmols) { return nmols <= 32 * 4 * 152 ? 32 : 128; }
+static int md_site_threads(int nsites) { return nsites <= 32 * 4 * 152 ? 32 : 256; }
+
+// Sums of K values over a block of up to 256 threads (whole warps), in a
+// fixed order; the results in thread 0.
+template <int K> __device__ __forceinline__ void md_block_sum(double (&v)[K], double (*sh)[8])
+{
+   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+   for (int k = 0; k < K; k++) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+      if (lane == 0) sh[k][w] = v[k];
+   }
+   if (nw == 1) return;
+   __syncthreads();
+   if (threadIdx.x == 0)
+      for (int j = 1; j < nw; j++)
+#pragma unroll
+         for (int k = 0; k < K; k++) v[k] += sh[k][j];
+}
+
 // Half step of the co-ordinates (leapf_all_coords, src/accel.c:360-372).
 // Under the thermostat (therm non-null) the steps are scaled by its
 // variable s, and each block writes to tpart its share of the thermostat
@@ -258,7 +287,7 @@ k_md_drift(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restric
            const int *__restrict__ mol_site0 = nullptr, const double *__restrict__ pf = nullptr,
            double *__restrict__ site = nullptr)
 {
-   __shared__ double sh[128];
+   __shared__ double sh[1][8];
    const int m = blockIdx.x * blockDim.x + threadIdx.x;
    const double sv = therm ? therm[TH_S] : 1.0;
    double dsm = 0.0;   // this molecule's increment of the thermostat momentum
@@ -342,27 +371,22 @@ k_md_drift(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restric
    }
    }
    if (!therm) return;
-   // fixed-shape block sum of the increments
-   sh[threadIdx.x] = dsm;
-   __syncthreads();
-   for (int w = 64; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-      __syncthreads();
-   }
-   if (threadIdx.x == 0) tpart[blockIdx.x] = sh[0];
+   double d[1] = {dsm};
+   md_block_sum(d, sh);
+   if (threadIdx.x == 0) tpart[blockIdx.x] = d[0];
 }
 
 // One thread per molecule: force and principal-frame torque from the site
 // forces, two half kicks, and the kinetic energy between them (block sums
 // of the translational and rotational parts in kpart).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 k_md_kick(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restrict__ mol_spec,
           const int *__restrict__ mol_q, const int *__restrict__ mol_site0, const double *__restrict__ pf,
           const double *__restrict__ force, const double *__restrict__ quat, double *__restrict__ mom,
           double *__restrict__ amom, double *__restrict__ kpart, double *__restrict__ molf,
           double *__restrict__ molt, const double *__restrict__ therm)
 {
-   __shared__ double sh[2][256];
+   __shared__ double sh[2][8];
    const int m = blockIdx.x * blockDim.x + threadIdx.x;
    const int N = P.nsites;
    double ket = 0.0, ker = 0.0;
@@ -439,20 +463,11 @@ k_md_kick(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restrict
       pm[1] = S.framework ? 0.0 : x[1];
       pm[2] = S.framework ? 0.0 : x[2];
    }
-   // fixed-shape block sums
-   sh[0][threadIdx.x] = ket;
-   sh[1][threadIdx.x] = ker;
-   __syncthreads();
-   for (int w = 128; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w) {
-         sh[0][threadIdx.x] += sh[0][threadIdx.x + w];
-         sh[1][threadIdx.x] += sh[1][threadIdx.x + w];
-      }
-      __syncthreads();
-   }
+   double d[2] = {ket, ker};
+   md_block_sum(d, sh);
    if (threadIdx.x == 0) {
-      kpart[2 * blockIdx.x] = sh[0][0];
-      kpart[2 * blockIdx.x + 1] = sh[1][0];
+      kpart[2 * blockIdx.x] = d[0];
+      kpart[2 * blockIdx.x + 1] = d[1];
    }
 }
 
@@ -572,7 +587,7 @@ __global__ void __launch_bounds__(128)
 k_md_kedyad(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restrict__ mol_spec,
             const double *__restrict__ mom, const double *__restrict__ therm, double *__restrict__ part)
 {
-   __shared__ double sh[9][128];
+   __shared__ double sh[9][8];
    const int m = blockIdx.x * blockDim.x + threadIdx.x;
    double d[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
    if (m < P.nmols) {
@@ -588,14 +603,9 @@ k_md_kedyad(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restri
       for (int i = 0; i < 3; i++)
          for (int j = 0; j < 3; j++) d[3 * i + j] = v[i] * v[j] * r;
    }
-   for (int k = 0; k < 9; k++) sh[k][threadIdx.x] = d[k];
-   __syncthreads();
-   for (int w = 64; w > 0; w >>= 1) {
-      if ((int)threadIdx.x < w)
-         for (int k = 0; k < 9; k++) sh[k][threadIdx.x] += sh[k][threadIdx.x + w];
-      __syncthreads();
-   }
-   if (threadIdx.x < 9) part[9 * blockIdx.x + threadIdx.x] = sh[threadIdx.x][0];
+   md_block_sum(d, sh);
+   if (threadIdx.x == 0)
+      for (int k = 0; k < 9; k++) part[9 * blockIdx.x + k] = d[k];
 }
 
 // ------------------------------------------------------------ dump records
@@ -608,7 +618,7 @@ k_md_virc(MdStepParams P, const int *__restrict__ site_mol, const int *__restric
           const double *__restrict__ pf, const int *__restrict__ mol_q, const double *__restrict__ quat,
           const double *__restrict__ force, double *__restrict__ part)
 {
-   __shared__ double sh[9][256];
+   __shared__ double sh[9][8];
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    const int N = P.nsites, t = threadIdx.x;
    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -626,31 +636,21 @@ k_md_virc(MdStepParams P, const int *__restrict__ site_mol, const int *__restric
       for (int a = 0; a < 3; a++)
          for (int b = 0; b < 3; b++) v[3 * a + b] = f[a] * d[b];
    }
-   for (int k = 0; k < 9; k++) sh[k][t] = v[k];
-   __syncthreads();
-   for (int w = 128; w > 0; w >>= 1) {
-      if (t < w)
-         for (int k = 0; k < 9; k++) sh[k][t] += sh[k][t + w];
-      __syncthreads();
-   }
-   if (t < 9) part[9 * (size_t)blockIdx.x + t] = sh[t][0];
+   md_block_sum(v, sh);
+   if (t == 0)
+      for (int k = 0; k < 9; k++) part[9 * (size_t)blockIdx.x + k] = v[k];
 }
 
 __global__ void __launch_bounds__(256) k_md_virc2(const double *__restrict__ part, int nb, double *__restrict__ virc)
 {
-   __shared__ double sh[9][256];
+   __shared__ double sh[9][8];
    const int t = threadIdx.x;
    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
    for (int b = t; b < nb; b += 256)
       for (int k = 0; k < 9; k++) v[k] += part[9 * (size_t)b + k];
-   for (int k = 0; k < 9; k++) sh[k][t] = v[k];
-   __syncthreads();
-   for (int w = 128; w > 0; w >>= 1) {
-      if (t < w)
-         for (int k = 0; k < 9; k++) sh[k][t] += sh[k][t + w];
-      __syncthreads();
-   }
-   if (t < 9) virc[t] = sh[t][0];
+   md_block_sum(v, sh);
+   if (t == 0)
+      for (int k = 0; k < 9; k++) virc[k] = v[k];
 }
 
 // Offsets of the parts of a record (-1: absent), in dump_convert's order.
@@ -888,13 +888,13 @@ extern "C" mdgpu_status mdgpu_md_init(mdgpu_ctx *c, const mdgpu_dynamics *dyn, c
    CK(D.site_pf.ensure(c->nsites));
    CK(D.pf.ensure(c->spec_pf.size()));
    CK(D.spec.ensure(nsp));
-   CK(D.kpart.ensure(2 * (size_t)((c->nmols + 255) / 256)));
+   CK(D.kpart.ensure(2 * (size_t)((c->nmols + 31) / 32)));
    CK(D.molf.ensure(3 * (size_t)c->nmols));
    CK(D.molt.ensure(3 * (size_t)nq + 3));
    CK(D.err.ensure(1));
    CK(D.counter.ensure(1));
    CK(D.therm.ensure(4));
-   CK(D.tpart.ensure(2 * (size_t)((c->nmols + 127) / 128)));
+   CK(D.tpart.ensure(2 * (size_t)((c->nmols + 31) / 32)));
    CK(cudaMemcpyAsync(D.cofm.p, c_of_m, 3 * (size_t)c->nmols * sizeof(double), cudaMemcpyHostToDevice, st));
    CK(cudaMemcpyAsync(D.mom.p, mom, 3 * (size_t)c->nmols * sizeof(double), cudaMemcpyHostToDevice, st));
    if (nq) {
@@ -925,14 +925,14 @@ static mdgpu_status md_enqueue_step(mdgpu_ctx *c, const MdStepParams &P, int cap
    const MdHost &H = c->mdh;
    MdDev &D = c->md;
    cudaStream_t st = c->stream;
-   const int N = c->nsites, M = c->nmols, nbm = (M + 255) / 256, nbd = (M + 127) / 128;
+   const int N = c->nsites, M = c->nmols, tm = md_threads(M), nbd = (M + tm - 1) / tm;
    double *th = P.therm ? D.therm.p : nullptr;
    if (th) {
       k_md_therm<<<1, 128, 0, st>>>(P, th, nullptr, 0, 0);
       c->launches += 1;
    }
    // half drift, and the sites of the force evaluation from its result
-   k_md_drift<<<nbd, 128, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
+   k_md_drift<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
                                    D.err.p, th, D.tpart.p, D.mol_site0.p, D.pf.p, c->site.p);
    CK(cudaGetLastError());
    c->launches += 1;
@@ -941,17 +941,17 @@ static mdgpu_status md_enqueue_step(mdgpu_ctx *c, const MdStepParams &P, int cap
    if (virc) {
       // molecular correction of the virial, with the quaternions of this
       // force evaluation (the drift after the kick moves them)
-      const int nbs = (N + 255) / 256;
-      k_md_virc<<<nbs, 256, 0, st>>>(P, D.site_mol.p, D.site_pf.p, D.pf.p, D.mol_q.p, D.quat.p, c->force.p,
+      const int ts = md_site_threads(N), nbs = (N + ts - 1) / ts;
+      k_md_virc<<<nbs, ts, 0, st>>>(P, D.site_mol.p, D.site_pf.p, D.pf.p, D.mol_q.p, D.quat.p, c->force.p,
                                      D.vpart.p);
-      k_md_virc2<<<1, 256, 0, st>>>(D.vpart.p, nbs, D.virc.p);
+      k_md_virc2<<<1, nbs <= 64 ? 32 : 256, 0, st>>>(D.vpart.p, nbs, D.virc.p);
       c->launches += 2;
    }
-   k_md_kick<<<nbm, 256, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.mol_site0.p, D.pf.p, c->force.p,
+   k_md_kick<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.mol_site0.p, D.pf.p, c->force.p,
                                   D.quat.p, D.mom.p, D.amom.p, D.kpart.p, D.molf.p, D.molt.p, th);
-   k_md_record<<<1, 128, 0, st>>>(D.counter.p, cap, c->small.p, D.kpart.p, nbm, dist_v, c->out.p, D.energies.p,
+   k_md_record<<<1, 128, 0, st>>>(D.counter.p, cap, c->small.p, D.kpart.p, nbd, dist_v, c->out.p, D.energies.p,
                                  D.err.p, P, th, D.tpart.p, nbd);
-   k_md_drift<<<nbd, 128, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
+   k_md_drift<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
                                    D.err.p, th, D.tpart.p + nbd);
    CK(cudaGetLastError());
    c->launches += 3;
@@ -1062,8 +1062,8 @@ static mdgpu_status ke_dyad_h(mdgpu_ctx *c, const MdStepParams &P, double *dyad)
 {
    MdDev &D = c->md;
    cudaStream_t st = c->stream;
-   const int nbd = (c->nmols + 127) / 128;
-   k_md_kedyad<<<nbd, 128, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mom.p, D.therm.p, D.kdpart.p);
+   const int tm = md_threads(c->nmols), nbd = (c->nmols + tm - 1) / tm;
+   k_md_kedyad<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mom.p, D.therm.p, D.kdpart.p);
    CK(cudaGetLastError());
    c->launches += 1;
    std::vector<double> &hp = c->mdh.kpart_h;
@@ -1089,7 +1089,7 @@ static mdgpu_status md_baro_step(mdgpu_ctx *c, int cap)
    MdHost &H = c->mdh;
    MdDev &D = c->md;
    cudaStream_t st = c->stream;
-   const int N = c->nsites, M = c->nmols, nbm = (M + 255) / 256, nbd = (M + 127) / 128;
+   const int N = c->nsites, M = c->nmols, tm = md_threads(M), nbd = (M + tm - 1) / tm;
    const bool uni = H.baro == 2, therm = H.therm;
    const double dt = 2.0 * H.half;
    double *th = D.therm.p;
@@ -1110,23 +1110,23 @@ static mdgpu_status md_baro_step(mdgpu_ctx *c, int cap)
    if (s) return s;
    update_hmom_h(0.5 * dt, ts, H.h, dyad, H.hmom, uni);
    // half drift, and the sites of the force evaluation from its result
-   k_md_drift<<<nbd, 128, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
+   k_md_drift<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
                                    D.err.p, th, D.tpart.p, D.mol_site0.p, D.pf.p, c->site.p);
    CK(cudaGetLastError());
    c->launches += 1;
    if ((s = mdgpu_forces_device(c, H.h, c->site.p, D.cofm.p, c->force.p, c->small.p, c->small.p + 2)) != MDGPU_OK)
       return s;
-   const int nbs = (N + 255) / 256;
-   k_md_virc<<<nbs, 256, 0, st>>>(P, D.site_mol.p, D.site_pf.p, D.pf.p, D.mol_q.p, D.quat.p, c->force.p, D.vpart.p);
-   k_md_virc2<<<1, 256, 0, st>>>(D.vpart.p, nbs, D.virc.p);
+   const int tv = md_site_threads(N), nbs = (N + tv - 1) / tv;
+   k_md_virc<<<nbs, tv, 0, st>>>(P, D.site_mol.p, D.site_pf.p, D.pf.p, D.mol_q.p, D.quat.p, c->force.p, D.vpart.p);
+   k_md_virc2<<<1, nbs <= 64 ? 32 : 256, 0, st>>>(D.vpart.p, nbs, D.virc.p);
    const double vol = det3(H.h);
    P.kecell = ke_cell_h(H.hmom, H.pmass);
    P.pv = H.pressure * vol;
    P.dsm_mid = dsm_mid;
    std::memcpy(P.hmom, H.hmom, sizeof P.hmom);
-   k_md_kick<<<nbm, 256, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.mol_site0.p, D.pf.p, c->force.p,
+   k_md_kick<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.mol_site0.p, D.pf.p, c->force.p,
                                   D.quat.p, D.mom.p, D.amom.p, D.kpart.p, D.molf.p, D.molt.p, th);
-   k_md_record<<<1, 128, 0, st>>>(D.counter.p, cap, c->small.p, D.kpart.p, nbm, H.dist / vol, c->out.p,
+   k_md_record<<<1, 128, 0, st>>>(D.counter.p, cap, c->small.p, D.kpart.p, nbd, H.dist / vol, c->out.p,
                                  D.energies.p, D.err.p, P, th, D.tpart.p, nbd);
    CK(cudaGetLastError());
    c->launches += 4;
@@ -1145,7 +1145,7 @@ static mdgpu_status md_baro_step(mdgpu_ctx *c, int cap)
    update_hmom_h(dt, ts, H.h, S, H.hmom, uni);
    if ((s = ke_dyad_h(c, P, dyad)) != MDGPU_OK) return s;
    update_hmom_h(0.5 * dt, ts, H.h, dyad, H.hmom, uni);
-   k_md_drift<<<nbd, 128, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
+   k_md_drift<<<nbd, tm, 0, st>>>(P, D.spec.p, D.mol_spec.p, D.mol_q.p, D.cofm.p, D.mom.p, D.quat.p, D.amom.p,
                                    D.err.p, th, D.tpart.p + nbd);
    CK(cudaGetLastError());
    c->launches += 1;
@@ -1223,16 +1223,16 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
    const int nrec = records && nsteps >= first ? (nsteps - first) / interval + 1 : 0;
    int batch = 0;
    if (H.baro) {
-      CK(D.vpart.ensure(9 * (size_t)((c->nsites + 255) / 256)));
+      CK(D.vpart.ensure(9 * (size_t)((c->nsites + 31) / 32)));
       CK(D.virc.ensure(9));
-      CK(D.kdpart.ensure(9 * (size_t)((c->nmols + 127) / 128)));
+      CK(D.kdpart.ensure(9 * (size_t)((c->nmols + 31) / 32)));
    }
    if (nrec > 0) {
       // device batch of records: up to 256 MiB
       batch = (int)std::min<size_t>((size_t)nrec, std::max<size_t>(1, ((size_t)64 << 20) / (size_t)dsize));
       CK(D.rec.ensure((size_t)batch * dsize));
       if (level & 8) {
-         CK(D.vpart.ensure(9 * (size_t)((c->nsites + 255) / 256)));
+         CK(D.vpart.ensure(9 * (size_t)((c->nsites + 31) / 32)));
          CK(D.virc.ensure(9));
       }
    }
