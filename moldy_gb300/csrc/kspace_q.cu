@@ -1393,21 +1393,17 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    if (c->nsm <= 0) CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
    if (q.ns == ns || c->kl.nk == 0) return MDGPU_OK;
    build_qlist(c->kl, ns);
-   cudaStream_t st = c->stream;
-   auto up = [&](auto &buf, const auto &v) -> cudaError_t {
-      cudaError_t e = buf.ensure(v.size());
-      if (e == cudaSuccess && !v.empty())
-         e = cudaMemcpyAsync(buf.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st);
-      return e;
-   };
-   CK(up(d.q_units, q.units));
-   CK(up(d.q_coeff, q.coeff));
-   CK(up(d.q_tiles, q.tiles));
-   CK(up(d.q_segs, q.segs));
-   CK(up(d.q_fu, q.fu));
+   TablePack &k = d.q_lists;
+   k.begin();
+   const size_t o[5] = {k.add(q.units), k.add(q.coeff), k.add(q.tiles), k.add(q.segs), k.add(q.fu)};
+   CK(k.send(c->stream));
+   k.at(d.q_units.p, o[0]);
+   k.at(d.q_coeff.p, o[1]);
+   k.at(d.q_tiles.p, o[2]);
+   k.at(d.q_segs.p, o[3]);
+   k.at(d.q_fu.p, o[4]);
    d.q_fblk = q.fblk;
    d.q_nfblk = q.fblk.empty() ? 0 : (int)q.fblk.size() - 1;
-   CK(cudaStreamSynchronize(st));
    d.tc_ver++;
    return MDGPU_OK;
 }

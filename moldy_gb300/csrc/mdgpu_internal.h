@@ -6,6 +6,7 @@
 
 #include <cstdint>
 #include <string>
+#include <cstring>
 #include <vector>
 
 #include "../../include/moldy_gb300.h"
@@ -162,6 +163,34 @@ struct DBuf {
    }
 };
 
+// Host tables that change together (with the cell shape, every step of a
+// constant-pressure run), gathered here and sent in one copy: a copy costs the
+// host 3 to 5 us to issue whatever its size, and waiting for it a round trip.
+// (The source is ordinary memory, which the driver has read when the call
+// returns.)
+struct TablePack {
+   std::vector<unsigned char> h;
+   DBuf<unsigned char> d;
+   void begin() { h.clear(); }
+   template <typename T> size_t add(const std::vector<T> &v)   // its offset
+   {
+      const size_t o = (h.size() + 255) & ~(size_t)255;
+      h.resize(o + v.size() * sizeof(T));
+      if (!v.empty()) std::memcpy(h.data() + o, v.data(), v.size() * sizeof(T));
+      return o;
+   }
+   cudaError_t send(cudaStream_t st)
+   {
+      cudaError_t e = d.ensure(h.size());
+      if (e == cudaSuccess && !h.empty()) e = cudaMemcpyAsync(d.p, h.data(), h.size(), cudaMemcpyHostToDevice, st);
+      return e;
+   }
+   template <typename T> void at(T *&p, size_t o) const { p = reinterpret_cast<T *>(d.p + o); }
+};
+template <typename T> struct DView {   // a table of a pack
+   T *p = nullptr;
+};
+
 // Device-resident outputs of one evaluation (all FP64).
 struct DevOut {
    double pe_rs;          // sum of pair energies (before eintra)
@@ -197,8 +226,9 @@ struct RsDev {
    DBuf<int2> tag;         // sorted: site id, molecule
    DBuf<int> molmap, siteid, ent_mol;
    DBuf<double> chg, cofm;
-   DBuf<int4> full;
-   DBuf<float4> off_hi, off_lo;
+   TablePack geom;         // the link-cell tables: full .. off_lo, cols .. coff
+   DView<int4> full;
+   DView<float4> off_hi, off_lo;
    DBuf<double> pot64;
    DBuf<float> pot32;
    DBuf<double> part;      // per-block partial energies/virials
@@ -209,9 +239,9 @@ struct RsDev {
    // columns and their offsets (where it runs with two interaction classes
    // the slots are laid class by class: cell_start then holds class 0's
    // cells, class 1's, and the end)
-   DBuf<int4> cols;
-   DBuf<int> col_base;
-   DBuf<float4> coff;      // [e][2]: the column offsets' hi and lo parts side by side (32 B per entry)
+   DView<int4> cols;
+   DView<int> col_base;
+   DView<float4> coff;     // [e][2]: the column offsets' hi and lo parts side by side (32 B per entry)
    DBuf<int2> tagc;        // per slot: site id with the cell's z index above 16 bits, molecule
    DBuf<int> site_cls;     // interaction class of every site
    DBuf<int> rank, unsorted;   // place of a site among its cell's, slots before the sort within cells
@@ -259,10 +289,11 @@ struct KsDev {
    // operand; z as the mixed force pass's A operand or in FP64); the
    // structure-factor partials; per (quad, t) A and B; the force passes'
    // coefficient operands
-   DBuf<int4> q_units, q_fu;
-   DBuf<double2> q_coeff;
-   DBuf<QTile> q_tiles;
-   DBuf<QSeg> q_segs;
+   TablePack q_lists;      // q_units .. q_segs
+   DView<int4> q_units, q_fu;
+   DView<double2> q_coeff;
+   DView<QTile> q_tiles;
+   DView<QSeg> q_segs;
    DBuf<QItem> q_items;
    DBuf<int> q_x32, q_y32, q_bexp;
    DBuf<long long> q_x64, q_y64;

@@ -2172,24 +2172,21 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
       }
       CK(d.cell_start.ensure(2 * (size_t)g.ncells + 1));
       CK(d.blocksum.ensure((2 * (size_t)g.ncells + 1 + 1023) / 1024 + 2));
-      CK(d.full.ensure(g.full.size()));
-      CK(d.off_hi.ensure(g.full.size()));
-      CK(d.off_lo.ensure(g.full.size()));
-      CK(cudaMemcpyAsync(d.full.p, g.full.data(), g.full.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.off_hi.p, g.off_hi.data(), g.off_hi.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.off_lo.p, g.off_lo.data(), g.off_lo.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-      CK(d.cols.ensure(g.cols.size()));
-      CK(d.col_base.ensure(g.col_base.size()));
       std::vector<float4> coff(2 * g.coff_hi.size());
       for (size_t e = 0; e < g.coff_hi.size(); e++) {
          coff[2 * e] = g.coff_hi[e];
          coff[2 * e + 1] = g.coff_lo[e];
       }
-      CK(d.coff.ensure(coff.size()));
-      CK(cudaMemcpyAsync(d.cols.p, g.cols.data(), g.cols.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.col_base.p, g.col_base.data(), g.col_base.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-      CK(cudaMemcpyAsync(d.coff.p, coff.data(), coff.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-      CK(cudaStreamSynchronize(st));
+      TablePack &k = d.geom;
+      k.begin();
+      const size_t o[6] = {k.add(g.full), k.add(g.off_hi), k.add(g.off_lo), k.add(g.cols), k.add(g.col_base), k.add(coff)};
+      CK(k.send(st));
+      k.at(d.full.p, o[0]);
+      k.at(d.off_hi.p, o[1]);
+      k.at(d.off_lo.p, o[2]);
+      k.at(d.cols.p, o[3]);
+      k.at(d.col_base.p, o[4]);
+      k.at(d.coff.p, o[5]);
       c->rs_uploaded = true;
    }
    const int nb = (N + PAIR_WARPS - 1) / PAIR_WARPS;
