@@ -483,6 +483,7 @@ struct mdgpu_ctx {
    // every identifier is in class 0.
    std::vector<int> cls_of_id;
    int ncls = 1;
+   int cls_pot = 0, cls_chg = 0;    // bit k: class k has a potential, charges among its sites
    // bumped by every call that changes what a captured step would launch
    // (system, control, parameters, precision, stream, dynamics state)
    uint64_t gen = 1;

@@ -44,6 +44,8 @@ struct RsParams {
    int ncols;             // stencil columns (k_pairs_col)
    int chunk;             // home slots a block takes at a time (ColHome)
    int one_class;         // the slots are in link-cell order, one interaction class
+   int ex, ey, z0, z1;    // the stencil's extents: |dx|, |dy|, dz from z0 to z1
+   int cls_pot, cls_chg;  // bit k: sites of class k have a potential among them, charges
    double hinv[9];
    double h[9];
    double rn[3];          // 1/nx, 1/ny, 1/nz
@@ -509,7 +511,8 @@ template <> struct PairMath<double, true> {
 // One pair of kernel(): f = -U'(r)/r and U, with the erfc real-space Ewald
 // term by the A&S polynomial when EW (src/kernel.c:182-353 / 355-460).
 template <int PT, bool EW, typename R, bool FAST = false>
-__device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm, R &f, R &u)
+__device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm, R &f, R &u, bool hp = true,
+                                        bool hc = true)
 {
    typedef PairMath<R, FAST> M;
    R t = R(0), ef = R(0), r = R(0), r_r = R(0), rs_r;
@@ -525,7 +528,7 @@ __device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm,
    } else {
       rs_r = M::rcp(r2);
    }
-   if (EW) {
+   if (EW && hc) {
       if (FAST && sizeof(R) == 8) {   // one product fewer (FP64)
          t = M::rcp(fma((R(ASP) * alpha), r, R(1)));
          ef = qq * M::ex(-(alpha * alpha) * r2);
@@ -536,6 +539,11 @@ __device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm,
       }
       t = (t * (R(AS1) + t * (R(AS2) + t * (R(AS3) + t * (R(AS4) + t * R(AS5)))))) * ef * r_r;
       ef = t + norm * ef;
+   }
+   if (EW && FAST && !hp) {   // (warp-uniform: the home site's class has none)
+      u = t;
+      f = rs_r * ef;
+      return;
    }
    if (EW && FAST && sizeof(R) == 8) {
       // FP64: a potential whose parameters are all zero adds exactly nothing
@@ -1020,7 +1028,7 @@ __global__ void __launch_bounds__(256) k_reduce_rs2(const double *__restrict__ p
 // k_tooclose_x.
 constexpr int COL_E = 3;                    // stencil columns per lane in one pass
 constexpr int COL_ROWS = 32 * COL_E * 2;    // slot runs per pass (two per column at most)
-constexpr int COL_WIN = 256;                // candidates decoded per window
+constexpr int COL_WIN = 384;                // candidates decoded per window (most stencils' whole list)
 constexpr int COL_CHUNK = 16;               // most consecutive home slots a block takes at a time
 
 // The home slots of a block's warp w: chunks of `chunk` consecutive slots
@@ -1079,6 +1087,102 @@ __device__ __forceinline__ ColRuns col_runs(const RsParams &P, int cx, int cy, i
    return r;
 }
 
+// The walk of the column kernels: calls visit(j, inf) for every slot j of the
+// home cell (cx, cy, cz)'s stencil (the home slot among them), inf = index
+// base << 5 | image code: the offset-table entry of slot j in cell c (its z
+// alone with ZREL) is c + (inf >> 5).  csk: the cell starts of the class
+// walked.  Listing the candidates costs as much as the mixed form's pair
+// arithmetic (32,000-site water: 2327 instructions a home site, 10 rounds of
+// about 110 of them arithmetic; 2046 so, pairs of
+// 131,072-site water 356 -> 314 us), hence: the runs of a lane's
+// columns stay in registers (in shared memory only where the candidates do
+// not fit one window), a second run per column is looked at only where some
+// column wraps the cell, and cells whose whole stencil lies inside the grid
+// take a path without images.
+struct ColRows {
+   int *inc, *jb, *inf, *cand;
+};
+template <bool ZREL, class Visit>
+__device__ __forceinline__ void walk_columns(const RsParams &P, const int *__restrict__ csk,
+                                             const int4 *__restrict__ cols, const int *__restrict__ col_base,
+                                             int cx, int cy, int cz, int lane, const ColRows &w, Visit &&visit)
+{
+   const bool inside = cx >= P.ex && cx + P.ex < P.nx && cy >= P.ey && cy + P.ey < P.ny && cz + P.z0 >= 0 &&
+                       cz + P.z1 < P.nz;
+   for (int base = 0; base < P.ncols; base += 32 * COL_E) {
+      int T, nrow;   // candidates; runs per column
+      {
+         int cnt[2 * COL_E], jb[2 * COL_E], tot = 0, ns = 1;
+#pragma unroll
+         for (int u = 0; u < COL_E; u++) {
+            const int q0 = lane * 2 * COL_E + 2 * u, col = base + lane * COL_E + u;
+            cnt[2 * u] = cnt[2 * u + 1] = jb[2 * u] = jb[2 * u + 1] = 0;
+            if (col < P.ncols) {
+               const int4 cd = __ldg(&cols[col]);
+               const int ob = __ldg(&col_base[col]);
+               if (inside) {
+                  const int cc = P.nz * (cy + cd.y + P.ny * (cx + cd.x)), z = cz + cd.z;
+                  jb[2 * u] = __ldg(&csk[cc + z]);
+                  cnt[2 * u] = __ldg(&csk[cc + z + cd.w]) - jb[2 * u];
+                  w.inf[q0] = (ob - z - (ZREL ? 0 : cc)) * 32 | 13;
+               } else {
+                  const ColRuns cr = col_runs(P, cx, cy, cz, cd);
+#pragma unroll
+                  for (int s = 0; s < 2; s++)
+                     if (s < cr.ns) {
+                        jb[2 * u + s] = __ldg(&csk[cr.cc + cr.za[s]]);
+                        cnt[2 * u + s] = __ldg(&csk[cr.cc + cr.zb[s] + 1]) - jb[2 * u + s];
+                        const int eb = ob - cd.z - cz + cr.iz[s] * P.nz - (ZREL ? 0 : cr.cc);
+                        w.inf[q0 + s] = eb * 32 | (9 * (cr.ix + 1) + 3 * (cr.iy + 1) + (cr.iz[s] + 1));
+                     }
+                  ns = max(ns, cr.ns);
+               }
+               tot += cnt[2 * u] + cnt[2 * u + 1];
+            }
+         }
+         nrow = inside ? 1 : __reduce_max_sync(0xffffffffu, ns);
+         const int linc = warp_incl_scan(tot);
+         T = __shfl_sync(0xffffffffu, linc, 31);
+         int run = linc - tot;
+         // the runs end to end: the first window's candidates (slot | run << 24)
+#pragma unroll
+         for (int r = 0; r < 2 * COL_E; r++)
+            if ((r & 1) == 0 || nrow == 2) {
+               const int q = lane * 2 * COL_E + r, e = run + cnt[r], jq = jb[r] - run;
+               if (T > COL_WIN) {   // later windows read the runs again
+                  w.jb[q] = jq;
+                  w.inc[q] = e;
+               }
+               const int b = min(e, COL_WIN);
+               for (int t = run; t < b; t++) w.cand[t] = (jq + t) | (q << 24);
+               run = e;
+            }
+      }
+      __syncwarp();
+      for (int w0 = 0; w0 < T; w0 += COL_WIN) {
+         const int w1 = min(T, w0 + COL_WIN);
+         if (w0 > 0) {
+#pragma unroll
+            for (int r = 0; r < 2 * COL_E; r++)
+               if ((r & 1) == 0 || nrow == 2) {
+                  const int q = lane * 2 * COL_E + r, q1 = q - (nrow == 2 ? 1 : 2);   // the run before
+                  const int a = max(q1 >= 0 ? w.inc[q1] : 0, w0), b = min(w.inc[q], w1), jq = w.jb[q];
+                  for (int t = a; t < b; t++) w.cand[t - w0] = (jq + t) | (q << 24);
+               }
+            __syncwarp();
+         }
+         for (int r0 = w0; r0 < w1; r0 += 32) {
+            const int idx = r0 + lane;
+            if (idx < w1) {
+               const int v = w.cand[idx - w0];
+               visit(v & 0xffffff, w.inf[(unsigned)v >> 24]);
+            }
+         }
+         __syncwarp();
+      }
+   }
+}
+
 // Each warp takes home slots of the class-major layout in turn (eight
 // blocks per SM, the grid's warps striding over the slots, so that the
 // block's set-up and energy reduction are paid once per block).  Per home
@@ -1112,7 +1216,7 @@ k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__r
 
    const int N = P.nsites, n0 = P.one_class ? N : cs[P.ncells];
    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   int *inc = s_inc[w], *jbr = s_jb[w], *infr = s_inf[w], *cand = s_cand[w];
+   const ColRows rows{s_inc[w], s_jb[w], s_inf[w], s_cand[w]};
    // the lane's energy and virial over all its home sites (per-site sums
    // added in: two levels of FP32), kept in shared memory, which the
    // candidate loop's registers leave no room for
@@ -1137,113 +1241,53 @@ k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__r
       const R alpha = P.alphaf, norm = P.normf;
       const int oi = sortc[p];
       const R cut100 = (R)P.cut100;
-      for (int base = 0; base < P.ncols; base += 32 * COL_E) {
-         // this lane's runs go straight to its rows (counts in inc for now)
-         int tot = 0;
-#pragma unroll
-         for (int u = 0; u < COL_E; u++) {
-            const int q0 = lane * 2 * COL_E + 2 * u;
-            inc[q0] = inc[q0 + 1] = 0;
-            jbr[q0] = jbr[q0 + 1] = 0;
-            infr[q0] = infr[q0 + 1] = 0;
-            const int col = base + lane * COL_E + u;
-            if (col < P.ncols) {
-               const int4 cd = __ldg(&cols[col]);
-               const int ob = __ldg(&col_base[col]);
-               const ColRuns cr = col_runs(P, cx, cy, cz, cd);
-#pragma unroll
-               for (int s = 0; s < 2; s++) {
-                  if (s < cr.ns) {
-                     const int a = __ldg(&csk[cr.cc + cr.za[s]]), b = __ldg(&csk[cr.cc + cr.zb[s] + 1]);
-                     inc[q0 + s] = b - a;
-                     jbr[q0 + s] = a;
-                     tot += b - a;
-                     // offset-table index of a candidate in cell z: z + eb
-                     const int eb = ob - cd.z - cz + cr.iz[s] * P.nz;
-                     infr[q0 + s] = (eb * 32) | (9 * (cr.ix + 1) + 3 * (cr.iy + 1) + (cr.iz[s] + 1));
-                  }
-               }
-            }
+      const bool hp = P.cls_pot >> (p >= n0) & 1, hc = P.cls_chg >> (p >= n0) & 1;
+      walk_columns<true>(P, csk, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf_q) {
+         const int kimg = inf_q & 31;
+         if (j == p && kimg == 13) return;
+         const int2 tj = __ldg(&tagc[j]);
+         const int e = (tj.x >> 16) + (inf_q >> 5);
+         const float4 xj = __ldg(&posc[j]);
+         float4 h4, l4;
+         ld_coff(coff + 2 * e, h4, l4);
+         const R rx = (h4.x + (xj.x - xi.x)) + l4.x;
+         const R ry = (h4.y + (xj.y - xi.y)) + l4.y;
+         const R rz = (h4.z + (xj.z - xi.z)) + l4.z;
+         R r2 = rx * rx + ry * ry + rz * rz;
+         const bool intra = ti.y == tj.y;
+         bool too_close, clip;
+         pair_flags<true>(P, r2, oi, j, kimg, sortc, site, too_close, clip);
+         if (too_close && !intra) {
+            const int oj = sortc[j];
+            if (oi < oj) note_too_close(out, oi, oj);
          }
-         const int linc = warp_incl_scan(tot);
-         const int T = __shfl_sync(0xffffffffu, linc, 31);
-         int run = linc - tot;
+         const R r2a = r2;
+         if (clip) r2 = cut100;
+         R pp[NP];
+         const R *pj = prow + (size_t)(tj.x & 0xffff) * NPOTP;
 #pragma unroll
-         for (int r = 0; r < 2 * COL_E; r++) {
-            const int q = lane * 2 * COL_E + r;
-            jbr[q] -= run;               // slot = jbr[q] + candidate index
-            run += inc[q];
-            inc[q] = run;                // the row's inclusive end
+         for (int k = 0; k < NP; k++) pp[k] = pj[k];
+         R f, u;
+         pair_fu<PT, EW, R, true>(r2, xj.w * qi, pp, alpha, norm, f, u, hp, hc);
+         if (intra) {
+            // as in k_pairs: an intramolecular pair's energy is
+            // what the intramolecular correction subtracts again
+            R fa, ua = R(0);
+            if (clip) pair_fu<PT, EW, R, true>(r2a, xj.w * qi, pp, alpha, norm, fa, ua, hp, hc);
+            u = clip ? u - ua : R(0);
          }
-         __syncwarp();
-         for (int w0 = 0; w0 < T; w0 += COL_WIN) {
-            const int w1 = min(T, w0 + COL_WIN);
-            // decode this lane's runs that fall in [w0, w1)
-#pragma unroll
-            for (int r = 0; r < 2 * COL_E; r++) {
-               const int q = lane * 2 * COL_E + r;
-               const int e1 = inc[q], e0 = q > 0 ? inc[q - 1] : 0;
-               const int a = max(e0, w0), b = min(e1, w1);
-               const int jq = jbr[q];
-               for (int t = a; t < b; t++) cand[t - w0] = (jq + t) | (q << 24);
-            }
-            __syncwarp();
-            for (int r0 = w0; r0 < w1; r0 += 32) {
-               const int idx = r0 + lane;
-               if (idx < w1) {
-                  const int v = cand[idx - w0];
-                  const int j = v & 0xffffff, q = (unsigned)v >> 24;
-                  const int inf_q = infr[q];
-                  const int kimg = inf_q & 31;
-                  if (j != p || kimg != 13) {
-                     const int2 tj = __ldg(&tagc[j]);
-                     const int e = (tj.x >> 16) + (inf_q >> 5);
-                     const float4 xj = __ldg(&posc[j]);
-                     float4 h4, l4;
-                     ld_coff(coff + 2 * e, h4, l4);
-                     const R rx = (h4.x + (xj.x - xi.x)) + l4.x;
-                     const R ry = (h4.y + (xj.y - xi.y)) + l4.y;
-                     const R rz = (h4.z + (xj.z - xi.z)) + l4.z;
-                     R r2 = rx * rx + ry * ry + rz * rz;
-                     const bool intra = ti.y == tj.y;
-                     bool too_close, clip;
-                     pair_flags<true>(P, r2, oi, j, kimg, sortc, site, too_close, clip);
-                     if (too_close && !intra) {
-                        const int oj = sortc[j];
-                        if (oi < oj) note_too_close(out, oi, oj);
-                     }
-                     const R r2a = r2;
-                     if (clip) r2 = cut100;
-                     R pp[NP];
-                     const R *pj = prow + (size_t)(tj.x & 0xffff) * NPOTP;
-#pragma unroll
-                     for (int k = 0; k < NP; k++) pp[k] = pj[k];
-                     R f, u;
-                     pair_fu<PT, EW, R, true>(r2, xj.w * qi, pp, alpha, norm, f, u);
-                     if (intra) {
-                        // as in k_pairs: an intramolecular pair's energy is
-                        // what the intramolecular correction subtracts again
-                        R fa, ua = R(0);
-                        if (clip) pair_fu<PT, EW, R, true>(r2a, xj.w * qi, pp, alpha, norm, fa, ua);
-                        u = clip ? u - ua : R(0);
-                     }
-                     const R hf = R(0.5) * f;
-                     fx -= f * rx;
-                     fy -= f * ry;
-                     fz -= f * rz;
-                     pe += R(0.5) * u;
-                     v0 += hf * rx * rx;
-                     v1 += hf * rx * ry;
-                     v2 += hf * rx * rz;
-                     v3 += hf * ry * ry;
-                     v4 += hf * ry * rz;
-                     v5 += hf * rz * rz;
-                  }
-               }
-            }
-            __syncwarp();
-         }
-      }
+         const R wx = f * rx, wy = f * ry, wz = f * rz;
+         fx -= wx;
+         fy -= wy;
+         fz -= wz;
+         pe += u;
+         v0 += wx * rx;
+         v1 += wx * ry;
+         v2 += wx * rz;
+         v3 += wy * ry;
+         v4 += wy * rz;
+         v5 += wz * rz;
+      });
       R Fx = fx, Fy = fy, Fz = fz;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) {
@@ -1256,13 +1300,14 @@ k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__r
          force[N + oi] = (double)Fy;
          force[2 * N + oi] = (double)Fz;
       }
-      s_tot[0][threadIdx.x] += pe;
-      s_tot[1][threadIdx.x] += v0;
-      s_tot[2][threadIdx.x] += v1;
-      s_tot[3][threadIdx.x] += v2;
-      s_tot[4][threadIdx.x] += v3;
-      s_tot[5][threadIdx.x] += v4;
-      s_tot[6][threadIdx.x] += v5;
+      // (half of each evaluation)
+      s_tot[0][threadIdx.x] += R(0.5) * pe;
+      s_tot[1][threadIdx.x] += R(0.5) * v0;
+      s_tot[2][threadIdx.x] += R(0.5) * v1;
+      s_tot[3][threadIdx.x] += R(0.5) * v2;
+      s_tot[4][threadIdx.x] += R(0.5) * v3;
+      s_tot[5][threadIdx.x] += R(0.5) * v4;
+      s_tot[6][threadIdx.x] += R(0.5) * v5;
    }
    __shared__ R wred[7][PAIR_WARPS];
    R vv[7];
@@ -1284,79 +1329,6 @@ k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__r
    reduce_pairs_last(part, gridDim.x, sync, out, fin);
 }
 
-// The walk of k_pairs_col as a function: calls visit(j, inf) for every slot
-// j of the home cell (cx, cy, cz)'s stencil (the home slot among them), inf
-// = (offset index less the partner column's first cell) << 5 | image code:
-// the offset-table entry of slot j in cell c is c + (inf >> 5).  csk: the
-// cell starts of the slots walked.
-struct ColRows {
-   int *inc, *jb, *inf, *cand;
-};
-template <class Visit>
-__device__ __forceinline__ void walk_columns(const RsParams &P, const int *__restrict__ csk,
-                                             const int4 *__restrict__ cols, const int *__restrict__ col_base,
-                                             int cx, int cy, int cz, int lane, const ColRows &w, Visit &&visit)
-{
-   for (int base = 0; base < P.ncols; base += 32 * COL_E) {
-      int tot = 0;
-#pragma unroll
-      for (int u = 0; u < COL_E; u++) {
-         const int q0 = lane * 2 * COL_E + 2 * u;
-         w.inc[q0] = w.inc[q0 + 1] = 0;
-         w.jb[q0] = w.jb[q0 + 1] = 0;
-         w.inf[q0] = w.inf[q0 + 1] = 0;
-         const int col = base + lane * COL_E + u;
-         if (col < P.ncols) {
-            const int4 cd = __ldg(&cols[col]);
-            const int ob = __ldg(&col_base[col]);
-            const ColRuns cr = col_runs(P, cx, cy, cz, cd);
-#pragma unroll
-            for (int s = 0; s < 2; s++) {
-               if (s < cr.ns) {
-                  const int a = __ldg(&csk[cr.cc + cr.za[s]]), b = __ldg(&csk[cr.cc + cr.zb[s] + 1]);
-                  w.inc[q0 + s] = b - a;
-                  w.jb[q0 + s] = a;
-                  tot += b - a;
-                  const int eb = ob - cd.z - cz + cr.iz[s] * P.nz - cr.cc;
-                  w.inf[q0 + s] = eb * 32 | (9 * (cr.ix + 1) + 3 * (cr.iy + 1) + (cr.iz[s] + 1));
-               }
-            }
-         }
-      }
-      const int linc = warp_incl_scan(tot);
-      const int T = __shfl_sync(0xffffffffu, linc, 31);
-      int run = linc - tot;
-#pragma unroll
-      for (int r = 0; r < 2 * COL_E; r++) {
-         const int q = lane * 2 * COL_E + r;
-         w.jb[q] -= run;
-         run += w.inc[q];
-         w.inc[q] = run;
-      }
-      __syncwarp();
-      for (int w0 = 0; w0 < T; w0 += COL_WIN) {
-         const int w1 = min(T, w0 + COL_WIN);
-#pragma unroll
-         for (int r = 0; r < 2 * COL_E; r++) {
-            const int q = lane * 2 * COL_E + r;
-            const int e1 = w.inc[q], e0 = q > 0 ? w.inc[q - 1] : 0;
-            const int a = max(e0, w0), b = min(e1, w1);
-            const int jq = w.jb[q];
-            for (int t = a; t < b; t++) w.cand[t - w0] = (jq + t) | (q << 24);
-         }
-         __syncwarp();
-         for (int r0 = w0; r0 < w1; r0 += 32) {
-            const int idx = r0 + lane;
-            if (idx < w1) {
-               const int v = w.cand[idx - w0];
-               visit(v & 0xffffff, w.inf[(unsigned)v >> 24]);
-            }
-         }
-         __syncwarp();
-      }
-   }
-}
-
 // a < b for non-negative doubles, by their bits (a compare would take the
 // FP64 pipe); false when a is NaN
 __device__ __forceinline__ bool less_bits(double a, double b)
@@ -1370,8 +1342,8 @@ __device__ __forceinline__ bool less_bits(double a, double b)
 // The FP64 pipe bounds it (79 % busy at 32,000 sites): 131,072-site water
 // (real-space phase) 9.75 ms with k_pairs (every class, 110 FP64 instructions
 // per pair), 4.61 ms with 81 of them, 3.79 ms without those of a potential of
-// zero parameters and with the shorter exponential; 2048-site water
-// 0.220 -> 0.105 ms.
+// zero parameters and with the shorter exponential, 3.62 ms without the
+// charges' part in a class that has none; 2048-site water 0.220 -> 0.099 ms.
 template <int PT, bool EW>
 __global__ void __launch_bounds__(PAIR_WARPS * 32, 5)
 k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__restrict__ cols,
@@ -1408,7 +1380,8 @@ k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *_
       const double *prow = pot + (size_t)(ti.x & 0xffff) * P.max_id * NPOTP;
       const double4 xi = posc[p];
       const int oi = sortc[p];
-      walk_columns(P, csk, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
+      const bool hp = P.cls_pot >> (p >= n0) & 1, hc = P.cls_chg >> (p >= n0) & 1;
+      walk_columns<false>(P, csk, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
          const int kimg = inf & 31;
          if (j == p && kimg == 13) return;
          const double4 xj = posc[j];
@@ -1428,7 +1401,7 @@ k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *_
 #pragma unroll
          for (int k = 0; k < NP; k++) pp[k] = pj[k];
          double f, u;
-         pair_fu<PT, EW, double, true>(r2, xj.w * xi.w, pp, P.alpha, P.norm, f, u);
+         pair_fu<PT, EW, double, true>(r2, xj.w * xi.w, pp, P.alpha, P.norm, f, u, hp, hc);
          const double wx = f * rx, wy = f * ry, wz = f * rz;
          fx -= wx;
          fy -= wy;
@@ -1900,7 +1873,7 @@ k_pairs_adj_col(RsParams P, AdjParams A, const int *__restrict__ cell_start, con
       }
       const int oi = sorted[p];
       R gqs = 0, gas = 0;
-      walk_columns(P, cell_start, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
+      walk_columns<false>(P, cell_start, cols, col_base, cx, cy, cz, lane, rows, [&](int j, int inf) {
          const int kimg = inf & 31;
          if (j == p && kimg == 13) return;
          const int2 tj = __ldg(&tag[j]);
@@ -2048,6 +2021,15 @@ k_rdf(RsParams P, const int *__restrict__ cell_start, const int *__restrict__ sl
 }
 
 // -------------------------------------------------------------- host side
+// The slots class by class, or one list of every class.
+static void set_one_class(RsParams &P, bool one)
+{
+   P.one_class = one;
+   if (one) {
+      P.cls_pot = P.cls_pot != 0;
+      P.cls_chg = P.cls_chg != 0;
+   }
+}
 static bool col_walk_ok(const mdgpu_ctx *c);
 
 static RsParams make_params(mdgpu_ctx *c)
@@ -2064,6 +2046,16 @@ static RsParams make_params(mdgpu_ctx *c)
    P.rn[0] = 1.0 / g.nx; P.rn[1] = 1.0 / g.ny; P.rn[2] = 1.0 / g.nz;
    P.nfull = (int)g.full.size();
    P.ncols = (int)g.cols.size();
+   P.z0 = g.nz;
+   P.z1 = -g.nz;
+   for (const int4 &cd : g.cols) {
+      P.ex = std::max(P.ex, std::abs(cd.x));
+      P.ey = std::max(P.ey, std::abs(cd.y));
+      P.z0 = std::min(P.z0, cd.z);
+      P.z1 = std::max(P.z1, cd.z + cd.w - 1);
+   }
+   P.cls_pot = c->cls_pot;
+   P.cls_chg = c->cls_chg;
    P.max_id = c->max_id;
    P.molpbc = c->ctl.molpbc;
    P.strict = c->ctl.strict_cutoff;
@@ -2149,6 +2141,15 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
             }
          for (int a = 0; a < M; a++)
             if (pop[a] == 0) c->cls_of_id[a] = 0;
+         // which classes have a potential, and charges, among their sites
+         c->cls_pot = c->cls_chg = 0;
+         for (int a = 0; a < M; a++) {
+            if (pop[a] == 0) continue;
+            if (charged[a]) c->cls_chg |= 1 << c->cls_of_id[a];
+            for (int b = 0; b < M; b++)
+               for (int k = 0; pop[b] > 0 && k < npar; k++)
+                  if (c->potpar[((size_t)a * M + b) * NPOTP + k] != 0.0) c->cls_pot |= 1 << c->cls_of_id[a];
+         }
          std::vector<int> sc(N);
          for (int i = 0; i < N; i++) sc[i] = c->cls_of_id[c->site_id[i]];
          CK(d.site_cls.ensure(N));
@@ -2464,7 +2465,7 @@ static mdgpu_status rs_pairs_col(mdgpu_ctx *c, RsParams P, double *d_force, bool
    cudaStream_t st = c->stream;
    const int N = c->nsites;
    const bool two = c->class_major;
-   P.one_class = !two;
+   set_one_class(P, !two);
    // eight resident blocks per SM (the kernel's launch bounds), each warp
    // looping over home sites: the per-block set-up and energy reduction once
    // per block instead of once per four sites
@@ -2502,7 +2503,7 @@ mdgpu_status rs_count_pairs(mdgpu_ctx *c)
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)
    if (!c->npairs_pending) return MDGPU_OK;
    RsParams P = make_params(c);
-   P.one_class = !c->class_major;
+   set_one_class(P, !c->class_major);
    cudaStream_t st = c->stream;
    DevOut *out = c->out.p;
    CK(cudaMemsetAsync(&out->npairs2, 0, sizeof(out->npairs2), st));
