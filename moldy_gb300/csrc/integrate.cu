@@ -646,7 +646,7 @@ __global__ void __launch_bounds__(256) k_md_virc2(const double *__restrict__ par
    __shared__ double sh[9][8];
    const int t = threadIdx.x;
    double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-   for (int b = t; b < nb; b += 256)
+   for (int b = t; b < nb; b += blockDim.x)
       for (int k = 0; k < 9; k++) v[k] += part[9 * (size_t)b + k];
    md_block_sum(v, sh);
    if (t == 0)
