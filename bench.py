@@ -90,10 +90,8 @@ def measured_peaks():
         return {"hbm_gbs": 6800.0, "bf16": 1900.0, "bf16_sustained": 1700.0, "source": "fallback"}
 
 
-def tc_item_counts(sysm):
-    """Counts of the tensor-core items (runs of up to 64 l values per (h,k)
-    column of the k-list), largest first, padded with empty items to a
-    multiple of 128 -- as the library builds them."""
+def k_columns(sysm):
+    """(h, k, its l values) of every column of the k-list."""
     import math
     h = np.asarray(sysm.h, np.float64).reshape(9)
     kc = sysm.control.k_cutoff
@@ -101,31 +99,49 @@ def tc_item_counts(sysm):
     kmax = int(math.floor(kc / (2 * math.pi) * math.sqrt(h[1] ** 2 + h[4] ** 2)))
     lmax = int(math.floor(kc / (2 * math.pi) * math.sqrt(h[2] ** 2 + h[5] ** 2 + h[8] ** 2)))
     hi = (2 * math.pi * np.linalg.inv(h.reshape(3, 3))).reshape(9)
-    counts = []
     for hh in range(hmax + 1):
         for k in range(0 if hh == 0 else -kmax, kmax + 1):
             kx, ky, kzt = hh * hi[0] + k * hi[3], hh * hi[1] + k * hi[4], hh * hi[2] + k * hi[5]
             ls = np.arange(1 if hh == 0 and k == 0 else -lmax, lmax + 1)
-            n = int(np.count_nonzero((kzt + ls * hi[8]) ** 2 + kx * kx + ky * ky < kc * kc))
-            while n > 0:
-                counts.append(min(n, 64))
-                n -= 64
+            yield hh, k, ls[(kzt + ls * hi[8]) ** 2 + kx * kx + ky * ky < kc * kc]
+
+
+def tc_item_counts(sysm):
+    """Counts of runs of up to 64 l values per (h,k) column of the k-list,
+    largest first, padded with empty ones to a multiple of 128 -- as
+    mdgpu_tc_items lists them."""
+    counts = []
+    for _, _, ls in k_columns(sysm):
+        n = len(ls)
+        while n > 0:
+            counts.append(min(n, 64))
+            n -= 64
     counts = sorted(counts, reverse=True)
     return counts + [0] * (-len(counts) % 128)
 
 
 def tc_mma_flops(sysm, nq):
-    """Tensor-core work the two reciprocal-space kernels issue per launch
-    (bf16 MMA flops, the split-operand term products and the padding of
-    items to 16-column multiples included), from the k-list columns exactly
-    as the library builds them (tc_item_counts): 128 items per
-    structure-factor tile, 32 per force tile."""
-    counts = tc_item_counts(sysm)
-    np32 = (nq + 31) // 32 * 32
-    # per 128-item tile and 16 sites: Ar and Ai times [Zr | Zi], six term products, N = 128
-    sfac = (len(counts) // 128) * (np32 // 16) * 12 * 2 * 128 * 128 * 16
-    force = ((nq + 127) // 128) * sum(12 * ((counts[t] + 15) // 16) * 2 * 128 * 128 * 16
-                                      for t in range(0, len(counts), 32))
+    """Tensor-core work the mixed form's two reciprocal-space kernels issue
+    per launch (MMA flops, padding included).  Units are four (h, |k|) quads
+    with the t = |l| range that covers them; structure factor: 16 units a
+    row tile (256 rows) of each 32-wide t-block, six digit products; force
+    pass: four units an item tile (128 columns) of each 64-wide t-block in
+    order of falling t range, 8 t a K-step, six term products."""
+    tr = {}
+    for hh, k, ls in k_columns(sysm):
+        if len(ls):
+            u = (hh, abs(k) // 4)
+            tr[u] = max(tr.get(u, 0), int(np.abs(ls).max()) + 1)
+    t = sorted(tr.values(), reverse=True)
+    tp = (t[0] + 7) // 8 * 8
+    sfac = force = 0.0
+    for b in range(0, tp, 32):
+        tiles = (sum(x > b for x in t) + 15) // 16
+        sfac += tiles * ((nq + 31) // 32) * 2 * 6 * 2 * 256 * (2 * min(32, tp - b)) * 16
+    for b in range(0, tp, 64):
+        f = [x for x in t if x > b]
+        steps = sum(min((x - b + 7) // 8, 8) for x in f[::4])
+        force += ((nq + 127) // 128) * steps * 6 * 2 * 128 * 128 * 16
     return {"sfac": float(sfac), "kforce": float(force)}
 
 
@@ -468,15 +484,15 @@ def run_gpu(args):
     dom = max(work, key=lambda k: phases.get(k, 0.0))
     achieved = work[dom] / (phases[dom] * 1e-3) / 1e12
     traffic = traffic_from_profiles().get(dom)
-    kernel_names = {"kforce": "k_force_tc", "sfac": "k_sfac_tc", "pairs": "k_pairs_col<LJ,erfc>"}
+    kernel_names = {"kforce": "k_force_tc", "sfac": "k_sfac_q", "pairs": "k_pairs_col<LJ,erfc>"}
     peaks = measured_peaks()
     mma = tc_mma_flops(sysA, n_q)
     if dom in mma:
         # tensor-core kernels: the bound is the bf16 tensor pipe (sustained,
         # as the kernel runs inside a long step); achieved counts the
         # reference's own FP32 operations, the MMA work they expand to (three
-        # bf16 terms per operand, six term products, complex arithmetic as
-        # real products, padded columns) is reported beside it
+        # terms or digits per operand, six products, padded rows and columns)
+        # is reported beside it
         peak, unit, bound = peaks["bf16_sustained"], "TFLOP/s", "tensor"
         peak_source = (f"{peaks['source']} cuBLAS bf16 GEMM throughput, sustained "
                        f"(MEASURED_PEAKS.json bf16_tflops_sustained)")
