@@ -836,11 +836,16 @@ __global__ void k_fsum(int n3, int nsplit, const double *__restrict__ fpart, dou
 // (partials by slot of the charged-site list; the other sites get nothing),
 // times the site's charge when chg is given
 // (and the evaluation's result: every sum is complete here)
-__global__ void k_fsum_slots(int n, int N, int nsplit, const double *__restrict__ fpart,
-                             const int *__restrict__ slots, const double *__restrict__ chg, double *__restrict__ force,
+// Grid y: the groups of sites (a framework's after the others).
+__global__ void k_fsum_slots(int na, int nb, int N, int nsplit, const double *__restrict__ fparta,
+                             const double *__restrict__ fpartb, const int *__restrict__ slotsa,
+                             const int *__restrict__ slotsb, const double *__restrict__ chg, double *__restrict__ force,
                              FinArgs fin, DevOut *out)
 {
-   if (fin.on && blockIdx.x == 0 && threadIdx.x == blockDim.x - 1) finalize_eval(out, fin);
+   if (fin.on && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == blockDim.x - 1) finalize_eval(out, fin);
+   const int n = blockIdx.y ? nb : na;
+   const double *__restrict__ fpart = blockIdx.y ? fpartb : fparta;
+   const int *__restrict__ slots = blockIdx.y ? slotsb : slotsa;
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
    if (i >= 3 * n) return;
    const int comp = i / n, j = i - comp * n;
@@ -1188,22 +1193,21 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
       sh.splits = ks_force_tc_splits(d);
       int np = 0;
       for (int i = 0; i < d.q_nfblk; i++) np = std::max(np, d.q_fblk[i + 1] - d.q_fblk[i]);
-      CK(d.utab.ensure(ks_tc_utab_len(np)));
-      CK(d.tc_coef.ensure((size_t)np * 8));
-      if (nfc) CK(d.fpartf.ensure((size_t)sh.splits * 3 * nfc));
+      const int ngrp = nfc ? 2 : 1;
+      CK(d.utab.ensure(ngrp * ks_tc_utab_len(np)));
+      CK(d.tc_coef.ensure((size_t)ngrp * np * 8));
    }
-   if (!tc || mixed) CK(d.fpart.ensure((size_t)sh.splits * 3 * Nk));
+   if (!tc || mixed) CK(d.fpart.ensure((size_t)sh.splits * 3 * (Nk + nfc)));   // (the framework's after the others')
+   double *const fpart2 = d.fpart.p + (size_t)sh.splits * 3 * Nk;
    phase_mark(c, MDGPU_PH_KFORCE);
    dim3 gf((Nk + 255) / 256, sh.splits);
    const int obase = compact ? -1 : 0;   // partial rows by slot of the charged list, or by site
    if (tc && mixed) {
-      int nl = 0;
-      for (int f = 0; f < 2 && nl >= 0; f++)
-         if (f ? nfc : Nk) {
-            const int k = ks_force_tc(st, f ? nfc : Nk, f ? f0 : 0, kl.q.g, d, f ? d.q_abf32.p : d.q_ab32.p, false, c->nsm,
-                                      f ? d.fpartf.p : d.fpart.p, &out->err);
-            nl = k < 0 ? -1 : nl + k;
-         }
+      KsForceSites grp[2];
+      int ng = 0;
+      if (Nk) grp[ng++] = KsForceSites{Nk, 0, d.q_ab32.p, d.fpart.p};
+      if (nfc) grp[ng++] = KsForceSites{nfc, f0, d.q_abf32.p, fpart2};
+      const int nl = ks_force_tc(st, grp, ng, kl.q.g, d, false, c->nsm, &out->err);
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl - 1;
    } else if (tc) {
@@ -1222,18 +1226,17 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    if (join) CK(cudaStreamWaitEvent(st, join, 0));
    if (compact || tc) {
       if (!accumulate) CK(cudaMemsetAsync(d_force, 0, 3 * (size_t)N * sizeof(double), st));
-      for (int f = 0; f < 2; f++) {
-         const int n = f ? nfc : Nk;
-         if (n == 0) continue;
-         FinArgs fin = c->fin;
-         fin.on = fin.on && (f || !nfc);   // by the last of them
-         if (tc && !mixed) {
+      if (tc && !mixed) {
+         for (int f = 0; f < 2; f++) {
+            const int n = f ? nfc : Nk;
+            if (n == 0) continue;
+            FinArgs fin = c->fin;
+            fin.on = fin.on && (f || !nfc);   // by the last of them
             if ((s = ks_q_fsum64(c, n, f ? f0 : 0, slots, d_force, fin)) != MDGPU_OK) return s;
-         } else {
-            k_fsum_slots<<<(3 * n + 255) / 256, 256, 0, st>>>(n, N, sh.splits, f ? d.fpartf.p : d.fpart.p,
-                                                              slots + (f ? f0 : 0), tc ? c->rd.chg.p : nullptr, d_force,
-                                                              fin, out);
          }
+      } else {
+         k_fsum_slots<<<dim3((3 * std::max(Nk, nfc) + 255) / 256, nfc ? 2 : 1), 256, 0, st>>>(
+            Nk, nfc, N, sh.splits, d.fpart.p, fpart2, slots, slots + f0, tc ? c->rd.chg.p : nullptr, d_force, c->fin, out);
       }
       c->fin.on = 0;
    } else {

@@ -1654,7 +1654,8 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
          qs * std::ldexp(1.0 / k4, -30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
       const int sp = ks_force_tc_splits(d);
       CK(a.gkpart.ensure((size_t)sp * 3 * N));
-      const int nl = ks_force_tc(st, N, 0, g, d, a.ab32.p, true, c->nsm, a.gkpart.p, &c->out.p->err);
+      const KsForceSites grp{N, 0, a.ab32.p, a.gkpart.p};
+      const int nl = ks_force_tc(st, &grp, 1, g, d, true, c->nsm, &c->out.p->err);
       if (nl < 0) return fail(c, MDGPU_E_NOMEM, "device allocation failed (force-pass work ranges)");
       c->launches += nl;
       k_qadj_site<true, float4><<<(N + 255) / 256, 256, 0, st>>>(N, sp, g, d.fpart.p, a.gkpart.p, a.res32.p,

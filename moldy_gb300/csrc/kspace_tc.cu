@@ -64,9 +64,68 @@ constexpr int FTC_XBYTES = 2 * FTC_EG * 128 * 3 * 4 + FTC_EW * FTC_IPW * 16;   /
 // 0.346 ms at 208 KB, 0.377 ms with a third coefficient stage, 226 KB).
 __host__ __device__ constexpr int ftc_smem(int aterm) { return 3 * aterm + 2 * FTC_NSB * FTC_SBYTES + FTC_XBYTES; }
 constexpr int FTC_THREADS = 32 * (FTC_EW + 3);     // epilogue warps, a bulk-copy warp, two MMA warps
+__host__ __device__ constexpr size_t ftc_utab_len(int nitems) { return (size_t)(nitems / FTC_NI) * 8 * (FTC_BBYTES / 16); }
 static_assert(FTC_IPW % 4 == 0, "an epilogue warp reads its items' columns 16 at a time");
 constexpr int FTC_SPLITS = 2;                      // force slots per site (two CTAs at most per site tile)
 constexpr int FTC_ERR = 16;                        // error-word bit: a force-pass wait expired
+
+// A launch takes one or two groups of sites (grid y): all, or with a framework
+// molecule the others and the framework's charged sites, each with its own
+// coefficients.  On a small system a launch of its own costs each kernel as
+// much as its work (water on a charged wall, 1044 sites: an evaluation 144 us
+// with launches for each, 125 us so).
+struct FtcRanges {          // a group's work ranges
+   int build, tiles, G;     // to be made; site tiles, ranges
+   int *ustart;
+};
+struct FtcSecond {          // the second group: sites, ranges, and its data from the first's on
+   int n, G;
+   const int *ustart;
+   size_t x, y, z, fpart;
+};
+
+// K-steps (8 t each) of an item tile in the t-block from t0: its first unit's
+// t range is the longest (units in order of falling range)
+__device__ __forceinline__ int ftc_ksteps(int4 un, int t0)
+{
+   return un.w < 0 ? 0 : min(max(un.z - t0 + 7, 0) >> 3, 8);
+}
+
+// Work ranges of the persistent force pass.  Unit u is (site tile u / ntl,
+// item tile u % ntl); CTA c takes units ustart[c] .. ustart[c + 1] - 1, a
+// contiguous run over the site tiles.  The runs split the units' weights
+// (an item tile's K-steps plus one for its epilogue) evenly over G CTAs,
+// with G <= the number of site tiles (or G = twice that, each CTA then half
+// a tile), so no run lies strictly inside a site tile and a tile is shared
+// by two CTAs at most.  One block; pre (after ustart[G]) holds the prefix
+// weights of the item tiles.
+__device__ __forceinline__ void ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *ustart)
+{
+   int *pre = ustart + G + 1;
+   if (threadIdx.x == 0) {
+      int sum = 0;
+      pre[0] = 0;
+      for (int t = 0; t < ntl; t++) {
+         sum += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
+         pre[t + 1] = sum;
+      }
+   }
+   __syncthreads();
+   const long long wt = pre[ntl], wall = wt * nsite_tiles;
+   for (int c = threadIdx.x; c <= G; c += blockDim.x) {
+      const long long target = (long long)c * wall / G;
+      const long long tile = target / wt, rem = target - tile * wt;
+      int lo = 0, hi = ntl;   // the first item tile whose prefix weight reaches rem
+      while (lo < hi) {
+         const int mid = (lo + hi) >> 1;
+         if (pre[mid] >= rem)
+            hi = mid;
+         else
+            lo = mid + 1;
+      }
+      ustart[c] = (int)(tile * ntl + lo);
+   }
+}
 
 // Coefficient rows of each item from the dense per-(quad, t) A and B
 // (k_qreduce): one warp per item, 64 t from t0.  Item 8 j + 2 q + s is quad
@@ -74,12 +133,24 @@ constexpr int FTC_ERR = 16;                        // error-word bit: a force-pa
 // [cosines, sines][row group 16][8 rows][8 t] bf16, row 8 q + 2 c + s for
 // the items (q, s) of the tile: the two signs of k side by side, as the
 // epilogue takes them in paired FP32 instructions; the force coefficients
-// likewise, per q (x+ x- y+ y-), (z0+ z0- dz+ dz-).
+// likewise, per q (x+ x- y+ y-), (z0+ z0- dz+ dz-).  The block after the last
+// makes the group's work ranges (a cell that changes every step needs them
+// every step: a launch of their own took 3-4 us).
 __global__ void __launch_bounds__(256)
 k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, const float4 *__restrict__ ab,
-          uint4 *__restrict__ utab, float *__restrict__ coef)
+          const float4 *__restrict__ ab2, uint4 *__restrict__ utab, float *__restrict__ coef, FtcRanges ra, FtcRanges rb)
 {
    __shared__ float4 sv[8][64];
+   if (blockIdx.x == gridDim.x - 1) {   // (uniform)
+      const FtcRanges r = blockIdx.y ? rb : ra;
+      if (r.build) ftc_ranges(fu, t0, nitems / FTC_NI, r.tiles, r.G, r.ustart);
+      return;
+   }
+   if (blockIdx.y) {
+      ab = ab2;
+      utab += ftc_utab_len(nitems);
+      coef += (size_t)nitems * 4;
+   }
    const int wl = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int i = blockIdx.x * 8 + wl;
    if (i >= nitems) return;   // (warp-uniform)
@@ -160,50 +231,7 @@ __device__ __forceinline__ void kahan_add_tc(float &s, float &c, float x)
    s = t;
 }
 
-// K-steps (8 t each) of an item tile in the t-block from t0: its first unit's
-// t range is the longest (units in order of falling range)
-__device__ __forceinline__ int ftc_ksteps(int4 un, int t0)
-{
-   return un.w < 0 ? 0 : min(max(un.z - t0 + 7, 0) >> 3, 8);
-}
-
-// Work ranges of the persistent force pass.  Unit u is (site tile u / ntl,
-// item tile u % ntl); CTA c takes units ustart[c] .. ustart[c + 1] - 1, a
-// contiguous run over the site tiles.  The runs split the units' weights
-// (an item tile's K-steps plus one for its epilogue) evenly over G CTAs,
-// with G <= the number of site tiles (or G = twice that, each CTA then half
-// a tile), so no run lies strictly inside a site tile and a tile is shared
-// by two CTAs at most.  One block; pre (after ustart[G]) holds the prefix
-// weights of the item tiles.
-__global__ void k_ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *__restrict__ ustart)
-{
-   int *pre = ustart + G + 1;
-   if (threadIdx.x == 0) {
-      int sum = 0;
-      pre[0] = 0;
-      for (int t = 0; t < ntl; t++) {
-         sum += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
-         pre[t + 1] = sum;
-      }
-   }
-   __syncthreads();
-   const long long wt = pre[ntl], wall = wt * nsite_tiles;
-   for (int c = threadIdx.x; c <= G; c += blockDim.x) {
-      const long long target = (long long)c * wall / G;
-      const long long tile = target / wt, rem = target - tile * wt;
-      int lo = 0, hi = ntl;   // the first item tile whose prefix weight reaches rem
-      while (lo < hi) {
-         const int mid = (lo + hi) >> 1;
-         if (pre[mid] >= rem)
-            hi = mid;
-         else
-            lo = mid + 1;
-      }
-      ustart[c] = (int)(tile * ntl + lo);
-   }
-}
-
-// Persistent: one CTA per work range (k_ftc_ranges).  Per site tile of the
+// Persistent: one CTA per work range (ftc_ranges).  Per site tile of the
 // range the CTA loads its z tables once (after the MMAs of the previous tile
 // have completed) and runs its item tiles as before; the epilogue writes the
 // tile's forces into slot 0 of fpart, or slot 1 when the range starts inside
@@ -211,7 +239,8 @@ __global__ void k_ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int n
 __global__ void __launch_bounds__(FTC_THREADS, 1)
 k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef, int nitems, int t0,
            const int *__restrict__ X, const int *__restrict__ Y, const uint4 *__restrict__ zsite,
-           const uint4 *__restrict__ utab, int n, const int *__restrict__ ustart, double *__restrict__ fpart, int *__restrict__ err)
+           const uint4 *__restrict__ utab, int n, int G, const int *__restrict__ ustart, double *__restrict__ fpart,
+           FtcSecond s2, int *__restrict__ err)
 {
    using namespace tc;
    extern __shared__ __align__(1024) unsigned char sm[];
@@ -222,6 +251,18 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    __shared__ int abort_s;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
    const int ntl = nitems / FTC_NI;   // item tiles per site tile
+   if (blockIdx.y) {
+      n = s2.n;
+      G = s2.G;
+      ustart = s2.ustart;
+      X += s2.x;
+      Y += s2.y;
+      zsite += s2.z;
+      fpart += s2.fpart;
+      utab += ftc_utab_len(nitems);
+      coef += nitems;
+   }
+   if ((int)blockIdx.x >= G) return;   // (uniform)
    const int u0 = ustart[blockIdx.x], u1 = ustart[blockIdx.x + 1];
    if (u1 <= u0) return;              // an empty range (uniform)
    const int T0 = u0 / ntl, T1 = (u1 - 1) / ntl;
@@ -499,42 +540,51 @@ k_force_tc(QGeom g, const int4 *__restrict__ fu, const float4 *__restrict__ coef
    }
 }
 
-// The force pass of one t-block, sites from slot f0 on (its units fu0 .. fu0 + npos - 1 of the
-// list, a multiple of four) into slots 0 and 1 of fpart; returns the
-// launches, -1 if out of memory.
-static int force_tc_block(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int blk,
-                          int fu0, int npos, int nsm, double *fpart, int *err)
+// The force pass of one t-block (its units fu0 .. fu0 + npos - 1 of the
+// list, a multiple of four) into slots 0 and 1 of each group's fpart (one
+// buffer, the second group's after the first's); returns
+// the launches, -1 if out of memory.
+static int force_tc_block(cudaStream_t st, const KsForceSites *grp, int ngrp, const QGeom &g, KsDev &d, bool scalar, int blk,
+                          int fu0, int npos, int nsm, int *err)
 {
-   const int T = (nsites + 127) / 128, ntl = npos * 8 / FTC_NI, t0 = 64 * blk;
-   const int G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
+   const int ntl = npos * 8 / FTC_NI, t0 = 64 * blk;
    const int4 *fu = d.q_fu.p + fu0;
-   const int f = f0 > 0;
-   k_utab_tc<<<npos, 256, 0, st>>>(npos * 8, g, t0, scalar ? 1 : 0, fu, reinterpret_cast<const float4 *>(ab), d.utab.p,
-                                   reinterpret_cast<float *>(d.tc_coef.p));
-   int launches = 2;
-   if (blk > 0 || d.tc_rkey[f][0] != T || d.tc_rkey[f][1] != ntl || d.tc_rkey[f][2] != G || d.tc_rver[f] != d.tc_ver) {
-      if (d.tc_ustart[f].ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
-      k_ftc_ranges<<<1, 256, 0, st>>>(fu, t0, ntl, T, G, d.tc_ustart[f].p);
-      d.tc_rkey[f][0] = T;
-      d.tc_rkey[f][1] = ntl;
-      d.tc_rkey[f][2] = G;
-      d.tc_rver[f] = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
-      launches++;
+   FtcRanges r[2] = {};
+   for (int k = 0; k < ngrp; k++) {
+      const int f = grp[k].f0 > 0, T = (grp[k].n + 127) / 128, G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
+      int *key = d.tc_rkey[f];
+      if (blk > 0 || key[0] != T || key[1] != ntl || key[2] != G || d.tc_rver[f] != d.tc_ver) {
+         if (d.tc_ustart[f].ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
+         r[k].build = 1;
+         key[0] = T;
+         key[1] = ntl;
+         key[2] = G;
+         d.tc_rver[f] = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
+      }
+      r[k].tiles = T;
+      r[k].G = G;
+      r[k].ustart = d.tc_ustart[f].p;
    }
-   k_force_tc<<<G, FTC_THREADS, ftc_smem(256 * std::min(128, 2 * (g.TP - t0))), st>>>(g, fu, d.tc_coef.p, npos * 8, t0,
-                                                d.q_x32.p + (size_t)f0 / 32 * 2 * g.hrows * 36, d.q_y32.p + (size_t)f0 / 32 * 2 * g.mrows * 36,
-                                                d.zsite.p + (size_t)f0 / 128 * 2 * g.TP * 48,
-                                                d.utab.p, nsites, d.tc_ustart[f].p, fpart, err);
-   return launches;
+   auto xat = [&](int k) { return (size_t)grp[k].f0 / 32 * 2 * g.hrows * 36; };
+   auto yat = [&](int k) { return (size_t)grp[k].f0 / 32 * 2 * g.mrows * 36; };
+   auto zat = [&](int k) { return (size_t)grp[k].f0 / 128 * 2 * g.TP * 48; };
+   auto fat = [&](int k) { return grp[k].fpart + (size_t)blk * FTC_SPLITS * 3 * grp[k].n; };
+   FtcSecond s2 = {};
+   if (ngrp > 1) s2 = FtcSecond{grp[1].n, r[1].G, r[1].ustart, xat(1) - xat(0), yat(1) - yat(0), zat(1) - zat(0), (size_t)(fat(1) - fat(0))};
+   k_utab_tc<<<dim3(npos + 1, ngrp), 256, 0, st>>>(
+      npos * 8, g, t0, scalar ? 1 : 0, fu, reinterpret_cast<const float4 *>(grp[0].ab),
+      reinterpret_cast<const float4 *>(ngrp > 1 ? grp[1].ab : nullptr), d.utab.p, reinterpret_cast<float *>(d.tc_coef.p), r[0], r[1]);
+   k_force_tc<<<dim3(std::max(r[0].G, r[1].G), ngrp), FTC_THREADS, ftc_smem(256 * std::min(128, 2 * (g.TP - t0))), st>>>(
+      g, fu, d.tc_coef.p, npos * 8, t0, d.q_x32.p + xat(0), d.q_y32.p + yat(0), d.zsite.p + zat(0), d.utab.p, grp[0].n, r[0].G,
+      r[0].ustart, fat(0), s2, err);
+   return 2;
 }
 
-int ks_force_tc(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
-                double *fpart, int *err)
+int ks_force_tc(cudaStream_t st, const KsForceSites *grp, int ngrp, const QGeom &g, KsDev &d, bool scalar, int nsm, int *err)
 {
    int launches = 0;
    for (int b = 0; b < d.q_nfblk; b++) {
-      const int nl = force_tc_block(st, nsites, f0, g, d, ab, scalar, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm,
-                                    fpart + (size_t)b * FTC_SPLITS * 3 * nsites, err);
+      const int nl = force_tc_block(st, grp, ngrp, g, d, scalar, b, d.q_fblk[b], d.q_fblk[b + 1] - d.q_fblk[b], nsm, err);
       if (nl < 0) return -1;
       launches += nl;
    }
@@ -542,7 +592,7 @@ int ks_force_tc(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, c
 }
 
 int ks_force_tc_splits(const KsDev &d) { return FTC_SPLITS * d.q_nfblk; }
-size_t ks_tc_utab_len(int npos) { return (size_t)((npos + 3) / 4) * 8 * (FTC_BBYTES / 16); }
+size_t ks_tc_utab_len(int npos) { return ftc_utab_len((npos + 3) / 4 * FTC_NI); }
 
 cudaError_t ks_force_tc_init()
 {

@@ -312,7 +312,7 @@ struct KsDev {
    DBuf<uint4> zsite;      // force pass: z tables as the A operand, per 128 sites
    DBuf<uint4> utab;       // force pass: per-item coefficient rows (B operand)
    DBuf<float4> tc_coef;   // per item: kx s1, ky s1, kz0 s1, dkz s2 (row scales s)
-   DBuf<int> tc_ustart[2]; // force pass: the CTAs' work ranges (k_ftc_ranges), of the framework's sites
+   DBuf<int> tc_ustart[2]; // force pass: the CTAs' work ranges (ftc_ranges), of the framework's sites
    long long tc_ver = 0;   // uploads of the quad list so far
    int tc_rkey[2][3] = {{-1, -1, -1}, {-1, -1, -1}};   // (site tiles, item tiles, CTAs) of tc_ustart
    long long tc_rver[2] = {-1, -1};                    // tc_ver of tc_ustart
@@ -541,8 +541,14 @@ mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw);
 // sites from slot f0 (zero or the framework's first) on
 mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0);
 mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, int f0, const int *slots, double *d_force, const FinArgs &fin);
-int ks_force_tc(cudaStream_t st, int nsites, int f0, const QGeom &g, KsDev &d, const float *ab, bool scalar, int nsm,
-                double *fpart, int *err);
+// a group of sites of the mixed force pass: n from slot f0 on, their A and B
+// per (quad, t), their force sums
+struct KsForceSites {
+   int n, f0;
+   const float *ab;
+   double *fpart;
+};
+int ks_force_tc(cudaStream_t st, const KsForceSites *grp, int ngrp, const QGeom &g, KsDev &d, bool scalar, int nsm, int *err);
 mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq, int *nblocks);
 int ks_force_tc_splits(const KsDev &d);
 size_t ks_tc_utab_len(int npos);
