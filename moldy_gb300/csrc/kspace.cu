@@ -1,5 +1,8 @@
 // Reciprocal-space Ewald sum on the GPU (the work of ewald(),
-// src/ewald.c:280-589).
+// src/ewald.c:280-589): the order of the passes (ks_launch) and the CUDA-core
+// passes, which run for the adjoint with a framework molecule and with
+// MDGPU_KSPACE_TC=0; the tensor-core passes are in kspace_q.cu and
+// kspace_tc.cu.
 //
 // Phases.  With s = h^-1 r the fractional co-ordinate of a site, the phase of
 // k-vector (h,k,l) is k.r = 2 pi (h s_x + k s_y + l s_z) (the reference's

@@ -5,17 +5,22 @@
 //   1. k_bin        FP64 binning of every site (or molecule centre of mass in
 //                   molecular-cutoff mode) with the reference's arithmetic and
 //                   edge fix-ups (cellbin, src/force.c:119-137);
-//   2. scan         cell counts -> cell starts (3-kernel block scan);
-//   3. k_scatter +  sites placed cell by cell, then each cell's members put
-//      k_cellsort   in ascending site order (deterministic layout);
-//   4. k_gather     per-slot records: FP64 (x,y,z,q), or FP32 co-ordinates
-//                   relative to the cell origin plus q, and (site id, molecule);
-//   5. k_pairs      one warp per site walks the full neighbour-cell stencil
-//                   (the reference's half-space list and its mirror) and
-//                   evaluates every candidate pair the reference evaluates,
-//                   accumulating the force on its own site only; energy and
-//                   virial take half of each evaluation.  No atomics on forces.
-//   6. k_reduce_rs  per-block energy/virial partials summed in fixed order.
+//   2. scan         cell counts -> cell starts (in k_bin's last block on small
+//                   grids, else two kernels);
+//   3. k_scatter    sites placed cell by cell (in k_bin's last block on small
+//                   systems);
+//   4. k_place      each cell's members in ascending site order (deterministic
+//                   layout) and per-slot records: FP64 (x,y,z,q), or FP32
+//                   co-ordinates relative to the cell origin plus q, and (site
+//                   id, molecule);
+//   5. k_pairs_col  one warp per home site walks the stencil by columns over
+//      k_pairs_col64  one interaction class at a time, accumulating the force
+//                   on its own site only; energy and virial take half of each
+//                   evaluation, summed in a fixed order by the last block.  No
+//                   atomics on forces.  k_pairs and k_reduce_rs walk it cell
+//                   by cell with frameworks, molecular cut-offs, the pair-key
+//                   listing and stencils that wrap the cell more than once;
+//   6. k_tooclose_x pairs across the classes below the too-close distance.
 //
 // The pair set is the reference's exactly: every site pair of a cell and of
 // each stencil cell, with no per-pair cutoff in lazy mode and r^2 clamped to
