@@ -1048,13 +1048,24 @@ struct ColHome {
       p = ((it / chunk) * (int)gridDim.x + (int)blockIdx.x) * chunk + it % chunk + w;
    }
 };
-// Chunks of 16 (neighbouring sites share candidates and column starts in
-// L1), shorter where the grid then had blocks without a site: 500-site argon
-// in FP64 57 us with 16 against 18 us with 4.
+// Sites per chunk: of 16, 12, 8 and 4 the one with which the busiest block
+// has the fewest sites, the largest of equals (neighbouring sites share
+// candidates and column starts in L1): with fewer blocks than chunks of 16 a
+// second round of few blocks was a tail (16,384-site water, mixed, 24 sites in
+// place of 16: 63 -> 61 us, 92 -> 83 us in link order; 32,768 ions 88 -> 82
+// us), and blocks without a site idle (500-site argon in FP64 57 us with 16,
+// 18 us with 4).
 static int col_chunk(int N, int nblk)
 {
-   const int per = (N + nblk - 1) / nblk;
-   return std::max(PAIR_WARPS, std::min(COL_CHUNK, per / PAIR_WARPS * PAIR_WARPS));
+   int best = COL_CHUNK, most = 1 << 30;
+   for (int ch = COL_CHUNK; ch >= PAIR_WARPS; ch -= PAIR_WARPS) {
+      const int chunks = (N + ch - 1) / ch, m = (chunks + nblk - 1) / nblk * ch;
+      if (m < most) {
+         most = m;
+         best = ch;
+      }
+   }
+   return best;
 }
 
 // A column offset's hi and lo parts (32 bytes, 32-byte aligned) in one load.
@@ -1826,11 +1837,11 @@ k_pairs_adj(RsParams P, AdjParams A, const int *__restrict__ cell_start,
 // shared memory (a column of its own: no conflicts), and only the gradient
 // asked for (LOSS: of G, else of the energy).  FP64 form: the cheaper
 // primitives of PairMath<double, true>.  One walk instead of one per
-// identifier: 16,384-site water, mixed, 458 -> 137 us; 2048 sites, FP64,
-// 735 -> 250 us.  Dynamic shared memory: slot sums
+// identifier: 16,384-site water, mixed, 458 -> 137 us (92 with eight blocks per
+// SM); 2048 sites, FP64, 735 -> 190 us.  Dynamic shared memory: slot sums
 // [nslot] FP64, lane sums [types NP][threads], the potential table.
 template <int PT, bool EW, bool MIXED, bool LOSS>
-__global__ void __launch_bounds__(PAIR_WARPS * 32, MIXED ? 6 : 4)
+__global__ void __launch_bounds__(PAIR_WARPS * 32, MIXED ? 8 : 4)
 k_pairs_adj_col(RsParams P, AdjParams A, const int *__restrict__ cell_start, const int *__restrict__ slot_cell,
                 const int4 *__restrict__ cols, const int *__restrict__ col_base, const float4 *__restrict__ coff,
                 const double4 *__restrict__ pos64, const float4 *__restrict__ pos32, const int2 *__restrict__ tag,
@@ -2308,8 +2319,15 @@ mdgpu_status rs_adjoint(mdgpu_ctx *c, bool loss)
    A.nslot = 2 * c->max_id * c->max_id * np + 2;
    A.ntype = 0;
    for (int b = 0; b < MDGPU_ADJ_MAX_ID; b++) A.type_index[b] = (unsigned char)((A.type_mask >> b) & 1u ? A.ntype++ : 0);
-   int nblk = (N + PAIR_WARPS - 1) / PAIR_WARPS;
-   if (nblk > 4 * 152) nblk = 4 * 152;
+   // as many blocks as are resident: the kernel's launch bounds, or what its
+   // shared memory (with many identifiers) leaves room for (the walk waits for
+   // its gathers: 16,384-site water, mixed, 134 us with four blocks per SM, 92
+   // us with eight)
+   const size_t smem = (size_t)A.nslot * sizeof(double) + 20 * 1024 +
+                       ((size_t)A.ntype * np * PAIR_WARPS * 32 + (size_t)c->max_id * c->max_id * NPOTP) *
+                          (mixed ? sizeof(float) : sizeof(double));
+   const int per_sm = std::max(1, std::min(mixed ? 8 : 4, (int)(227 * 1024 / smem)));
+   const int nblk = std::min((N + PAIR_WARPS - 1) / PAIR_WARPS, per_sm * 152);
    P.chunk = col_chunk(N, nblk);
    CK(a.gq.ensure(2 * (size_t)N));
    CK(a.gpart.ensure((size_t)nblk * A.nslot));
