@@ -1394,7 +1394,7 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    if (q.ns == ns || c->kl.nk == 0) return MDGPU_OK;
    build_qlist(c->kl, ns);
    TablePack &k = d.q_lists;
-   k.begin();
+   CK(k.begin());
    const size_t o[5] = {k.add(q.units), k.add(q.coeff), k.add(q.tiles), k.add(q.segs), k.add(q.fu)};
    CK(k.send(c->stream));
    k.at(d.q_units.p, o[0]);

@@ -166,12 +166,29 @@ struct DBuf {
 // Host tables that change together (with the cell shape, every step of a
 // constant-pressure run), gathered here and sent in one copy: a copy costs the
 // host 3 to 5 us to issue whatever its size, and waiting for it a round trip.
-// (The source is ordinary memory, which the driver has read when the call
-// returns.)
+// The source may be read after send() returns (a GPU that reads pageable
+// memory in place need not stage it), so begin() waits for the copy before it
+// is rewritten: done long before, where an evaluation lies between.
 struct TablePack {
    std::vector<unsigned char> h;
    DBuf<unsigned char> d;
-   void begin() { h.clear(); }
+   cudaEvent_t sent = nullptr;
+   TablePack() = default;
+   TablePack(const TablePack &) = delete;
+   TablePack &operator=(const TablePack &) = delete;
+   ~TablePack()
+   {
+      if (sent) {
+         cudaEventSynchronize(sent);
+         cudaEventDestroy(sent);
+      }
+   }
+   cudaError_t begin()
+   {
+      const cudaError_t e = sent ? cudaEventSynchronize(sent) : cudaEventCreateWithFlags(&sent, cudaEventDisableTiming);
+      if (e == cudaSuccess) h.clear();
+      return e;
+   }
    template <typename T> size_t add(const std::vector<T> &v)   // its offset
    {
       const size_t o = (h.size() + 255) & ~(size_t)255;
@@ -181,9 +198,13 @@ struct TablePack {
    }
    cudaError_t send(cudaStream_t st)
    {
-      cudaError_t e = d.ensure(h.size());
+      // a capture would keep reading h when replayed: refused, as a wait would be
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      cudaError_t e = cudaStreamIsCapturing(st, &cap);
+      if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+      if (e == cudaSuccess) e = d.ensure(h.size());
       if (e == cudaSuccess && !h.empty()) e = cudaMemcpyAsync(d.p, h.data(), h.size(), cudaMemcpyHostToDevice, st);
-      return e;
+      return e == cudaSuccess ? cudaEventRecord(sent, st) : e;
    }
    template <typename T> void at(T *&p, size_t o) const { p = reinterpret_cast<T *>(d.p + o); }
 };

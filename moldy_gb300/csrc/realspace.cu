@@ -2195,7 +2195,7 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
          coff[2 * e + 1] = g.coff_lo[e];
       }
       TablePack &k = d.geom;
-      k.begin();
+      CK(k.begin());
       const size_t o[6] = {k.add(g.full), k.add(g.off_hi), k.add(g.off_lo), k.add(g.cols), k.add(g.col_base), k.add(coff)};
       CK(k.send(st));
       k.at(d.full.p, o[0]);
