@@ -1189,6 +1189,7 @@ static mdgpu_status md_capture(mdgpu_ctx *c, const MdStepParams &P, int cap, dou
    H.graph_launches = c->launches - l0;
    c->launches = l0;
    H.graph_gen = c->gen;
+   H.graph_moves = c->moves.n;
    return MDGPU_OK;
 }
 
@@ -1214,11 +1215,7 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
    MdStepParams P;
    step_params(c, P);
    const int cap = nsteps > 0 ? nsteps : 1;
-   if (D.energies.n < 4 * (size_t)cap) {
-      // a larger record buffer moves the pointer a captured step holds
-      CK(D.energies.ensure(4 * (size_t)cap));
-      H.graph_gen = 0;
-   }
+   CK(D.energies.ensure(4 * (size_t)cap));
    CK(c->small.ensure(16));
    const int nrec = records && nsteps >= first ? (nsteps - first) / interval + 1 : 0;
    int batch = 0;
@@ -1246,9 +1243,12 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
       // a step runs directly until one has run since the configuration last
       // changed (every buffer is then allocated); later ones replay a
       // captured step (a step whose record needs the virial correction also
-      // runs directly)
+      // runs directly).  Other evaluations of the context in between may
+      // have moved buffers (a gradient runs over more sites, another cell
+      // has larger tables): the step is captured again then.  One that failed
+      // may have left cell counts behind: the direct step clears them.
       const bool virc = dump && (level & 8);
-      const bool replay = (i > 0 || H.warm_gen == c->gen) && !c->timing && !virc && !H.baro;
+      const bool replay = (i > 0 || H.warm_gen == c->gen) && c->counts_clean && !c->timing && !virc && !H.baro;
       if (H.baro) {
          // constant pressure: every step direct, h and the tables change
          if ((s = md_baro_step(c, cap)) != MDGPU_OK) return s;
@@ -1257,7 +1257,7 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
          dist_v = H.dist / v;
          distp_v = H.distp / v;
          c->gen++;
-      } else if (replay && (!H.graph || H.graph_gen != c->gen || H.graph_cap != cap)) {
+      } else if (replay && (!H.graph || H.graph_gen != c->gen || H.graph_moves != c->moves.n || H.graph_cap != cap)) {
          if ((s = md_capture(c, P, cap, dist_v)) != MDGPU_OK) return s;
          H.graph_cap = cap;
       }

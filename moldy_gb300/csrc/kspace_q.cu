@@ -975,9 +975,12 @@ k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *
    }
 }
 
-// Grid: (site tiles of 128, sets, items).  hpart[item][set][n].
+// Grid: (site tiles of 128, sets, runs of up to per segments of one t-block).
+// hpart[run][set][n].  The run is found from the t-blocks' first segments
+// (seg0) here: a list of runs kept on the device would be another call's by
+// the time a captured evaluation is replayed.
 __global__ void __launch_bounds__(Q_THREADS, 1)
-k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restrict__ items,
+k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restrict__ seg0, int per,
           const int4 *__restrict__ units, const long long *__restrict__ X, const long long *__restrict__ Y,
           const double *__restrict__ zd, const unsigned char *__restrict__ bq, const int *__restrict__ bexp, int n,
           double *__restrict__ hpart, int *__restrict__ err)
@@ -993,9 +996,19 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const QItem *__restr
    unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
    const int tile = blockIdx.x, set = blockIdx.y;
-   const QItem it = items[blockIdx.z];
-   const int nst = (it.seg1 - it.seg0) * SEG;
-   const int blk = segs[it.seg0].blk, nT = q_blkcols(g, blk);
+   struct {
+      int seg0, seg1;
+   } it;
+   int blk = 0, run = blockIdx.z;
+   for (; blk < g.nblk - 1; blk++) {
+      const int nr = (seg0[blk + 1] - seg0[blk] + per - 1) / per;
+      if (run < nr) break;
+      run -= nr;
+   }
+   it.seg0 = seg0[blk] + run * per;
+   it.seg1 = min(it.seg0 + per, seg0[blk + 1]);
+   const int nst = (it.seg1 - it.seg0) * SEG, nT = q_blkcols(g, blk);
+   if (nst <= 0) return;   // (uniform; the grid has no such run)
    if (tid == 0) {
       q_init(B);
       abort_s = 0;
@@ -1395,16 +1408,16 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    build_qlist(c->kl, ns);
    TablePack &k = d.q_lists;
    CK(k.begin());
-   const size_t o[5] = {k.add(q.units), k.add(q.coeff), k.add(q.tiles), k.add(q.segs), k.add(q.fu)};
+   const size_t o[6] = {k.add(q.units), k.add(q.coeff), k.add(q.tiles), k.add(q.segs), k.add(q.fu), k.add(q.seg0)};
    CK(k.send(c->stream));
    k.at(d.q_units.p, o[0]);
    k.at(d.q_coeff.p, o[1]);
    k.at(d.q_tiles.p, o[2]);
    k.at(d.q_segs.p, o[3]);
    k.at(d.q_fu.p, o[4]);
+   k.at(d.q_seg0.p, o[5]);
    d.q_fblk = q.fblk;
    d.q_nfblk = q.fblk.empty() ? 0 : (int)q.fblk.size() - 1;
-   d.tc_ver++;
    return MDGPU_OK;
 }
 
@@ -1528,44 +1541,35 @@ mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw)
    return MDGPU_OK;
 }
 
-// (a framework's sites take the runs chosen for the others')
+// Runs of segments of the FP64 force pass over T site tiles: the length for
+// which the waves of (site tile, set, run) CTAs come out shortest.
+static void q_runs(mdgpu_ctx *c, int T)
+{
+   KsDev &d = c->kd;
+   const QList &q = c->kl.q;
+   long long best = -1;
+   int mx = 1;
+   for (size_t b = 0; b + 1 < q.seg0.size(); b++) mx = std::max(mx, q.seg0[b + 1] - q.seg0[b]);
+   for (int p = 1; p <= mx; p++) {
+      int k = 0;
+      for (size_t b = 0; b + 1 < q.seg0.size(); b++) k += (q.seg0[b + 1] - q.seg0[b] + p - 1) / p;
+      if (k > 16 && p < mx) continue;
+      const long long cost = (3LL * T * k + c->nsm - 1) / c->nsm * (4LL * p + 7);
+      if (best < 0 || cost < best) {
+         best = cost;
+         d.q_per = p;
+         d.q_nitems = k;
+      }
+   }
+}
+
+// (a framework's sites take the runs chosen for the others', if there are any)
 mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0)
 {
    KsDev &d = c->kd;
    const QList &q = c->kl.q;
    const int nseg = (int)q.segs.size(), T = (n + 127) / 128;
-   // runs of segments: the length for which the waves of (site tile, set,
-   // run) CTAs come out shortest
-   if ((d.q_items_for[0] != T && f0 == 0) || d.q_items_for[1] != (int)d.tc_ver || d.q_items_for[2] != c->nsm) {
-      int per = 1;
-      long long best = -1;
-      int mx = 1;
-      for (size_t b = 0; b + 1 < q.seg0.size(); b++) mx = std::max(mx, q.seg0[b + 1] - q.seg0[b]);
-      auto count = [&](int p) {
-         int k = 0;
-         for (size_t b = 0; b + 1 < q.seg0.size(); b++) k += (q.seg0[b + 1] - q.seg0[b] + p - 1) / p;
-         return k;
-      };
-      for (int p = 1; p <= mx; p++) {
-         const int k = count(p);
-         if (k > 16 && p < mx) continue;
-         const long long cost = (3LL * T * k + c->nsm - 1) / c->nsm * (4LL * p + 7);
-         if (best < 0 || cost < best) {
-            best = cost;
-            per = p;
-         }
-      }
-      std::vector<QItem> items;
-      for (size_t b = 0; b + 1 < q.seg0.size(); b++)
-         for (int s = q.seg0[b]; s < q.seg0[b + 1]; s += per) items.push_back(QItem{s, std::min(s + per, q.seg0[b + 1])});
-      CK(d.q_items.ensure(items.size()));
-      CK(cudaMemcpyAsync(d.q_items.p, items.data(), items.size() * sizeof(QItem), cudaMemcpyHostToDevice, c->stream));
-      CK(cudaStreamSynchronize(c->stream));
-      d.q_nitems = (int)items.size();
-      d.q_items_for[0] = T;
-      d.q_items_for[1] = (int)d.tc_ver;
-      d.q_items_for[2] = c->nsm;
-   }
+   if (f0 == 0 || c->ncharged == c->ncharged_fw) q_runs(c, T);
    CK(d.q_bq.ensure((size_t)3 * nseg * 4 * QCfg<7>::NTMAX * Q_KS * 2 * 7));
    CK(d.q_bexp.ensure((size_t)3 * nseg));
    DBuf<double> &hpart = f0 > 0 ? d.fpartf : d.fpart;
@@ -1573,7 +1577,7 @@ mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0)
    k_qcoef<<<dim3(nseg, 3), 256, 0, c->stream>>>(q.g, 0, d.q_segs.p, nseg, d.q_units.p,
                                                  f0 > 0 ? d.q_abf64.p : d.q_ab64.p, d.q_bq.p, d.q_bexp.p);
    k_force_q<<<dim3(T, 3, d.q_nitems), Q_THREADS, Q_FSMEM, c->stream>>>(
-      q.g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p + (size_t)f0 / 32 * 2 * q.g.hrows * QCfg<7>::RS,
+      q.g, d.q_segs.p, nseg, d.q_seg0.p, d.q_per, d.q_units.p, d.q_x64.p + (size_t)f0 / 32 * 2 * q.g.hrows * QCfg<7>::RS,
       d.q_y64.p + (size_t)f0 / 32 * 2 * q.g.mrows * QCfg<7>::RS, d.q_zd.p + (size_t)f0 / 32 * 2 * q.g.TP * 32, d.q_bq.p,
       d.q_bexp.p, n, hpart.p, &c->out.p->err);
    CK(cudaGetLastError());
@@ -1668,7 +1672,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
       CK(a.gkpart.ensure((size_t)d.q_nitems * N));
       k_qcoef<<<dim3(nseg, 1), 256, 0, st>>>(g, 3, d.q_segs.p, nseg, d.q_units.p, a.ab64.p, d.q_bq.p, d.q_bexp.p);
       k_force_q<<<dim3(T, 1, d.q_nitems), Q_THREADS, Q_FSMEM, st>>>(
-         g, d.q_segs.p, nseg, d.q_items.p, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, N,
+         g, d.q_segs.p, nseg, d.q_seg0.p, d.q_per, d.q_units.p, d.q_x64.p, d.q_y64.p, d.q_zd.p, d.q_bq.p, d.q_bexp.p, N,
          a.gkpart.p, &c->out.p->err);
       c->launches += 2;
       k_qadj_site<false, double4><<<(N + 255) / 256, 256, 0, st>>>(N, d.q_nitems, g, d.fpart.p, a.gkpart.p, a.res64.p,

@@ -75,7 +75,7 @@ constexpr int FTC_ERR = 16;                        // error-word bit: a force-pa
 // much as its work (water on a charged wall, 1044 sites: an evaluation 144 us
 // with launches for each, 125 us so).
 struct FtcRanges {          // a group's work ranges
-   int build, tiles, G;     // to be made; site tiles, ranges
+   int tiles, G;            // site tiles, ranges
    int *ustart;
 };
 struct FtcSecond {          // the second group: sites, ranges, and its data from the first's on
@@ -97,18 +97,32 @@ __device__ __forceinline__ int ftc_ksteps(int4 un, int t0)
 // (an item tile's K-steps plus one for its epilogue) evenly over G CTAs,
 // with G <= the number of site tiles (or G = twice that, each CTA then half
 // a tile), so no run lies strictly inside a site tile and a tile is shared
-// by two CTAs at most.  One block; pre (after ustart[G]) holds the prefix
-// weights of the item tiles.
+// by two CTAs at most.  One block of 256; pre (after ustart[G]) holds the
+// prefix weights of the item tiles.  Made by every evaluation: ranges kept for
+// the next one would be another call's (the gradient runs over all sites) by
+// the time a captured evaluation is replayed.
 __device__ __forceinline__ void ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *ustart)
 {
    int *pre = ustart + G + 1;
-   if (threadIdx.x == 0) {
-      int sum = 0;
-      pre[0] = 0;
-      for (int t = 0; t < ntl; t++) {
-         sum += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
-         pre[t + 1] = sum;
-      }
+   __shared__ int wsum[8];
+   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+   const int run = (ntl + 255) / 256, ta = min(ntl, tid * run), tb = min(ntl, ta + run);   // this thread's tiles
+   int sum = 0;
+   for (int t = ta; t < tb; t++) sum += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
+   int inc = sum;   // inclusive over the threads
+#pragma unroll
+   for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+   }
+   if (lane == 31) wsum[w] = inc;
+   __syncthreads();
+   int at = inc - sum;
+   for (int k = 0; k < w; k++) at += wsum[k];
+   if (tid == 0) pre[0] = 0;
+   for (int t = ta; t < tb; t++) {
+      at += ftc_ksteps(fu[t * (FTC_NI / 8)], t0) + 1;
+      pre[t + 1] = at;
    }
    __syncthreads();
    const long long wt = pre[ntl], wall = wt * nsite_tiles;
@@ -143,7 +157,7 @@ k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, 
    __shared__ float4 sv[8][64];
    if (blockIdx.x == gridDim.x - 1) {   // (uniform)
       const FtcRanges r = blockIdx.y ? rb : ra;
-      if (r.build) ftc_ranges(fu, t0, nitems / FTC_NI, r.tiles, r.G, r.ustart);
+      ftc_ranges(fu, t0, nitems / FTC_NI, r.tiles, r.G, r.ustart);
       return;
    }
    if (blockIdx.y) {
@@ -552,15 +566,7 @@ static int force_tc_block(cudaStream_t st, const KsForceSites *grp, int ngrp, co
    FtcRanges r[2] = {};
    for (int k = 0; k < ngrp; k++) {
       const int f = grp[k].f0 > 0, T = (grp[k].n + 127) / 128, G = 2 * T <= nsm ? 2 * T : std::min(nsm, T);
-      int *key = d.tc_rkey[f];
-      if (blk > 0 || key[0] != T || key[1] != ntl || key[2] != G || d.tc_rver[f] != d.tc_ver) {
-         if (d.tc_ustart[f].ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
-         r[k].build = 1;
-         key[0] = T;
-         key[1] = ntl;
-         key[2] = G;
-         d.tc_rver[f] = d.q_nfblk > 1 ? -1 : d.tc_ver;   // rebuilt per block when there are several
-      }
+      if (d.tc_ustart[f].ensure((size_t)G + ntl + 2) != cudaSuccess) return -1;
       r[k].tiles = T;
       r[k].G = G;
       r[k].ustart = d.tc_ustart[f].p;

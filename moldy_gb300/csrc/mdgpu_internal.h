@@ -75,13 +75,10 @@ struct QTile {
    int unit[16];
 };
 // Eight units of one t-block (the K-rows between two read-backs of the FP64
-// force pass), and a run of segments.
+// force pass).
 struct QSeg {
    int blk;
    int unit[8];
-};
-struct QItem {
-   int seg0, seg1;
 };
 struct QList {
    int ns = 0;                     // digits it was built for (3 mixed, 7 FP64)
@@ -137,19 +134,33 @@ double det3(const double *a);
 void inv3(const double *a, double *b);
 
 // ---- device buffers ----------------------------------------------------------
+// How often a buffer of a context has been freed for a larger one: a captured
+// step holds the pointers of its time and is good for the count of its time
+// only.  The buffers find their context's count while it is being constructed
+// (it is the context's first member; the context's constructor ends that).
+struct BufferMoves {
+   uint64_t n = 0;
+   static inline thread_local uint64_t *of_new = nullptr;
+   BufferMoves() { of_new = &n; }
+};
+
 // Owned by the context: freed by release() or when the context is deleted
 // (on its device: mdgpu_destroy selects it first).
 template <typename T>
 struct DBuf {
    T *p = nullptr;
    size_t n = 0;
+   uint64_t *moves = BufferMoves::of_new;
    DBuf() = default;
    DBuf(const DBuf &) = delete;
    DBuf &operator=(const DBuf &) = delete;
    ~DBuf() { release(); }
    cudaError_t ensure(size_t want) {
       if (want <= n && p) return cudaSuccess;
-      if (p) cudaFree(p);
+      if (p) {
+         cudaFree(p);
+         if (moves) ++*moves;
+      }
       p = nullptr;
       n = 0;
       cudaError_t e = cudaMalloc(&p, (want ? want : 1) * sizeof(T));
@@ -315,7 +326,7 @@ struct KsDev {
    DView<double2> q_coeff;
    DView<QTile> q_tiles;
    DView<QSeg> q_segs;
-   DBuf<QItem> q_items;
+   DView<int> q_seg0;
    DBuf<int> q_x32, q_y32, q_bexp;
    DBuf<long long> q_x64, q_y64;
    DBuf<unsigned char> q_ztab, q_bq, q_part;
@@ -323,8 +334,7 @@ struct KsDev {
    DBuf<float> q_ab32;
    int q_nfblk = 0;                 // mixed force pass: t-blocks and their entries of q_fu
    std::vector<int> q_fblk;
-   int q_items_for[3] = {-1, -1, -1};   // (site tiles, list upload, SMs) of q_items
-   int q_nitems = 0;
+   int q_per = 1, q_nitems = 0;     // FP64 force pass of this evaluation: segments per run, runs
    int q_nranges = 0, q_nrangesf = 0;   // site ranges of q_part, the framework's after them
    DBuf<double> q_abf64;   // the framework sites' coefficients (whole S(k) without the framework's)
    DBuf<float> q_abf32;
@@ -334,9 +344,6 @@ struct KsDev {
    DBuf<uint4> utab;       // force pass: per-item coefficient rows (B operand)
    DBuf<float4> tc_coef;   // per item: kx s1, ky s1, kz0 s1, dkz s2 (row scales s)
    DBuf<int> tc_ustart[2]; // force pass: the CTAs' work ranges (ftc_ranges), of the framework's sites
-   long long tc_ver = 0;   // uploads of the quad list so far
-   int tc_rkey[2][3] = {{-1, -1, -1}, {-1, -1, -1}};   // (site tiles, item tiles, CTAs) of tc_ustart
-   long long tc_rver[2] = {-1, -1};                    // tc_ver of tc_ustart
 };
 
 // Buffers of the adjoint (parameter-gradient) passes.
@@ -391,7 +398,7 @@ struct MdHost {
    int nosym = 0, saxis = 0, nmols_r = 0;
    // one captured step (CUDA graph), replayed by mdgpu_md_run
    cudaGraphExec_t graph = nullptr;
-   uint64_t graph_gen = 0;
+   uint64_t graph_gen = 0, graph_moves = 0;   // configuration and buffers it was captured with
    int64_t graph_launches = 0;       // kernels one replay launches
    int graph_cap = 0;                // record capacity it was captured with
    uint64_t warm_gen = 0;            // configuration of the last direct step
@@ -426,6 +433,8 @@ struct MdDev {
 }  // namespace mdgpu
 
 struct mdgpu_ctx {
+   mdgpu::BufferMoves moves;   // (first: the buffers below count in it)
+   mdgpu_ctx() { mdgpu::BufferMoves::of_new = nullptr; }
    int device = 0;
    int nsm = 0;        // multiprocessors of the device (read when first needed)
    cudaStream_t own_stream = nullptr, stream = nullptr;
