@@ -23,6 +23,7 @@ mdgpu_status fail(mdgpu_ctx *c, mdgpu_status s, const std::string &msg)
 mdgpu_status cuda_check(mdgpu_ctx *c, cudaError_t e, const char *what)
 {
    if (e == cudaSuccess) return MDGPU_OK;
+   cudaGetLastError();   // reported here: not the next call's
    std::string m = std::string(what) + ": " + cudaGetErrorString(e);
    return fail(c, e == cudaErrorMemoryAllocation ? MDGPU_E_NOMEM : MDGPU_E_CUDA, m);
 }

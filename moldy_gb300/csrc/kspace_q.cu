@@ -1406,6 +1406,7 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    if (c->nsm <= 0) CK(cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, c->device));
    if (q.ns == ns || c->kl.nk == 0) return MDGPU_OK;
    build_qlist(c->kl, ns);
+   q.ns = 0;   // not there until the copy is on its way: it may be refused
    TablePack &k = d.q_lists;
    CK(k.begin());
    const size_t o[6] = {k.add(q.units), k.add(q.coeff), k.add(q.tiles), k.add(q.segs), k.add(q.fu), k.add(q.seg0)};
@@ -1418,6 +1419,7 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
    k.at(d.q_seg0.p, o[5]);
    d.q_fblk = q.fblk;
    d.q_nfblk = q.fblk.empty() ? 0 : (int)q.fblk.size() - 1;
+   q.ns = ns;
    return MDGPU_OK;
 }
 
