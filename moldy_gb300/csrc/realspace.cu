@@ -2216,6 +2216,15 @@ mdgpu_status rs_prepare(mdgpu_ctx *c)
    return MDGPU_OK;
 }
 
+// Opts a pair kernel in to dyn bytes of dynamic shared memory.  The 48 KB a
+// block has without that cover static and dynamic memory together, and these
+// kernels have 6 to 28 KB of static memory.
+template <class F> static cudaError_t allow_smem(F *kfn, size_t dyn)
+{
+   if (dyn <= 16 * 1024) return cudaSuccess;
+   return cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+}
+
 template <int PT, bool EW, bool MIXED, int MODE>
 static cudaError_t launch_pairs_t(const RsParams &P, mdgpu_ctx *c, double *force, DevOut *out,
                                   unsigned long long *keys, long long key_cap, size_t smem)
@@ -2223,10 +2232,8 @@ static cudaError_t launch_pairs_t(const RsParams &P, mdgpu_ctx *c, double *force
    RsDev &d = c->rd;
    const int nb = (P.nsites + PAIR_WARPS - 1) / PAIR_WARPS;
    auto kfn = k_pairs<PT, EW, MIXED, MODE>;
-   if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-   }
+   const cudaError_t e = allow_smem(kfn, smem);
+   if (e != cudaSuccess) return e;
    kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, d.cell_start.p, d.slot_cell.p, d.full.p, d.off_hi.p, d.off_lo.p,
                                      d.pos64.p, d.pos32.p, d.tag.p, d.sorted.p, c->cur_site,
                                      d.pot64.p, d.pot32.p, d.chg.p, force, d.part.p, out, keys, key_cap);
@@ -2252,10 +2259,8 @@ static cudaError_t launch_adj_col_t(const RsParams &P, const AdjParams &A, mdgpu
    RsDev &d = c->rd;
    AdjDev &a = c->ad;
    auto kfn = k_pairs_adj_col<PT, EW, MIXED, LOSS>;
-   if (smem > 24 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-   }
+   const cudaError_t e = allow_smem(kfn, smem);
+   if (e != cudaSuccess) return e;
    kfn<<<nblk, PAIR_WARPS * 32, smem, c->stream>>>(P, A, d.cell_start.p, d.slot_cell.p, d.cols.p, d.col_base.p,
                                                    d.coff.p, d.pos64.p, d.pos32.p, d.tag.p, d.sorted.p, c->cur_site,
                                                    d.pot64.p, d.pot32.p, a.res64.p, a.res32.p, a.gq.p, a.gpart.p);
@@ -2459,20 +2464,16 @@ static cudaError_t launch_col_t(const RsParams &P, mdgpu_ctx *c, double *force, 
    fin.on = fin.on && !fin.has_ewald;
    if (!mixed) {
       auto kfn = k_pairs_col64<PT, EW>;
-      if (smem > 16 * 1024) {
-         cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-         if (e != cudaSuccess) return e;
-      }
+      const cudaError_t e = allow_smem(kfn, smem);
+      if (e != cudaSuccess) return e;
       kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, fin, d.cell_start.p, d.cols.p, d.col_base.p, d.pos64.p, d.tagc.p,
                                                     d.slot_cell.p, d.sorted.p, d.pot64.p, force, d.part.p, d.sync.p,
                                                     c->out.p);
       return cudaGetLastError();
    }
    auto kfn = k_pairs_col<PT, EW>;
-   if (smem > 48 * 1024) {
-      cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-   }
+   const cudaError_t e = allow_smem(kfn, smem);
+   if (e != cudaSuccess) return e;
    kfn<<<nb, PAIR_WARPS * 32, smem, c->stream>>>(P, fin, d.cell_start.p, d.cols.p, d.col_base.p, d.coff.p, d.pos32.p,
                                                  d.tagc.p, d.slot_cell.p, d.sorted.p, c->cur_site, d.pot32.p, force,
                                                  d.part.p, d.sync.p, c->out.p);
