@@ -996,20 +996,17 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restric
    unsigned char *Abuf = sm, *Sbuf = sm + 2 * Q_A<NS>;
    const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
    const int tile = blockIdx.x, set = blockIdx.y;
-   struct {
-      int seg0, seg1;
-   } it;
-   int blk = 0, run = blockIdx.z;
-   for (; blk < g.nblk - 1; blk++) {
-      const int nr = (seg0[blk + 1] - seg0[blk] + per - 1) / per;
-      if (run < nr) break;
-      run -= nr;
-   }
-   it.seg0 = seg0[blk] + run * per;
-   it.seg1 = min(it.seg0 + per, seg0[blk + 1]);
-   const int nst = (it.seg1 - it.seg0) * SEG, nT = q_blkcols(g, blk);
-   if (nst <= 0) return;   // (uniform; the grid has no such run)
+   __shared__ int s_run[3];   // first segment, segments, t-block
    if (tid == 0) {
+      int b = 0, run = blockIdx.z;
+      for (; b < g.nblk - 1; b++) {
+         const int nr = (seg0[b + 1] - seg0[b] + per - 1) / per;
+         if (run < nr) break;
+         run -= nr;
+      }
+      s_run[0] = seg0[b] + run * per;
+      s_run[1] = min(per, seg0[b + 1] - s_run[0]);
+      s_run[2] = b;
       q_init(B);
       abort_s = 0;
    }
@@ -1019,11 +1016,12 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restric
    __syncthreads();
    fence_after_sync();
    const unsigned int tmem = tmem_s;
+   const int sg0 = s_run[0], nst = s_run[1] * SEG, blk = s_run[2], nT = q_blkcols(g, blk);
 
    if (w == Q_BW) {
       if (lane == 0) {
          const unsigned int bb = (unsigned int)(nT * Q_KS * 2 * NS);
-         const unsigned char *src = bq + ((size_t)set * nseg + it.seg0) * SEG * BST;
+         const unsigned char *src = bq + ((size_t)set * nseg + sg0) * SEG * BST;
          int issued = 0;
          for (int st = 0; st < nst; st++) {
             const int s = st % NB;
@@ -1063,7 +1061,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restric
             return false;
          }
          fence_after_sync();
-         const int sh = emax - bexp[set * nseg + it.seg0 + seg];
+         const int sh = emax - bexp[set * nseg + sg0 + seg];
 #pragma unroll
          for (int ch = 0; ch < MAXC; ch++)
             if (4 * ch < ncw) {
@@ -1086,7 +1084,7 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restric
       // a stage's table values are fetched a stage ahead, its unit two stages
       long long xv[2], yv[4];
       auto unit = [&](int st) {
-         const int u = segs[it.seg0 + st / SEG].unit[2 * (st % SEG) + (kg >> 1)];
+         const int u = segs[sg0 + st / SEG].unit[2 * (st % SEG) + (kg >> 1)];
          return u >= 0 ? *reinterpret_cast<const int2 *>(units + u) : make_int2(0, 0);
       };
       auto fetch = [&](int2 un) {
