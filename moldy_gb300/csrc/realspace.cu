@@ -349,18 +349,27 @@ template <> struct NPar<3> { static constexpr int v = 6; };
 template <> struct NPar<4> { static constexpr int v = 3; };
 template <> struct NPar<6> { static constexpr int v = 7; };
 
-// Reciprocal square root, reciprocal and exponential: correctly rounded
+// Square root and its reciprocal, reciprocal and exponential: correctly rounded
 // (FAST false), or the FP32 hardware approximations (FAST true: rsqrt and
 // reciprocal within 2 ulp, exp within a few ulp over the arguments of the
 // potentials here), which the column-walk pair kernel of the mixed form
 // uses.
 template <typename R, bool FAST> struct PairMath {
-   static __device__ __forceinline__ R rsqrt(R x) { return R(1) / dsqrt<R>(x); }
+   // r = sqrt(x), r_r = 1 / r
+   static __device__ __forceinline__ void root(R x, R &r, R &r_r)
+   {
+      r = dsqrt<R>(x);
+      r_r = R(1) / r;
+   }
    static __device__ __forceinline__ R rcp(R x) { return R(1) / x; }
    static __device__ __forceinline__ R ex(R x) { return dexp<R>(x); }
 };
 template <> struct PairMath<float, true> {
-   static __device__ __forceinline__ float rsqrt(float x) { return rsqrtf(x); }
+   static __device__ __forceinline__ void root(float x, float &r, float &r_r)
+   {
+      r_r = rsqrtf(x);
+      r = x * r_r;
+   }
    static __device__ __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
    static __device__ __forceinline__ float ex(float x) { return __expf(x); }
 };
@@ -469,14 +478,20 @@ __device__ const double2 g_exp2_tab[256] = {
    {1.9945921121709402, 8.979134e-18},
 };
 constexpr double EXP_HI = 0.00270760617331689, EXP_LO = 7.453964567463233e-13, EXP_INV = 369.3299304675746;
-__device__ __forceinline__ double rsqrt_n(double x)
+__device__ __forceinline__ void root_n(double x, double &r, double &r_r)
 {
    // (range checks on the exponent bits: a compare would take the FP64 pipe)
-   if ((unsigned int)__double2hiint(x) - 0x04000000u >= 0x78000000u) return 1.0 / sqrt(x);
+   if ((unsigned int)__double2hiint(x) - 0x04000000u >= 0x78000000u) {
+      // (zero among them: r = 0, r_r infinite, where x r_r would be NaN)
+      r = sqrt(x);
+      r_r = 1.0 / r;
+      return;
+   }
    double y;
    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
    const double e = fma(-x, y * y, 1.0);
-   return fma(y * e, fma(0.375, e, 0.5), y);
+   r_r = fma(y * e, fma(0.375, e, 0.5), y);
+   r = x * r_r;
 }
 __device__ __forceinline__ double rcp_n(double x)
 {
@@ -508,7 +523,7 @@ __device__ __forceinline__ double exp_n(double x)
    return __hiloint2double(__double2hiint(r) + ((n >> 8) << 20), __double2loint(r));
 }
 template <> struct PairMath<double, true> {
-   static __device__ __forceinline__ double rsqrt(double x) { return rsqrt_n(x); }
+   static __device__ __forceinline__ void root(double x, double &r, double &r_r) { root_n(x, r, r_r); }
    static __device__ __forceinline__ double rcp(double x) { return rcp_n(x); }
    static __device__ __forceinline__ double ex(double x) { return exp_n(x); }
 };
@@ -522,13 +537,7 @@ __device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm,
    typedef PairMath<R, FAST> M;
    R t = R(0), ef = R(0), r = R(0), r_r = R(0), rs_r;
    if (EW || PT != 0) {
-      if (FAST) {
-         r_r = M::rsqrt(r2);
-         r = r2 * r_r;
-      } else {
-         r = dsqrt<R>(r2);
-         r_r = R(1) / r;
-      }
+      M::root(r2, r, r_r);
       rs_r = r_r * r_r;
    } else {
       rs_r = M::rcp(r2);
@@ -1345,11 +1354,17 @@ k_pairs_col(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *__r
    reduce_pairs_last(part, gridDim.x, sync, out, fin);
 }
 
-// a < b for non-negative doubles, by their bits (a compare would take the
-// FP64 pipe); false when a is NaN
-__device__ __forceinline__ bool less_bits(double a, double b)
+// r2 < b and r2 > b by their bits (a compare would take the FP64 pipe), for
+// r2 a sum of squares and b positive and finite; both false when r2 is NaN, of
+// either sign, as the compares are.
+__device__ __forceinline__ bool r2_below(double r2, double b)
 {
-   return __double_as_longlong(a) < __double_as_longlong(b);
+   return (unsigned long long)__double_as_longlong(r2) < (unsigned long long)__double_as_longlong(b);
+}
+__device__ __forceinline__ bool r2_above(double r2, double b)
+{
+   const unsigned long long i = (unsigned long long)__double_as_longlong(b);
+   return (unsigned long long)__double_as_longlong(r2) - i - 1 < 0x7ff0000000000000ull - i;
 }
 
 // The FP64 form by columns over one interaction class at a time: k_pairs'
@@ -1407,11 +1422,11 @@ k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *_
          const double rz = __dadd_rn(__dsub_rn(xj.z, xi.z), rl[2]);
          double r2 = __dadd_rn(__dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)), __dmul_rn(rz, rz));
          const int2 tj = __ldg(&tagc[j]);
-         if (less_bits(r2, TOO_CLOSE) && ti.y != tj.y) {
+         if (r2_below(r2, TOO_CLOSE) && ti.y != tj.y) {
             const int oj = sortc[j];
             if (oi < oj) note_too_close(out, oi, oj);
          }
-         if (strict && less_bits(P.cut2, r2)) r2 = P.cut100;
+         if (strict && r2_above(r2, P.cut2)) r2 = P.cut100;
          double pp[NP];
          const double *pj = prow + (size_t)(tj.x & 0xffff) * NPOTP;
 #pragma unroll
@@ -1600,8 +1615,9 @@ template <int PT, bool EW, typename R, bool FAST = false>
 __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, PairGrad<NPar<PT>::v, R> &g)
 {
    typedef PairMath<R, FAST> M;
-   const R r_f = FAST ? M::rsqrt(r2) : R(0);
-   const R r = FAST ? r2 * r_f : dsqrt<R>(r2), r_r = FAST ? r_f : R(1) / r, rs_r = r_r * r_r;
+   R r, r_r;
+   M::root(r2, r, r_r);
+   const R rs_r = r_r * r_r;
    g.uc = g.fc = g.duc = g.dfc = R(0);
    if (EW) {
       const R x = alpha * r;
