@@ -968,17 +968,19 @@ static void count_charged(mdgpu_ctx *c)
    if (c->ncharged_gen == c->gen) return;
    int n = 0, nfw = 0;
    double qm = 0;
+   bool finite = true;
    for (size_t i = 0; i < c->chg.size(); i++) {
       const double q = c->chg[i];
       n += q != 0.0;
       nfw += q != 0.0 && (int)i >= c->fw_site0;
+      finite = finite && std::isfinite(q);
       qm = std::max(qm, std::fabs(q));
    }
    c->ncharged = n;
    c->ncharged_fw = nfw;
    c->n_class0 = 0;
    for (int id : c->site_id) c->n_class0 += c->cls_of_id[id] == 0;
-   c->qmax = qm;
+   c->qmax = finite ? qm : NAN;
    c->ncharged_gen = c->gen;
 }
 

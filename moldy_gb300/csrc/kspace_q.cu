@@ -57,6 +57,7 @@ constexpr int Q_OP = 128 * Q_KS * 2;              // one digit of a 128-row oper
 constexpr int Q_BW = 16;                          // operand / read-back warps
 constexpr int Q_THREADS = 32 * (Q_BW + 3);        // and a bulk-copy warp, two MMA warps
 constexpr int Q_ERR = 8, Q_FERR = 16;             // error-word bits: structure factor, force pass
+constexpr int Q_NOT_FINITE = 8192;                // scale exponent: a value is infinite or NaN
 
 template <int NS> struct QCfg;
 template <> struct QCfg<3> {
@@ -913,17 +914,19 @@ __device__ __forceinline__ void q_coefs(const double *ab, int set, int h, int m,
 }
 
 // Grid: (segments, sets from set0).  The segment's B operand, [stage 4][digit]
-// [col group][kg 4][8 cols][8 K], and its scale exponent.
+// [col group][kg 4][8 cols][8 K], and its scale exponent.  Digits hold no NaN
+// or infinity: where a coefficient is one, the exponent says so, and the force
+// pass hands NaN on.
 __global__ void __launch_bounds__(256)
 k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *__restrict__ units,
         const double *__restrict__ ab, unsigned char *__restrict__ bq, int *__restrict__ bexp)
 {
    constexpr int NS = 7;
-   __shared__ double smax[8];
+   __shared__ long long smax[8];
    const int seg = blockIdx.x, set = blockIdx.y, tid = threadIdx.x;
    const QSeg &sg = segs[seg];
    const int nT = q_blkcols(g, sg.blk), tw = nT / 2, t0 = sg.blk * g.TW;
-   double mx = 0.0;
+   long long mb = 0;   // the largest magnitude's bits (infinity and NaN are the largest)
    for (int i = tid; i < 32 * tw; i += 256) {
       const int ql = i / tw, t = t0 + i % tw, u = sg.unit[ql >> 2];
       if (u < 0) continue;
@@ -932,15 +935,20 @@ k_qcoef(QGeom g, int set0, const QSeg *__restrict__ segs, int nseg, const int4 *
       double v[8];
       q_coefs(ab + ((size_t)(4 * u + (ql & 3)) * g.TP + t) * 8, set0 + set, un.x, un.y + (ql & 3), t, v);
 #pragma unroll
-      for (int k = 0; k < 8; k++) mx = fmax(mx, fabs(v[k]));
+      for (int k = 0; k < 8; k++) mb = max(mb, __double_as_longlong(fabs(v[k])));
    }
 #pragma unroll
-   for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-   if ((tid & 31) == 0) smax[tid >> 5] = mx;
+   for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+   if ((tid & 31) == 0) smax[tid >> 5] = mb;
    __syncthreads();
-   mx = smax[0];
-   for (int k = 1; k < 8; k++) mx = fmax(mx, smax[k]);
+   mb = smax[0];
+   for (int k = 1; k < 8; k++) mb = max(mb, smax[k]);
+   double mx = __longlong_as_double(mb);
    int e = -4096;
+   if (mb >= 0x7ff0000000000000ll) {
+      e = Q_NOT_FINITE;
+      mx = 0.0;
+   }
    if (mx > 0.0) frexp(mx, &e);
    if (tid == 0) bexp[set * nseg + seg] = e;
    const double sc = mx > 0.0 ? ldexp(Q_KAPPA * Q_KAPPA, 63 - e) : 0.0;
@@ -1140,7 +1148,9 @@ k_force_q(QGeom g, const QSeg *__restrict__ segs, int nseg, const int *__restric
          if (i < n && !q_aborted(&abort_s)) {
             const double s = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
             // units of the product: 2^-62 over the four table scales, times the coefficients' scale
-            const double sc = emax > -4096 ? ldexp(1.0 / (Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA), emax - 62) : 0.0;
+            const double sc = emax >= Q_NOT_FINITE ? __longlong_as_double(0x7ff8000000000000ll)
+                              : emax > -4096       ? ldexp(1.0 / (Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA), emax - 62)
+                                                   : 0.0;
             hpart[((size_t)blockIdx.z * gridDim.y + set) * n + i] = s * sc;
          }
       }
@@ -1424,9 +1434,11 @@ mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns)
 // The scale of the charges: FP64, a power of two above the largest; mixed,
 // the largest itself (its 31-bit fixed point then holds charges in simple
 // ratios, rigid water's 1 : -2, exactly: their rounding is the same at every
-// site of a kind and does not average out).
+// site of a kind and does not average out).  NaN where a charge is not finite,
+// which the digits cannot hold: the sums' scale then makes every result NaN.
 static double q_charge_scale(const mdgpu_ctx *c, int ns)
 {
+   if (std::isnan(c->qmax)) return c->qmax;
    int e = 0;
    const double q = c->qmax > 0 ? c->qmax : 1.0;
    std::frexp(q, &e);

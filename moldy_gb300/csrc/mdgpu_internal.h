@@ -499,7 +499,7 @@ struct mdgpu_ctx {
    int ncharged = 0;                // sites with a nonzero charge
    int ncharged_fw = 0;             // of them, of the framework molecule
    int n_class0 = 0;                // sites of interaction class 0
-   double qmax = 0;                 // and their largest |q|
+   double qmax = 0;                 // and their largest |q| (NaN if one is not finite)
    cudaEvent_t ev[MDGPU_NPHASES + 1] = {};
    // second (high-priority) stream: the k-space passes run on it beside
    // the pair kernel
