@@ -1190,33 +1190,38 @@ k_fsum_q(int n, int N, int nitems, QGeom g, const double *__restrict__ hpart, co
 // charges in the mixed form (residual weights spread over decades: a few
 // close contacts dominate them, and the digits' grid is that of the largest).
 
-// wmax[a]: bits of an FP32 upper bound of max |q v_a| (zeroed before)
+// wmax[a]: high word of max |q v_a| (zeroed before): its FP64 exponent, so that
+// no weight of the FP64 form is out of range, and above every finite one where
+// a weight is infinite or NaN
 template <typename V4>
 __global__ void __launch_bounds__(256)
 k_qwmax(int n, const int *__restrict__ slots, const double *__restrict__ chg, const V4 *__restrict__ res,
         unsigned int *__restrict__ wmax)
 {
    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-   float m[3] = {0.f, 0.f, 0.f};
+   unsigned int m[3] = {0u, 0u, 0u};
    if (i < n) {
       const double q = chg[slots[i]];
       const V4 v = res[i];
-      m[0] = __double2float_ru(fabs(q * (double)v.x));
-      m[1] = __double2float_ru(fabs(q * (double)v.y));
-      m[2] = __double2float_ru(fabs(q * (double)v.z));
+      m[0] = (unsigned int)__double2hiint(fabs(q * (double)v.x));
+      m[1] = (unsigned int)__double2hiint(fabs(q * (double)v.y));
+      m[2] = (unsigned int)__double2hiint(fabs(q * (double)v.z));
    }
 #pragma unroll
    for (int a = 0; a < 3; a++) {
-      const unsigned int x = __reduce_max_sync(0xffffffffu, __float_as_uint(m[a]));
+      const unsigned int x = __reduce_max_sync(0xffffffffu, m[a]);
       if ((threadIdx.x & 31) == 0 && x) atomicMax(&wmax[a], x);
    }
 }
-__device__ __forceinline__ int q_wexp(unsigned int bits)   // a power of two above
+__device__ __forceinline__ int q_wexp(unsigned int hi)   // a power of two above (subnormal ones too)
 {
-   int e = 0;
-   const float m = __uint_as_float(bits);
-   if (m > 0.f) frexp((double)m, &e);
-   return e;
+   return (int)(hi >> 20) - 1022;
+}
+// the channel's scale, NaN where a weight is not finite (its digits are not
+// either then)
+__device__ __forceinline__ double q_wscale(double scale, unsigned int hi)
+{
+   return hi >= 0x7ff00000u ? __longlong_as_double(0x7ff8000000000000ll) : ldexp(scale, q_wexp(hi));
 }
 
 // Operand B of the three weighted channels, per 32-site stage as in k_qtab.
@@ -1300,7 +1305,7 @@ k_qadj(QGeom g, const int4 *__restrict__ units, const double2 *__restrict__ coef
       const size_t at = ((size_t)quad * 4 + (w >> 1)) * row + 16 * (t >> 3) + 8 * (w & 1) + (t & 7);
       sq[0][w][lane] = live ? scale0 * q_rangesum(part + at, plane, nr0) : 0.0;
       for (int ch = 1; ch < 4; ch++)
-         sq[ch][w][lane] = live && loss ? ldexp(scalev, q_wexp(wmax[ch - 1])) *
+         sq[ch][w][lane] = live && loss ? q_wscale(scalev, wmax[ch - 1]) *
                                              q_rangesum(partv + (size_t)(ch - 1) * nrv * plane + at, plane, nrv)
                                         : 0.0;
    }
