@@ -204,15 +204,9 @@ mdgpu_status mdgpu::sync_out(mdgpu_ctx *c)
    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
    if (e != cudaSuccess) return cuda_check(c, e, "synchronise");
    fill_info(c);
-   if (c->h_out->err & 1)
-      return fail(c, MDGPU_E_RANGE, "Co-ordinate out of range in BIN (fill_cells)");
-   if (c->h_out->err & 4)
-      return fail(c, MDGPU_E_CUDA, "a structure-factor tile copy did not complete (bounded wait expired)");
-   if (c->h_out->err & 8)
-      return fail(c, MDGPU_E_CUDA, "a tensor-core structure-factor stage did not complete (bounded wait expired)");
-   if (c->h_out->err & 16)
-      return fail(c, MDGPU_E_CUDA, "a tensor-core force-pass stage did not complete (bounded wait expired)");
-   return MDGPU_OK;
+   mdgpu_status s;
+   const char *m = eval_error(c->h_out->err, s);
+   return m ? fail(c, s, m) : MDGPU_OK;
 }
 
 #define CKR(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) return cuda_check(c, e_, #x); } while (0)

@@ -355,7 +355,7 @@ k_md_drift(MdStepParams P, const MdSpec *__restrict__ spec, const int *__restric
    double norm = 0.0;
    for (int k = 0; k < 4; k++) norm = DA(norm, DM(q[k], q[k]));
    norm = sqrt(norm);
-   if (fabs(norm - 1.0) > QNORM_TOL) atomicOr(err, 2);
+   if (fabs(norm - 1.0) > QNORM_TOL) atomicOr(err, MD_ERR_QNORM);
    double qn[4];
    const double rnorm = 1.0 / norm;   // one division (the FP64 pipe bounds this kernel)
    for (int k = 0; k < 4; k++) {
@@ -531,7 +531,7 @@ k_md_record(int *__restrict__ counter, int cap, const double *__restrict__ pe, c
    }
    const int step = *counter;
    *counter = step + 1;
-   if (out->err & 1) *err |= 1;
+   if (out->err) *err = md_err_add(*err, out->err);
    if (step >= cap) return;
    double *e = energies + 4 * (size_t)step;
    e[0] = pe[0] + dist_v;
@@ -1293,8 +1293,8 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
       CK(cudaMemcpyAsync(energies, D.energies.p, 4 * (size_t)nsteps * sizeof(double), cudaMemcpyDeviceToHost, st));
    CK(cudaMemcpyAsync(&err, D.err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
    if ((s = sync_out(c)) != MDGPU_OK) return s;
-   if (err & 1) return fail(c, MDGPU_E_RANGE, "Co-ordinate out of range in BIN (fill_cells)");
-   if (err & 2) return fail(c, MDGPU_E_RANGE, "quaternion normalisation error (QNORM2)");
+   if (const char *m = eval_error(err >> MD_ERR_EVAL, s)) return fail(c, s, m);
+   if (err & MD_ERR_QNORM) return fail(c, MDGPU_E_RANGE, "quaternion normalisation error (QNORM2)");
    return MDGPU_OK;
 }
 

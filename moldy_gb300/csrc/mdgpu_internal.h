@@ -238,6 +238,21 @@ struct DevOut {
    double fin[11];        // energies [2] and stress [9] of mdgpu_forces
 };
 
+// DevOut::err as a status and its message (null: no error).
+inline const char *eval_error(int err, mdgpu_status &s)
+{
+   s = err & 1 ? MDGPU_E_RANGE : err ? MDGPU_E_CUDA : MDGPU_OK;
+   if (err & 1) return "Co-ordinate out of range in BIN (fill_cells)";
+   if (err & 4) return "a structure-factor tile copy did not complete (bounded wait expired)";
+   if (err & 8) return "a tensor-core structure-factor stage did not complete (bounded wait expired)";
+   if (err & 16) return "a tensor-core force-pass stage did not complete (bounded wait expired)";
+   return err ? "unknown device error" : nullptr;
+}
+// The error word of a dynamics run: bit 1 its own (quaternions), from bit 8 on
+// the errors of every step's evaluation (the next one clears DevOut).
+constexpr int MD_ERR_QNORM = 2, MD_ERR_EVAL = 8;
+__host__ __device__ inline int md_err_add(int run, int eval) { return run | eval << MD_ERR_EVAL; }
+
 // What the last kernel of an evaluation adds up (finalize_eval): the
 // first-call constants and where the energies and the stress go besides
 // DevOut::fin (pe null: nowhere).  on: the kernel's last block does it.
