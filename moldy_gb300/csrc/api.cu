@@ -223,8 +223,19 @@ static bool stage(mdgpu_ctx *c, size_t n)
    return true;
 }
 
-// parts[k][N], k < np, to dst[np][N] (the staging buffer's last use is over:
-// every host call that stages also waits)
+// A host call's copies from its arrays or the staging buffer are over when it
+// returns, with an error too: the caller may free the arrays, the next call
+// rewrites the buffer.
+struct CopiesOver {
+   cudaStream_t st;
+   bool waited = false;
+   ~CopiesOver()
+   {
+      if (!waited && cudaStreamSynchronize(st) != cudaSuccess) cudaGetLastError();   // (the call's own error is returned)
+   }
+};
+
+// parts[k][N], k < np, to dst[np][N]
 static mdgpu_status copy_in(mdgpu_ctx *c, double *dst, const double *const *parts, int np, size_t at, bool staged)
 {
    const size_t N = c->nsites;
@@ -259,7 +270,6 @@ static mdgpu_status copy_out_sync(mdgpu_ctx *c, double *const force[3], bool sta
 static mdgpu_status upload_cofm(mdgpu_ctx *c, const double *c_of_m)
 {
    if (c->ctl.molpbc) {
-      if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       c->last_cofm.assign(c_of_m, c_of_m + 3 * (size_t)c->nmols);
       CKR(cudaMemcpyAsync(c->cofm_in.p, c->last_cofm.data(), 3 * c->nmols * sizeof(double),
                           cudaMemcpyHostToDevice, c->stream));
@@ -569,9 +579,9 @@ mdgpu_status mdgpu_forces(mdgpu_ctx *c, const double *h, const double *site_soa,
    mdgpu_status s = ensure_ready(c, h, true, true);
    if (s) return s;
    const size_t N = c->nsites;
+   if (c->ctl.molpbc && !c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
    CKR(cudaMemcpyAsync(c->site.p, site_soa, 3 * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    if (c->ctl.molpbc) {
-      if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c_of_m, 3 * c->nmols * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    }
    CKR(c->small.ensure(16));
@@ -595,7 +605,9 @@ mdgpu_status mdgpu_force_calc(mdgpu_ctx *c, const double *h, double *const site[
    mdgpu_status s = ensure_ready(c, h, true, false);
    if (s) return s;
    const size_t N = c->nsites;
+   if (c->ctl.molpbc && !c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
    const bool staged = stage(c, 6 * N);
+   CopiesOver over{c->stream};
    if ((s = copy_in(c, c->site.p, site, 3, 0, staged)) != MDGPU_OK || (s = upload_cofm(c, c_of_m)) != MDGPU_OK ||
        (s = copy_in(c, c->force_in.p, site_force, 3, 3 * N, staged)) != MDGPU_OK)
       return s;
@@ -608,6 +620,7 @@ mdgpu_status mdgpu_force_calc(mdgpu_ctx *c, const double *h, double *const site[
    CKR(cudaGetLastError());
    s = copy_out_sync(c, site_force, staged);
    if (s) return s;
+   over.waited = true;
    const DevOut &o = *c->h_out;
    *pe -= eintra_subtracted(c);
    *pe += o.pe_rs;
@@ -625,12 +638,13 @@ mdgpu_status mdgpu_ewald(mdgpu_ctx *c, const double *h, double *const site[3],
    mdgpu_status s = ensure_ready(c, h, true, true);
    if (s) return s;
    const size_t N = c->nsites;
+   if (c->ctl.molpbc && c->last_cofm.size() != 3 * (size_t)c->nmols)
+      return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass (call force_calc first)");
    const bool staged = stage(c, 6 * N);
+   CopiesOver over{c->stream};
    if ((s = copy_in(c, c->site.p, site, 3, 0, staged)) != MDGPU_OK || (s = copy_in(c, c->force.p, site_force, 3, 3 * N, staged)) != MDGPU_OK)
       return s;
    if (c->ctl.molpbc) {   // binning by molecule: the centres of mass are on the host record only
-      if (c->last_cofm.size() != 3 * (size_t)c->nmols)
-         return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass (call force_calc first)");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c->last_cofm.data(), 3 * c->nmols * sizeof(double),
                           cudaMemcpyHostToDevice, c->stream));
    }
@@ -640,6 +654,7 @@ mdgpu_status mdgpu_ewald(mdgpu_ctx *c, const double *h, double *const site[3],
    if (s) return s;
    s = copy_out_sync(c, site_force, staged);
    if (s) return s;
+   over.waited = true;
    const DevOut &o = *c->h_out;
    const double sv = c->sheet_energy / c->kl.vol;
    *pe -= c->self_energy;
@@ -677,9 +692,9 @@ mdgpu_status mdgpu_rdf_counts(mdgpu_ctx *c, const double *h, const double *site_
    mdgpu_status s = ensure_ready(c, h, true, false);
    if (s) return s;
    const size_t N = c->nsites;
+   if (c->ctl.molpbc && !c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
    CKR(cudaMemcpyAsync(c->site.p, site_soa, 3 * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    if (c->ctl.molpbc) {
-      if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c_of_m, 3 * c->nmols * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    }
    c->link_order = true;
@@ -743,9 +758,9 @@ mdgpu_status mdgpu_pair_keys(mdgpu_ctx *c, const double *h, const double *site_s
    mdgpu_status s = ensure_ready(c, h, true, false);
    if (s) return s;
    const size_t N = c->nsites;
+   if (c->ctl.molpbc && !c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
    CKR(cudaMemcpyAsync(c->site.p, site_soa, 3 * N * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    if (c->ctl.molpbc) {
-      if (!c_of_m) return fail(c, MDGPU_E_ARG, "molecular cutoff needs the centres of mass");
       CKR(cudaMemcpyAsync(c->cofm_in.p, c_of_m, 3 * c->nmols * sizeof(double), cudaMemcpyHostToDevice, c->stream));
    }
    CKR(c->rd.keys.ensure(cap > 0 ? (size_t)cap : 1));
