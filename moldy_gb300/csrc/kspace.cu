@@ -984,15 +984,18 @@ static void count_charged(mdgpu_ctx *c)
    c->ncharged_gen = c->gen;
 }
 
+// The passes are those on the tensor cores (the adjoint with a framework
+// molecule runs on the CUDA-core ones).
+static bool ks_on_tc(const mdgpu_ctx *c) { return c->tc_sfac && (c->fw_site0 == c->nsites || !c->ks_all_sites); }
+
 mdgpu_status ks_prepare(mdgpu_ctx *c)
 {
    KsDev &d = c->kd;
    cudaStream_t st = c->stream;
    const int N = c->nsites;
-   if (c->tc_sfac) {
-      const mdgpu_status s = ks_q_prepare(c, c->prec == MDGPU_MIXED ? 3 : 7);
-      if (s) return s;
-   }
+   // (the tables here, not with the passes: a captured step only replays those)
+   const mdgpu_status s = ks_on_tc(c) ? ks_q_prepare(c, c->prec == MDGPU_MIXED ? 3 : 7) : ks_upload_list(c);
+   if (s) return s;
    // a framework's charged sites: their slots never change (the fillers
    // before them neither)
    if (c->tc_sfac && c->fw_site0 < N && d.kslots_gen != c->gen) {
@@ -1068,7 +1071,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    // pass takes them with the other sites' coefficients (water on a charged
    // wall, 1044 sites, mixed: an evaluation took 200 us with two CUDA-core
    // structure-factor passes and a correcting force pass, 146 us so).
-   const bool tc = c->tc_sfac && (nf <= 0 || !c->ks_all_sites);
+   const bool tc = ks_on_tc(c);
    const bool compact = (nf <= 0 || tc) && !c->ks_all_sites;
    int Nk = N;
    const int *slots = c->rd.sorted.p;
@@ -1099,7 +1102,6 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    }
    const int ns = mixed ? 3 : 7;
    mdgpu_status s;
-   if (!tc && (s = ks_upload_list(c)) != MDGPU_OK) return s;
    if (tc) {
       if ((s = ks_q_tables(c, ns, nfc ? f0 + nfc : Nk, nf > 0, slots, d_site)) != MDGPU_OK) return s;
       if (cudaStream_t main = c->pairs_after_tables) {

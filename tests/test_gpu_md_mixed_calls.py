@@ -66,3 +66,12 @@ def test_run_between_other_calls(n, call, before, form, tol):
         ff.close()
     for a, b in zip(*out):
         assert np.abs(a - b).max() <= tol * np.abs(a).max()
+
+
+@pytest.mark.parametrize("form,tol", [("fp64", 1e-11), ("mixed", 1e-6)])
+@pytest.mark.parametrize("before", [3, 1])
+@pytest.mark.parametrize("call", [gradient, other_cell], ids=lambda v: v.__name__)
+def test_run_between_other_calls_cuda_core_passes(call, before, form, tol, monkeypatch):
+    """The k-list tables of the CUDA-core passes are the run's own again."""
+    monkeypatch.setenv("MDGPU_KSPACE_TC", "0")
+    test_run_between_other_calls(6, call, before, form, tol)
