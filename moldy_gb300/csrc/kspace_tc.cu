@@ -97,13 +97,17 @@ __device__ __forceinline__ int ftc_ksteps(int4 un, int t0)
 // (an item tile's K-steps plus one for its epilogue) evenly over G CTAs,
 // with G <= the number of site tiles (or G = twice that, each CTA then half
 // a tile), so no run lies strictly inside a site tile and a tile is shared
-// by two CTAs at most.  One block of 256; pre (after ustart[G]) holds the
-// prefix weights of the item tiles.  Made by every evaluation: ranges kept for
+// by two CTAs at most.  One block of 256; pre holds the prefix weights of the
+// item tiles, in shared memory (sh, FTC_PRE entries; with the search's reads, one
+// after the other, from global memory an evaluation of 1044 sites took 127
+// us in place of 125.5) or, for more tiles, after ustart[G].  Made by every evaluation: ranges kept for
 // the next one would be another call's (the gradient runs over all sites) by
 // the time a captured evaluation is replayed.
-__device__ __forceinline__ void ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *ustart)
+constexpr int FTC_PRE = 2048;
+__device__ __forceinline__ void ftc_ranges(const int4 *__restrict__ fu, int t0, int ntl, int nsite_tiles, int G, int *ustart,
+                                           int *sh)
 {
-   int *pre = ustart + G + 1;
+   int *pre = ntl < FTC_PRE ? sh : ustart + G + 1;
    __shared__ int wsum[8];
    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
    const int run = (ntl + 255) / 256, ta = min(ntl, tid * run), tb = min(ntl, ta + run);   // this thread's tiles
@@ -155,9 +159,10 @@ k_utab_tc(int nitems, QGeom g, int t0, int scalar, const int4 *__restrict__ fu, 
           const float4 *__restrict__ ab2, uint4 *__restrict__ utab, float *__restrict__ coef, FtcRanges ra, FtcRanges rb)
 {
    __shared__ float4 sv[8][64];
+   static_assert(sizeof sv >= FTC_PRE * sizeof(int), "the ranges' prefix weights");
    if (blockIdx.x == gridDim.x - 1) {   // (uniform)
       const FtcRanges r = blockIdx.y ? rb : ra;
-      ftc_ranges(fu, t0, nitems / FTC_NI, r.tiles, r.G, r.ustart);
+      ftc_ranges(fu, t0, nitems / FTC_NI, r.tiles, r.G, r.ustart, reinterpret_cast<int *>(sv));
       return;
    }
    if (blockIdx.y) {
