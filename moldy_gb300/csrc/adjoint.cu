@@ -446,7 +446,7 @@ static mdgpu_status ks_adjoint(mdgpu_ctx *c, bool loss)
       CK(cudaMemsetAsync(a.scal.p + 1, 0, 2 * sizeof(double), st));
       return MDGPU_OK;
    }
-   if (c->tc_sfac && !fw) {
+   if (ks_on_tc(c) && !fw) {
       int nb = 0;
       const mdgpu_status s = ks_q_adjoint(c, loss, c->rd.sorted.p, a.gq.p + (loss ? N : 0), &nb);
       if (s != MDGPU_OK) return s;

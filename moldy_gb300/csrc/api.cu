@@ -539,7 +539,7 @@ mdgpu_status mdgpu_forces_device(mdgpu_ctx *c, const double *h, const double *d_
       // priority) start before the pair blocks take every SM: those then fill
       // what is left.  Below 8 x 152 x 4 sites both start at once (131,072-site
       // water, mixed: 1.153 ms with the pair kernel first, 1.138 ms so).
-      c->pairs_after_tables = c->nsites >= 32 * 152 && c->tc_sfac && c->nsites == c->fw_site0 ? main : nullptr;
+      c->pairs_after_tables = c->nsites >= 32 * 152 && ks_on_tc(c) && c->nsites == c->fw_site0 ? main : nullptr;
       if (!c->pairs_after_tables) {
          s = rs_pairs(c, d_force, nullptr, 0);
          if (s) return s;

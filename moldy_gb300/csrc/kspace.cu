@@ -963,11 +963,22 @@ static mdgpu_status ks_upload_list(mdgpu_ctx *c)
 // begins there, never the first one (slot 0 on are the others).
 static int fw_slot0(int n) { return std::max(128, (n + 127) & ~127); }
 
+// The tensor-core structure factor holds q z on a fixed grid below the largest
+// charge (2^-56 of it, mixed 2^-24), where FP64 and FP32 rounded every charge's
+// term by its own size: with a largest charge of c times the root mean square the
+// grid's error grows with c against theirs.  Error of the k-space force on the
+// large charges, 1000 to 4000 ions, CUDA-core FP64 passes / digits: c = 1, 1.4, 10,
+// 22: 5.5 / 5.3, 7.0 / 7.9, 5.5 / 7.5, 14 / 12 e-16; c = 32, 63: 8.1e-15 / 2.5e-14,
+// 3.9e-13 / 4.5e-12.  Beyond 16 the FP64 form takes the CUDA-core passes and the
+// mixed one four digits, 2^-32 (three there: 4.8e-5 with its former operands / 5.0e-5,
+// 5.0e-3 / 6.3e-3).
+constexpr double Q_CREST = 16;
+
 static void count_charged(mdgpu_ctx *c)
 {
    if (c->ncharged_gen == c->gen) return;
    int n = 0, nfw = 0;
-   double qm = 0;
+   double qm = 0, sq = 0;
    bool finite = true;
    for (size_t i = 0; i < c->chg.size(); i++) {
       const double q = c->chg[i];
@@ -975,18 +986,24 @@ static void count_charged(mdgpu_ctx *c)
       nfw += q != 0.0 && (int)i >= c->fw_site0;
       finite = finite && std::isfinite(q);
       qm = std::max(qm, std::fabs(q));
+      sq += q * q;
    }
    c->ncharged = n;
    c->ncharged_fw = nfw;
    c->n_class0 = 0;
    for (int id : c->site_id) c->n_class0 += c->cls_of_id[id] == 0;
    c->qmax = finite ? qm : NAN;
+   c->q_spread = finite && n * (qm * qm) > Q_CREST * Q_CREST * sq;
    c->ncharged_gen = c->gen;
 }
 
-// The passes are those on the tensor cores (the adjoint with a framework
-// molecule runs on the CUDA-core ones).
-static bool ks_on_tc(const mdgpu_ctx *c) { return c->tc_sfac && (c->fw_site0 == c->nsites || !c->ks_all_sites); }
+// (the adjoint with a framework molecule runs on the CUDA-core passes)
+bool ks_on_tc(mdgpu_ctx *c)
+{
+   if (!c->tc_sfac || (c->fw_site0 < c->nsites && c->ks_all_sites)) return false;
+   count_charged(c);
+   return c->prec == MDGPU_MIXED || !c->q_spread;
+}
 
 mdgpu_status ks_prepare(mdgpu_ctx *c)
 {
@@ -998,8 +1015,7 @@ mdgpu_status ks_prepare(mdgpu_ctx *c)
    if (s) return s;
    // a framework's charged sites: their slots never change (the fillers
    // before them neither)
-   if (c->tc_sfac && c->fw_site0 < N && d.kslots_gen != c->gen) {
-      count_charged(c);
+   if (ks_on_tc(c) && c->fw_site0 < N && d.kslots_gen != c->gen) {
       const int n = c->ncharged - c->ncharged_fw, f0 = fw_slot0(n);
       std::vector<int> v((size_t)f0 - n, -1);
       for (int i = c->fw_site0; i < N; i++)
@@ -1071,7 +1087,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    // pass takes them with the other sites' coefficients (water on a charged
    // wall, 1044 sites, mixed: an evaluation took 200 us with two CUDA-core
    // structure-factor passes and a correcting force pass, 146 us so).
-   const bool tc = ks_on_tc(c);
+   const bool tc = ks_on_tc(c), wide = nf > 0 || c->q_spread;
    const bool compact = (nf <= 0 || tc) && !c->ks_all_sites;
    int Nk = N;
    const int *slots = c->rd.sorted.p;
@@ -1103,7 +1119,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    const int ns = mixed ? 3 : 7;
    mdgpu_status s;
    if (tc) {
-      if ((s = ks_q_tables(c, ns, nfc ? f0 + nfc : Nk, nf > 0, slots, d_site)) != MDGPU_OK) return s;
+      if ((s = ks_q_tables(c, ns, nfc ? f0 + nfc : Nk, wide, slots, d_site)) != MDGPU_OK) return s;
       if (cudaStream_t main = c->pairs_after_tables) {
          CK(cudaEventRecord(c->ev_fork, st));
          CK(cudaStreamWaitEvent(main, c->ev_fork, 0));
@@ -1141,7 +1157,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    phase_mark(c, MDGPU_PH_SFAC);
    const dim3 gs((ni + 127) / 128, sh.chunks);
    if (tc) {
-      if ((s = ks_q_sfac(c, ns, Nk, nf > 0, f0, nfc)) != MDGPU_OK) return s;
+      if ((s = ks_q_sfac(c, ns, Nk, wide, f0, nfc)) != MDGPU_OK) return s;
    } else if (mixed) {
       CK(d.part32.ensure((size_t)sh.chunks * nk));
       k_sfac32<<<gs, 128, 0, st>>>(d.item.p, d.item_k0.p, ni, d.ph32.p, d.zp32.p, Nk, sh.chunk, nk, d.part32.p,
@@ -1167,7 +1183,7 @@ mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool
    CK(d.blk.ensure((size_t)nbk * 8));
    phase_mark(c, MDGPU_PH_KREDUCE);
    if (tc) {
-      if ((s = ks_q_reduce(c, ns, nf > 0)) != MDGPU_OK) return s;
+      if ((s = ks_q_reduce(c, ns, nf > 0, wide)) != MDGPU_OK) return s;
    } else if (nf > 0) {
       if (mixed) {
          CK(d.kdatf32.ensure(nk));

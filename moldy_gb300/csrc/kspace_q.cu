@@ -519,7 +519,8 @@ __device__ __forceinline__ double q_value(const Q96 &v)
 // Grid: (row tiles, site ranges, channels).  The first r0 ranges share stages
 // 0 .. n0 - 1, the others those from s1 to nstages - 1 (a framework's).  part[channel][range][quad row 4
 // quad + p][2 TP]; channel c reads its own digits, zstride further on each.
-// NA = 4 (mixed form with a framework molecule): 32-bit operands.  The energy
+// NA = 4 (mixed form with a framework molecule, or charges of very different
+// size): 32-bit operands.  The energy
 // and stress there are differences of the framework's large and the other
 // sites' small sums, and charges of any ratio share the digits' grid: with
 // three digits the stress of a clay (500 sites) was 1.5e-5 off, with FP32
@@ -1450,20 +1451,19 @@ static double q_charge_scale(const mdgpu_ctx *c, int ns)
    return ns == 3 ? q : std::ldexp(1.0, e);
 }
 
-// (fw: the mixed form's structure factor in four digits)
-mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool fw, const int *slots, const double *d_site)
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool wide, const int *slots, const double *d_site)
 {
    KsDev &d = c->kd;
    const QGeom &g = c->kl.q.g;
    const size_t S = q_stages(n);
    const double *hi = c->kl.hinv;
    const double qinv = 1.0 / q_charge_scale(c, ns);
-   CK(d.q_ztab.ensure(S * 2 * g.TP * Q_KS * 2 * (ns == 3 && fw ? 4 : ns)));
+   CK(d.q_ztab.ensure(S * 2 * g.TP * Q_KS * 2 * (ns == 3 && wide ? 4 : ns)));
    if (ns == 3) {
       CK(d.q_x32.ensure(S * 2 * g.hrows * QCfg<3>::RS));
       CK(d.q_y32.ensure(S * 2 * g.mrows * QCfg<3>::RS));
       CK(d.zsite.ensure(S / 4 * 2 * g.TP * 48));
-      if (fw) {
+      if (wide) {
          CK(d.q_xw32.ensure(S * 2 * g.hrows * QCfg<3>::RS));
          k_qtab<3, 4><<<(unsigned int)S, 256, 0, c->stream>>>(n, c->nsites, g, slots, d_site, c->rd.chg.p, hi[0], hi[1], hi[2],
                                                            hi[3], hi[4], hi[5], hi[6], hi[7], hi[8], qinv, d.q_x32.p,
@@ -1488,7 +1488,7 @@ mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool fw, const int *slots,
 // Site ranges: the count for which the waves of (tile, range) CTAs, each its
 // stages plus a start-up of about six, come out shortest.  A framework's
 // sites (slots f0 on) have ranges of their own.
-mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool fw, int f0, int nf)
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool wide, int f0, int nf)
 {
    KsDev &d = c->kd;
    const QList &q = c->kl.q;
@@ -1508,7 +1508,7 @@ mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool fw, int f0, int nf)
    const int R0 = (n0 + per - 1) / per, R = R0 + (nstf + per - 1) / per;
    CK(d.q_part.ensure(R * plane * psz));
    const dim3 grid(nt, R);
-   if (ns == 3 && fw)
+   if (ns == 3 && wide)
       k_sfac_q<3, 4, 4><<<grid, Q_THREADS, Q_SMEM<3, 4, 4>, c->stream>>>(q.g, 256u, d.q_tiles.p, d.q_units.p,
          (const unsigned char *)d.q_xw32.p, (const unsigned char *)d.q_y32.p, d.q_ztab.p, 0, R0, n0, s1, s1 + nstf, per,
          (float *)d.q_part.p, &c->out.p->err);
@@ -1534,14 +1534,14 @@ static void q_reduce(mdgpu_ctx *c, int nb, double scale, DBuf<R> &ab, DBuf<R> &a
                                                (const R *)d.q_part.p, d.q_nrangesf, ab.p, abf.p, d.blk.p,
                                                c->rd.sync.p, c->out.p);
 }
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw)
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw, bool wide)
 {
    KsDev &d = c->kd;
    const QGeom &g = c->kl.q.g;
    const size_t nqt = (size_t)g.nquads * g.TP;
    const int nb = (int)std::min<size_t>((nqt + 31) / 32, 4 * (size_t)c->nsm);
    const double k4 = Q_KAPPA * Q_KAPPA * Q_KAPPA * Q_KAPPA;
-   const double scale = q_charge_scale(c, ns) * std::ldexp(1.0 / k4, ns == 7 ? -62 : fw ? -38 : -30);
+   const double scale = q_charge_scale(c, ns) * std::ldexp(1.0 / k4, ns == 7 ? -62 : wide ? -38 : -30);
    CK(d.blk.ensure((size_t)nb * 8));
    if (ns == 3) {
       CK(d.q_ab32.ensure(nqt * 8));
@@ -1672,7 +1672,7 @@ mdgpu_status ks_q_adjoint(mdgpu_ctx *c, bool loss, const int *slots, double *gq,
    if (ns == 3) {
       CK(a.ab32.ensure(nqt * 8));
       k_qadj<float><<<nb, 256, 0, st>>>(g, d.q_units.p, d.q_coeff.p, c->ctl.alpha, loss ? 1 : 0, d.q_nranges,
-         qs * std::ldexp(1.0 / k4, -30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
+         qs * std::ldexp(1.0 / k4, c->q_spread ? -38 : -30), (const float *)d.q_part.p, R, std::ldexp(1.0 / k4, -38), a.wmax.p, (const float *)a.partv.p, a.ab32.p, a.blk.p);
       const int sp = ks_force_tc_splits(d);
       CK(a.gkpart.ensure((size_t)sp * 3 * N));
       const KsForceSites grp{N, 0, a.ab32.p, a.gkpart.p};

@@ -515,6 +515,7 @@ struct mdgpu_ctx {
    int ncharged_fw = 0;             // of them, of the framework molecule
    int n_class0 = 0;                // sites of interaction class 0
    double qmax = 0;                 // and their largest |q| (NaN if one is not finite)
+   bool q_spread = false;           // largest far above the root mean square (see ks_on_tc)
    cudaEvent_t ev[MDGPU_NPHASES + 1] = {};
    // second (high-priority) stream: the k-space passes run on it beside
    // the pair kernel
@@ -563,6 +564,8 @@ int pot_nparams(int ptype);     // parameters the potential type reads
 mdgpu_status rs_rdf(mdgpu_ctx *c, double limit, int nbins);
 // kspace.cu
 mdgpu_status ks_prepare(mdgpu_ctx *c);
+// The passes of the current system and form are those on the tensor cores.
+bool ks_on_tc(mdgpu_ctx *c);
 // join: an event the final force sum waits for (the pair kernel running on
 // another stream writes d_force first), or null.
 mdgpu_status ks_launch(mdgpu_ctx *c, const double *d_site, double *d_force, bool accumulate,
@@ -579,10 +582,11 @@ KsShape ks_shape(int N, int nitems, int ipt, int spt);
 // fpart[split][3][nsites], or with scalar the sum over k of A sin - B cos
 // into its first component (returns the launches, -1 if out of memory).
 mdgpu_status ks_q_prepare(mdgpu_ctx *c, int ns);
-mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool fw, const int *slots, const double *d_site);
+// (wide: the mixed form's structure factor in four digits)
+mdgpu_status ks_q_tables(mdgpu_ctx *c, int ns, int n, bool wide, const int *slots, const double *d_site);
 // n sites and, from slot f0 (a multiple of 128) on, nf of a framework molecule
-mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool fw, int f0, int nf);
-mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw);
+mdgpu_status ks_q_sfac(mdgpu_ctx *c, int ns, int n, bool wide, int f0, int nf);
+mdgpu_status ks_q_reduce(mdgpu_ctx *c, int ns, bool fw, bool wide);
 // sites from slot f0 (zero or the framework's first) on
 mdgpu_status ks_q_force64(mdgpu_ctx *c, int n, int f0);
 mdgpu_status ks_q_fsum64(mdgpu_ctx *c, int n, int f0, const int *slots, double *d_force, const FinArgs &fin);
