@@ -2461,7 +2461,9 @@ mdgpu_status rs_launch(mdgpu_ctx *c, const double *d_site, const double *d_cofm,
 }
 
 // The column walk serves both forms without a framework molecule or
-// molecular cut-off, where every stencil column wraps the cell at most once.
+// molecular cut-off, where every stencil column wraps the cell at most once
+// and its packed words hold the grid: 27 bits of a cell index (walk_columns'
+// index base), 15 of a z index (tagc).
 static bool col_walk_ok(const mdgpu_ctx *c)
 {
    static const bool off = [] {
@@ -2469,6 +2471,7 @@ static bool col_walk_ok(const mdgpu_ctx *c)
       return e && e[0] == '0';
    }();
    return !off && c->rs.cols_ok && c->fw_mol < 0 && !c->ctl.molpbc && c->nsites < (1 << 24) &&
+          c->rs.ncells < (1 << 25) && c->rs.nz <= (1 << 15) &&
           c->max_id < (1 << 16) && c->rs.cols.size() > 0;
 }
 
