@@ -1188,6 +1188,8 @@ static mdgpu_status md_capture(mdgpu_ctx *c, const MdStepParams &P, int cap, dou
    CK(ei);
    H.graph_launches = c->launches - l0;
    c->launches = l0;
+   H.graph_class_major = c->class_major;
+   H.graph_npairs_pending = c->npairs_pending;
    H.graph_gen = c->gen;
    H.graph_moves = c->moves.n;
    return MDGPU_OK;
@@ -1265,6 +1267,9 @@ static mdgpu_status md_run_impl(mdgpu_ctx *c, int nsteps, double *energies, int 
       } else if (replay) {
          CK(cudaGraphLaunch(H.graph, st));
          c->launches += H.graph_launches;
+         // (what other calls in between have set)
+         c->class_major = H.graph_class_major;
+         c->npairs_pending = H.graph_npairs_pending;
       } else {
          if ((s = md_enqueue_step(c, P, cap, dist_v, virc)) != MDGPU_OK) return s;
          H.warm_gen = c->gen;

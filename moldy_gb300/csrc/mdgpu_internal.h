@@ -415,6 +415,7 @@ struct MdHost {
    cudaGraphExec_t graph = nullptr;
    uint64_t graph_gen = 0, graph_moves = 0;   // configuration and buffers it was captured with
    int64_t graph_launches = 0;       // kernels one replay launches
+   bool graph_class_major = false, graph_npairs_pending = false;   // how it leaves the slots, the pair count
    int graph_cap = 0;                // record capacity it was captured with
    uint64_t warm_gen = 0;            // configuration of the last direct step
    // constant temperature (mdgpu_md_set_thermostat)

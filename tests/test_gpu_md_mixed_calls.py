@@ -75,3 +75,23 @@ def test_run_between_other_calls_cuda_core_passes(call, before, form, tol, monke
     """The k-list tables of the CUDA-core passes are the run's own again."""
     monkeypatch.setenv("MDGPU_KSPACE_TC", "0")
     test_run_between_other_calls(6, call, before, form, tol)
+
+
+@pytest.mark.parametrize("form", ["fp64", "mixed"])
+@pytest.mark.parametrize("call", [None, gradient, other_cell], ids=lambda v: getattr(v, "__name__", "info"))
+def test_pair_count_after_replayed_steps(call, form):
+    """The count is taken from the slots as the last step left them: class by
+    class, where a gradient leaves them in plain order, and again for steps
+    after one that has been counted.  Exact."""
+    counts = []
+    for between in (False, True):
+        ff, md = start(6, form)
+        md.run(3)
+        if between:
+            assert ff.info()["npairs"] > 0
+            if call:
+                call(ff)
+        md.run(2)
+        counts.append(ff.info()["npairs"])
+        ff.close()
+    assert counts[0] == counts[1] > 0
