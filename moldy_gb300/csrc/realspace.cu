@@ -349,14 +349,24 @@ template <> struct NPar<3> { static constexpr int v = 6; };
 template <> struct NPar<4> { static constexpr int v = 3; };
 template <> struct NPar<6> { static constexpr int v = 7; };
 
+// The potential holds an exponential of r (not of r^2): 6-exp, MCY, generic, Morse.
+// Its argument multiplies r's rounding by up to ten, and rock salt's forces are a
+// thousandth of the terms they are sums of: for these forms r is rounded correctly
+// and the erfc arguments are alpha r as the cell-by-cell kernel has them.  Force of
+// 1728 ions against extended precision: cell by cell 4.83-5.02e-15, r from the
+// reciprocal root alone 5.8-6.0e-15, corrected 4.96-5.2e-15, with alpha r
+// 4.88-5.07e-15 (32,768 ions: pairs 1.023, 1.050, 1.062 ms); water and MCY, without
+// either, are below the cell-by-cell kernel's error.
+template <int PT> struct ExpOfR { static constexpr bool v = PT != 0 && PT != 4; };
+
 // Square root and its reciprocal, reciprocal and exponential: correctly rounded
 // (FAST false), or the FP32 hardware approximations (FAST true: rsqrt and
 // reciprocal within 2 ulp, exp within a few ulp over the arguments of the
 // potentials here), which the column-walk pair kernel of the mixed form
 // uses.
 template <typename R, bool FAST> struct PairMath {
-   // r = sqrt(x), r_r = 1 / r
-   static __device__ __forceinline__ void root(R x, R &r, R &r_r)
+   // r = sqrt(x), r_r = 1 / r; XR: r is an argument of an exponential
+   template <bool XR> static __device__ __forceinline__ void root(R x, R &r, R &r_r)
    {
       r = dsqrt<R>(x);
       r_r = R(1) / r;
@@ -365,7 +375,7 @@ template <typename R, bool FAST> struct PairMath {
    static __device__ __forceinline__ R ex(R x) { return dexp<R>(x); }
 };
 template <> struct PairMath<float, true> {
-   static __device__ __forceinline__ void root(float x, float &r, float &r_r)
+   template <bool XR> static __device__ __forceinline__ void root(float x, float &r, float &r_r)
    {
       r_r = rsqrtf(x);
       r = x * r_r;
@@ -378,12 +388,13 @@ template <> struct PairMath<float, true> {
 // the pair loops, so the correctly rounded square root, divisions and exp
 // (about 55 of 110 FP64 instructions per pair) are replaced by
 //   rsqrt, rcp: the hardware's 20-bit approximation and one third-order
-//     Newton (Householder) step, e -> e^3: 5 and 3 FP64 instructions, about
-//     1 ulp;
+//     Newton (Householder) step, e -> e^3: 5 and 3 FP64 instructions, 0.507
+//     ulp at most (measured, 4 million arguments, as the figures below);
+//   sqrt: x rsqrt(x), 1.5 ulp at most (mean 0.35), or with a Newton step 0.5;
 //   exp: Tang's table method (ACM TOMS 15, 144, 1989): x = (256 k + j)
 //     ln2/256 + f, exp(x) = 2^k 2^(j/256) e^f, |f| <= ln2/512, degree 4, the
-//     rounding residue of 2^(j/256) added to f: 10 instructions, 0.52 ulp (a
-//     64-entry table without residues and degree 6 took 12, for 0.87 ulp).
+//     rounding residue of 2^(j/256) added to f: 10 instructions, 0.545 ulp (a
+//     64-entry table without residues and degree 6 took 12).
 //     The table is in shared memory.
 // Arguments outside their range (r^2 zero or subnormal, |x| > 700) take the
 // general functions.
@@ -478,7 +489,7 @@ __device__ const double2 g_exp2_tab[256] = {
    {1.9945921121709402, 8.979134e-18},
 };
 constexpr double EXP_HI = 0.00270760617331689, EXP_LO = 7.453964567463233e-13, EXP_INV = 369.3299304675746;
-__device__ __forceinline__ void root_n(double x, double &r, double &r_r)
+template <bool XR> __device__ __forceinline__ void root_n(double x, double &r, double &r_r)
 {
    // (range checks on the exponent bits: a compare would take the FP64 pipe)
    if ((unsigned int)__double2hiint(x) - 0x04000000u >= 0x78000000u) {
@@ -492,6 +503,7 @@ __device__ __forceinline__ void root_n(double x, double &r, double &r_r)
    const double e = fma(-x, y * y, 1.0);
    r_r = fma(y * e, fma(0.375, e, 0.5), y);
    r = x * r_r;
+   if (XR) r = fma(0.5 * r_r, fma(-r, r, x), r);
 }
 __device__ __forceinline__ double rcp_n(double x)
 {
@@ -523,7 +535,10 @@ __device__ __forceinline__ double exp_n(double x)
    return __hiloint2double(__double2hiint(r) + ((n >> 8) << 20), __double2loint(r));
 }
 template <> struct PairMath<double, true> {
-   static __device__ __forceinline__ void root(double x, double &r, double &r_r) { root_n(x, r, r_r); }
+   template <bool XR> static __device__ __forceinline__ void root(double x, double &r, double &r_r)
+   {
+      root_n<XR>(x, r, r_r);
+   }
    static __device__ __forceinline__ double rcp(double x) { return rcp_n(x); }
    static __device__ __forceinline__ double ex(double x) { return exp_n(x); }
 };
@@ -537,13 +552,13 @@ __device__ __forceinline__ void pair_fu(R r2, R qq, const R *p, R alpha, R norm,
    typedef PairMath<R, FAST> M;
    R t = R(0), ef = R(0), r = R(0), r_r = R(0), rs_r;
    if (EW || PT != 0) {
-      M::root(r2, r, r_r);
+      M::template root<ExpOfR<PT>::v>(r2, r, r_r);
       rs_r = r_r * r_r;
    } else {
       rs_r = M::rcp(r2);
    }
    if (EW && hc) {
-      if (FAST && sizeof(R) == 8) {   // one product fewer (FP64)
+      if (FAST && sizeof(R) == 8 && !ExpOfR<PT>::v) {   // one product fewer (FP64)
          t = M::rcp(fma((R(ASP) * alpha), r, R(1)));
          ef = qq * M::ex(-(alpha * alpha) * r2);
       } else {
@@ -1434,9 +1449,9 @@ k_pairs_col64(RsParams P, FinArgs fin, const int *__restrict__ cs, const int4 *_
          double f, u;
          pair_fu<PT, EW, double, true>(r2, xj.w * xi.w, pp, P.alpha, P.norm, f, u, hp, hc);
          const double wx = f * rx, wy = f * ry, wz = f * rz;
-         fx -= wx;
-         fy -= wy;
-         fz -= wz;
+         fx = fma(-f, rx, fx);   // (not w: one rounding fewer at the same cost)
+         fy = fma(-f, ry, fy);
+         fz = fma(-f, rz, fz);
          pe += u;
          v0 = fma(wx, rx, v0);
          v1 = fma(wx, ry, v1);
@@ -1616,7 +1631,7 @@ __device__ __forceinline__ void pair_grad(R r2, const R *p, R alpha, R norm, Pai
 {
    typedef PairMath<R, FAST> M;
    R r, r_r;
-   M::root(r2, r, r_r);
+   M::template root<ExpOfR<PT>::v>(r2, r, r_r);
    const R rs_r = r_r * r_r;
    g.uc = g.fc = g.duc = g.dfc = R(0);
    if (EW) {
