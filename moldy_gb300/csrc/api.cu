@@ -537,7 +537,9 @@ mdgpu_status mdgpu_forces_device(mdgpu_ctx *c, const double *h, const double *d_
       // A pair kernel that fills the GPU waits for the k-space tables, so that
       // the structure factor's CTAs (one per SM, on the stream of higher
       // priority) start before the pair blocks take every SM: those then fill
-      // what is left.  Below 8 x 152 x 4 sites both start at once (131,072-site
+      // what is left beside them (mixed: a block per SM; beside the force pass
+      // and the FP64 kernels, 19 warps of 96 registers, no pair block fits, so
+      // there they run before and after).  Below 8 x 152 x 4 sites both start at once (131,072-site
       // water, mixed: 1.153 ms with the pair kernel first, 1.138 ms so).
       c->pairs_after_tables = c->nsites >= 32 * 152 && ks_on_tc(c) && c->nsites == c->fw_site0 ? main : nullptr;
       if (!c->pairs_after_tables) {

@@ -1,7 +1,8 @@
 // Reciprocal-space Ewald sum on the GPU (the work of ewald(),
 // src/ewald.c:280-589): the order of the passes (ks_launch) and the CUDA-core
-// passes, which run for the adjoint with a framework molecule and with
-// MDGPU_KSPACE_TC=0; the tensor-core passes are in kspace_q.cu and
+// passes, which run for the adjoint with a framework molecule, in the FP64 form
+// for charges of very different size (ks_on_tc), and with MDGPU_KSPACE_TC=0; the
+// tensor-core passes are in kspace_q.cu and
 // kspace_tc.cu.
 //
 // Phases.  With s = h^-1 r the fractional co-ordinate of a site, the phase of
@@ -970,8 +971,8 @@ static int fw_slot0(int n) { return std::max(128, (n + 127) & ~127); }
 // large charges, 1000 to 4000 ions, CUDA-core FP64 passes / digits: c = 1, 1.4, 10,
 // 22: 5.5 / 5.3, 7.0 / 7.9, 5.5 / 7.5, 14 / 12 e-16; c = 32, 63: 8.1e-15 / 2.5e-14,
 // 3.9e-13 / 4.5e-12.  Beyond 16 the FP64 form takes the CUDA-core passes and the
-// mixed one four digits, 2^-32 (three there: 4.8e-5 with its former operands / 5.0e-5,
-// 5.0e-3 / 6.3e-3).
+// mixed one four digits, 2^-32 (c = 32, 63: three digits 5.0e-5 and 6.3e-3, bf16
+// triples of every charge 4.8e-5 and 5.0e-3, four digits 9.4e-6 and 2.3e-3).
 constexpr double Q_CREST = 16;
 
 static void count_charged(mdgpu_ctx *c)
